@@ -101,7 +101,7 @@ struct ProdBatch {
   void add(const cplx* X, cplx* Y, const cplx* M, int ldm, int conjT, const std::vector<int>& shape, int mode,
            int nout, cplx alpha, int accumulate, int xfmt = TF_C64, int yfmt = TF_C64) {
     if (yfmt != TF_C64 && (accumulate || alpha.x != 1.0 || alpha.y != 0.0))
-      throw StatusError(MCTDH_EARG, "split-format output needs alpha = 1 without accumulation");
+      throw StatusError(MCTDH_EARG, "FP32 output needs alpha = 1 without accumulation");
     ProdDesc pd;
     memset(&pd, 0, sizeof(pd));
     pd.xfmt = xfmt;
@@ -137,21 +137,26 @@ struct ProdBatch {
   }
 };
 
-// Blocks per contraction: one block per HOLE_TPB fibre tiles, at most HOLE_CAP
-// blocks; the partial buffers hold up to HOLE_NBLK_MAX blocks so that the
+// Blocks per contraction: one block per tpb tiles of 32 fibres x 8 x 8 pairs (every
+// block's four warps then have at least four 16-fibre steps at HOLE_TPB 4), at most
+// `cap` blocks; the partial buffers hold up to HOLE_NBLK_MAX blocks so that the
 // ensemble autotuner can re-tile without re-planning.
-#define HOLE_TPB 8
-#define HOLE_CAP 64
+#define HOLE_TPB 4
+#define HOLE_CAP 32
 #define HOLE_NBLK_MAX 128
-inline int hole_nblk(long long ntiles, int tpb, int cap) {
-  return (int)std::min<long long>(std::max<long long>(ntiles / tpb, 1), std::min(cap, HOLE_NBLK_MAX));
+inline int hole_nblk(const HoleDesc& d, int tpb, int cap) {
+  const long long ntiles = (d.L * d.R + HOLE_TILE - 1) / HOLE_TILE;
+  const long long work = ntiles * ((d.n1 + 7) / 8) * ((d.n2 + 7) / 8);
+  return (int)std::min({std::max(work / tpb, 1LL), ntiles, (long long)std::min(cap, HOLE_NBLK_MAX)});
 }
 
 struct HoleBatch {
   std::vector<HoleDesc> h;
   HoleDesc* d = nullptr;
   long long nblocks = 0;
-  int prec = 0;                  // 0 FP64, 2 compensated split FP32
+  int maxn = 0;                  // largest n1, n2
+  bool f32 = false;              // some operand is complex FP32
+  int prec = 0;                  // 1 FP32 sums, else FP64 accuracy
   double flops = 0, bytes = 0;
   // returns index of the hole
   int add(DevArena& ar, const cplx* X, const cplx* Y, long long L, long long R, int n1, int n2,
@@ -167,21 +172,29 @@ struct HoleBatch {
     if (L * R >= (1LL << 31)) throw StatusError(MCTDH_EUNSUPPORTED, "more than 2^31 fibres in one contraction");
     hd.n1 = n1;
     hd.n2 = n2;
-    long long ntiles = (L * R + HOLE_TILE - 1) / HOLE_TILE;
-    hd.nblk = hole_nblk(ntiles, HOLE_TPB, HOLE_CAP);
-    hd.partial = ar.calloc_c((long long)hole_nblk(ntiles, 1, HOLE_NBLK_MAX) * n1 * n2);
+    hd.nblk = hole_nblk(hd, HOLE_TPB, HOLE_CAP);
+    hd.partial = ar.calloc_c((long long)hole_nblk(hd, 1, HOLE_NBLK_MAX) * n1 * n2);
     h.push_back(hd);
     return (int)h.size() - 1;
   }
   void finalize(DevArena& ar) {
     nblocks = 0;
+    maxn = 0;
     flops = bytes = 0;
     for (auto& hd : h) {
       hd.block_start = nblocks;
       nblocks += hd.nblk;
+      hd.nred = prec == 1 ? hd.nblk : 1;
+      maxn = std::max(maxn, std::max(hd.n1, hd.n2));
+      f32 = f32 || hd.xfmt == TF_F32 || hd.yfmt == TF_F32;
       const double fib = (double)hd.L * (double)hd.R;
       flops += 8.0 * hd.n1 * hd.n2 * fib;
       bytes += (elem_bytes(hd.xfmt) * hd.n1 + (hd.X == hd.Y ? 0.0 : elem_bytes(hd.yfmt) * hd.n2)) * fib;
+    }
+    if (!h.empty()) {
+      unsigned* cnt = (unsigned*)ar.alloc(sizeof(unsigned) * h.size());
+      CK(cudaMemset(cnt, 0, sizeof(unsigned) * h.size()));
+      for (size_t i = 0; i < h.size(); ++i) h[i].counter = cnt + i;
     }
     d = upload_vec(ar, h);
   }
@@ -190,7 +203,8 @@ struct HoleBatch {
     if (h.empty()) return;
     nblocks = 0;
     for (auto& hd : h) {
-      hd.nblk = hole_nblk((hd.L * hd.R + HOLE_TILE - 1) / HOLE_TILE, tpb, cap);
+      hd.nblk = hole_nblk(hd, tpb, cap);
+      hd.nred = prec == 1 ? hd.nblk : 1;
       hd.block_start = nblocks;
       nblocks += hd.nblk;
     }
@@ -221,7 +235,7 @@ struct RedBatch {
     RedTerm rt;
     memset(&rt, 0, sizeof(rt));
     rt.partial = hd.partial;
-    rt.nblk = hd.nblk;
+    rt.nblk = hd.nred;
     rt.alpha = alpha;
     rt.conjT = conjT;
     pending[target].push_back(rt);
@@ -243,8 +257,8 @@ struct RedBatch {
     for (auto& rt : terms)
       for (const HoleBatch* hb : hbs)
         for (const auto& hd : hb->h)
-          if (hd.partial == rt.partial && rt.nblk != hd.nblk) {
-            rt.nblk = hd.nblk;
+          if (hd.partial == rt.partial && rt.nblk != hd.nred) {
+            rt.nblk = hd.nred;
             changed = true;
           }
     if (changed) CK(cudaMemcpyAsync(d_terms, terms.data(), sizeof(RedTerm) * terms.size(), cudaMemcpyHostToDevice, st));
@@ -465,9 +479,6 @@ struct Ctx {
   cplx* d_hbin = nullptr;
   cplx* d_hbin32 = nullptr;   // precision 1: d_hbin as complex FP32, the input of the H_B products
   cplx* d_in32 = nullptr;     // precision 1: the coefficients of d_in as complex FP32 (chain inputs)
-  // compensated contractions (and precision-2 chains): the coefficients of d_in as
-  // FP32 split pairs, converted once per evaluation instead of at every staging
-  cplx* d_insplit = nullptr;
   FusedDot hb_dot{nullptr, nullptr, nullptr, nullptr};    // <d_hbin | H_B d_hbin> in the term sum
   FusedDot lan_nrm{nullptr, nullptr, nullptr, nullptr};   // ||Kn||^2 in the Lanczos axpy
   std::vector<ProdBatch> hb_chains;
@@ -1112,13 +1123,6 @@ void plan_eom(Ctx& c) {
   c.xh1_d = upload_vec(c.ar, c.xh1_h);
   if (!c.modes_gwp.empty()) plan_gwp_setup(c);
 
-  if (c.hole_prec == 2 && !c.member && c.modes_gwp.empty() && !c.mixture)
-    c.d_insplit = c.ar.calloc_c(c.naconftot);
-  // the contractions' operand for A itself: its split copy where there is one
-  auto hole_in = [&](const cplx* p, int fmt, int s) -> std::pair<const cplx*, int> {
-    if (c.d_insplit && p == c.d_in + c.aoff[s]) return std::make_pair((const cplx*)(c.d_insplit + c.aoff[s]), (int)TF_SPLIT);
-    return std::make_pair(p, fmt);
-  };
   // density matrices (Calc_rho1mode, gmctdh_objects.f90:408-477)
   std::vector<HoleRef> hrefs;       // mean-field contractions (c.holes)
   std::vector<HoleRef> rrefs;       // density-matrix contractions (c.rho_holes, FP64)
@@ -1143,9 +1147,8 @@ void plan_eom(Ctx& c) {
         if (!weighted.count(key)) weighted[key] = plan_s_weighted(c, s, key.second);
         Y = weighted[key];
       }
-      const auto hy = hole_in(Y, TF_C64, s), hx = hole_in(c.d_in + c.aoff[s], TF_C64, s);
-      int hidx = c.rho_holes.add(c.ar, hy.first, hx.first, prod_range(sh, 0, m),
-                                 prod_range(sh, m + 1, (int)sh.size()), n, n, hy.second, hx.second);
+      int hidx = c.rho_holes.add(c.ar, Y, c.d_in + c.aoff[s], prod_range(sh, 0, m),
+                                 prod_range(sh, m + 1, (int)sh.size()), n, n);
       rho_hole[m][s] = hidx;
       int tg = c.red.add_target(c.rho[m][s], n, n, n, 1);
       rrefs.push_back(HoleRef{hidx, tg, mkc(1, 0)});
@@ -1162,8 +1165,8 @@ void plan_eom(Ctx& c) {
   // reference's left/right chains.
   c.chains.assign(f + 1, ProdBatch());
   std::vector<std::vector<SumSrc>> srcs(c.nstates);
-  // chain intermediates: complex FP32 in precision 1, FP32 split pairs in precision 2
-  const int chain_fmt = c.precision == 1 ? TF_F32 : (c.precision ? TF_SPLIT : TF_C64);
+  // chain intermediates: complex FP32 in precision 1, else complex FP64
+  const int chain_fmt = c.precision == 1 ? TF_F32 : TF_C64;
   // precision 1: the products read the coefficients converted once to complex FP32
   // (the contractions keep the FP64 coefficients)
   if (c.precision == 1 && !c.member) c.d_in32 = c.ar.calloc_c((c.naconftot + 1) / 2);
@@ -1171,8 +1174,6 @@ void plan_eom(Ctx& c) {
     if (c.d_in32 && X.p == c.d_in + c.aoff[s])   // 8-byte elements: offsets count float2
       return std::make_pair(reinterpret_cast<const cplx*>(reinterpret_cast<float2*>(c.d_in32) + c.aoff[s]),
                             (int)TF_F32);
-    if (c.precision == 2 && c.d_insplit && X.p == c.d_in + c.aoff[s])
-      return std::make_pair((const cplx*)(c.d_insplit + c.aoff[s]), (int)TF_SPLIT);
     return std::make_pair((const cplx*)X.p, X.fmt);
   };
   std::map<std::pair<int, int>, int> mf_target;   // (m,k) -> red target
@@ -1373,9 +1374,7 @@ void plan_eom(Ctx& c) {
       const TRef& X = L[im];
       const TRef& Y = R[f - 1 - im];
       long long Ll = prod_range(X.shape, 0, im), Rr = prod_range(X.shape, im + 1, (int)X.shape.size());
-      const auto hx = c.mf_hole_prec == 2 ? hole_in(X.p, X.fmt, s1) : std::make_pair((const cplx*)X.p, X.fmt);
-      const auto hy = c.mf_hole_prec == 2 ? hole_in(Y.p, Y.fmt, s2) : std::make_pair((const cplx*)Y.p, Y.fmt);
-      int hidx = c.holes.add(c.ar, hx.first, hy.first, Ll, Rr, X.shape[im], Y.shape[im], hx.second, hy.second);
+      int hidx = c.holes.add(c.ar, X.p, Y.p, Ll, Rr, X.shape[im], Y.shape[im], X.fmt, Y.fmt);
       term_hole[std::make_pair(t, im)] = hidx;
       hrefs.push_back(HoleRef{hidx, mf_tg(im, k), c.ae[t]});
     }
@@ -1629,8 +1628,8 @@ void plan_hb(Ctx& c) {
     }
   }
   std::vector<std::vector<SumSrc>> srcs(c.nstates);
-  // FP32 products keep complex FP32 intermediates; compensated ones the split pairs
-  const int chain_fmt = c.hb_prec == 1 ? TF_F32 : (c.hb_prec ? TF_SPLIT : TF_C64);
+  // FP32 products keep complex FP32 intermediates
+  const int chain_fmt = c.hb_prec == 1 ? TF_F32 : TF_C64;
   // FP32 products read the Krylov vector once converted to complex FP32 (8-byte
   // elements: state offsets count float2)
   const int hb_in_fmt = c.hb_prec == 1 ? TF_F32 : TF_C64;
@@ -1817,8 +1816,6 @@ void plan_ovl(Ctx& c, OvlPlan& P, cplx* y1, cplx* y2, int prec, bool norm_only, 
     cplx* a1 = y1 + c.aoff[s];
     cplx* a2 = y2 + c.aoff[s];
     cplx* cur[3] = {a1, a2, a2};
-    int curfmt[3] = {TF_C64, TF_C64, TF_C64};
-    const int cfmt = prec ? TF_SPLIT : TF_C64;
     // each chain alternates between two buffers (depth i reads i - 1's output);
     // plans run on the context stream share them (c.ovl_pool: one plan runs at a
     // time), the CMF2 error overlap, which runs beside other work, has its own
@@ -1837,20 +1834,19 @@ void plan_ovl(Ctx& c, OvlPlan& P, cplx* y1, cplx* y2, int prec, bool norm_only, 
           if (shared) c.ovl_pool[std::make_tuple(s, q, (int)(i & 1))] = buf;
         }
         cplx* out = buf;
-        P.chain[i + 1].add(cur[q], out, mats[q], n, 0, sh, m, n, mkc(1, 0), 0, curfmt[q], cfmt);
+        P.chain[i + 1].add(cur[q], out, mats[q], n, 0, sh, m, n, mkc(1, 0), 0);
         cur[q] = out;
-        curfmt[q] = cfmt;
       }
     }
     const long long n1 = c.n1[s];
     for (int w = 0; w < c.npk; ++w) {
       const long long o = n1 * w;
-      drefs.push_back(HoleRef{P.dots.add(c.ar, a1 + o, cur[0] + o, n1, 1, 1, 1, TF_C64, curfmt[0]), tgt[3 * w],
+      drefs.push_back(HoleRef{P.dots.add(c.ar, a1 + o, cur[0] + o, n1, 1, 1, 1), tgt[3 * w],
                               mkc(1, 0)});
       if (norm_only) continue;
-      drefs.push_back(HoleRef{P.dots.add(c.ar, a2 + o, cur[1] + o, n1, 1, 1, 1, TF_C64, curfmt[1]), tgt[3 * w + 1],
+      drefs.push_back(HoleRef{P.dots.add(c.ar, a2 + o, cur[1] + o, n1, 1, 1, 1), tgt[3 * w + 1],
                               mkc(1, 0)});
-      drefs.push_back(HoleRef{P.dots.add(c.ar, a1 + o, cur[2] + o, n1, 1, 1, 1, TF_C64, curfmt[2]), tgt[3 * w + 2],
+      drefs.push_back(HoleRef{P.dots.add(c.ar, a1 + o, cur[2] + o, n1, 1, 1, 1), tgt[3 * w + 2],
                               mkc(1, 0)});
     }
   }
@@ -2021,7 +2017,7 @@ void run_prod(Ctx& c, const ProdBatch& b) {
 void run_hole(Ctx& c, const HoleBatch& b) {
   if (b.h.empty()) return;
   ProfScope ps(c, KP_HOLE, b.flops, b.bytes);
-  launch_hole(b.d, (int)b.h.size(), b.nblocks, c.st, b.prec);
+  launch_hole(b.d, (int)b.h.size(), b.nblocks, b.maxn, b.f32, c.st, b.prec);
   c.count();
 }
 void run_red(Ctx& c, const RedBatch& b) {
@@ -2099,10 +2095,6 @@ void eom(Ctx& c, cplx* out, bool mf_only = false, bool reginv = true) {
   if (gwp) gwp_setup_run(c);
   if (c.d_in32) {
     launch_to_f32(c.d_in32, c.d_in, c.naconftot, c.st);
-    c.count();
-  }
-  if (c.d_insplit) {
-    launch_to_split(c.d_insplit, c.d_in, c.naconftot, c.st);
     c.count();
   }
   {
@@ -3725,10 +3717,6 @@ void cmf2(Ctx& c, double t, double htry, double* hdid_out, double* hnext_out, lo
       // would magnify a prediction error in the weakly occupied directions by up to
       // 1 / eps_rho^2); the mean fields come from the prediction
       copy_dev(c, c.d_in, c.d_y, c.naconftot);
-      if (c.d_insplit) {
-        launch_to_split(c.d_insplit, c.d_in, c.naconftot, c.st);
-        c.count();
-      }
       run_hole(c, c.rho_holes);
       run_red(c, c.red);
       launch_snap(M->segs_d, (int)M->segs_h.size(), M->pred0, M->E, 2, c.st);
@@ -4264,7 +4252,7 @@ void ens_run_prod(Ens& E, const ProdBatch& b) {
 }
 void ens_run_hole(Ens& E, const HoleBatch& b) {
   if (b.h.empty()) return;
-  launch_hole(b.d, (int)b.h.size(), b.nblocks, E.st, b.prec, E.persist_hole);
+  launch_hole(b.d, (int)b.h.size(), b.nblocks, b.maxn, b.f32, E.st, b.prec, E.persist_hole);
   ++E.launches;
 }
 void ens_run_red(Ens& E, const RedBatch& b) {

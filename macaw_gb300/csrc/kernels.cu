@@ -29,7 +29,8 @@ __device__ __forceinline__ int find_desc(const D* descs, int ndesc) {
 }
 
 // ---------------------------------------------------------------------------
-// Batched mode product (Mult_HeM_MatV / Mult_GM_MatV, gmctdh_objects.f90:1407-1468)
+// Batched mode product in FP32 (Mult_HeM_MatV / Mult_GM_MatV,
+// gmctdh_objects.f90:1407-1468; FP64 accuracy in fixed.cu)
 // One thread owns one fibre (l, :, r): it reads the nin inputs once into
 // registers and writes the nout outputs.
 // ---------------------------------------------------------------------------
@@ -47,47 +48,15 @@ __device__ __forceinline__ void df_fma(float& sh, float& sl, float ah, float al,
   sl += t + e;
 }
 
-// acc (hi, lo) += a * b for plain FP32 a, b (no low parts): the same compensated
-// sum as df_fma without the two correction products that vanish.
-__device__ __forceinline__ void df_fma0(float& sh, float& sl, float a, float b) {
-  const float p = a * b;
-  const float e = fmaf(a, b, -p);
-  const float s = sh + p;
-  const float bp = s - sh;
-  const float t = (sh - (s - bp)) + (p - bp);
-  sh = s;
-  sl += t + e;
-}
-
-// acc += conj(x) y for complex split operands (re hi, im hi, re lo, im lo):
-// re = xr yr + xi yi, im = xr yi - xi yr, each real product compensated
-__device__ __forceinline__ void df_cfma(float* h, float* l, const float4& x, const float4& y) {
-  df_fma(h[0], l[0], x.x, x.z, y.x, y.z);
-  df_fma(h[0], l[0], x.y, x.w, y.y, y.w);
-  df_fma(h[1], l[1], x.x, x.z, y.y, y.w);
-  df_fma(h[1], l[1], -x.y, -x.w, y.x, y.z);
-}
-// the same for complex FP32 operands (no low parts)
-__device__ __forceinline__ void df_cfma0(float* h, float* l, const float2& x, const float2& y) {
-  df_fma0(h[0], l[0], x.x, y.x);
-  df_fma0(h[0], l[0], x.y, y.y);
-  df_fma0(h[1], l[1], x.x, y.y);
-  df_fma0(h[1], l[1], -x.y, y.x);
-}
-
-// PREC 0: FP64.  PREC 1: FP32 -- the products of the FP32-rounded x and M are
-// accumulated in FP32 (~1e-7 relative; the split's correction products would sit
-// at the accumulation's own rounding level), outputs complex FP32 (TF_F32) or
-// FP64.  PREC 2: x and M split into hi + lo FP32 parts, x*M = xh*Mh + xh*Ml + xl*Mh
-// with the sum carried as an FP32 hi/lo pair (compensated), ~1e-13 relative.
+// FP32 products: the FP32-rounded x and M are multiplied and accumulated in FP32
+// (~1e-7 relative; the split's correction products would sit at the accumulation's
+// own rounding level), outputs complex FP32 (TF_F32) or FP64.
 // Block `bb` of the batch (blockIdx.x of the plain launch; persistent CTAs walk
 // the blocks).
-template <int MAXN, int PREC>
+template <int MAXN>
 __device__ __forceinline__ void prod_block(const ProdDesc* __restrict__ descs, int ndesc, long long bb) {
   __shared__ int s_di;
-  __shared__ cplx Ms[PREC == 0 ? MAXN * MAXN : 1];
-  __shared__ cplxf Mh[PREC == 0 ? 1 : MAXN * MAXN];
-  __shared__ cplxf Ml[PREC == 0 ? 1 : MAXN * MAXN];
+  __shared__ cplxf Mh[MAXN * MAXN];
   if (threadIdx.x == 0) s_di = find_desc_at(descs, ndesc, bb);
   __syncthreads();
   const ProdDesc& d = descs[s_di];
@@ -95,19 +64,10 @@ __device__ __forceinline__ void prod_block(const ProdDesc* __restrict__ descs, i
   for (int e = threadIdx.x; e < nin * nout; e += blockDim.x) {
     int jo = e % nout, ji = e / nout;
     cplx v = d.conjT ? cconj(d.M[ji + (long long)d.ldm * jo]) : d.M[jo + (long long)d.ldm * ji];
-    if (PREC == 0) {
-      Ms[jo + MAXN * ji] = v;
-    } else {
-      float hx, lx, hy, ly;
-      split_d2f(v.x, hx, lx);
-      split_d2f(v.y, hy, ly);
-      if (PREC == 1) {
-        Mh[jo + MAXN * ji] = make_float2(hx + lx, hy + ly);   // rounded to nearest
-      } else {
-        Mh[jo + MAXN * ji] = make_float2(hx, hy);
-        Ml[jo + MAXN * ji] = make_float2(lx, ly);
-      }
-    }
+    float hx, lx, hy, ly;
+    split_d2f(v.x, hx, lx);
+    split_d2f(v.y, hy, ly);
+    Mh[jo + MAXN * ji] = make_float2(hx + lx, hy + ly);   // rounded to nearest
   }
   __syncthreads();
   const long long p = (bb - d.block_start) * blockDim.x + threadIdx.x;
@@ -118,86 +78,40 @@ __device__ __forceinline__ void prod_block(const ProdDesc* __restrict__ descs, i
   const long long xi0 = l + L * (long long)nin * r;
   cplx* y0 = d.Y + l + L * (long long)nout * r;
   const cplx alpha = d.alpha;
-  if (PREC == 0) {
-    cplx x[MAXN];
+  cplxf xh[MAXN];
 #pragma unroll
-    for (int j = 0; j < MAXN; ++j) x[j] = (j < nin) ? load_c(d.X, xi0 + L * j, d.xfmt) : mkc(0.0, 0.0);
-    for (int jo = 0; jo < nout; ++jo) {
-      cplx acc = mkc(0.0, 0.0);
+  for (int j = 0; j < MAXN; ++j) {
+    const float4 w = (j < nin) ? load_split(d.X, xi0 + L * j, d.xfmt) : make_float4(0.f, 0.f, 0.f, 0.f);
+    xh[j] = make_float2(w.x + w.z, w.y + w.w);   // rounded to nearest
+  }
+  const bool unit_alpha = (alpha.x == 1.0 && alpha.y == 0.0);
+  for (int jo = 0; jo < nout; ++jo) {
+    cplxf acc = make_float2(0.f, 0.f);
 #pragma unroll
-      for (int j = 0; j < MAXN; ++j)
-        if (j < nin) cfma(acc, Ms[jo + MAXN * j], x[j]);
-      cplx v = cmul(alpha, acc);
-      if (d.accumulate) v = cadd(v, y0[L * jo]);
-      y0[L * jo] = v;
+    for (int j = 0; j < MAXN; ++j)
+      if (j < nin) acc = cfmaf_(acc, Mh[jo + MAXN * j], xh[j]);
+    if (d.yfmt == TF_F32) {   // 8-byte elements: index from the tensor's base
+      reinterpret_cast<float2*>(d.Y)[l + L * ((long long)nout * r + jo)] = acc;
+      continue;
     }
-  } else {
-    cplxf xh[MAXN], xl[MAXN];
-#pragma unroll
-    for (int j = 0; j < MAXN; ++j) {
-      const float4 w = (j < nin) ? load_split(d.X, xi0 + L * j, d.xfmt) : make_float4(0.f, 0.f, 0.f, 0.f);
-      if (PREC == 1) {
-        xh[j] = make_float2(w.x + w.z, w.y + w.w);   // rounded to nearest
-      } else {
-        xh[j] = make_float2(w.x, w.y);
-        xl[j] = make_float2(w.z, w.w);
-      }
-    }
-    const bool unit_alpha = (alpha.x == 1.0 && alpha.y == 0.0);
-    float4* y0f = reinterpret_cast<float4*>(y0);
-    for (int jo = 0; jo < nout; ++jo) {
-      cplx accd;
-      if (PREC == 1) {
-        // FP32 values rounded to nearest: hi + lo of the split, added in FP32
-        cplxf acc = make_float2(0.f, 0.f);
-#pragma unroll
-        for (int j = 0; j < MAXN; ++j)
-          if (j < nin) acc = cfmaf_(acc, Mh[jo + MAXN * j], xh[j]);
-        if (d.yfmt == TF_F32) {   // 8-byte elements: index from the tensor's base
-          reinterpret_cast<float2*>(d.Y)[l + L * ((long long)nout * r + jo)] = acc;
-          continue;
-        }
-        if (d.yfmt) {
-          y0f[L * jo] = make_float4(acc.x, acc.y, 0.f, 0.f);
-          continue;
-        }
-        accd = mkc(f2d_exact(acc.x), f2d_exact(acc.y));
-      } else {
-        float rh = 0.f, rl = 0.f, ih = 0.f, il = 0.f;
-#pragma unroll
-        for (int j = 0; j < MAXN; ++j)
-          if (j < nin) {
-            const cplxf mh = Mh[jo + MAXN * j], ml = Ml[jo + MAXN * j];
-            // real: mr*xr - mi*xi ; imag: mr*xi + mi*xr
-            df_fma(rh, rl, mh.x, ml.x, xh[j].x, xl[j].x);
-            df_fma(rh, rl, -mh.y, -ml.y, xh[j].y, xl[j].y);
-            df_fma(ih, il, mh.x, ml.x, xh[j].y, xl[j].y);
-            df_fma(ih, il, mh.y, ml.y, xh[j].x, xl[j].x);
-          }
-        if (d.yfmt) {
-          y0f[L * jo] = make_float4(rh, ih, rl, il);
-          continue;
-        }
-        accd = mkc(f2d_exact(rh) + f2d_exact(rl), f2d_exact(ih) + f2d_exact(il));
-      }
-      cplx v = unit_alpha ? accd : cmul(alpha, accd);
-      if (d.accumulate) v = cadd(v, y0[L * jo]);
-      y0[L * jo] = v;
-    }
+    const cplx accd = mkc(f2d_exact(acc.x), f2d_exact(acc.y));
+    cplx v = unit_alpha ? accd : cmul(alpha, accd);
+    if (d.accumulate) v = cadd(v, y0[L * jo]);
+    y0[L * jo] = v;
   }
 }
 
-template <int MAXN, int PREC>
+template <int MAXN>
 __global__ void __launch_bounds__(128) prod_kernel(const ProdDesc* __restrict__ descs, int ndesc) {
-  prod_block<MAXN, PREC>(descs, ndesc, (long long)blockIdx.x);
+  prod_block<MAXN>(descs, ndesc, (long long)blockIdx.x);
 }
 
 // Persistent form: gridDim.x CTAs walk the batch's blocks in a fixed stride.
-template <int MAXN, int PREC>
+template <int MAXN>
 __global__ void __launch_bounds__(128) prod_kernel_persistent(const ProdDesc* __restrict__ descs, int ndesc,
                                                               long long nblocks) {
   for (long long bb = blockIdx.x; bb < nblocks; bb += gridDim.x) {
-    prod_block<MAXN, PREC>(descs, ndesc, bb);
+    prod_block<MAXN>(descs, ndesc, bb);
     __syncthreads();   // the block's shared operands are rewritten by the next one
   }
 }
@@ -213,131 +127,63 @@ bool tc_enabled() {
   return on == 1;
 }
 
+// prec 0 and 2: FP64 accuracy (fixed.cu); prec 1: FP32 products.
 // tc: 0 CUDA-core kernel, 1 tensor cores from the configured SPF count on,
 // 2 tensor cores for every size they take (the ensemble autotuner's candidate).
 // persist > 0: at most that many persistent CTAs walk the blocks.
 void launch_prod(const ProdDesc* d_descs, int ndesc, long long nblocks, int maxn, cudaStream_t st, int prec,
                  int tc, int persist) {
   if (ndesc <= 0 || nblocks <= 0) return;
-  if (prec == 1 && tc && tc_enabled() && launch_prod_tc(d_descs, ndesc, nblocks, maxn, st, tc == 2)) return;
+  if (prec != 1) {
+    launch_prod_fx(d_descs, ndesc, nblocks, maxn, st, persist);
+    return;
+  }
+  if (tc && tc_enabled() && launch_prod_tc(d_descs, ndesc, nblocks, maxn, st, tc == 2)) return;
+  // register arrays sized for the batch's largest SPF count: no dead unrolled
+  // iterations and fewer registers (more resident warps) at 8 SPFs and below
   if (persist > 0 && nblocks > persist) {
     const unsigned g = (unsigned)persist;
-    if (maxn <= 8) {
-      if (prec == 0) prod_kernel_persistent<8, 0><<<g, 128, 0, st>>>(d_descs, ndesc, nblocks);
-      else if (prec == 1) prod_kernel_persistent<8, 1><<<g, 128, 0, st>>>(d_descs, ndesc, nblocks);
-      else prod_kernel_persistent<8, 2><<<g, 128, 0, st>>>(d_descs, ndesc, nblocks);
-    } else if (maxn <= 12) {
-      if (prec == 0) prod_kernel_persistent<12, 0><<<g, 128, 0, st>>>(d_descs, ndesc, nblocks);
-      else if (prec == 1) prod_kernel_persistent<12, 1><<<g, 128, 0, st>>>(d_descs, ndesc, nblocks);
-      else prod_kernel_persistent<12, 2><<<g, 128, 0, st>>>(d_descs, ndesc, nblocks);
-    } else {
-      if (prec == 0) prod_kernel_persistent<MAXN_SPF, 0><<<g, 128, 0, st>>>(d_descs, ndesc, nblocks);
-      else if (prec == 1) prod_kernel_persistent<MAXN_SPF, 1><<<g, 128, 0, st>>>(d_descs, ndesc, nblocks);
-      else prod_kernel_persistent<MAXN_SPF, 2><<<g, 128, 0, st>>>(d_descs, ndesc, nblocks);
-    }
+    if (maxn <= 8) prod_kernel_persistent<8><<<g, 128, 0, st>>>(d_descs, ndesc, nblocks);
+    else if (maxn <= 12) prod_kernel_persistent<12><<<g, 128, 0, st>>>(d_descs, ndesc, nblocks);
+    else prod_kernel_persistent<MAXN_SPF><<<g, 128, 0, st>>>(d_descs, ndesc, nblocks);
     return;
   }
   const unsigned nb = (unsigned)nblocks;
-  // register arrays sized for the batch's largest SPF count: no dead unrolled
-  // iterations and fewer registers (more resident warps) at 8 SPFs and below
-  if (maxn <= 8) {
-    if (prec == 0) prod_kernel<8, 0><<<nb, 128, 0, st>>>(d_descs, ndesc);
-    else if (prec == 1) prod_kernel<8, 1><<<nb, 128, 0, st>>>(d_descs, ndesc);
-    else prod_kernel<8, 2><<<nb, 128, 0, st>>>(d_descs, ndesc);
-  } else if (maxn <= 12) {
-    if (prec == 0) prod_kernel<12, 0><<<nb, 128, 0, st>>>(d_descs, ndesc);
-    else if (prec == 1) prod_kernel<12, 1><<<nb, 128, 0, st>>>(d_descs, ndesc);
-    else prod_kernel<12, 2><<<nb, 128, 0, st>>>(d_descs, ndesc);
-  } else {
-    if (prec == 0) prod_kernel<MAXN_SPF, 0><<<nb, 128, 0, st>>>(d_descs, ndesc);
-    else if (prec == 1) prod_kernel<MAXN_SPF, 1><<<nb, 128, 0, st>>>(d_descs, ndesc);
-    else prod_kernel<MAXN_SPF, 2><<<nb, 128, 0, st>>>(d_descs, ndesc);
-  }
+  if (maxn <= 8) prod_kernel<8><<<nb, 128, 0, st>>>(d_descs, ndesc);
+  else if (maxn <= 12) prod_kernel<12><<<nb, 128, 0, st>>>(d_descs, ndesc);
+  else prod_kernel<MAXN_SPF><<<nb, 128, 0, st>>>(d_descs, ndesc);
 }
 
 // ---------------------------------------------------------------------------
-// Batched single-hole contraction, first stage (zher2k / zgemm('T','N') loops of
-// Calc_rho1mode and Calc_MeanField, gmctdh_objects.f90:452-457, :595-600).
+// Batched single-hole contraction with FP32 sums (precision modes 3 and 6; the
+// others in fixed.cu), first stage (gmctdh_objects.f90:452-457, :595-600): FP32
+// operands (rounded to nearest), FP32 products and sums (~1e-7 relative), the
+// block partials widened to FP64 for the deterministic reduction.
 // Block b of a descriptor handles fibre tiles b, b + nblk, ...; every thread owns
 // one (j1, j2) pair and a fibre group; groups are summed in shared memory.
 // ---------------------------------------------------------------------------
-// 1 x 1 contractions (inner products): every thread strides over elements with
-// coalesced loads, the block reduces in shared memory.
-template <int PREC>
-__device__ void dot_block(const HoleDesc& d, int b, cplx* red) {
-  const long long n = d.L * d.R;
-  const int tid = threadIdx.x;
-  cplx acc = mkc(0, 0);
-  for (long long i = (long long)b * HOLE_THREADS + tid; i < n; i += (long long)d.nblk * HOLE_THREADS)
-    cfma_conj(acc, load_c(d.X, i, d.xfmt), load_c(d.Y, i, d.yfmt));
-  red[tid] = acc;
-  __syncthreads();
-  for (int s = HOLE_THREADS / 2; s > 0; s >>= 1) {
-    if (tid < s) red[tid] = cadd(red[tid], red[tid + s]);
-    __syncthreads();
-  }
-  if (tid == 0) d.partial[b] = red[0];
-}
-
-// PREC 0: FP64.  PREC 2: operands split into FP32 hi + lo parts, products and sums
-// carried as compensated FP32 pairs (df_fma), ~1e-13 relative; complex-FP32
-// operands on both sides skip the vanishing low-part products (df_fma0).
-// PREC 1: FP32 operands (rounded to nearest), FP32 products and sums (~1e-7
-// relative), the block partials widened to FP64 for the deterministic reduction.
-template <int PREC>
 __device__ __forceinline__ void hole_block(const HoleDesc* __restrict__ descs, int ndesc, long long bb) {
   __shared__ int s_di;
-  __shared__ cplx Xs[HOLE_TILE * MAXN_SPF];
-  __shared__ cplx Ys[HOLE_TILE * MAXN_SPF];
-  float4* Xf = reinterpret_cast<float4*>(Xs);   // PREC 2: (re hi, im hi, re lo, im lo)
-  float4* Yf = reinterpret_cast<float4*>(Ys);
-  float2* X1 = reinterpret_cast<float2*>(Xs);   // PREC 1 and complex-FP32 operands: (re, im)
-  float2* Y1 = reinterpret_cast<float2*>(Ys);
+  __shared__ float2 X1[HOLE_TILE * MAXN_SPF];
+  __shared__ float2 Y1[HOLE_TILE * MAXN_SPF];
+  __shared__ cplx red[HOLE_THREADS];
   if (threadIdx.x == 0) s_di = find_desc_at(descs, ndesc, bb);
   __syncthreads();
   const HoleDesc& d = descs[s_di];
   const int b = (int)(bb - d.block_start);
   const int n1 = d.n1, n2 = d.n2, npairs = n1 * n2;
-  if (npairs == 1 && d.L * d.R >= HOLE_THREADS) {
-    dot_block<PREC>(d, b, Xs);
-    return;
-  }
   const long long L = d.L, nfib = d.L * d.R;
   const long long ntiles = (nfib + HOLE_TILE - 1) / HOLE_TILE;
   const int tid = threadIdx.x;
-  // PREC 2 with complex-FP32 operands on both sides: exact products of plain FP32
-  // numbers into the compensated sums (the staging keeps (re, im) pairs)
-  const bool f32in = PREC == 2 && d.xfmt == TF_F32 && d.yfmt == TF_F32;
   const bool small = npairs <= HOLE_THREADS;
   const int G = small ? HOLE_THREADS / npairs : 1;
   const int pair0 = small ? tid % npairs : tid;
   const int g = small ? tid / npairs : 0;
-  // PREC 2 with even n1, n2: every thread owns a 2 x 2 block of (j1, j2) pairs, so
-  // each staged value it reads feeds two products (half the shared-memory reads
-  // per product and four independent accumulation chains)
-  const bool quad = PREC == 2 && small && ((n1 | n2) & 1) == 0;
-  // X = Y (density matrices, SPF overlaps): C is Hermitian, so only the blocks on
-  // and above the diagonal are computed (the others are their conjugates) and the
-  // tensor is staged once
-  const bool sym = quad && d.X == d.Y && n1 == n2 && d.xfmt == d.yfmt;
-  const int h1 = n1 >> 1, nq = sym ? h1 * (h1 + 1) / 2 : h1 * (n2 >> 1);
-  const int Gq = quad ? HOLE_THREADS / nq : 0;
-  const int qd = quad ? tid % nq : 0, gq = quad ? tid / nq : 0;
-  int i1 = 2 * (qd % (h1 > 0 ? h1 : 1)), i2 = 2 * (qd / (h1 > 0 ? h1 : 1));
-  if (sym) {   // qd -> (qi <= qj), qj-major: qd = qj (qj + 1) / 2 + qi
-    int rem = qd, qj = 0;
-    while (rem > qj) { rem -= qj + 1; ++qj; }
-    i1 = 2 * rem;
-    i2 = 2 * qj;
-  }
-  cplx acc[4] = {mkc(0, 0), mkc(0, 0), mkc(0, 0), mkc(0, 0)};
   float ah[4][2] = {{0.f, 0.f}, {0.f, 0.f}, {0.f, 0.f}, {0.f, 0.f}};
-  float al[4][2] = {{0.f, 0.f}, {0.f, 0.f}, {0.f, 0.f}, {0.f, 0.f}};
   // Staging: thread tid always loads fibre q = tid % HOLE_TILE of a tile and the
   // columns j = tid / HOLE_TILE, + HOLE_THREADS / HOLE_TILE, ...; its fibre's
   // (l, r) is carried from tile to tile instead of divided out per element.
   static_assert(HOLE_THREADS % HOLE_TILE == 0, "staging assumes whole tiles per thread row");
-  static_assert(4 * HOLE_THREADS <= HOLE_TILE * MAXN_SPF, "the 2 x 2 partials fit the staging tile");
   const int qt = tid % HOLE_TILE, jt = tid / HOLE_TILE, jstep = HOLE_THREADS / HOLE_TILE;
   long long pcur = (long long)b * HOLE_TILE + qt;
   long long lcur = pcur % L, rcur = pcur / L;
@@ -350,56 +196,15 @@ __device__ __forceinline__ void hole_block(const HoleDesc* __restrict__ descs, i
     lcur += dl;
     rcur += dr;
     if (lcur >= L) { lcur -= L; rcur += 1; }
-    const int q = qt;
     for (int j = jt; j < n1; j += jstep) {
-      const long long idx = in_range ? xb + L * j : -1;
-      if (PREC == 0) {
-        Xs[q * MAXN_SPF + j] = (idx >= 0) ? load_c(d.X, idx, d.xfmt) : mkc(0, 0);
-      } else if (PREC == 1 || f32in) {
-        const float4 w = (idx >= 0) ? load_split(d.X, idx, d.xfmt) : make_float4(0.f, 0.f, 0.f, 0.f);
-        X1[q * MAXN_SPF + j] = make_float2(w.x + w.z, w.y + w.w);
-      } else {
-        Xf[q * MAXN_SPF + j] = (idx >= 0) ? load_split(d.X, idx, d.xfmt) : make_float4(0.f, 0.f, 0.f, 0.f);
-      }
+      const float4 w = in_range ? load_split(d.X, xb + L * j, d.xfmt) : make_float4(0.f, 0.f, 0.f, 0.f);
+      X1[qt * MAXN_SPF + j] = make_float2(w.x + w.z, w.y + w.w);
     }
-    for (int j = jt; j < (sym ? 0 : n2); j += jstep) {
-      const long long idx = in_range ? yb + L * j : -1;
-      if (PREC == 0) {
-        Ys[q * MAXN_SPF + j] = (idx >= 0) ? load_c(d.Y, idx, d.yfmt) : mkc(0, 0);
-      } else if (PREC == 1 || f32in) {
-        const float4 w = (idx >= 0) ? load_split(d.Y, idx, d.yfmt) : make_float4(0.f, 0.f, 0.f, 0.f);
-        Y1[q * MAXN_SPF + j] = make_float2(w.x + w.z, w.y + w.w);
-      } else {
-        Yf[q * MAXN_SPF + j] = (idx >= 0) ? load_split(d.Y, idx, d.yfmt) : make_float4(0.f, 0.f, 0.f, 0.f);
-      }
+    for (int j = jt; j < n2; j += jstep) {
+      const float4 w = in_range ? load_split(d.Y, yb + L * j, d.yfmt) : make_float4(0.f, 0.f, 0.f, 0.f);
+      Y1[qt * MAXN_SPF + j] = make_float2(w.x + w.z, w.y + w.w);
     }
     __syncthreads();
-    if (quad) {
-      // pairs (i1, i2), (i1 + 1, i2), (i1, i2 + 1), (i1 + 1, i2 + 1) in ah/al[0..3]
-      const float2* Y1r = sym ? X1 : Y1;
-      const float4* Yfr = sym ? Xf : Yf;
-      if (gq < Gq) {
-        for (int q = gq; q < HOLE_TILE; q += Gq) {
-          if (f32in) {
-            const float2 xa = X1[q * MAXN_SPF + i1], xb = X1[q * MAXN_SPF + i1 + 1];
-            const float2 ya = Y1r[q * MAXN_SPF + i2], yb = Y1r[q * MAXN_SPF + i2 + 1];
-            df_cfma0(ah[0], al[0], xa, ya);
-            df_cfma0(ah[1], al[1], xb, ya);
-            df_cfma0(ah[2], al[2], xa, yb);
-            df_cfma0(ah[3], al[3], xb, yb);
-          } else {
-            const float4 xa = Xf[q * MAXN_SPF + i1], xb = Xf[q * MAXN_SPF + i1 + 1];
-            const float4 ya = Yfr[q * MAXN_SPF + i2], yb = Yfr[q * MAXN_SPF + i2 + 1];
-            df_cfma(ah[0], al[0], xa, ya);
-            df_cfma(ah[1], al[1], xb, ya);
-            df_cfma(ah[2], al[2], xa, yb);
-            df_cfma(ah[3], al[3], xb, yb);
-          }
-        }
-      }
-      __syncthreads();
-      continue;
-    }
 #pragma unroll
     for (int k = 0; k < 4; ++k) {
       int pr, q0, qs;
@@ -413,56 +218,20 @@ __device__ __forceinline__ void hole_block(const HoleDesc* __restrict__ descs, i
       }
       const int j1 = pr % n1, j2 = pr / n1;
       for (int q = q0; q < HOLE_TILE; q += qs) {
-        if (PREC == 0) {
-          cfma_conj(acc[k], Xs[q * MAXN_SPF + j1], Ys[q * MAXN_SPF + j2]);
-        } else if (PREC == 1) {
-          const float2 x = X1[q * MAXN_SPF + j1], y = Y1[q * MAXN_SPF + j2];
-          ah[k][0] = fmaf(x.x, y.x, ah[k][0]);
-          ah[k][0] = fmaf(x.y, y.y, ah[k][0]);
-          ah[k][1] = fmaf(x.x, y.y, ah[k][1]);
-          ah[k][1] = fmaf(-x.y, y.x, ah[k][1]);
-        } else if (f32in) {
-          // complex FP32 operands on both sides (no low parts)
-          const float2 x = X1[q * MAXN_SPF + j1], y = Y1[q * MAXN_SPF + j2];
-          df_fma0(ah[k][0], al[k][0], x.x, y.x);
-          df_fma0(ah[k][0], al[k][0], x.y, y.y);
-          df_fma0(ah[k][1], al[k][1], x.x, y.y);
-          df_fma0(ah[k][1], al[k][1], -x.y, y.x);
-        } else {
-          // conj(x) y: re = xr yr + xi yi, im = xr yi - xi yr
-          const float4 x = Xf[q * MAXN_SPF + j1], y = Yf[q * MAXN_SPF + j2];
-          df_fma(ah[k][0], al[k][0], x.x, x.z, y.x, y.z);
-          df_fma(ah[k][0], al[k][0], x.y, x.w, y.y, y.w);
-          df_fma(ah[k][1], al[k][1], x.x, x.z, y.y, y.w);
-          df_fma(ah[k][1], al[k][1], -x.y, -x.w, y.x, y.z);
-        }
+        const float2 x = X1[q * MAXN_SPF + j1], y = Y1[q * MAXN_SPF + j2];
+        ah[k][0] = fmaf(x.x, y.x, ah[k][0]);
+        ah[k][0] = fmaf(x.y, y.y, ah[k][0]);
+        ah[k][1] = fmaf(x.x, y.y, ah[k][1]);
+        ah[k][1] = fmaf(-x.y, y.x, ah[k][1]);
       }
     }
     __syncthreads();
   }
-  if (PREC != 0) {
+  cplx acc[4];
 #pragma unroll
-    for (int k = 0; k < 4; ++k)
-      acc[k] = mkc(f2d_exact(ah[k][0]) + f2d_exact(al[k][0]), f2d_exact(ah[k][1]) + f2d_exact(al[k][1]));
-  }
+  for (int k = 0; k < 4; ++k) acc[k] = mkc(f2d_exact(ah[k][0]), f2d_exact(ah[k][1]));
   cplx* out = d.partial + (long long)b * npairs;
-  if (quad) {
-    cplx* red = Xs;   // 4 * HOLE_THREADS <= HOLE_TILE * MAXN_SPF entries
-#pragma unroll
-    for (int k = 0; k < 4; ++k) red[4 * tid + k] = acc[k];
-    __syncthreads();
-    if (tid < npairs) {
-      int j1 = tid % n1, j2 = tid / n1;
-      const bool lower = sym && (j1 >> 1) > (j2 >> 1);   // conj of the transposed pair
-      if (lower) { const int tmp = j1; j1 = j2; j2 = tmp; }
-      const int qq = sym ? (j2 >> 1) * ((j2 >> 1) + 1) / 2 + (j1 >> 1) : (j1 >> 1) + h1 * (j2 >> 1);
-      const int k = (j1 & 1) + 2 * (j2 & 1);
-      cplx s = mkc(0, 0);
-      for (int gg = 0; gg < Gq; ++gg) s = cadd(s, red[4 * (gg * nq + qq) + k]);
-      out[tid] = lower ? cconj(s) : s;
-    }
-  } else if (small) {
-    cplx* red = Xs;   // reuse (HOLE_TILE*MAXN_SPF >= HOLE_THREADS)
+  if (small) {
     red[tid] = acc[0];
     __syncthreads();
     if (tid < npairs) {
@@ -479,37 +248,32 @@ __device__ __forceinline__ void hole_block(const HoleDesc* __restrict__ descs, i
   }
 }
 
-template <int PREC>
 __global__ void __launch_bounds__(HOLE_THREADS, 4) hole_kernel(const HoleDesc* __restrict__ descs, int ndesc) {
-  hole_block<PREC>(descs, ndesc, (long long)blockIdx.x);
+  hole_block(descs, ndesc, (long long)blockIdx.x);
 }
 
 // Persistent form: gridDim.x CTAs walk the batch's blocks in a fixed stride (each
 // block still writes its own partial, so the sums do not depend on the grid).
-template <int PREC>
 __global__ void __launch_bounds__(HOLE_THREADS, 4) hole_kernel_persistent(const HoleDesc* __restrict__ descs,
                                                                        int ndesc, long long nblocks) {
   for (long long bb = blockIdx.x; bb < nblocks; bb += gridDim.x) {
-    hole_block<PREC>(descs, ndesc, bb);
+    hole_block(descs, ndesc, bb);
     __syncthreads();   // the staging tiles are rewritten by the next block
   }
 }
 
-void launch_hole(const HoleDesc* d_descs, int ndesc, long long nblocks, cudaStream_t st, int prec, int persist) {
+// maxn: the batch's largest n1, n2; f32: some operand is complex FP32; prec 1: FP32 sums, else FP64 accuracy (fixed.cu)
+void launch_hole(const HoleDesc* d_descs, int ndesc, long long nblocks, int maxn, bool f32, cudaStream_t st, int prec,
+                 int persist) {
   if (ndesc <= 0 || nblocks <= 0) return;
-  if (persist > 0 && nblocks > persist) {
-    const unsigned g = (unsigned)persist;
-    if (prec == 0) hole_kernel_persistent<0><<<g, HOLE_THREADS, 0, st>>>(d_descs, ndesc, nblocks);
-    else if (prec == 1) hole_kernel_persistent<1><<<g, HOLE_THREADS, 0, st>>>(d_descs, ndesc, nblocks);
-    else hole_kernel_persistent<2><<<g, HOLE_THREADS, 0, st>>>(d_descs, ndesc, nblocks);
+  if (prec != 1) {
+    launch_hole_fx(d_descs, ndesc, nblocks, maxn, f32, st, persist);
     return;
   }
-  if (prec == 0)
-    hole_kernel<0><<<(unsigned)nblocks, HOLE_THREADS, 0, st>>>(d_descs, ndesc);
-  else if (prec == 1)
-    hole_kernel<1><<<(unsigned)nblocks, HOLE_THREADS, 0, st>>>(d_descs, ndesc);
+  if (persist > 0 && nblocks > persist)
+    hole_kernel_persistent<<<(unsigned)persist, HOLE_THREADS, 0, st>>>(d_descs, ndesc, nblocks);
   else
-    hole_kernel<2><<<(unsigned)nblocks, HOLE_THREADS, 0, st>>>(d_descs, ndesc);
+    hole_kernel<<<(unsigned)nblocks, HOLE_THREADS, 0, st>>>(d_descs, ndesc);
 }
 
 // ---------------------------------------------------------------------------
@@ -1860,21 +1624,6 @@ __global__ void to_f32_kernel(float2* __restrict__ out, const cplx* __restrict__
   split_d2f(v.x, hx, lx);
   split_d2f(v.y, hy, ly);
   out[i] = make_float2(hx + lx, hy + ly);
-}
-// complex128 -> FP32 split pairs (re hi, im hi, re lo, im lo), the exact split
-// of load_split done once per element
-__global__ void to_split_kernel(float4* __restrict__ out, const cplx* __restrict__ in, long long n) {
-  const long long i = (long long)blockIdx.x * blockDim.x + threadIdx.x;
-  if (i >= n) return;
-  const cplx v = in[i];
-  float4 w;
-  split_d2f(v.x, w.x, w.z);
-  split_d2f(v.y, w.y, w.w);
-  out[i] = w;
-}
-void launch_to_split(cplx* out, const cplx* in, long long n, cudaStream_t st) {
-  if (n <= 0) return;
-  to_split_kernel<<<(unsigned)((n + 255) / 256), 256, 0, st>>>(reinterpret_cast<float4*>(out), in, n);
 }
 void launch_to_f32(cplx* out, const cplx* in, long long n, cudaStream_t st) {
   if (n <= 0) return;

@@ -15,11 +15,8 @@
 #define HOLE_THREADS 256
 
 // Y = alpha * (M_eff x_mode X) (+ Y when accumulate)
-// Tensor storage formats.  TF_C64: complex128 (re, im).  TF_SPLIT: the same 16
-// bytes per element as FP32 (re hi, im hi, re lo, im lo), re = hi + lo to
-// ~2^-48 relative: intermediates of the split-precision chains stay in this
-// form, so neither side of a chain step converts through the FP64 pipe.
-enum { TF_C64 = 0, TF_SPLIT = 1, TF_F32 = 2 };
+// Tensor storage formats.  TF_C64: complex128 (re, im).  TF_F32: complex FP32.
+enum { TF_C64 = 0, TF_F32 = 1 };
 
 struct ProdDesc {
   const cplx* X;
@@ -30,7 +27,7 @@ struct ProdDesc {
   int conjT;               // 0: M_eff(j',j) = M[j' + ldm*j];  1: M_eff(j',j) = conj(M[j + ldm*j'])
   cplx alpha;
   int accumulate;
-  int xfmt, yfmt;          // TF_*: TF_SPLIT output only with alpha = 1, no accumulation, PREC > 0
+  int xfmt, yfmt;          // TF_*: TF_F32 output only of FP32 products with alpha = 1, no accumulation
   int pad;
   long long block_start;
 };
@@ -45,7 +42,8 @@ struct HoleDesc {
   long long block_start;
   int nblk;
   int xfmt, yfmt;          // TF_*
-  int pad;
+  int nred;                // partial blocks left to add: 1 (the contraction adds its own) or nblk
+  unsigned* counter;       // blocks done (zero between launches)
 };
 
 // out (n1 x n2, leading dim ld) = [out +] sum_t alpha_t * sum_blocks partial_t
@@ -234,8 +232,14 @@ int tc_timeout_flag(bool clear);
 // persist > 0: at most `persist` persistent CTAs walk the batch's blocks
 void launch_prod(const ProdDesc* d_descs, int ndesc, long long nblocks, int maxn, cudaStream_t st,
                  int prec = 0, int tc = 1, int persist = 0);
-void launch_hole(const HoleDesc* d_descs, int ndesc, long long nblocks, cudaStream_t st, int prec = 0,
-                 int persist = 0);
+void launch_hole(const HoleDesc* d_descs, int ndesc, long long nblocks, int maxn, bool f32, cudaStream_t st,
+                 int prec = 0, int persist = 0);
+// FP64 accuracy as exact digit products on the tensor cores (fixed.cu); launched by
+// launch_prod / launch_hole
+void launch_prod_fx(const ProdDesc* d_descs, int ndesc, long long nblocks, int maxn, cudaStream_t st, int persist);
+// f32: operands may be complex FP32
+void launch_hole_fx(const HoleDesc* d_descs, int ndesc, long long nblocks, int maxn, bool f32, cudaStream_t st,
+                    int persist);
 void launch_reduce(const RedTarget* d_tg, int ntg, const RedTerm* d_terms, cudaStream_t st);
 // with_h: also h1mode (second launch: the Hermitian part of same-state matrices);
 // prec > 0: the operator products and phi^H (O phi) in compensated split FP32
@@ -327,7 +331,6 @@ void launch_copy_scale(cplx* out, const cplx* in, cplx s, long long n, cudaStrea
 void launch_axpy(cplx* y, const cplx* x, cplx a, long long n, cudaStream_t st);
 // out (complex FP32, TF_F32 storage) = in rounded to nearest
 void launch_to_f32(cplx* out, const cplx* in, long long n, cudaStream_t st);
-void launch_to_split(cplx* out, const cplx* in, long long n, cudaStream_t st);
 void launch_gemv_cols(cplx* out, const cplx* basis, long long ld, const cplx* coef, int ncol, long long n,
                       cudaStream_t st);
 void launch_jacobi_tridiag(const double* alpha, const double* beta, int n, double* evals, double* evecs,
