@@ -637,7 +637,84 @@ __device__ void jacobi_herm(cplx* A, cplx* V, int n, int ld, JacRot* R, bool* ok
   *ok = converged;
 }
 
-// Four warps per (mode, state): the Jacobi sweeps run on the first (its
+// 1 / d for d > 0 by Newton's iteration on the hardware's approximate reciprocal:
+// four dependent FP64 instructions instead of a full division (443 cycles of latency).
+__device__ __forceinline__ double newton_rcp(double d) {
+  double y;
+  asm("rcp.approx.ftz.f64 %0, %1;" : "=d"(y) : "d"(d));
+  y = fma(y, fma(-d, y, 1.0), y);
+  return fma(y, fma(-d, y, 1.0), y);
+}
+
+// Inverse of a Hermitian positive definite n x n matrix (n <= 32) by n symmetric sweeps
+// (Gauss-Jordan elimination of the upper triangle, whose every intermediate is
+// Hermitian): A -> A^-1 in place, A[i + ld j], both triangles filled.  A thread holds EPT
+// elements of the triangle; per sweep one column passes through shared memory
+// (v, two buffers of 32).  One sweep costs a reciprocal and six dependent FP64
+// instructions, against the rotations of six to ten Jacobi sweeps of n - 1 rounds.
+// Returns false (on every thread) at a pivot that is not positive; all threads call it.
+template <int EPT>
+__device__ __forceinline__ bool sweep_inverse(cplx* A, int n, int ld, cplx (*v)[MAXN_SPF]) {
+  cplx a[EPT];
+  int ei[EPT], ej[EPT];
+#pragma unroll
+  for (int q = 0; q < EPT; ++q) {
+    int e = threadIdx.x + q * blockDim.x, j = 0;
+    if (e >= n * (n + 1) / 2) {
+      ei[q] = ej[q] = -1;
+      a[q] = mkc(0, 0);
+      continue;
+    }
+    while (e > j) e -= ++j;   // e -> (i <= j), j-major
+    ei[q] = e;
+    ej[q] = j;
+    a[q] = A[e + ld * j];
+    if (e == 0) v[0][j] = cconj(a[q]);
+  }
+  bool ok = true;
+  for (int k = 0; k < n; ++k) {
+    __syncthreads();
+    const cplx* vk = v[k & 1];
+    const double d = vk[k].x;
+    ok = ok && d > 0.0;
+    const double p = newton_rcp(d);
+#pragma unroll
+    for (int q = 0; q < EPT; ++q) {
+      const int i = ei[q], j = ej[q];
+      if (i < 0) continue;
+      const bool row = i == k, col = j == k;
+      const cplx vj = vk[j];
+      const cplx w = cscale(row ? cconj(vj) : vk[i], p);
+      if (row || col) {
+        a[q] = (row && col) ? mkc(-p, 0.0) : w;
+      } else {
+        a[q].x = fma(-w.x, vj.x, fma(-w.y, vj.y, a[q].x));
+        a[q].y = fma(-w.y, vj.x, fma(w.x, vj.y, a[q].y));
+        if (i == j) a[q].y = 0.0;
+      }
+      if (i == k + 1) v[(k + 1) & 1][j] = cconj(a[q]);
+      else if (j == k + 1) v[(k + 1) & 1][i] = a[q];
+    }
+  }
+  __syncthreads();
+#pragma unroll
+  for (int q = 0; q < EPT; ++q) {
+    if (ei[q] < 0) continue;
+    A[ei[q] + ld * ej[q]] = mkc(-a[q].x, -a[q].y);
+    A[ej[q] + ld * ei[q]] = mkc(-a[q].x, a[q].y);
+  }
+  __syncthreads();
+  return ok;
+}
+
+// Where every eigenvalue of rho is at least eps the 'poly' regularisation is the plain
+// inverse, 1 / w; the inverse itself shows it: positive pivots, and |rho^-1|_F <= 1 / eps
+// bounds its largest eigenvalue.  Then no eigen-decomposition is needed (8 x 8: 63 -> 9 us
+// a launch of 18 matrices); otherwise the Jacobi path below.  blockIdx.y: the blocks
+// of a matrix share its rho^-1 MF products, one warp per operator at a time, each
+// inverting for itself.
+//
+// Jacobi path: four warps per (mode, state), the sweeps on the first (its
 // rotations are one round per warp-wide step), the warm-start products, the
 // regularised inverse and the rho^-1 MF products on all four (independent
 // FP64 dot products, so more of them in flight against the FP64 latency).
@@ -648,6 +725,8 @@ __global__ void __launch_bounds__(128) reginv_kernel(const RegInvDesc* __restric
   __shared__ cplx Inv[MAXN_SPF * MAXN_SPF];
   __shared__ double w[MAXN_SPF];
   __shared__ JacRot R[MAXN_SPF / 2];
+  __shared__ cplx vcol[2][MAXN_SPF];
+  __shared__ float fro[4];
   const RegInvDesc& d = descs[blockIdx.x];
   const int n = d.n, ld = MAXN_SPF;
   for (int e = threadIdx.x; e < n * n; e += blockDim.x) {
@@ -656,8 +735,38 @@ __global__ void __launch_bounds__(128) reginv_kernel(const RegInvDesc* __restric
     cplx v = (i <= j) ? d.A[i + n * j] : cconj(d.A[j + n * i]);
     if (i == j) v.y = 0.0;
     A[i + ld * j] = v;
+    Inv[i + ld * j] = v;
   }
   __syncthreads();
+  if (d.regtype == 0) {
+    const bool pos = n <= 15 ? sweep_inverse<1>(Inv, n, ld, vcol) : sweep_inverse<5>(Inv, n, ld, vcol);
+    float f2 = 0.f;
+    for (int e = threadIdx.x; e < n * n; e += blockDim.x) {
+      const cplx v = Inv[e % n + ld * (e / n)];
+      const float x = (float)v.x, y = (float)v.y;
+      f2 = fmaf(x, x, fmaf(y, y, f2));
+    }
+    for (int o = 16; o > 0; o >>= 1) f2 += __shfl_down_sync(0xffffffffu, f2, o);
+    if ((threadIdx.x & 31) == 0) fro[threadIdx.x >> 5] = f2;
+    __syncthreads();
+    const float lim = 0.999f / (float)d.eps;
+    if (pos && fro[0] + fro[1] + fro[2] + fro[3] <= lim * lim) {
+      if (d.inv_out && blockIdx.y == 0)
+        for (int e = threadIdx.x; e < n * n; e += blockDim.x) d.inv_out[e] = Inv[e % n + ld * (e / n)];
+      const int lane = threadIdx.x & 31;
+      for (int o = blockIdx.y * 4 + (threadIdx.x >> 5); o < d.op_count; o += 4 * gridDim.y) {
+        const MFOp& op = ops[d.op_first + o];
+        for (int e = lane; e < n * op.n2; e += 32) {
+          const int i = e % n, j = e / n;
+          cplx s = mkc(0, 0);
+          for (int k = 0; k < n; ++k) cfma(s, Inv[i + ld * k], op.mf[k + n * j]);
+          op.out[e] = s;
+        }
+      }
+      return;
+    }
+  }
+  if (blockIdx.y > 0) return;   // the first block's alone (it keeps the warm-start vectors)
   // Warm start: rho changes little between consecutive calls (the mean-field
   // evaluations of one propagation), so the previous eigenvectors Vp nearly
   // diagonalise it; Jacobi then runs on Vp^H A Vp and the eigenvectors are Vp V.
@@ -745,7 +854,9 @@ __global__ void __launch_bounds__(128) reginv_kernel(const RegInvDesc* __restric
 
 void launch_reginv(const RegInvDesc* d_descs, int ndesc, const MFOp* d_ops, int* d_status, cudaStream_t st) {
   if (ndesc <= 0) return;
-  reginv_kernel<<<ndesc, 128, 0, st>>>(d_descs, d_ops, d_status);
+  // up to four blocks per matrix while the GPU has SMs for them
+  const unsigned split = (unsigned)std::max(1, std::min(4, 152 / ndesc));
+  reginv_kernel<<<dim3(ndesc, split), 128, 0, st>>>(d_descs, d_ops, d_status);
 }
 
 // ---------------------------------------------------------------------------
@@ -1220,45 +1331,59 @@ __global__ void __launch_bounds__(512) spf_tile_split2_kernel(const SpfDesc* __r
 }
 
 // (phi^H phi) X = phi^H dphi (zposv 'U') by Gauss-Jordan elimination of [S | O]
-// without pivoting, which is stable for the Hermitian positive definite S: each of
-// the n steps is one pivot reciprocal, then one scale and one update per element
-// across all threads (a short dependent path, unlike the column-serial Cholesky
-// and the per-right-hand-side triangular solves).  A non-positive pivot is the
-// zposv failure (DEVST_CHOL_FAIL).
-__global__ void __launch_bounds__(256) spf_solve_kernel(const SpfDesc* __restrict__ descs, int* status) {
-  __shared__ cplx M[MAXN_SPF * 2 * MAXN_SPF];   // M[i + ld * c], c < n: S, c >= n: O
-  __shared__ cplx s_pinv;
-  __shared__ int s_fail;
-  const SpfDesc& d = descs[blockIdx.x];
-  const int n = d.n, ld = MAXN_SPF;
-  if (threadIdx.x == 0) s_fail = 0;
-  for (int pr = threadIdx.x; pr < 2 * n * n; pr += blockDim.x) {
-    const int which = pr / (n * n), q = pr % (n * n);
-    const int j1 = q % n, j2 = q / n;
-    cplx s = mkc(0, 0);
-    for (int t = 0; t < d.ntile; ++t) s = cadd(s, d.partial[(long long)t * 2 * n * n + pr]);
-    M[j1 + ld * (j2 + which * n)] = s;
+// without pivoting, which is stable for the Hermitian positive definite S.  Pivots
+// are real; a thread holds its elements in registers, and per pivot one column and one
+// row pass through shared memory (two buffers, one barrier).  A non-positive pivot is
+// the zposv failure (DEVST_CHOL_FAIL).
+template <int EPT>
+__device__ __forceinline__ bool solve_elimination(const SpfDesc& d, cplx (*colb)[MAXN_SPF], cplx (*rowb)[2 * MAXN_SPF]) {
+  const int n = d.n;
+  cplx a[EPT];
+#pragma unroll
+  for (int q = 0; q < EPT; ++q) {
+    const int e = threadIdx.x + q * blockDim.x;
+    a[q] = mkc(0, 0);
+    if (e >= 2 * n * n) continue;
+    for (int t = 0; t < d.ntile; ++t) a[q] = cadd(a[q], d.partial[(long long)t * 2 * n * n + e]);
+    const int i = e % n, c = e / n;
+    if (c == 0) colb[0][i] = a[q];
+    if (i == 0) rowb[0][c] = a[q];
   }
-  __syncthreads();
+  bool ok = true;
   for (int k = 0; k < n; ++k) {
-    if (threadIdx.x == 0) {
-      const cplx p = M[k + ld * k];
-      if (!(p.x > 0.0)) s_fail = 1;
-      const double den = p.x * p.x + p.y * p.y;
-      s_pinv = (den > 0.0) ? mkc(p.x / den, -p.y / den) : mkc(0.0, 0.0);
+    __syncthreads();
+    const int b = k & 1;
+    const double p = rowb[b][k].x;
+    ok = ok && p > 0.0;
+    const double pinv = newton_rcp(p);
+#pragma unroll
+    for (int q = 0; q < EPT; ++q) {
+      const int e = threadIdx.x + q * blockDim.x, i = e % n, c = e / n;
+      if (e >= 2 * n * n || c <= k) continue;
+      const cplx r = cscale(rowb[b][c], pinv);   // the scaled pivot row
+      if (i == k) {
+        a[q] = r;
+      } else {
+        const cplx f = colb[b][i];
+        a[q].x = fma(-f.x, r.x, fma(f.y, r.y, a[q].x));
+        a[q].y = fma(-f.x, r.y, fma(-f.y, r.x, a[q].y));
+      }
+      if (c == k + 1) colb[b ^ 1][i] = a[q];
+      if (i == k + 1) rowb[b ^ 1][c] = a[q];
     }
-    __syncthreads();
-    for (int c = k + 1 + (int)threadIdx.x; c < 2 * n; c += blockDim.x) M[k + ld * c] = cmul(s_pinv, M[k + ld * c]);
-    __syncthreads();
-    for (int e = threadIdx.x; e < n * 2 * n; e += blockDim.x) {
-      const int i = e % n, c = e / n;
-      if (i == k || c <= k) continue;
-      M[i + ld * c] = csub(M[i + ld * c], cmul(M[i + ld * k], M[k + ld * c]));
-    }
-    __syncthreads();
   }
-  if (threadIdx.x == 0 && s_fail) atomicOr(status, DEVST_CHOL_FAIL);
-  for (int e = threadIdx.x; e < n * n; e += blockDim.x) d.X[e] = M[(e % n) + ld * (n + e / n)];
+#pragma unroll
+  for (int q = 0; q < EPT; ++q) {
+    const int e = threadIdx.x + q * blockDim.x;
+    if (e >= n * n && e < 2 * n * n) d.X[e - n * n] = a[q];
+  }
+  return ok;
+}
+__global__ void __launch_bounds__(256) spf_solve_kernel(const SpfDesc* __restrict__ descs, int* status) {
+  __shared__ cplx colb[2][MAXN_SPF], rowb[2][2 * MAXN_SPF];
+  const SpfDesc& d = descs[blockIdx.x];
+  const bool ok = d.n <= 11 ? solve_elimination<1>(d, colb, rowb) : solve_elimination<8>(d, colb, rowb);
+  if (threadIdx.x == 0 && !ok) atomicOr(status, DEVST_CHOL_FAIL);
 }
 
 __global__ void __launch_bounds__(256) spf_proj_kernel(const SpfDesc* __restrict__ descs, int ndesc,
