@@ -212,6 +212,33 @@ struct HoleBatch {
   }
 };
 
+void merge_prod(ProdBatch& d, const ProdBatch& s) {
+  d.h.insert(d.h.end(), s.h.begin(), s.h.end());
+  d.prec = s.prec;
+}
+void merge_hole(HoleBatch& d, const HoleBatch& s) {
+  d.h.insert(d.h.end(), s.h.begin(), s.h.end());
+  d.prec = s.prec;
+}
+// depth i of both chain sets, and the one-mode products with depth 1, as one batch each
+void merge_full(std::vector<ProdBatch>& full, const std::vector<ProdBatch>& a, const std::vector<ProdBatch>& b,
+                const ProdBatch& first, DevArena& ar) {
+  full.assign(std::max<size_t>(std::max(a.size(), b.size()), 2), ProdBatch());
+  for (size_t i = 1; i < a.size(); ++i) merge_prod(full[i], a[i]);
+  for (size_t i = 1; i < b.size(); ++i) merge_prod(full[i], b[i]);
+  merge_prod(full[1], first);
+  for (auto& x : full) {
+    x.prec = first.prec;
+    x.finalize(ar);
+  }
+}
+void merge_holes(HoleBatch& all, const HoleBatch& a, const HoleBatch& b, DevArena& ar) {
+  if (a.prec != b.prec || a.h.empty() || b.h.empty()) return;
+  merge_hole(all, a);
+  merge_hole(all, b);
+  all.finalize(ar);
+}
+
 struct RedBatch {
   std::vector<RedTarget> tg;
   std::vector<RedTerm> terms;
@@ -474,6 +501,12 @@ struct Ctx {
   MatSumDesc* msum_d = nullptr;
   MatSumSrc* msum_src_d = nullptr;
   std::map<std::pair<int, int>, cplx*> gmat;   // (s, m) -> G_{s,m}
+  // a full evaluation's products: depth i of both chain sets in one launch, the
+  // G_{s,m} products with the first (they are as independent as the chains are of
+  // each other; 6 + 6 + 1 launches of a six-mode model become 6)
+  std::vector<ProdBatch> full;
+  // rho_holes and holes in one launch (one precision), else empty
+  HoleBatch all_holes;
   ProdBatch gprods;                            // G_{s,m} x_m A_s
   // H_B * B plan for CMF2 (Calc_DHD_B): reads d_hbin, writes d_hb
   cplx* d_hbin = nullptr;
@@ -1252,7 +1285,7 @@ void plan_eom(Ctx& c) {
         continue;
       }
       const int k = c.ioper[mact + f * t];
-      gsumk[c.kind[t]][std::make_pair(s1, mact)].push_back(MatSumSrc{c.hmat[mact][k], c.ae[t]});
+      gsumk[c.kind[t]][std::make_pair(s1, mact)].push_back(MatSumSrc{c.hmat[mact][k], c.ae[t], 0, 0});
       if (!c.is_identity[mact + f * k]) rrefs.push_back(HoleRef{rho_hole[mact][s1], mf_tg(mact, k), c.ae[t]});
       continue;
     }
@@ -1390,7 +1423,14 @@ void plan_eom(Ctx& c) {
     md.n2 = n;
     md.first = (int)c.msum_src_h.size();
     md.count = (int)kv.second.size();
-    for (auto& x : kv.second) c.msum_src_h.push_back(x);
+    for (auto x : kv.second) {
+      for (const H1Desc& hd : c.h1_h)   // the operator's raw projection, made Hermitian in the sum
+        if (hd.h == x.src && hd.same_state) {
+          x.src = hd.X;
+          x.herm = 1;
+        }
+      c.msum_src_h.push_back(x);
+    }
     c.msum_h.push_back(md);
     if (kd == 0) c.gmat[kv.first] = md.out;   // H_B of CMF2 takes the Hamiltonian's operators only
     std::vector<int> sh = c.shape_of(s);
@@ -1430,6 +1470,8 @@ void plan_eom(Ctx& c) {
   c.holes.finalize(c.ar);
   // density matrices: compensated split FP32 (~1e-13 relative) in the split modes
   c.rho_holes.prec = c.hole_prec;
+  merge_full(c.full, c.chains, c.chains_full, c.gprods, c.ar);
+  merge_holes(c.all_holes, c.rho_holes, c.holes, c.ar);
   c.rho_holes.finalize(c.ar);
   for (auto& hr : rrefs) c.red.add_term(hr.target, c.rho_holes.h[hr.hole], hr.alpha);
   for (auto& hr : hrefs) c.red.add_term(hr.target, c.holes.h[hr.hole], hr.alpha, hr.conjT);
@@ -2100,20 +2142,21 @@ void eom(Ctx& c, cplx* out, bool mf_only = false, bool reginv = true) {
   {
     RtScope rt(c, RT_H1MODE);
     ProfScope ps(c, KP_H1);
-    launch_h1(c.h1_d, (int)c.h1_h.size(), c.h1_maxn2, c.h1_smem, true, c.st, c.precision);
-    launch_matsum(c.msum_d, (int)c.msum_h.size(), c.msum_src_d, c.st);
-    c.count(3);
+    launch_h1(c.h1_d, (int)c.h1_h.size(), c.h1_maxn2, c.h1_smem, true, c.st, c.precision, c.msum_d, (int)c.msum_h.size(),
+              c.msum_src_d);
+    c.count(2);
   }
   RtScope rt_mf(c, RT_MEANFIELD);   // gmctdh_objects.f90:511-1140
   // the deepest level holds only the full products H_t A of the right chains (dA)
   const size_t depth_end = mf_only ? c.chains.size() - 1 : c.chains.size();
-  for (size_t i = 1; i < depth_end; ++i) run_prod(c, c.chains[i]);
-  if (!mf_only)
-    for (size_t i = 1; i < c.chains_full.size(); ++i) run_prod(c, c.chains_full[i]);
-  if (!mf_only) run_prod(c, c.gprods);
+  for (size_t i = 1; i < depth_end; ++i) run_prod(c, mf_only ? c.chains[i] : c.full[i]);
   for (auto& b : c.gwp_rho_chain) run_prod(c, b);
-  run_hole(c, c.rho_holes);
-  run_hole(c, c.holes);
+  if (c.all_holes.h.empty()) {
+    run_hole(c, c.rho_holes);
+    run_hole(c, c.holes);
+  } else {
+    run_hole(c, c.all_holes);
+  }
   run_red(c, c.red);
   if (c.pk_on) run_packets(c);
   if (reginv || !mf_only) run_reginv(c);
@@ -2160,12 +2203,13 @@ void run_ovl(Ctx& c, OvlPlan& P) {
 }
 
 void check_status(Ctx& c) {
-  int st = 0;
-  CK(cudaMemcpyAsync(&st, c.d_status, sizeof(int), cudaMemcpyDeviceToHost, c.st));
+  int* pinned = reinterpret_cast<int*>(c.h_scal + 32);
+  CK(cudaMemcpyAsync(pinned, c.d_status, sizeof(int), cudaMemcpyDeviceToHost, c.st));
   CK(cudaStreamSynchronize(c.st));
   if (st != 0) {
     CK(cudaMemsetAsync(c.d_status, 0, sizeof(int), c.st));
     if (st & DEVST_EIG_NOCONV) throw StatusError(MCTDH_EEIG, "Jacobi eigensolver did not converge");
+  const int st = *pinned;
     if (st & DEVST_CHOL_FAIL) throw StatusError(MCTDH_EEIG, "SPF overlap matrix is not positive definite");
     throw StatusError(MCTDH_ENONFINITE, "device status " + std::to_string(st));
   }
@@ -2830,9 +2874,9 @@ void h1_only(Ctx& c, const cplx* y) {
     launch_gwp_h1(c.gh1_d, (int)c.gh1_h.size(), c.st);
     c.count(2);
   }
-  launch_h1(c.h1_d, (int)c.h1_h.size(), c.h1_maxn2, c.h1_smem, true, c.st, c.precision);
-  launch_matsum(c.msum_d, (int)c.msum_h.size(), c.msum_src_d, c.st);
-  c.count(3);
+  launch_h1(c.h1_d, (int)c.h1_h.size(), c.h1_maxn2, c.h1_smem, true, c.st, c.precision, c.msum_d, (int)c.msum_h.size(),
+            c.msum_src_d);
+  c.count(2);
 }
 
 // SPF integration of all DVR modes with frozen mean fields, in lockstep: one
@@ -3982,9 +4026,9 @@ struct Ens {
   cplx der = mkc(0, -1);
   double min_stepsize = 0, writetime = 0;
   // merged EOM plan
-  std::vector<ProdBatch> chains, chains_full;
+  std::vector<ProdBatch> chains, chains_full, full;
   ProdBatch gprods;
-  HoleBatch rho_holes, holes;
+  HoleBatch rho_holes, holes, all_holes;
   RedBatch red;
   std::vector<H1Desc> h1_h;
   H1Desc* h1_d = nullptr;
@@ -4077,14 +4121,6 @@ void ens_graph(Ens& E, int k, F body) {
   E.eom_count += E.graph_eoms[k];
 }
 
-void merge_prod(ProdBatch& d, const ProdBatch& s) {
-  d.h.insert(d.h.end(), s.h.begin(), s.h.end());
-  d.prec = s.prec;
-}
-void merge_hole(HoleBatch& d, const HoleBatch& s) {
-  d.h.insert(d.h.end(), s.h.begin(), s.h.end());
-  d.prec = s.prec;
-}
 void merge_red(RedBatch& d, const RedBatch& s) {
   d.tg.insert(d.tg.end(), s.tg.begin(), s.tg.end());
   d.pending.insert(d.pending.end(), s.pending.begin(), s.pending.end());
@@ -4205,6 +4241,8 @@ Ens* ens_create(const mctdh_setup_t* setups, int n) {
     E->reg_d = upload_vec(E->ar, E->reg_h);
     E->mfop_d = upload_vec(E->ar, E->mfop_h);
     E->spf_d = upload_vec(E->ar, E->spf_h);
+    merge_full(E->full, E->chains, E->chains_full, E->gprods, E->ar);
+    merge_holes(E->all_holes, E->rho_holes, E->holes, E->ar);
     for (auto& x : E->spf_h) E->spf_nf = std::max(E->spf_nf, x.n);
     for (auto& x : E->spfop_h) E->spf_nf = std::max(E->spf_nf, x.n2);
     E->spfop_d = upload_vec(E->ar, E->spfop_h);
@@ -4263,14 +4301,16 @@ void ens_run_red(Ens& E, const RedBatch& b) {
 
 // EOM of every member: IN -> out (same layout as the ensemble vectors).
 void ens_eom(Ens& E, cplx* out) {
-  launch_h1(E.h1_d, (int)E.h1_h.size(), E.h1_maxn2, E.h1_smem, true, E.st, E.precision);
-  launch_matsum(E.msum_d, (int)E.msum_h.size(), E.msum_src_d, E.st);
-  E.launches += 3;
-  for (size_t i = 1; i < E.chains.size(); ++i) ens_run_prod(E, E.chains[i]);
-  for (size_t i = 1; i < E.chains_full.size(); ++i) ens_run_prod(E, E.chains_full[i]);
-  ens_run_prod(E, E.gprods);
-  ens_run_hole(E, E.rho_holes);
-  ens_run_hole(E, E.holes);
+  launch_h1(E.h1_d, (int)E.h1_h.size(), E.h1_maxn2, E.h1_smem, true, E.st, E.precision, E.msum_d, (int)E.msum_h.size(),
+            E.msum_src_d);
+  E.launches += 2;
+  for (size_t i = 1; i < E.full.size(); ++i) ens_run_prod(E, E.full[i]);
+  if (E.all_holes.h.empty()) {
+    ens_run_hole(E, E.rho_holes);
+    ens_run_hole(E, E.holes);
+  } else {
+    ens_run_hole(E, E.all_holes);
+  }
   ens_run_red(E, E.red);
   launch_reginv(E.reg_d, (int)E.reg_h.size(), E.mfop_d, E.status_d, E.st);
   launch_termsum(out, E.sum_d, (int)E.sum_h.size(), E.src_d, E.total, E.st, E.precision);
@@ -4281,7 +4321,7 @@ void ens_eom(Ens& E, cplx* out) {
 
 // Contraction tiling of every merged contraction batch and their reductions.
 void ens_retile(Ens& E, int tpb, int cap) {
-  for (HoleBatch* hb : {&E.rho_holes, &E.holes, &E.ov_spf_holes, &E.ov_dots}) hb->retile(tpb, cap, E.st);
+  for (HoleBatch* hb : {&E.rho_holes, &E.holes, &E.all_holes, &E.ov_spf_holes, &E.ov_dots}) hb->retile(tpb, cap, E.st);
   E.red.sync_nblk({&E.rho_holes, &E.holes}, E.st);
   E.ov_spf_red.sync_nblk({&E.ov_spf_holes}, E.st);
   E.ov_dot_red.sync_nblk({&E.ov_dots}, E.st);
@@ -4866,7 +4906,7 @@ int64_t mctdh_calc_derivs(mctdh_ctx_t* ctx, const double* A, const double* psi, 
   return guarded(c, [&] {
     (void)t;
     upload(*c, c->d_in, A, psi);
-    eom(*c, c->d_out);
+    run_graphed(*c, 20, nullptr, [&] { eom(*c, c->d_out); });
     check_status(*c);
     download(*c, c->d_out, dA, dpsi);
   });

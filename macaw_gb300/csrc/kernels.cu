@@ -507,8 +507,26 @@ __global__ void __launch_bounds__(256) h1_split_kernel(const H1Desc* __restrict_
   }
 }
 
-// Same-state h1mode = (X + X^H) / 2 (the zher2k form, hamilton.f90:500-506).
-__global__ void h1_herm_kernel(const H1Desc* __restrict__ descs) {
+// Blocks 0 .. nh - 1: same-state h1mode = (X + X^H) / 2 (the zher2k form,
+// hamilton.f90:500-506).  The others: operators pre-summed per state and mode,
+// out = sum_k coeff_k src_k, from the same X.
+__global__ void h1_finish_kernel(const H1Desc* __restrict__ descs, int nh, const MatSumDesc* __restrict__ sums,
+                                 const MatSumSrc* __restrict__ srcs) {
+  if ((int)blockIdx.x >= nh) {
+    const MatSumDesc& m = sums[blockIdx.x - nh];
+    for (int e = threadIdx.x; e < m.n1 * m.n2; e += blockDim.x) {
+      const int j1 = e % m.n1, j2 = e / m.n1, eT = j2 + m.n1 * j1;
+      cplx acc = mkc(0, 0);
+      for (int k = 0; k < m.count; ++k) {
+        const MatSumSrc& x = srcs[m.first + k];
+        cplx v = x.src[e];
+        if (x.herm) v = cscale(cadd(v, cconj(x.src[eT])), 0.5);
+        cfma(acc, x.coeff, v);
+      }
+      m.out[e] = acc;
+    }
+    return;
+  }
   const H1Desc& d = descs[blockIdx.x];
   if (d.h == nullptr || !d.same_state) return;
   const int n1 = d.n1;
@@ -519,17 +537,19 @@ __global__ void h1_herm_kernel(const H1Desc* __restrict__ descs) {
 }
 
 void launch_h1(const H1Desc* d_descs, int ndesc, int maxn2, size_t smem_bytes, bool with_h, cudaStream_t st,
-               int prec) {
-  if (ndesc <= 0) return;
-  static size_t configured = 0;
-  if (smem_bytes > 48 * 1024 && smem_bytes > configured) {
-    cudaFuncSetAttribute(h1_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem_bytes);
-    cudaFuncSetAttribute(h1_split_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem_bytes);
-    configured = smem_bytes;
+               int prec, const MatSumDesc* sums, int nsums, const MatSumSrc* srcs) {
+  if (ndesc > 0) {
+    static size_t configured = 0;
+    if (smem_bytes > 48 * 1024 && smem_bytes > configured) {
+      cudaFuncSetAttribute(h1_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem_bytes);
+      cudaFuncSetAttribute(h1_split_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem_bytes);
+      configured = smem_bytes;
+    }
+    if (prec > 0) h1_split_kernel<<<dim3(ndesc, maxn2), 256, smem_bytes, st>>>(d_descs);
+    else h1_kernel<<<dim3(ndesc, maxn2), 256, smem_bytes, st>>>(d_descs);
   }
-  if (prec > 0) h1_split_kernel<<<dim3(ndesc, maxn2), 256, smem_bytes, st>>>(d_descs);
-  else h1_kernel<<<dim3(ndesc, maxn2), 256, smem_bytes, st>>>(d_descs);
-  if (with_h) h1_herm_kernel<<<ndesc, 128, 0, st>>>(d_descs);
+  const int nh = with_h ? ndesc : 0;
+  if (nh + nsums > 0) h1_finish_kernel<<<nh + nsums, 128, 0, st>>>(d_descs, nh, sums, srcs);
 }
 
 // ---------------------------------------------------------------------------
@@ -1771,19 +1791,6 @@ void launch_gemv_cols(cplx* out, const cplx* basis, long long ld, const cplx* co
                       cudaStream_t st) {
   if (n <= 0) return;
   gemv_cols_kernel<<<(unsigned)((n + 255) / 256), 256, 0, st>>>(out, basis, ld, coef, ncol, n);
-}
-
-__global__ void matsum_kernel(const MatSumDesc* __restrict__ descs, const MatSumSrc* __restrict__ srcs) {
-  const MatSumDesc& d = descs[blockIdx.x];
-  for (int e = threadIdx.x; e < d.n1 * d.n2; e += blockDim.x) {
-    cplx acc = mkc(0, 0);
-    for (int k = 0; k < d.count; ++k) cfma(acc, srcs[d.first + k].coeff, srcs[d.first + k].src[e]);
-    d.out[e] = acc;
-  }
-}
-void launch_matsum(const MatSumDesc* d_descs, int ndesc, const MatSumSrc* d_srcs, cudaStream_t st) {
-  if (ndesc <= 0) return;
-  matsum_kernel<<<ndesc, 128, 0, st>>>(d_descs, d_srcs);
 }
 
 // ---------------------------------------------------------------------------

@@ -154,6 +154,8 @@ struct MatSumDesc {
 struct MatSumSrc {
   const cplx* src;
   cplx coeff;
+  int herm;                // 1: the source's Hermitian part
+  int pad;
 };
 
 struct SpfErrDesc {
@@ -241,10 +243,11 @@ void launch_prod_fx(const ProdDesc* d_descs, int ndesc, long long nblocks, int m
 void launch_hole_fx(const HoleDesc* d_descs, int ndesc, long long nblocks, int maxn, bool f32, cudaStream_t st,
                     int persist);
 void launch_reduce(const RedTarget* d_tg, int ntg, const RedTerm* d_terms, cudaStream_t st);
-// with_h: also h1mode (second launch: the Hermitian part of same-state matrices);
-// prec > 0: the operator products and phi^H (O phi) in compensated split FP32
+// with_h: also h1mode (second launch: the Hermitian part of same-state matrices, and
+// the operator sums `sums`); prec > 0: the operator products and phi^H (O phi) in
+// compensated split FP32
 void launch_h1(const H1Desc* d_descs, int ndesc, int maxn2, size_t smem_bytes, bool with_h, cudaStream_t st,
-               int prec);
+               int prec, const MatSumDesc* sums = nullptr, int nsums = 0, const MatSumSrc* srcs = nullptr);
 void launch_reginv(const RegInvDesc* d_descs, int ndesc, const MFOp* d_ops, int* d_status, cudaStream_t st);
 // prec > 0: the tile products in compensated split FP32 (spf_tile_split_kernel)
 // nf: the largest SPF count of the descriptors and their operators (<= 16: the
@@ -335,7 +338,6 @@ void launch_gemv_cols(cplx* out, const cplx* basis, long long ld, const cplx* co
                       cudaStream_t st);
 void launch_jacobi_tridiag(const double* alpha, const double* beta, int n, double* evals, double* evecs,
                            int* d_status, cudaStream_t st);
-void launch_matsum(const MatSumDesc* d_descs, int ndesc, const MatSumSrc* d_srcs, cudaStream_t st);
 void launch_stage_modes(cplx* out, const cplx* base, const StageArgs& a, const double* dt_mode,
                         const unsigned char* elem_mode, long long off, long long n, cudaStream_t st);
 void launch_masked_copy(cplx* y, const cplx* src, const unsigned char* elem_mode, const int* accept, long long off,
