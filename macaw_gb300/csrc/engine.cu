@@ -482,12 +482,11 @@ struct Ctx {
   RegInvDesc* reg_d = nullptr;
   MFOp* mfop_d = nullptr;
   std::vector<SpfDesc> spf_h;
-  std::vector<SpfOp> spfop_h;
+  std::vector<SpfStep> spfstep_h;
   SpfDesc* spf_d = nullptr;
-  SpfOp* spfop_d = nullptr;
-  size_t spf_smem = 0;
+  SpfStep* spfstep_d = nullptr;
+  HoleBatch spf_holes;     // phi^H phi and phi^H dphi of every SPF derivative block
   long long spf_tiles = 0;
-  int spf_nf = 0;          // largest SPF count of the SPF derivative blocks and their operators
   std::vector<SumRange> sum_h;
   std::vector<SumSrc> src_h;
   SumRange* sum_d = nullptr;
@@ -501,13 +500,13 @@ struct Ctx {
   MatSumDesc* msum_d = nullptr;
   MatSumSrc* msum_src_d = nullptr;
   std::map<std::pair<int, int>, cplx*> gmat;   // (s, m) -> G_{s,m}
+  ProdBatch gprods;                            // G_{s,m} x_m A_s
   // a full evaluation's products: depth i of both chain sets in one launch, the
   // G_{s,m} products with the first (they are as independent as the chains are of
   // each other; 6 + 6 + 1 launches of a six-mode model become 6)
   std::vector<ProdBatch> full;
   // rho_holes and holes in one launch (one precision), else empty
   HoleBatch all_holes;
-  ProdBatch gprods;                            // G_{s,m} x_m A_s
   // H_B * B plan for CMF2 (Calc_DHD_B): reads d_hbin, writes d_hb
   cplx* d_hbin = nullptr;
   cplx* d_hbin32 = nullptr;   // precision 1: d_hbin as complex FP32, the input of the H_B products
@@ -1470,9 +1469,9 @@ void plan_eom(Ctx& c) {
   c.holes.finalize(c.ar);
   // density matrices: compensated split FP32 (~1e-13 relative) in the split modes
   c.rho_holes.prec = c.hole_prec;
+  c.rho_holes.finalize(c.ar);
   merge_full(c.full, c.chains, c.chains_full, c.gprods, c.ar);
   merge_holes(c.all_holes, c.rho_holes, c.holes, c.ar);
-  c.rho_holes.finalize(c.ar);
   for (auto& hr : rrefs) c.red.add_term(hr.target, c.rho_holes.h[hr.hole], hr.alpha);
   for (auto& hr : hrefs) c.red.add_term(hr.target, c.holes.h[hr.hole], hr.alpha, hr.conjT);
   c.red.finalize(c.ar);
@@ -1513,7 +1512,6 @@ void plan_eom(Ctx& c) {
   c.mfop_d = upload_vec(c.ar, c.mfop_h);
 
   // SPF derivatives (derivatives.f90:96-153)
-  size_t ssmem = 0;
   for (int m : c.modes_dvr) {
     std::vector<int> states;
     if (c.multiset[m]) for (int s = 0; s < c.nstates; ++s) states.push_back(s);
@@ -1525,32 +1523,31 @@ void plan_eom(Ctx& c) {
       sd.out_offset = c.naconftot + c.ipsi[m + f * s];
       sd.G = c.gmode[m];
       sd.n = c.m_of(m, s);
-      sd.op_first = (int)c.spfop_h.size();
+      sd.step_first = (int)c.spfstep_h.size();
       for (int k = 0; k < c.noper[m]; ++k) {
         if (c.is_identity[m + f * k] || !c.ham_op[m][k]) continue;
         if (c.multiset[m] && c.oper[m][k][0] != s) continue;
-        SpfOp op;
-        memset(&op, 0, sizeof(op));
-        op.ophi = c.ophi[m][k];
-        op.rm = c.rhom1mf[m][k];
-        op.n2 = c.m_of(m, c.oper[m][k][1]);
-        c.spfop_h.push_back(op);
+        const int n2 = c.m_of(m, c.oper[m][k][1]);
+        for (int j = 0; j < n2; j += 8)
+          c.spfstep_h.push_back(SpfStep{c.ophi[m][k] + (long long)sd.G * j, c.rhom1mf[m][k] + (long long)sd.n * j,
+                                        std::min(8, n2 - j), 0});
       }
-      sd.op_count = (int)c.spfop_h.size() - sd.op_first;
-      sd.ntile = (sd.G + SPF_TILE - 1) / SPF_TILE;
+      sd.step_count = (int)c.spfstep_h.size() - sd.step_first;
       sd.block_start = c.spf_tiles;
-      c.spf_tiles += sd.ntile;
-      sd.partial = c.ar.calloc_c((long long)sd.ntile * 2 * sd.n * sd.n);
-      sd.X = c.ar.calloc_c((long long)sd.n * sd.n);
+      c.spf_tiles += (sd.G + SPF_ROWS - 1) / SPF_ROWS;
       c.spf_h.push_back(sd);
-      ssmem = std::max(ssmem, sizeof(cplx) * (size_t)(2 * sd.G * sd.n));
+      c.spf_holes.add(c.ar, sd.phi, sd.phi, sd.G, 1, sd.n, sd.n);
+      const int h = c.spf_holes.add(c.ar, sd.phi, nullptr, sd.G, 1, sd.n, sd.n);
+      c.spf_holes.h[h].yoff = sd.out_offset;
     }
   }
-  c.spf_smem = ssmem;
+  c.spf_holes.finalize(c.ar);
+  for (size_t i = 0; i < c.spf_h.size(); ++i) {
+    c.spf_h[i].S = c.spf_holes.h[2 * i].partial;
+    c.spf_h[i].O = c.spf_holes.h[2 * i + 1].partial;
+  }
   c.spf_d = upload_vec(c.ar, c.spf_h);
-  for (auto& x : c.spf_h) c.spf_nf = std::max(c.spf_nf, x.n);
-  for (auto& x : c.spfop_h) c.spf_nf = std::max(c.spf_nf, x.n2);
-  c.spfop_d = upload_vec(c.ar, c.spfop_h);
+  c.spfstep_d = upload_vec(c.ar, c.spfstep_h);
 
   // dA = f * sum_t ae_t * (H_t A)   (conjugate of Adot_tmp, gmctdh_objects.f90:578; derivatives.f90:155-156)
   for (int s = 0; s < c.nstates; ++s) {
@@ -2131,6 +2128,13 @@ void run_packets(Ctx& c) {
   run_red(c, c.aux_red);
 }
 
+// SPF derivatives into out's psi part (derivatives.f90:94-153)
+void run_spf(Ctx& c, cplx* out) {
+  launch_spf(c.spf_d, (int)c.spf_h.size(), c.spf_tiles, c.spf_holes.maxn, c.spfstep_d, c.spf_holes.d,
+             (int)c.spf_holes.h.size(), c.spf_holes.nblocks, out, c.der, c.d_status, c.st);
+  c.count(3);
+}
+
 void eom(Ctx& c, cplx* out, bool mf_only = false, bool reginv = true) {
   RtScope rt_all(c, RT_CALCDERIVS, true, !mf_only);   // derivatives.f90:92-476
   const bool gwp = !c.modes_gwp.empty();
@@ -2172,8 +2176,7 @@ void eom(Ctx& c, cplx* out, bool mf_only = false, bool reginv = true) {
   {
     RtScope rt(c, RT_SPF_DVR);
     ProfScope ps(c, KP_SPF);
-    launch_spf(c.spf_d, (int)c.spf_h.size(), c.spf_tiles, c.spfop_d, out, c.der, c.d_status, c.st, c.precision, c.spf_nf);
-    c.count(3);
+    run_spf(c, out);
   }
   if (gwp) gwp_derivs_run(c, out);
   // Lagrange multipliers: dA += A (multLagDiag I + i multLag) (derivatives.f90:238-242)
@@ -2206,10 +2209,10 @@ void check_status(Ctx& c) {
   int* pinned = reinterpret_cast<int*>(c.h_scal + 32);
   CK(cudaMemcpyAsync(pinned, c.d_status, sizeof(int), cudaMemcpyDeviceToHost, c.st));
   CK(cudaStreamSynchronize(c.st));
+  const int st = *pinned;
   if (st != 0) {
     CK(cudaMemsetAsync(c.d_status, 0, sizeof(int), c.st));
     if (st & DEVST_EIG_NOCONV) throw StatusError(MCTDH_EEIG, "Jacobi eigensolver did not converge");
-  const int st = *pinned;
     if (st & DEVST_CHOL_FAIL) throw StatusError(MCTDH_EEIG, "SPF overlap matrix is not positive definite");
     throw StatusError(MCTDH_ENONFINITE, "device status " + std::to_string(st));
   }
@@ -2990,9 +2993,9 @@ void spf_eval_all(Ctx& c, CmfState& S, cplx* out, cplx* Dout) {
     }
     {
       ProfScope ps(c, KP_SPF);
-      launch_spf(c.spf_d, (int)c.spf_h.size(), c.spf_tiles, c.spfop_d, out, c.der, c.d_status, c.st, c.precision, c.spf_nf);
+      run_spf(c, out);
     }
-    c.count(4);
+    c.count();
   }
   if (S.gwp) {
     RtScope rt(c, RT_SPF_GWP);
@@ -4043,11 +4046,11 @@ struct Ens {
   RegInvDesc* reg_d = nullptr;
   MFOp* mfop_d = nullptr;
   std::vector<SpfDesc> spf_h;
-  std::vector<SpfOp> spfop_h;
+  std::vector<SpfStep> spfstep_h;
   SpfDesc* spf_d = nullptr;
-  SpfOp* spfop_d = nullptr;
+  SpfStep* spfstep_d = nullptr;
+  HoleBatch spf_holes;
   long long spf_tiles = 0;
-  int spf_nf = 0;          // largest SPF count of the SPF derivative blocks and their operators
   std::vector<SumRange> sum_h;
   std::vector<SumSrc> src_h;
   SumRange* sum_d = nullptr;
@@ -4204,13 +4207,17 @@ Ens* ens_create(const mctdh_setup_t* setups, int n) {
       }
       E->mfop_h.insert(E->mfop_h.end(), c->mfop_h.begin(), c->mfop_h.end());
       for (SpfDesc sd : c->spf_h) {
-        sd.op_first += (int)E->spfop_h.size();
+        sd.step_first += (int)E->spfstep_h.size();
         sd.out_offset += o;
-        sd.block_start = E->spf_tiles;
-        E->spf_tiles += sd.ntile;
+        sd.block_start += E->spf_tiles;
         E->spf_h.push_back(sd);
       }
-      E->spfop_h.insert(E->spfop_h.end(), c->spfop_h.begin(), c->spfop_h.end());
+      E->spf_tiles += c->spf_tiles;
+      E->spfstep_h.insert(E->spfstep_h.end(), c->spfstep_h.begin(), c->spfstep_h.end());
+      for (HoleDesc hd : c->spf_holes.h) {
+        if (!hd.Y) hd.yoff += o;
+        E->spf_holes.h.push_back(hd);
+      }
       for (SumRange r : c->sum_h) {
         r.offset += o;
         r.first += (int)E->src_h.size();
@@ -4234,6 +4241,8 @@ Ens* ens_create(const mctdh_setup_t* setups, int n) {
     E->gprods.finalize(E->ar);
     E->rho_holes.finalize(E->ar);
     E->holes.finalize(E->ar);
+    merge_full(E->full, E->chains, E->chains_full, E->gprods, E->ar);
+    merge_holes(E->all_holes, E->rho_holes, E->holes, E->ar);
     E->red.finalize(E->ar);
     E->h1_d = upload_vec(E->ar, E->h1_h);
     E->msum_d = upload_vec(E->ar, E->msum_h);
@@ -4241,11 +4250,8 @@ Ens* ens_create(const mctdh_setup_t* setups, int n) {
     E->reg_d = upload_vec(E->ar, E->reg_h);
     E->mfop_d = upload_vec(E->ar, E->mfop_h);
     E->spf_d = upload_vec(E->ar, E->spf_h);
-    merge_full(E->full, E->chains, E->chains_full, E->gprods, E->ar);
-    merge_holes(E->all_holes, E->rho_holes, E->holes, E->ar);
-    for (auto& x : E->spf_h) E->spf_nf = std::max(E->spf_nf, x.n);
-    for (auto& x : E->spfop_h) E->spf_nf = std::max(E->spf_nf, x.n2);
-    E->spfop_d = upload_vec(E->ar, E->spfop_h);
+    E->spfstep_d = upload_vec(E->ar, E->spfstep_h);
+    E->spf_holes.finalize(E->ar);
     E->sum_d = upload_vec(E->ar, E->sum_h);
     split_coeffs(E->src_h);
     E->src_d = upload_vec(E->ar, E->src_h);
@@ -4314,7 +4320,8 @@ void ens_eom(Ens& E, cplx* out) {
   ens_run_red(E, E.red);
   launch_reginv(E.reg_d, (int)E.reg_h.size(), E.mfop_d, E.status_d, E.st);
   launch_termsum(out, E.sum_d, (int)E.sum_h.size(), E.src_d, E.total, E.st, E.precision);
-  launch_spf(E.spf_d, (int)E.spf_h.size(), E.spf_tiles, E.spfop_d, out, E.der, E.status_d, E.st, E.precision, E.spf_nf);
+  launch_spf(E.spf_d, (int)E.spf_h.size(), E.spf_tiles, E.spf_holes.maxn, E.spfstep_d, E.spf_holes.d,
+             (int)E.spf_holes.h.size(), E.spf_holes.nblocks, out, E.der, E.status_d, E.st);
   E.launches += 5;
   E.eom_count++;
 }

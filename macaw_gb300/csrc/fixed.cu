@@ -282,7 +282,7 @@ static __device__ void dot_block(const HoleDesc& d, int b, cplx* red) {
 
 // The block's contraction in FP64 from global memory, for operands outside the
 // exponent range (fibres p0 .. p1).
-static __device__ __noinline__ void hole_block_fp64(const HoleDesc& d, int b, unsigned p0, unsigned p1) {
+static __device__ __noinline__ void hole_block_fp64(const HoleDesc& d, const cplx* Y, int b, unsigned p0, unsigned p1) {
   const long long L = d.L;
   for (int pr = threadIdx.x; pr < d.n1 * d.n2; pr += blockDim.x) {
     const int j1 = pr % d.n1, j2 = pr / d.n1;
@@ -290,7 +290,7 @@ static __device__ __noinline__ void hole_block_fp64(const HoleDesc& d, int b, un
     for (long long p = p0; p < p1; ++p) {
       const long long r = p / L, l = p - r * L;
       cfma_conj(acc, load_c(d.X, l + L * (j1 + (long long)d.n1 * r), d.xfmt),
-                load_c(d.Y, l + L * (j2 + (long long)d.n2 * r), d.yfmt));
+                load_c(Y, l + L * (j2 + (long long)d.n2 * r), d.yfmt));
     }
     d.partial[(long long)b * d.n1 * d.n2 + pr] = acc;
   }
@@ -298,12 +298,13 @@ static __device__ __noinline__ void hole_block_fp64(const HoleDesc& d, int b, un
 
 // F32: operands may be complex FP32
 template <bool F32>
-__device__ __forceinline__ void hole_fx_block(const HoleDesc& d, int b) {
+__device__ __forceinline__ void hole_fx_block(const HoleDesc& d, int b, const cplx* ybase) {
   constexpr int NS = HOLE_NS, ND = HOLE_ND;
   extern __shared__ cplx red[];   // [pair blocks][FS][64]
   __shared__ int s_slow;
+  const cplx* Yp = d.Y ? d.Y : ybase + d.yoff;
   const int n1 = d.n1, n2 = d.n2, npairs = n1 * n2;
-  if (npairs == 1 && d.L * d.R >= HOLE_MTHREADS) {
+  if (npairs == 1 && d.Y && d.L * d.R >= HOLE_MTHREADS) {
     dot_block(d, b, red);
     return;
   }
@@ -349,7 +350,7 @@ __device__ __forceinline__ void hole_fx_block(const HoleDesc& d, int b) {
         const bool in = p + (f & 1) + 8 * (f >> 1) < nfib;
         x[f] = y[f] = mkc(0.0, 0.0);
         if (in && jx < n1) x[f] = load_c(d.X, l[f] + (long long)L * (jx + (long long)n1 * r[f]), xfmt);
-        if (!same && in && jy < n2) y[f] = load_c(d.Y, l[f] + (long long)L * (jy + (long long)n2 * r[f]), yfmt);
+        if (!same && in && jy < n2) y[f] = load_c(Yp, l[f] + (long long)L * (jy + (long long)n2 * r[f]), yfmt);
         l[f] += dl;
         r[f] += dr;
         if (l[f] >= L) { l[f] -= L; r[f] += 1; }
@@ -451,7 +452,7 @@ __device__ __forceinline__ void hole_fx_block(const HoleDesc& d, int b) {
   if (slow) s_slow = 1;
   __syncthreads();
   if (s_slow) {
-    hole_block_fp64(d, b, 16u * g0, min(16u * g1, nfib));
+    hole_block_fp64(d, Yp, b, 16u * g0, min(16u * g1, nfib));
     return;
   }
   cplx* out = d.partial + (long long)b * npairs;
@@ -499,19 +500,20 @@ static __device__ __forceinline__ void hole_sum_blocks(const HoleDesc& d) {
 // form (each block writes its own partial, so the sums do not depend on the grid).
 template <bool F32>
 __global__ void __launch_bounds__(HOLE_MTHREADS, 3)
-    hole_fx_kernel(const HoleDesc* __restrict__ descs, int ndesc, long long nblocks) {
+    hole_fx_kernel(const HoleDesc* __restrict__ descs, int ndesc, long long nblocks, const cplx* ybase) {
   for (long long bb = blockIdx.x; bb < nblocks; bb += gridDim.x) {
     const HoleDesc& d = descs[warp_find_desc(descs, ndesc, bb)];
     if (bb != blockIdx.x) __syncthreads();   // the shared sums are rewritten
-    hole_fx_block<F32>(d, (int)(bb - d.block_start));
+    hole_fx_block<F32>(d, (int)(bb - d.block_start), ybase);
     hole_sum_blocks(d);
   }
 }
 
-void launch_hole_fx(const HoleDesc* d, int nd, long long nblocks, int maxn, bool f32, cudaStream_t st, int persist) {
+void launch_hole_fx(const HoleDesc* d, int nd, long long nblocks, int maxn, bool f32, cudaStream_t st, int persist,
+                    const cplx* ybase) {
   // the most tasks (pair blocks x fibre shares) of any n1, n2 <= maxn: 1 x 4, 3 x 4, 9 x 4
   const int smem = (int)sizeof(cplx) * 64 * (maxn <= 8 ? 4 : (maxn <= 16 ? 12 : 36));
   const unsigned grid = (unsigned)(persist > 0 ? std::min<long long>(nblocks, persist) : nblocks);
-  if (f32) hole_fx_kernel<true><<<grid, HOLE_MTHREADS, smem, st>>>(d, nd, nblocks);
-  else hole_fx_kernel<false><<<grid, HOLE_MTHREADS, smem, st>>>(d, nd, nblocks);
+  if (f32) hole_fx_kernel<true><<<grid, HOLE_MTHREADS, smem, st>>>(d, nd, nblocks, ybase);
+  else hole_fx_kernel<false><<<grid, HOLE_MTHREADS, smem, st>>>(d, nd, nblocks, ybase);
 }

@@ -1068,426 +1068,6 @@ void launch_jacobi_tridiag(const double* alpha, const double* beta, int n, doubl
 }
 
 // ---------------------------------------------------------------------------
-// DVR SPF derivative with the (1 - P) projector (derivatives.f90:96-153), tiled
-// over the grid so every (mode, state) block spreads over many SMs:
-//  (1) spf_tile_kernel: dphi rows = f * sum_k ophi_k rhom1MF_k^T for SPF_TILE grid
-//      rows, plus this tile's share of phi^H phi and phi^H dphi;
-//  (2) spf_solve_kernel: sum the tile shares (fixed order), Cholesky solve
-//      (phi^H phi) X = phi^H dphi  (zposv 'U');
-//  (3) spf_proj_kernel: dphi rows -= phi rows * X.
-// ---------------------------------------------------------------------------
-__global__ void __launch_bounds__(256) spf_tile_kernel(const SpfDesc* __restrict__ descs, int ndesc,
-                                                       const SpfOp* __restrict__ ops, cplx* __restrict__ out,
-                                                       cplx der) {
-  __shared__ int s_di;
-  __shared__ cplx phs[SPF_TILE * MAXN_SPF];
-  __shared__ cplx dps[SPF_TILE * MAXN_SPF];
-  if (threadIdx.x == 0) s_di = find_desc(descs, ndesc);
-  __syncthreads();
-  const SpfDesc& d = descs[s_di];
-  const int t = (int)(blockIdx.x - d.block_start);
-  const int G = d.G, n = d.n;
-  const int g0 = t * SPF_TILE;
-  const int rows = min(SPF_TILE, G - g0);
-  cplx* o = out + d.out_offset;
-  for (int e = threadIdx.x; e < rows * n; e += blockDim.x) {
-    const int r = e % rows, j1 = e / rows;
-    const int g = g0 + r;
-    phs[r + SPF_TILE * j1] = d.phi[g + (long long)G * j1];
-    cplx acc = mkc(0, 0);
-    for (int q = 0; q < d.op_count; ++q) {
-      const SpfOp& op = ops[d.op_first + q];
-      const cplx* oph = op.ophi + g;
-      for (int j2 = 0; j2 < op.n2; ++j2) cfma(acc, oph[(long long)G * j2], op.rm[j1 + n * j2]);
-    }
-    acc = cmul(der, acc);
-    dps[r + SPF_TILE * j1] = acc;
-    o[g + (long long)G * j1] = acc;
-  }
-  __syncthreads();
-  cplx* part = d.partial + (long long)t * 2 * n * n;
-  for (int pr = threadIdx.x; pr < 2 * n * n; pr += blockDim.x) {
-    const int which = pr / (n * n), q = pr % (n * n);
-    const int j1 = q % n, j2 = q / n;
-    const cplx* a = phs + SPF_TILE * j1;
-    const cplx* b = (which == 0 ? phs : dps) + SPF_TILE * j2;
-    cplx s = mkc(0, 0);
-    for (int r = 0; r < rows; ++r) cfma_conj(s, a[r], b[r]);
-    part[pr] = s;
-  }
-}
-
-// Split-FP32 variant of spf_tile_kernel (precision modes 1 and 2): per operator,
-// the tile rows of ophi and the matrix rhom1MF are split once into FP32 hi/lo
-// pairs in shared memory, and every product is accumulated as a compensated
-// FP32 pair (df_fma, ~1e-13 relative), leaving the FP64 pipe one add per output.
-// PREC 1: the products of FP32-rounded operands accumulated in FP32 (~1e-7
-// relative); PREC 2: compensated pairs.  The tile's shares of phi^H phi and
-// phi^H dphi are compensated FP32 sums in both.
-template <int PREC>
-__global__ void __launch_bounds__(256) spf_tile_split_kernel(const SpfDesc* __restrict__ descs, int ndesc,
-                                                             const SpfOp* __restrict__ ops, cplx* __restrict__ out,
-                                                             cplx der) {
-  __shared__ int s_di;
-  // operator phase: ophi tile and rhom1MF as (hx, hy, lx, ly); epilogue: phi and dphi rows
-  __shared__ __align__(16) cplx smem_u[2 * SPF_TILE * MAXN_SPF];
-  float4* ops_s = reinterpret_cast<float4*>(smem_u);
-  float4* rm_s = ops_s + SPF_TILE * MAXN_SPF;
-  float4* phf = reinterpret_cast<float4*>(smem_u);                    // epilogue: phi rows, split
-  float4* dpf = reinterpret_cast<float4*>(smem_u) + SPF_TILE * MAXN_SPF; // epilogue: dphi rows, split
-  if (threadIdx.x == 0) s_di = find_desc(descs, ndesc);
-  __syncthreads();
-  const SpfDesc& d = descs[s_di];
-  const int t = (int)(blockIdx.x - d.block_start);
-  const int G = d.G, n = d.n;
-  const int g0 = t * SPF_TILE;
-  const int rows = min(SPF_TILE, G - g0);
-  cplx* o = out + d.out_offset;
-  // each thread owns up to 4 outputs (r, j1); SPF_TILE * MAXN_SPF <= 4 * 256
-  float ah[4][2], al[4][2];
-#pragma unroll
-  for (int u = 0; u < 4; ++u) ah[u][0] = ah[u][1] = al[u][0] = al[u][1] = 0.f;
-  for (int q = 0; q < d.op_count; ++q) {
-    const SpfOp& op = ops[d.op_first + q];
-    const int n2 = op.n2;
-    __syncthreads();
-    for (int e = threadIdx.x; e < rows * n2; e += blockDim.x) {
-      const int r = e % rows, j2 = e / rows;
-      const cplx v = op.ophi[g0 + r + (long long)G * j2];
-      float hx, lx, hy, ly;
-      split_d2f(v.x, hx, lx);
-      split_d2f(v.y, hy, ly);
-      ops_s[r + SPF_TILE * j2] = (PREC == 1) ? make_float4(hx + lx, hy + ly, 0.f, 0.f) : make_float4(hx, hy, lx, ly);
-    }
-    for (int e = threadIdx.x; e < n * n2; e += blockDim.x) {
-      const cplx v = op.rm[e];
-      float hx, lx, hy, ly;
-      split_d2f(v.x, hx, lx);
-      split_d2f(v.y, hy, ly);
-      rm_s[e] = (PREC == 1) ? make_float4(hx + lx, hy + ly, 0.f, 0.f) : make_float4(hx, hy, lx, ly);
-    }
-    __syncthreads();
-#pragma unroll
-    for (int u = 0; u < 4; ++u) {
-      const int e = threadIdx.x + u * blockDim.x;
-      if (e >= rows * n) continue;
-      const int r = e % rows, j1 = e / rows;
-      for (int j2 = 0; j2 < n2; ++j2) {
-        const float4 x = ops_s[r + SPF_TILE * j2];
-        const float4 m = rm_s[j1 + n * j2];
-        // (x.r + i x.i)(m.r + i m.i)
-        if (PREC == 1) {
-          ah[u][0] = fmaf(x.x, m.x, fmaf(-x.y, m.y, ah[u][0]));
-          ah[u][1] = fmaf(x.x, m.y, fmaf(x.y, m.x, ah[u][1]));
-        } else {
-          df_fma(ah[u][0], al[u][0], x.x, x.z, m.x, m.z);
-          df_fma(ah[u][0], al[u][0], -x.y, -x.w, m.y, m.w);
-          df_fma(ah[u][1], al[u][1], x.x, x.z, m.y, m.w);
-          df_fma(ah[u][1], al[u][1], x.y, x.w, m.x, m.z);
-        }
-      }
-    }
-  }
-  __syncthreads();
-#pragma unroll
-  for (int u = 0; u < 4; ++u) {
-    const int e = threadIdx.x + u * blockDim.x;
-    if (e >= rows * n) continue;
-    const int r = e % rows, j1 = e / rows;
-    const int g = g0 + r;
-    const cplx acc = cmul(der, mkc(f2d_exact(ah[u][0]) + f2d_exact(al[u][0]),
-                                   f2d_exact(ah[u][1]) + f2d_exact(al[u][1])));
-    const cplx ph = d.phi[g + (long long)G * j1];
-    float4 w;
-    split_d2f(ph.x, w.x, w.z);
-    split_d2f(ph.y, w.y, w.w);
-    phf[r + SPF_TILE * j1] = w;
-    split_d2f(acc.x, w.x, w.z);
-    split_d2f(acc.y, w.y, w.w);
-    dpf[r + SPF_TILE * j1] = w;
-    o[g + (long long)G * j1] = acc;
-  }
-  __syncthreads();
-  cplx* part = d.partial + (long long)t * 2 * n * n;
-  for (int pr = threadIdx.x; pr < 2 * n * n; pr += blockDim.x) {
-    const int which = pr / (n * n), q = pr % (n * n);
-    const int j1 = q % n, j2 = q / n;
-    const float4* a = phf + SPF_TILE * j1;
-    const float4* b = (which == 0 ? phf : dpf) + SPF_TILE * j2;
-    // conj(a) b as compensated FP32 pairs on the pre-split rows (the FP64 pipe is ~64x slower)
-    float rh = 0.f, rl = 0.f, ih = 0.f, il = 0.f;
-    for (int r = 0; r < rows; ++r) {
-      const float4 x = a[r], y = b[r];
-      df_fma(rh, rl, x.x, x.z, y.x, y.z);
-      df_fma(rh, rl, x.y, x.w, y.y, y.w);
-      df_fma(ih, il, x.x, x.z, y.y, y.w);
-      df_fma(ih, il, -x.y, -x.w, y.x, y.z);
-    }
-    part[pr] = mkc(f2d_exact(rh) + f2d_exact(rl), f2d_exact(ih) + f2d_exact(il));
-  }
-}
-
-// spf_tile_split_kernel<2> with the operator sum split between two groups of 256
-// threads (operators 0, 2, 4, .. and 1, 3, 5, ..; both groups pass every barrier),
-// for n <= 16: twice the warps per tile, the same compensated arithmetic; the
-// second group's (hi, lo) sums are added to the first's at the end.
-#define SPF_G2_N 16
-__global__ void __launch_bounds__(512) spf_tile_split2_kernel(const SpfDesc* __restrict__ descs, int ndesc,
-                                                              const SpfOp* __restrict__ ops,
-                                                              cplx* __restrict__ out, cplx der) {
-  __shared__ int s_di;
-  // per group: ophi tile [SPF_TILE][16] and rhom1MF [16][16], split; epilogue: phi and
-  // dphi rows alias them; red: the second group's sums
-  __shared__ __align__(16) float4 buf[2 * (SPF_TILE * SPF_G2_N + SPF_G2_N * SPF_G2_N)];
-  __shared__ __align__(16) float4 red[2 * 256];
-  const int grp = threadIdx.x >> 8, loc = threadIdx.x & 255;
-  float4* ops_s = buf + grp * (SPF_TILE * SPF_G2_N + SPF_G2_N * SPF_G2_N);
-  float4* rm_s = ops_s + SPF_TILE * SPF_G2_N;
-  float4* phf = buf;
-  float4* dpf = buf + SPF_TILE * SPF_G2_N;
-  if (threadIdx.x == 0) s_di = find_desc(descs, ndesc);
-  __syncthreads();
-  const SpfDesc& d = descs[s_di];
-  const int t = (int)(blockIdx.x - d.block_start);
-  const int G = d.G, n = d.n;
-  const int g0 = t * SPF_TILE;
-  const int rows = min(SPF_TILE, G - g0);
-  cplx* o = out + d.out_offset;
-  // each thread owns up to 2 outputs (r, j1) = loc, loc + 256 of its group
-  float ah[2][2], al[2][2];
-#pragma unroll
-  for (int u = 0; u < 2; ++u) ah[u][0] = ah[u][1] = al[u][0] = al[u][1] = 0.f;
-  const int iters = (d.op_count + 1) / 2;
-  for (int it = 0; it < iters; ++it) {
-    const int q = 2 * it + grp;
-    const bool act = q < d.op_count;
-    const SpfOp* op = act ? &ops[d.op_first + q] : nullptr;
-    const int n2 = act ? op->n2 : 0;
-    __syncthreads();
-    for (int e = loc; e < rows * n2; e += 256) {
-      const int r = e % rows, j2 = e / rows;
-      const cplx v = op->ophi[g0 + r + (long long)G * j2];
-      float hx, lx, hy, ly;
-      split_d2f(v.x, hx, lx);
-      split_d2f(v.y, hy, ly);
-      ops_s[r + SPF_TILE * j2] = make_float4(hx, hy, lx, ly);
-    }
-    for (int e = loc; e < n * n2; e += 256) {
-      const cplx v = op->rm[e];
-      float hx, lx, hy, ly;
-      split_d2f(v.x, hx, lx);
-      split_d2f(v.y, hy, ly);
-      rm_s[e] = make_float4(hx, hy, lx, ly);
-    }
-    __syncthreads();
-#pragma unroll
-    for (int u = 0; u < 2; ++u) {
-      const int e = loc + u * 256;
-      if (e >= rows * n) continue;
-      const int r = e % rows, j1 = e / rows;
-      for (int j2 = 0; j2 < n2; ++j2) {
-        const float4 x = ops_s[r + SPF_TILE * j2];
-        const float4 m = rm_s[j1 + n * j2];
-        df_fma(ah[u][0], al[u][0], x.x, x.z, m.x, m.z);
-        df_fma(ah[u][0], al[u][0], -x.y, -x.w, m.y, m.w);
-        df_fma(ah[u][1], al[u][1], x.x, x.z, m.y, m.w);
-        df_fma(ah[u][1], al[u][1], x.y, x.w, m.x, m.z);
-      }
-    }
-  }
-  if (grp == 1) {
-#pragma unroll
-    for (int u = 0; u < 2; ++u) red[loc + 256 * u] = make_float4(ah[u][0], ah[u][1], al[u][0], al[u][1]);
-  }
-  __syncthreads();   // the operator tiles are dead; red holds the second group's sums
-  if (grp == 0) {
-#pragma unroll
-    for (int u = 0; u < 2; ++u) {
-      const int e = loc + u * 256;
-      if (e >= rows * n) continue;
-      const float4 b = red[e];
-      float sh = ah[u][0], sl = al[u][0], th = ah[u][1], tl = al[u][1];
-      {
-        const float x = sh + b.x, bp = x - sh;
-        sl += ((sh - (x - bp)) + (b.x - bp)) + b.z;
-        sh = x;
-      }
-      {
-        const float x = th + b.y, bp = x - th;
-        tl += ((th - (x - bp)) + (b.y - bp)) + b.w;
-        th = x;
-      }
-      const int r = e % rows, j1 = e / rows;
-      const int g = g0 + r;
-      const cplx acc = cmul(der, mkc(f2d_exact(sh) + f2d_exact(sl), f2d_exact(th) + f2d_exact(tl)));
-      const cplx ph = d.phi[g + (long long)G * j1];
-      float4 w;
-      split_d2f(ph.x, w.x, w.z);
-      split_d2f(ph.y, w.y, w.w);
-      phf[r + SPF_TILE * j1] = w;
-      split_d2f(acc.x, w.x, w.z);
-      split_d2f(acc.y, w.y, w.w);
-      dpf[r + SPF_TILE * j1] = w;
-      o[g + (long long)G * j1] = acc;
-    }
-  }
-  __syncthreads();
-  cplx* part = d.partial + (long long)t * 2 * n * n;
-  for (int pr = threadIdx.x; pr < 2 * n * n; pr += blockDim.x) {
-    const int which = pr / (n * n), qq = pr % (n * n);
-    const int j1 = qq % n, j2 = qq / n;
-    const float4* a = phf + SPF_TILE * j1;
-    const float4* b = (which == 0 ? phf : dpf) + SPF_TILE * j2;
-    float rh = 0.f, rl = 0.f, ih = 0.f, il = 0.f;
-    for (int r = 0; r < rows; ++r) {
-      const float4 x = a[r], y = b[r];
-      df_fma(rh, rl, x.x, x.z, y.x, y.z);
-      df_fma(rh, rl, x.y, x.w, y.y, y.w);
-      df_fma(ih, il, x.x, x.z, y.y, y.w);
-      df_fma(ih, il, -x.y, -x.w, y.x, y.z);
-    }
-    part[pr] = mkc(f2d_exact(rh) + f2d_exact(rl), f2d_exact(ih) + f2d_exact(il));
-  }
-}
-
-// (phi^H phi) X = phi^H dphi (zposv 'U') by Gauss-Jordan elimination of [S | O]
-// without pivoting, which is stable for the Hermitian positive definite S.  Pivots
-// are real; a thread holds its elements in registers, and per pivot one column and one
-// row pass through shared memory (two buffers, one barrier).  A non-positive pivot is
-// the zposv failure (DEVST_CHOL_FAIL).
-template <int EPT>
-__device__ __forceinline__ bool solve_elimination(const SpfDesc& d, cplx (*colb)[MAXN_SPF], cplx (*rowb)[2 * MAXN_SPF]) {
-  const int n = d.n;
-  cplx a[EPT];
-#pragma unroll
-  for (int q = 0; q < EPT; ++q) {
-    const int e = threadIdx.x + q * blockDim.x;
-    a[q] = mkc(0, 0);
-    if (e >= 2 * n * n) continue;
-    for (int t = 0; t < d.ntile; ++t) a[q] = cadd(a[q], d.partial[(long long)t * 2 * n * n + e]);
-    const int i = e % n, c = e / n;
-    if (c == 0) colb[0][i] = a[q];
-    if (i == 0) rowb[0][c] = a[q];
-  }
-  bool ok = true;
-  for (int k = 0; k < n; ++k) {
-    __syncthreads();
-    const int b = k & 1;
-    const double p = rowb[b][k].x;
-    ok = ok && p > 0.0;
-    const double pinv = newton_rcp(p);
-#pragma unroll
-    for (int q = 0; q < EPT; ++q) {
-      const int e = threadIdx.x + q * blockDim.x, i = e % n, c = e / n;
-      if (e >= 2 * n * n || c <= k) continue;
-      const cplx r = cscale(rowb[b][c], pinv);   // the scaled pivot row
-      if (i == k) {
-        a[q] = r;
-      } else {
-        const cplx f = colb[b][i];
-        a[q].x = fma(-f.x, r.x, fma(f.y, r.y, a[q].x));
-        a[q].y = fma(-f.x, r.y, fma(-f.y, r.x, a[q].y));
-      }
-      if (c == k + 1) colb[b ^ 1][i] = a[q];
-      if (i == k + 1) rowb[b ^ 1][c] = a[q];
-    }
-  }
-#pragma unroll
-  for (int q = 0; q < EPT; ++q) {
-    const int e = threadIdx.x + q * blockDim.x;
-    if (e >= n * n && e < 2 * n * n) d.X[e - n * n] = a[q];
-  }
-  return ok;
-}
-__global__ void __launch_bounds__(256) spf_solve_kernel(const SpfDesc* __restrict__ descs, int* status) {
-  __shared__ cplx colb[2][MAXN_SPF], rowb[2][2 * MAXN_SPF];
-  const SpfDesc& d = descs[blockIdx.x];
-  const bool ok = d.n <= 11 ? solve_elimination<1>(d, colb, rowb) : solve_elimination<8>(d, colb, rowb);
-  if (threadIdx.x == 0 && !ok) atomicOr(status, DEVST_CHOL_FAIL);
-}
-
-__global__ void __launch_bounds__(256) spf_proj_kernel(const SpfDesc* __restrict__ descs, int ndesc,
-                                                       cplx* __restrict__ out) {
-  __shared__ int s_di;
-  __shared__ cplx Xs[MAXN_SPF * MAXN_SPF];
-  if (threadIdx.x == 0) s_di = find_desc(descs, ndesc);
-  __syncthreads();
-  const SpfDesc& d = descs[s_di];
-  const int n = d.n, G = d.G;
-  for (int e = threadIdx.x; e < n * n; e += blockDim.x) Xs[e] = d.X[e];
-  __syncthreads();
-  const int t = (int)(blockIdx.x - d.block_start);
-  const int g0 = t * SPF_TILE;
-  const int rows = min(SPF_TILE, G - g0);
-  cplx* o = out + d.out_offset;
-  for (int e = threadIdx.x; e < rows * n; e += blockDim.x) {
-    const int r = e % rows, j = e / rows;
-    const int g = g0 + r;
-    cplx v = o[g + (long long)G * j];
-    for (int k = 0; k < n; ++k) v = csub(v, cmul(d.phi[g + (long long)G * k], Xs[k + n * j]));
-    o[g + (long long)G * j] = v;
-  }
-}
-
-// Split modes: dphi -= phi X with the products as compensated FP32 pairs on split
-// operands (~1e-13 relative) and one FP64 subtraction per element.
-__global__ void __launch_bounds__(256) spf_proj_split_kernel(const SpfDesc* __restrict__ descs, int ndesc,
-                                                             cplx* __restrict__ out) {
-  __shared__ int s_di;
-  __shared__ float4 Xs[MAXN_SPF * MAXN_SPF];
-  if (threadIdx.x == 0) s_di = find_desc(descs, ndesc);
-  __syncthreads();
-  const SpfDesc& d = descs[s_di];
-  const int n = d.n, G = d.G;
-  for (int e = threadIdx.x; e < n * n; e += blockDim.x) {
-    const cplx v = d.X[e];
-    float4 w4;
-    split_d2f(v.x, w4.x, w4.z);
-    split_d2f(v.y, w4.y, w4.w);
-    Xs[e] = w4;
-  }
-  __syncthreads();
-  const int t = (int)(blockIdx.x - d.block_start);
-  const int g0 = t * SPF_TILE;
-  const int rows = min(SPF_TILE, G - g0);
-  cplx* o = out + d.out_offset;
-  for (int e = threadIdx.x; e < rows * n; e += blockDim.x) {
-    const int r = e % rows, j = e / rows;
-    const int g = g0 + r;
-    float rh = 0.f, rl = 0.f, ih = 0.f, il = 0.f;
-    for (int k = 0; k < n; ++k) {
-      const cplx ph = d.phi[g + (long long)G * k];
-      float xh, xl, yh, yl;
-      split_d2f(ph.x, xh, xl);
-      split_d2f(ph.y, yh, yl);
-      const float4 m = Xs[k + n * j];
-      df_fma(rh, rl, xh, xl, m.x, m.z);
-      df_fma(rh, rl, -yh, -yl, m.y, m.w);
-      df_fma(ih, il, xh, xl, m.y, m.w);
-      df_fma(ih, il, yh, yl, m.x, m.z);
-    }
-    const cplx v = o[g + (long long)G * j];
-    o[g + (long long)G * j] = mkc(v.x - (f2d_exact(rh) + f2d_exact(rl)), v.y - (f2d_exact(ih) + f2d_exact(il)));
-  }
-}
-
-void launch_spf(const SpfDesc* d_descs, int ndesc, long long ntiles, const SpfOp* d_ops, cplx* out,
-                cplx der_factor, int* d_status, cudaStream_t st, int prec, int nf) {
-  if (ndesc <= 0) return;
-  // both split modes: compensated (FP32 accumulation here makes the SPF error
-  // estimate noisier and the adaptive SPF integration take more steps)
-  if (prec > 0 && nf > 0 && nf <= SPF_G2_N)
-    spf_tile_split2_kernel<<<(unsigned)ntiles, 512, 0, st>>>(d_descs, ndesc, d_ops, out, der_factor);
-  else if (prec > 0)
-    spf_tile_split_kernel<2><<<(unsigned)ntiles, 256, 0, st>>>(d_descs, ndesc, d_ops, out, der_factor);
-  else
-    spf_tile_kernel<<<(unsigned)ntiles, 256, 0, st>>>(d_descs, ndesc, d_ops, out, der_factor);
-  spf_solve_kernel<<<ndesc, 256, 0, st>>>(d_descs, d_status);
-  if (prec > 0) spf_proj_split_kernel<<<(unsigned)ntiles, 256, 0, st>>>(d_descs, ndesc, out);
-  else spf_proj_kernel<<<(unsigned)ntiles, 256, 0, st>>>(d_descs, ndesc, out);
-}
-
-// ---------------------------------------------------------------------------
 // Elementwise helpers
 // ---------------------------------------------------------------------------
 // The launch-wide sum of one complex value per thread, in a fixed order: warps,
@@ -1537,9 +1117,11 @@ __device__ void grid_sum_c(cplx v, cplx* partial, unsigned* counter, cplx* out) 
 // holding i; with dot.v also the launch-wide <dot.v|out> (FP64 products of the
 // values written) into dot.res.  Each block streams a contiguous chunk of the
 // elements with the current range's source descriptors cached in shared memory.
-// PREC 0: FP64.  PREC 1: FP32 coefficients times FP32-rounded sources accumulated
-// in FP32 (the sources are FP32 products there).  PREC 2: compensated FP32 pairs
-// (df_fma, ~1e-13 relative).
+// PREC 0: FP64; a source with a real or an imaginary coefficient (every term of a
+// Hamiltonian with real coefficients) costs two FP64 instructions, which bound the
+// kernel, instead of four (8-SPF QVC model, about nine sources: 74 -> 34 us).
+// PREC 1: FP32 coefficients times FP32-rounded sources accumulated in FP32 (the
+// sources are FP32 products there).
 #define TERMSUM_CACHE 64
 template <int PREC>
 __global__ void __launch_bounds__(256) termsum_kernel(cplx* __restrict__ out, const SumRange* __restrict__ ranges,
@@ -1609,22 +1191,27 @@ __global__ void __launch_bounds__(256) termsum_kernel(cplx* __restrict__ out, co
     }
     for (long long i = base + threadIdx.x; i < seg_end; i += blockDim.x) {
       const long long li = i - rg.offset;
-      cplx val;
-      if (PREC == 0) {
-        val = mkc(0, 0);
-        for (int k = 0; k < rg.count; ++k) cfma(val, sp[k].coeff, load_c(sp[k].src, li, sp[k].fmt));
-      } else {
-        float rh = 0.f, rl = 0.f, ih = 0.f, il = 0.f;
-        for (int k = 0; k < rg.count; ++k) {
-          const float ch = sp[k].cs[0], cl = sp[k].cs[1], dh = sp[k].cs[2], dl = sp[k].cs[3];
-          const float4 x = load_split(sp[k].src, li, sp[k].fmt);
-          // (c + i d)(xr + i xi)
-          df_fma(rh, rl, ch, cl, x.x, x.z);
-          df_fma(rh, rl, -dh, -dl, x.y, x.w);
-          df_fma(ih, il, ch, cl, x.y, x.w);
-          df_fma(ih, il, dh, dl, x.x, x.z);
+      cplx val = mkc(0, 0);
+      for (int k0 = 0; k0 < rg.count; k0 += 4) {
+        cplx x[4];
+#pragma unroll
+        for (int k = 0; k < 4; ++k)
+          x[k] = k0 + k < rg.count ? load_c(sp[k0 + k].src, li, sp[k0 + k].fmt) : mkc(0, 0);
+#pragma unroll
+        for (int k = 0; k < 4; ++k) {
+          if (k0 + k >= rg.count) break;
+          const cplx c = sp[k0 + k].coeff;
+          const int kind = sp[k0 + k].kind;
+          if (kind == 1) {          // i c.y
+            val.x = fma(-c.y, x[k].y, val.x);
+            val.y = fma(c.y, x[k].x, val.y);
+          } else if (kind == 2) {   // c.x
+            val.x = fma(c.x, x[k].x, val.x);
+            val.y = fma(c.x, x[k].y, val.y);
+          } else {
+            cfma(val, c, x[k]);
+          }
         }
-        val = mkc(f2d_exact(rh) + f2d_exact(rl), f2d_exact(ih) + f2d_exact(il));
       }
       out[i] = val;
       if (dot.v) cfma_conj(d, dot.v[i], val);
@@ -1641,8 +1228,6 @@ void launch_termsum(cplx* out, const SumRange* d_ranges, int nranges, const SumS
   const unsigned nb = (unsigned)std::min<long long>((total + 255) / 256, FUSED_BLOCKS);
   if (prec == 1)
     termsum_kernel<1><<<nb, 256, 0, st>>>(out, d_ranges, nranges, d_srcs, total, dot);
-  else if (prec > 1)
-    termsum_kernel<2><<<nb, 256, 0, st>>>(out, d_ranges, nranges, d_srcs, total, dot);
   else
     termsum_kernel<0><<<nb, 256, 0, st>>>(out, d_ranges, nranges, d_srcs, total, dot);
 }

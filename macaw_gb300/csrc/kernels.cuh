@@ -44,6 +44,7 @@ struct HoleDesc {
   int xfmt, yfmt;          // TF_*
   int nred;                // partial blocks left to add: 1 (the contraction adds its own) or nblk
   unsigned* counter;       // blocks done (zero between launches)
+  long long yoff;          // Y null: Y = ybase of the launch + yoff
 };
 
 // out (n1 x n2, leading dim ld) = [out +] sum_t alpha_t * sum_blocks partial_t
@@ -103,23 +104,21 @@ struct MFOp {
 
 // SPF derivative of one DVR mode and state (derivatives.f90:96-153):
 // dphi = f * sum_k ophi_k * rhom1MF_k^T, then dphi -= phi (phi^H phi)^-1 phi^H dphi.
+#define SPF_ROWS 64          // grid rows per block
 struct SpfDesc {
   const cplx* phi;         // G x n
   long long out_offset;    // offset of the block in the output vector
   int G, n;
-  int op_first, op_count;
-  cplx* partial;           // [ntile][2 n^2]: per grid tile phi^H phi and phi^H dphi
-  cplx* X;                 // n x n: (phi^H phi)^-1 phi^H dphi
-  long long block_start;   // first tile block of this descriptor
-  int ntile;
-  int pad;
+  int step_first, step_count;
+  const cplx* S;           // phi^H phi, phi^H dphi: the contractions' sums (n x n)
+  const cplx* O;
+  long long block_start;   // first row block of this descriptor
 };
-#define SPF_TILE 32          // grid rows per block of the tiled SPF derivative
-struct SpfOp {
-  const cplx* ophi;        // G x n2
-  const cplx* rm;          // n x n2 (ld n)
-  int n2;
-  int pad;
+// up to eight columns j2 of one operator: x = ophi(:, j2) (G x nj), rm = rhom1MF(:, j2) (n x nj)
+struct SpfStep {
+  const cplx* x;
+  const cplx* rm;
+  int nj, pad;
 };
 
 // Elementwise weighted sum of source tensors into a range of the output vector.
@@ -131,12 +130,13 @@ struct SumSrc {
   const cplx* src;
   cplx coeff;
   int fmt;                 // TF_*
-  int pad;
+  int kind;                // coeff: 0 complex, 1 imaginary, 2 real (set by split_coeffs)
   float cs[4];             // coeff split into FP32 pairs (re hi, re lo, im hi, im lo), set by split_coeffs
 };
-// Fill SumSrc::cs from coeff for the compensated term sums (host, before upload).
+// Fill SumSrc::kind and SumSrc::cs from coeff (host, before upload).
 inline void split_coeffs(std::vector<SumSrc>& v) {
   for (auto& s : v) {
+    s.kind = s.coeff.x == 0.0 ? 1 : (s.coeff.y == 0.0 ? 2 : 0);
     const float rh = (float)s.coeff.x, ih = (float)s.coeff.y;
     s.cs[0] = rh;
     s.cs[1] = (float)(s.coeff.x - (double)rh);
@@ -241,7 +241,7 @@ void launch_hole(const HoleDesc* d_descs, int ndesc, long long nblocks, int maxn
 void launch_prod_fx(const ProdDesc* d_descs, int ndesc, long long nblocks, int maxn, cudaStream_t st, int persist);
 // f32: operands may be complex FP32
 void launch_hole_fx(const HoleDesc* d_descs, int ndesc, long long nblocks, int maxn, bool f32, cudaStream_t st,
-                    int persist);
+                    int persist, const cplx* ybase = nullptr);
 void launch_reduce(const RedTarget* d_tg, int ntg, const RedTerm* d_terms, cudaStream_t st);
 // with_h: also h1mode (second launch: the Hermitian part of same-state matrices, and
 // the operator sums `sums`); prec > 0: the operator products and phi^H (O phi) in
@@ -249,12 +249,11 @@ void launch_reduce(const RedTarget* d_tg, int ntg, const RedTerm* d_terms, cudaS
 void launch_h1(const H1Desc* d_descs, int ndesc, int maxn2, size_t smem_bytes, bool with_h, cudaStream_t st,
                int prec, const MatSumDesc* sums = nullptr, int nsums = 0, const MatSumSrc* srcs = nullptr);
 void launch_reginv(const RegInvDesc* d_descs, int ndesc, const MFOp* d_ops, int* d_status, cudaStream_t st);
-// prec > 0: the tile products in compensated split FP32 (spf_tile_split_kernel)
-// nf: the largest SPF count of the descriptors and their operators (<= 16: the
-// two-group split tile kernel)
-void launch_spf(const SpfDesc* d_descs, int ndesc, long long ntiles, const SpfOp* d_ops, cplx* out,
-                cplx der_factor, int* d_status, cudaStream_t st, int prec, int nf = 0);
-// prec > 0: compensated split-FP32 accumulation (termsum_split_kernel)
+// holes: the contractions phi^H phi and phi^H dphi of every block (Y null: at yoff of out)
+void launch_spf(const SpfDesc* d_descs, int ndesc, long long ntiles, int maxn, const SpfStep* d_steps,
+                const HoleDesc* d_holes, int nholes, long long hole_blocks, cplx* out, cplx der_factor, int* d_status,
+                cudaStream_t st);
+// prec 1: FP32 accumulation, else FP64
 // A sum over a whole launch fused into a streaming kernel: v the vector to dot
 // with (termsum: <v|out>; Lanczos axpy: any non-null v requests ||Kn||^2), partial
 // one complex per block of the launch, counter zero-initialised, result in res.

@@ -1,0 +1,331 @@
+// SPF derivatives of the grid modes (derivatives.f90:94-153) for sm_103a: exact digit
+// products on the tensor cores (fixed.cuh) for the operator sum and the projection,
+// FP64 for the small solve.  Three launches over all (mode, state) blocks:
+//  (1) spf_drive_kernel: dphi = f sum_k ophi_k rhom1MF_k^T, 64 grid rows per CTA;
+//  (2) the contractions phi^H phi and phi^H dphi (fixed.cu);
+//  (3) spf_project_kernel: solve (phi^H phi) X = phi^H dphi (zposv 'U'), dphi -= phi X.
+#include "kernels.cuh"
+#include "fixed.cuh"
+
+#define SPF_THREADS 128
+#define SPF_NS 8
+#define SPF_CHUNK 9      // steps of eight j2 between flushes: 9 x 16 x 7 x 2^14 < 2^24
+
+#define SPF_PITCH (SPF_ROWS + 2)   // staged rows of a column: the lanes' 16-byte reads meet no bank twice
+
+// Shared operands of row_products.
+struct RowShared {
+  cplx x[SPF_CHUNK][8][SPF_PITCH];         // the CTA's rows of a chunk of steps
+  uint2 W[SPF_CHUNK][2][SPF_NS][32];       // digits of eight columns of the matrix (j2 = q and q + 4)
+  unsigned colmag[MAXN_SPF];
+};
+
+__device__ __forceinline__ void copy_async16(void* dst, const void* src) {
+  asm volatile("cp.async.ca.shared.global [%0], [%1], 16;" ::"r"((unsigned)__cvta_generic_to_shared(dst)), "l"(src)
+               : "memory");
+}
+__device__ __forceinline__ void copy_async_wait() { asm volatile("cp.async.wait_all;" ::: "memory"); }
+
+// Rows row0 .. row0 + 63 of the steps [s0, s0 + ns) on their way into S.x (zeros beyond
+// G and nj); copy_async_wait and a barrier complete it.
+template <typename Step>
+__device__ __forceinline__ void stage_rows(RowShared& S, int s0, int ns, Step&& step, int G, int row0) {
+  const int row = threadIdx.x & (SPF_ROWS - 1), jr = threadIdx.x / SPF_ROWS;
+  for (int s = 0; s < ns; ++s) {
+    const SpfStep st = step(s0 + s);
+#pragma unroll
+    for (int j = 0; j < 8; j += SPF_THREADS / SPF_ROWS) {
+      cplx* to = &S.x[s][j + jr][row];
+      if (row0 + row < G && j + jr < st.nj) copy_async16(to, st.x + row0 + row + (long long)G * (j + jr));
+      else *to = mkc(0.0, 0.0);
+    }
+  }
+}
+
+// The CTA's rows row0 .. row0 + 63 of sum_steps sum_j x(row, j) rm(j1, j) for all
+// j1 < n: a warp owns 16 rows (the MMA's rows), its columns the (re, im) of four j1; a row
+// has one exponent per chunk of steps, a column j1 of the matrices another.  step(s)
+// returns the s-th step (up to eight j); the first chunk is staged already.
+// put(row, j1, value) takes the results; rows from G on are skipped.  Operands outside
+// the exponent range are multiplied in FP64.
+template <typename Step, typename Put>
+__device__ __forceinline__ void row_products(RowShared& S, int nsteps, Step&& step, int n, int G, int row0, Put&& put) {
+  constexpr int NS = SPF_NS;
+  const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5, g = lane >> 2, q = lane & 3;
+  const int lr = 16 * warp + g;   // the lane's rows: lr, lr + 8
+  for (int j0 = 0; j0 < n; j0 += 8) {   // eight outputs per pass
+    cplx sum[2][2];                     // [group of four j1][row]
+    for (int s0 = 0; s0 < nsteps; s0 += SPF_CHUNK) {
+      const int ns = min(SPF_CHUNK, nsteps - s0);
+      if (s0 || (j0 && nsteps > SPF_CHUNK)) {
+        __syncthreads();   // the previous chunk is read
+        stage_rows(S, s0, ns, step, G, row0);
+      }
+      if (tid < 8) S.colmag[tid] = 0u;
+      copy_async_wait();
+      __syncthreads();
+      unsigned mag[2] = {0u, 0u};
+      for (int s = 0; s < ns; ++s)
+#pragma unroll
+        for (int f = 0; f < 2; ++f)
+          mag[f] = max(mag[f], max(fx_mag(S.x[s][q][lr + 8 * f]), fx_mag(S.x[s][q + 4][lr + 8 * f])));
+      bool bad = false;
+#pragma unroll
+      for (int f = 0; f < 2; ++f) {
+        mag[f] = max(mag[f], __shfl_xor_sync(0xffffffffu, mag[f], 1));
+        mag[f] = max(mag[f], __shfl_xor_sync(0xffffffffu, mag[f], 2));
+        bad = bad || !fx_ok(mag[f]);
+      }
+      const unsigned eb[2] = {fx_ebits(mag[0]), fx_ebits(mag[1])};
+      const int nc = min(8, n - j0);
+      for (int e = tid; e < 64 * ns; e += SPF_THREADS) {   // (step, j, j1)
+        const int j1 = e & 7, j = (e >> 3) & 7;
+        const SpfStep st = step(s0 + (e >> 6));
+        if (j1 < nc && j < st.nj) atomicMax(&S.colmag[j1], fx_mag(st.rm[j0 + j1 + n * j]));
+      }
+      __syncthreads();
+      if (tid < nc) bad = bad || !fx_ok(S.colmag[tid]);
+      for (int w = warp; w < 2 * ns; w += 4) {
+        const int t = w & 1, s = w >> 1, j1 = 4 * t + (g >> 1);
+        if (4 * t >= nc) continue;
+        const SpfStep st = step(s0 + s);
+        unsigned d0[NS], d1[NS];
+        const cplx m0 = (j1 < nc && q < st.nj) ? st.rm[j0 + j1 + n * q] : mkc(0, 0);
+        const cplx m1 = (j1 < nc && q + 4 < st.nj) ? st.rm[j0 + j1 + n * (q + 4)] : mkc(0, 0);
+        const unsigned em = fx_ebits(S.colmag[j1]);
+        fx_digits<NS>(m0.x, m0.y, em, em, d0);
+        fx_digits<NS>(m1.x, m1.y, em, em, d1);
+#pragma unroll
+        for (int i = 0; i < NS; ++i) {   // column re: (Mr, -Mi); column im: (Mi, Mr)
+          const unsigned w0 = (g & 1) ? __byte_perm(d0[i], d0[i], 0x1032) : d0[i] ^ 0x80000000u;
+          const unsigned w1 = (g & 1) ? __byte_perm(d1[i], d1[i], 0x1032) : d1[i] ^ 0x80000000u;
+          S.W[s][t][i][lane] = make_uint2(w0, w1);
+        }
+      }
+      if (__syncthreads_or(bad)) {   // the pass in FP64
+        for (int e = tid; e < SPF_ROWS * nc; e += SPF_THREADS) {
+          const int row = row0 + (e & (SPF_ROWS - 1)), j1 = j0 + e / SPF_ROWS;
+          if (row >= G) continue;
+          cplx acc = mkc(0, 0);
+          for (int s = 0; s < nsteps; ++s) {
+            const SpfStep st = step(s);
+            for (int j = 0; j < st.nj; ++j) cfma(acc, st.x[row + (long long)G * j], st.rm[j1 + n * j]);
+          }
+          put(row, j1, acc);
+        }
+        goto next_pass;
+      }
+      {
+        float c[2][NS][4];
+#pragma unroll
+        for (int t = 0; t < 2; ++t)
+#pragma unroll
+          for (int i = 0; i < NS; ++i)
+#pragma unroll
+            for (int k = 0; k < 4; ++k) c[t][i][k] = 0.f;
+        for (int s = 0; s < ns; ++s) {
+          unsigned A[NS][4];
+#pragma unroll
+          for (int f = 0; f < 2; ++f)
+#pragma unroll
+            for (int h = 0; h < 2; ++h) {
+              unsigned d[NS];
+              const cplx x = S.x[s][q + 4 * h][lr + 8 * f];
+              fx_digits<NS>(x.x, x.y, eb[f], eb[f], d);
+#pragma unroll
+              for (int i = 0; i < NS; ++i) A[i][2 * h + f] = d[i];
+            }
+#pragma unroll
+          for (int t = 0; t < 2; ++t) {
+            if (4 * t < nc) {
+#pragma unroll
+              for (int i = 0; i < NS; ++i) {
+                const uint2 w = S.W[s][t][i][lane];
+#pragma unroll
+                for (int j = 0; j + i < NS; ++j) fx_mma16(c[t][i + j], A[j], w.x, w.y, false);
+              }
+            }
+          }
+        }
+#pragma unroll
+        for (int t = 0; t < 2; ++t) {
+          if (4 * t < nc) {
+            const int em = (int)fx_ebits(S.colmag[4 * t + q]);
+#pragma unroll
+            for (int f = 0; f < 2; ++f) {
+              const int es = em + (int)eb[f] - ((2044 + 12 + 43) << 20);
+              const cplx v =
+                  mkc(fx_double(fx_join_wide<NS, 1>(c[t], 2 * f), es), fx_double(fx_join_wide<NS, 1>(c[t], 2 * f + 1), es));
+              sum[t][f] = s0 ? cadd(sum[t][f], v) : v;
+            }
+          }
+        }
+      }
+      __syncthreads();   // colmag and W are read
+    }
+#pragma unroll
+    for (int t = 0; t < 2; ++t)
+#pragma unroll
+      for (int f = 0; f < 2; ++f)
+        if (j0 + 4 * t + q < n && row0 + lr + 8 * f < G)
+          put(row0 + lr + 8 * f, j0 + 4 * t + q, nsteps ? sum[t][f] : mkc(0, 0));
+  next_pass:;
+  }
+}
+
+__global__ void __launch_bounds__(SPF_THREADS) spf_drive_kernel(const SpfDesc* __restrict__ descs, int ndesc,
+                                                                const SpfStep* __restrict__ steps,
+                                                                cplx* __restrict__ out, cplx der) {
+  extern __shared__ __align__(16) unsigned char spf_sm[];
+  RowShared& S = *reinterpret_cast<RowShared*>(spf_sm);
+  __shared__ SpfStep st[SPF_CHUNK];
+  const SpfDesc& d = descs[warp_find_desc(descs, ndesc, (long long)blockIdx.x)];
+  const SpfStep* gst = steps + d.step_first;
+  const int nsteps = d.step_count;
+  // one chunk's steps in shared memory; longer lists are read where they are
+  const bool local = nsteps <= SPF_CHUNK;
+  if (local && (int)threadIdx.x < nsteps) st[threadIdx.x] = gst[threadIdx.x];
+  __syncthreads();
+  cplx* o = out + d.out_offset;
+  const int G = d.G, row0 = (int)(blockIdx.x - d.block_start) * SPF_ROWS;
+  const bool rot = der.x == 0.0 && der.y == -1.0, neg = der.x == -1.0 && der.y == 0.0;
+  auto step = [&](int s) { return local ? st[s] : gst[s]; };
+  stage_rows(S, 0, min(SPF_CHUNK, nsteps), step, G, row0);
+  row_products(S, nsteps, step, d.n, G, row0, [&](int row, int j1, cplx v) {
+    o[row + (long long)G * j1] = rot ? mkc(v.y, -v.x) : (neg ? mkc(-v.x, -v.y) : cmul(der, v));
+  });
+}
+
+// 1 / d for d > 0 by Newton's iteration on the hardware's approximate reciprocal
+__device__ __forceinline__ double newton_rcp(double d) {
+  double y;
+  asm("rcp.approx.ftz.f64 %0, %1;" : "=d"(y) : "d"(d));
+  y = fma(y, fma(-d, y, 1.0), y);
+  return fma(y, fma(-d, y, 1.0), y);
+}
+
+// (phi^H phi) X = phi^H dphi by Gauss-Jordan elimination of [S | O] without pivoting,
+// which is stable for the Hermitian positive definite S.  Pivots are real; a thread
+// holds EPT elements in registers, and per pivot one column and one row pass through
+// shared memory (two buffers, one barrier).  X transposed into Xt[j + n k] = X(k, j).
+// Returns false at a pivot that is not positive.
+template <int EPT>
+__device__ __forceinline__ bool solve_elimination(const SpfDesc& d, cplx (*colb)[MAXN_SPF], cplx (*rowb)[2 * MAXN_SPF],
+                                                  cplx* Xt) {
+  const int n = d.n;
+  cplx a[EPT];
+  int ei[EPT], ec[EPT];   // the element's row and column (column -1: none)
+#pragma unroll
+  for (int q = 0; q < EPT; ++q) {
+    const int e = threadIdx.x + q * SPF_THREADS;
+    a[q] = mkc(0, 0);
+    const int c = e / n, i = e - c * n;
+    ei[q] = i;
+    ec[q] = c < 2 * n ? c : -1;
+    if (ec[q] < 0) continue;
+    // the contraction's upper triangle is authoritative
+    a[q] = c < n ? (i <= c ? d.S[i + n * c] : cconj(d.S[c + n * i])) : d.O[i + n * (c - n)];
+    if (c == 0) colb[0][i] = a[q];
+    if (i == 0) rowb[0][c] = a[q];
+  }
+  bool ok = true;
+  for (int k = 0; k < n; ++k) {
+    __syncthreads();
+    const int b = k & 1;
+    const double p = rowb[b][k].x;
+    ok = ok && p > 0.0;
+    const double pinv = newton_rcp(p);
+#pragma unroll
+    for (int q = 0; q < EPT; ++q) {
+      const int i = ei[q], c = ec[q];
+      if (c <= k) continue;
+      const cplx r = cscale(rowb[b][c], pinv);   // the scaled pivot row
+      if (i == k) {
+        a[q] = r;
+      } else {
+        const cplx f = colb[b][i];
+        a[q].x = fma(-f.x, r.x, fma(f.y, r.y, a[q].x));
+        a[q].y = fma(-f.x, r.y, fma(-f.y, r.x, a[q].y));
+      }
+      if (c == k + 1) colb[b ^ 1][i] = a[q];
+      if (i == k + 1) rowb[b ^ 1][c] = a[q];
+    }
+  }
+#pragma unroll
+  for (int q = 0; q < EPT; ++q) {
+    if (ec[q] >= n) Xt[ec[q] - n + n * ei[q]] = a[q];
+  }
+  return ok;
+}
+
+// Every CTA solves for itself (64 rows each: one or two CTAs per (mode, state) and SM
+// at the sizes met), then subtracts its rows of phi X; its rows of phi and dphi are
+// copied meanwhile.  Up to eight SPFs the product is 8 n FP64 instructions a row and
+// column pair of warps, less than cutting and joining digits.
+__global__ void __launch_bounds__(SPF_THREADS) spf_project8_kernel(const SpfDesc* __restrict__ descs, int ndesc,
+                                                                   cplx* __restrict__ out, int* status) {
+  __shared__ cplx colb[2][MAXN_SPF], rowb[2][2 * MAXN_SPF], Xt[64], phs[8 * SPF_ROWS], dph[8 * SPF_ROWS];
+  const SpfDesc& d = descs[warp_find_desc(descs, ndesc, (long long)blockIdx.x)];
+  const int n = d.n, G = d.G, tile = (int)(blockIdx.x - d.block_start), row0 = tile * SPF_ROWS;
+  const int row = threadIdx.x & (SPF_ROWS - 1);
+  const bool in = row0 + row < G;
+  cplx* o = out + d.out_offset + row0 + row;
+  const cplx* phi = d.phi + row0 + row;
+  for (int j = threadIdx.x / SPF_ROWS; j < n && in; j += SPF_THREADS / SPF_ROWS) {
+    copy_async16(phs + row + SPF_ROWS * j, phi + (long long)G * j);
+    copy_async16(dph + row + SPF_ROWS * j, o + (long long)G * j);
+  }
+  const bool ok = solve_elimination<1>(d, colb, rowb, Xt);
+  if (threadIdx.x == 0 && tile == 0 && !ok) atomicOr(status, DEVST_CHOL_FAIL);
+  copy_async_wait();
+  __syncthreads();
+  for (int j = threadIdx.x / SPF_ROWS; j < n && in; j += SPF_THREADS / SPF_ROWS) {
+    cplx v = dph[row + SPF_ROWS * j];
+    for (int k = 0; k < n; ++k) {
+      const cplx x = phs[row + SPF_ROWS * k], c = Xt[j + n * k];
+      v.x = fma(-x.x, c.x, fma(x.y, c.y, v.x));
+      v.y = fma(-x.x, c.y, fma(-x.y, c.x, v.y));
+    }
+    o[(long long)G * j] = v;
+  }
+}
+__global__ void __launch_bounds__(SPF_THREADS) spf_project_kernel(const SpfDesc* __restrict__ descs, int ndesc,
+                                                                  cplx* __restrict__ out, int* status) {
+  extern __shared__ __align__(16) unsigned char spf_sm[];
+  RowShared& S = *reinterpret_cast<RowShared*>(spf_sm);
+  __shared__ cplx colb[2][MAXN_SPF], rowb[2][2 * MAXN_SPF];
+  const SpfDesc& d = descs[warp_find_desc(descs, ndesc, (long long)blockIdx.x)];
+  const int n = d.n, G = d.G, tile = (int)(blockIdx.x - d.block_start), row0 = tile * SPF_ROWS;
+  cplx* Xt = reinterpret_cast<cplx*>(spf_sm + sizeof(RowShared));   // [n][n]
+  cplx* dph = Xt + n * n;                                           // [n][SPF_ROWS]
+  cplx* o = out + d.out_offset;
+  const cplx* phi = d.phi;
+  auto step = [&](int s) { return SpfStep{phi + (long long)G * 8 * s, Xt + n * 8 * s, min(8, n - 8 * s), 0}; };
+  stage_rows(S, 0, (n + 7) / 8, step, G, row0);
+  for (int e = threadIdx.x; e < n * SPF_ROWS; e += SPF_THREADS)
+    if (row0 + (e & (SPF_ROWS - 1)) < G) copy_async16(dph + e, o + row0 + (e & (SPF_ROWS - 1)) + (long long)G * (e / SPF_ROWS));
+  const bool ok = n <= 8 ? solve_elimination<1>(d, colb, rowb, Xt)
+                         : (n <= 16 ? solve_elimination<4>(d, colb, rowb, Xt) : solve_elimination<16>(d, colb, rowb, Xt));
+  if (threadIdx.x == 0 && tile == 0 && !ok) atomicOr(status, DEVST_CHOL_FAIL);
+  __syncthreads();
+  row_products(S, (n + 7) / 8, step, n, G, row0, [&](int row, int j1, cplx v) {
+    o[row + (long long)G * j1] = csub(dph[row - row0 + SPF_ROWS * j1], v);
+  });
+}
+
+void launch_spf(const SpfDesc* d_descs, int ndesc, long long ntiles, int maxn, const SpfStep* d_steps,
+                const HoleDesc* d_holes, int nholes, long long hole_blocks, cplx* out, cplx der_factor, int* d_status,
+                cudaStream_t st) {
+  if (ndesc <= 0) return;
+  const int smem = (int)sizeof(RowShared), smem_x = smem + (int)sizeof(cplx) * maxn * (maxn + SPF_ROWS);
+  static const cudaError_t configured = [] {
+    constexpr int most = (int)(sizeof(RowShared) + sizeof(cplx) * MAXN_SPF * (MAXN_SPF + SPF_ROWS));
+    cudaFuncSetAttribute(spf_drive_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, most);
+    return cudaFuncSetAttribute(spf_project_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, most);
+  }();
+  (void)configured;
+  spf_drive_kernel<<<(unsigned)ntiles, SPF_THREADS, smem, st>>>(d_descs, ndesc, d_steps, out, der_factor);
+  launch_hole_fx(d_holes, nholes, hole_blocks, maxn, false, st, 0, out);
+  if (maxn <= 8) spf_project8_kernel<<<(unsigned)ntiles, SPF_THREADS, 0, st>>>(d_descs, ndesc, out, d_status);
+  else spf_project_kernel<<<(unsigned)ntiles, SPF_THREADS, smem_x, st>>>(d_descs, ndesc, out, d_status);
+}
