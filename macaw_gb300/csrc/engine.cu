@@ -530,7 +530,7 @@ struct Ctx {
   OvlPlan io_plan;     // d_in vs d_out (host API norm/ovl)
   // CMF2 / Lanczos
   cplx* d_krylov = nullptr;  // [ntotA x 21]
-  double* d_lan = nullptr;   // alpha[20], beta[20], evals[20], evecs[400]
+  double* d_lan = nullptr;   // alpha[20], beta[20]
   int lan_nk = 0;
   std::vector<double> lan_evals, lan_evecs;
   cplx* d_coef = nullptr;
@@ -997,7 +997,7 @@ void plan_packets(Ctx& c, std::vector<std::vector<SumSrc>>& srcs, std::vector<st
       for (auto& x : v[s]) ss.push_back(x);
       rr.push_back(r);
     }
-    split_coeffs(ss);
+    sort_sources(rr, ss);
     sp.n = (int)rr.size();
     sp.nsrc = (int)ss.size();
     sp.ranges = upload_vec(c.ar, rr);
@@ -1559,8 +1559,8 @@ void plan_eom(Ctx& c) {
     for (auto& x : srcs[s]) c.src_h.push_back(x);
     c.sum_h.push_back(r);
   }
+  sort_sources(c.sum_h, c.src_h);
   c.sum_d = upload_vec(c.ar, c.sum_h);
-  split_coeffs(c.src_h);
   c.src_d = upload_vec(c.ar, c.src_h);
   for (auto& b : c.gwp_rho_chain) b.finalize(c.ar);
   if (!c.modes_gwp.empty()) plan_gwp_derivs(c);
@@ -1763,8 +1763,8 @@ void plan_hb(Ctx& c) {
     for (auto& x : srcs[s]) c.hbsrc_h.push_back(x);
     ranges.push_back(r);
   }
+  sort_sources(ranges, c.hbsrc_h);
   c.hbsum_d = upload_vec(c.ar, ranges);
-  split_coeffs(c.hbsrc_h);
   c.hbsrc_d = upload_vec(c.ar, c.hbsrc_h);
 }
 
@@ -2799,19 +2799,68 @@ void lan_check(Ctx& c, LanRun& R) {
   }
 }
 
+// Eigenpairs of the real symmetric tridiagonal matrix (d, e): implicit QL with
+// Wilkinson's shift, rotations accumulated into z (n x n, column r the vector of d[r]).
+// On the host: at n <= 20 it takes a few microseconds where one warp of the GPU, whose
+// FP64 chains are serial, took 143 (n = 7).
+void tridiag_eig(int n, double* d, double* e, double* z) {
+  for (int i = 0; i < n; ++i)
+    for (int j = 0; j < n; ++j) z[j + n * i] = i == j ? 1.0 : 0.0;
+  if (n > 0) e[n - 1] = 0.0;
+  for (int l = 0; l < n; ++l) {
+    for (int it = 0;; ++it) {
+      // the unreduced block from l: up to the first negligible off-diagonal element
+      int m = l;
+      while (m + 1 < n && !(fabs(e[m]) <= 0x1p-53 * (fabs(d[m]) + fabs(d[m + 1])))) ++m;
+      if (m == l) break;
+      if (it == 60) throw StatusError(MCTDH_EEIG, "tridiagonal eigensolver did not converge");
+      // the eigenvalue of the leading 2 x 2 block nearer to d[l]
+      const double h = 0.5 * (d[l + 1] - d[l]), r = hypot(h, e[l]);
+      const double mu = d[l] - (h >= 0.0 ? e[l] / (h + r) : e[l] / (h - r)) * e[l];
+      // chase the bulge from the bottom of the block up
+      double g = d[m] - mu, bulge = 0.0;   // the pair to be rotated: (g, bulge) above row m
+      double s = 1.0, c = 1.0, p = 0.0;
+      bool split = false;
+      for (int i = m - 1; i >= l; --i) {
+        const double f = s * e[i], b = c * e[i];
+        bulge = hypot(f, g);
+        e[i + 1] = bulge;
+        if (bulge == 0.0) {
+          d[i + 1] -= p;
+          e[m] = 0.0;
+          split = true;
+          break;
+        }
+        s = f / bulge;
+        c = g / bulge;
+        g = d[i + 1] - p;
+        const double t = (d[i] - g) * s + 2.0 * c * b;
+        p = s * t;
+        d[i + 1] = g + p;
+        g = c * t - b;
+        for (int k = 0; k < n; ++k) {
+          const double z0 = z[k + n * i], z1 = z[k + n * (i + 1)];
+          z[k + n * (i + 1)] = s * z0 + c * z1;
+          z[k + n * i] = c * z0 - s * z1;
+        }
+      }
+      if (split) continue;
+      d[l] -= p;
+      e[l] = g;
+      e[m] = 0.0;
+    }
+  }
+}
+
 void lan_finish(Ctx& c, LanRun& R) {
   RtScope rt(c, RT_LANCZOS);   // one call per Lanczos run
   const int nk = R.nk;
-  launch_jacobi_tridiag(c.d_lan, c.d_lan + NKRYLOV_MAX, nk, c.d_lan + 2 * NKRYLOV_MAX,
-                        c.d_lan + 3 * NKRYLOV_MAX, c.d_status, c.st);
-  c.count();
-  c.lan_evals.assign(nk, 0.0);
+  double* ab = c.h_scal + 128;   // pinned: alpha, beta
+  CK(cudaMemcpyAsync(ab, c.d_lan, sizeof(double) * 2 * NKRYLOV_MAX, cudaMemcpyDeviceToHost, c.st));
+  check_status(c);               // waits for the stream
+  c.lan_evals.assign(ab, ab + nk);
   c.lan_evecs.assign(nk * nk, 0.0);
-  CK(cudaMemcpyAsync(c.lan_evals.data(), c.d_lan + 2 * NKRYLOV_MAX, sizeof(double) * nk, cudaMemcpyDeviceToHost, c.st));
-  CK(cudaMemcpyAsync(c.lan_evecs.data(), c.d_lan + 3 * NKRYLOV_MAX, sizeof(double) * nk * nk,
-                     cudaMemcpyDeviceToHost, c.st));
-  CK(cudaStreamSynchronize(c.st));
-  check_status(c);
+  tridiag_eig(nk, c.lan_evals.data(), ab + NKRYLOV_MAX, c.lan_evecs.data());
   c.lan_nk = nk;
 }
 
@@ -2832,8 +2881,8 @@ void lan_combine(Ctx& c, cplx* BT, double dt) {
     }
   }
   CK(cudaMemcpyAsync(c.d_coef, coef.data(), sizeof(cplx) * nk, cudaMemcpyHostToDevice, c.st));
-  launch_gemv_cols(BT, c.d_krylov, n, c.d_coef, nk, n, c.st);
-  launch_lan_normalize(BT, BT, dot_dev(c, BT, BT, n), nullptr, n, c.st);
+  launch_gemv_cols(BT, c.d_krylov, n, c.d_coef, nk, n, c.st, c.lan_nrm);
+  launch_lan_normalize(BT, BT, c.lan_nrm.res, nullptr, n, c.st);
   c.count(2);
 }
 
@@ -3181,7 +3230,7 @@ void plan_cmf(Ctx& c, CmfState& S) {
       S.opsave = c.ar.calloc_c(off);
     }
     S.krylov0 = c.ar.calloc_c(c.naconftot * (NKRYLOV_MAX + 1));
-    S.lan0 = (double*)c.ar.alloc(sizeof(double) * (3 * NKRYLOV_MAX + NKRYLOV_MAX * NKRYLOV_MAX));
+    S.lan0 = (double*)c.ar.alloc(sizeof(double) * (2 * NKRYLOV_MAX));
   }
   S.elem_mode = upload_vec(c.ar, em);
   // the SPF error norms: compensated split FP32 (~1e-13) in the split modes
@@ -3937,7 +3986,7 @@ Ctx* create(const mctdh_setup_t* s, const MemberBufs* mb = nullptr) {
       }
       c->d_hb = c->ar.calloc_c(c->naconftot);
       c->d_krylov = c->ar.calloc_c(c->naconftot * (NKRYLOV_MAX + 1));
-      c->d_lan = (double*)c->ar.alloc(sizeof(double) * (3 * NKRYLOV_MAX + NKRYLOV_MAX * NKRYLOV_MAX));
+      c->d_lan = (double*)c->ar.alloc(sizeof(double) * (2 * NKRYLOV_MAX));
       c->d_coef = c->ar.calloc_c(NKRYLOV_MAX);
       plan_hb(*c);
       c->d_ovl1 = c->ar.calloc_c(c->ntot);
@@ -4253,7 +4302,6 @@ Ens* ens_create(const mctdh_setup_t* setups, int n) {
     E->spfstep_d = upload_vec(E->ar, E->spfstep_h);
     E->spf_holes.finalize(E->ar);
     E->sum_d = upload_vec(E->ar, E->sum_h);
-    split_coeffs(E->src_h);
     E->src_d = upload_vec(E->ar, E->src_h);
     E->ov_spf_holes.finalize(E->ar);
     E->ov_spf_red.finalize(E->ar);

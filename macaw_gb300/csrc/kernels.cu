@@ -1036,62 +1036,39 @@ void launch_dot(const cplx* a, const cplx* b, long long n, cplx* partial, unsign
   dot_kernel<<<DOT_BLOCKS, 256, 0, st>>>(a, b, n, partial, counter, out);
 }
 
-// Tridiagonal eigenproblem of the Lanczos matrix (dstev, cmf2_integration.f90:85)
-__global__ void tridiag_kernel(const double* alpha, const double* beta, int n, double* evals, double* evecs,
-                               int* status) {
-  __shared__ cplx A[MAXN_SPF * MAXN_SPF];
-  __shared__ cplx V[MAXN_SPF * MAXN_SPF];
-  __shared__ JacRot R[MAXN_SPF / 2];
-  const int ld = MAXN_SPF;
-  for (int e = threadIdx.x; e < n * n; e += blockDim.x) {
-    int i = e % n, j = e / n;
-    double v = 0.0;
-    if (i == j) v = alpha[i];
-    else if (j == i + 1) v = beta[i];
-    else if (i == j + 1) v = beta[j];
-    A[i + ld * j] = mkc(v, 0.0);
-  }
-  __syncthreads();
-  bool ok;
-  jacobi_herm(A, V, n, ld, R, &ok);
-  if (!ok && threadIdx.x == 0) atomicOr(status, DEVST_EIG_NOCONV);
-  for (int e = threadIdx.x; e < n * n; e += blockDim.x) {
-    int i = e % n, j = e / n;
-    evecs[i + n * j] = V[i + ld * j].x;   // real symmetric input keeps V real
-  }
-  if (threadIdx.x < n) evals[threadIdx.x] = A[threadIdx.x + ld * threadIdx.x].x;
-}
-
-void launch_jacobi_tridiag(const double* alpha, const double* beta, int n, double* evals, double* evecs,
-                           int* d_status, cudaStream_t st) {
-  tridiag_kernel<<<1, 32, 0, st>>>(alpha, beta, n, evals, evecs, d_status);
-}
-
 // ---------------------------------------------------------------------------
 // Elementwise helpers
 // ---------------------------------------------------------------------------
-// The launch-wide sum of one complex value per thread, in a fixed order: warps,
-// then the block's warps into partial[blockIdx.x]; the last block to finish adds
-// the block sums in block order into *out and resets the counter (graph replays).
-// Every thread of every block calls it (no early returns before it).
-__device__ __forceinline__ cplx warp_sum_cd(cplx v) {
-  for (int off = 16; off > 0; off >>= 1) {
-    v.x += __shfl_down_sync(0xffffffffu, v.x, off);
-    v.y += __shfl_down_sync(0xffffffffu, v.y, off);
+// The launch-wide sum of one complex value per thread, in a fixed order: the block's
+// values in shared memory, the components by warps 0 and 1 into partial[blockIdx.x];
+// the last block to finish adds the block sums likewise into *out and resets the
+// counter (graph replays).  Every thread of every block (256 threads) calls it.  Two
+// warps add where a tree in every warp took 85 FP64 instructions per block instead of
+// 26 (LANAXPY_FIG).
+#define GRID_SUM_THREADS 256
+__device__ __forceinline__ void block_sum_c(cplx v, double (*sv)[GRID_SUM_THREADS], cplx* res) {
+  const int tid = threadIdx.x, lane = tid & 31;
+  sv[0][tid] = v.x;
+  sv[1][tid] = v.y;
+  __syncthreads();
+  if (tid < 64) {
+    const double* c = sv[tid >> 5];
+    double t = c[lane];
+#pragma unroll
+    for (int k = 32; k < GRID_SUM_THREADS; k += 32) t += c[lane + k];
+    for (int off = 16; off > 0; off >>= 1) t += __shfl_down_sync(0xffffffffu, t, off);
+    if (lane == 0) reinterpret_cast<double*>(res)[tid >> 5] = t;
   }
-  return v;
+  __syncthreads();
 }
 __device__ void grid_sum_c(cplx v, cplx* partial, unsigned* counter, cplx* out) {
-  __shared__ cplx ws[32];
+  __shared__ double sv[2][GRID_SUM_THREADS];
+  __shared__ cplx r;
   __shared__ bool last;
-  const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5, nw = (blockDim.x + 31) >> 5;
-  v = warp_sum_cd(v);
-  if (lane == 0) ws[warp] = v;
-  __syncthreads();
+  const int tid = threadIdx.x;
+  block_sum_c(v, sv, &r);
   if (tid == 0) {
-    cplx t = ws[0];
-    for (int w = 1; w < nw; ++w) t = cadd(t, ws[w]);
-    partial[blockIdx.x] = t;
+    partial[blockIdx.x] = r;
     __threadfence();
     last = (atomicAdd(counter, 1u) == gridDim.x - 1);
   }
@@ -1100,14 +1077,9 @@ __device__ void grid_sum_c(cplx v, cplx* partial, unsigned* counter, cplx* out) 
   __threadfence();
   const volatile double* pv = (const volatile double*)partial;
   cplx t = mkc(0.0, 0.0);
-  for (int q = tid; q < (int)gridDim.x; q += blockDim.x) t = cadd(t, mkc(pv[2 * q], pv[2 * q + 1]));
-  t = warp_sum_cd(t);
-  __syncthreads();
-  if (lane == 0) ws[warp] = t;
-  __syncthreads();
+  for (int q = tid; q < (int)gridDim.x; q += GRID_SUM_THREADS) t = cadd(t, mkc(pv[2 * q], pv[2 * q + 1]));
+  block_sum_c(t, sv, &r);
   if (tid == 0) {
-    cplx r = ws[0];
-    for (int w = 1; w < nw; ++w) r = cadd(r, ws[w]);
     *out = r;
     *counter = 0u;
   }
@@ -1115,109 +1087,97 @@ __device__ void grid_sum_c(cplx v, cplx* partial, unsigned* counter, cplx* out) 
 
 // out[i] = sum_k coeff_k src_k[i - offset] over the sources of the state range
 // holding i; with dot.v also the launch-wide <dot.v|out> (FP64 products of the
-// values written) into dot.res.  Each block streams a contiguous chunk of the
-// elements with the current range's source descriptors cached in shared memory.
-// PREC 0: FP64; a source with a real or an imaginary coefficient (every term of a
-// Hamiltonian with real coefficients) costs two FP64 instructions, which bound the
-// kernel, instead of four (8-SPF QVC model, about nine sources: 74 -> 34 us).
+// values written) into dot.res.  The warps of the launch take rows of 32 elements in
+// turn: contiguous shares per block left every thread a sixth, nearly empty round at
+// 786,432 elements.
+// PREC 0: FP64, bound by its instructions: two per source with a real or an imaginary
+// coefficient (every term of a Hamiltonian with real coefficients), four otherwise.
+// The sources come sorted by kind; told apart inside the loop they were issued under
+// predicates and all paid for (8-SPF QVC model, about ten sources a state: TERMSUM_FIG).
 // PREC 1: FP32 coefficients times FP32-rounded sources accumulated in FP32 (the
 // sources are FP32 products there).
 #define TERMSUM_CACHE 64
+// KIND 0 complex, 1 imaginary, 2 real
+template <int KIND>
+__device__ __forceinline__ void termsum_run(cplx& val, const SumSrc* sp, int n, long long li) {
+  for (int k0 = 0; k0 < n; k0 += 4) {
+    cplx x[4];
+#pragma unroll
+    for (int k = 0; k < 4; ++k)
+      if (k0 + k < n) x[k] = load_c(sp[k0 + k].src, li, sp[k0 + k].fmt);
+#pragma unroll
+    for (int k = 0; k < 4; ++k) {
+      if (k0 + k >= n) break;
+      const cplx c = sp[k0 + k].coeff;
+      if (KIND == 1) {
+        val.x = fma(-c.y, x[k].y, val.x);
+        val.y = fma(c.y, x[k].x, val.y);
+      } else if (KIND == 2) {
+        val.x = fma(c.x, x[k].x, val.x);
+        val.y = fma(c.x, x[k].y, val.y);
+      } else {
+        cfma(val, c, x[k]);
+      }
+    }
+  }
+}
 template <int PREC>
 __global__ void __launch_bounds__(256) termsum_kernel(cplx* __restrict__ out, const SumRange* __restrict__ ranges,
                                                       int nr, const SumSrc* __restrict__ srcs, long long total,
                                                       FusedDot dot) {
   __shared__ SumSrc ss[TERMSUM_CACHE];
-  __shared__ int s_rg;
-  const long long chunk = (total + gridDim.x - 1) / gridDim.x;
-  const long long start = (long long)blockIdx.x * chunk, end = min(total, start + chunk);
+  const int nsrc = ranges[nr - 1].first + ranges[nr - 1].count;
+  const bool cached = nsrc <= TERMSUM_CACHE;
+  if (cached)
+    for (int k = threadIdx.x; k < nsrc; k += blockDim.x) ss[k] = srcs[k];
+  __syncthreads();
+  const SumSrc* all = cached ? ss : srcs;
   cplx d = mkc(0, 0);
-  long long base = start;
-  while (base < end) {
-    if (threadIdx.x == 0) {
-      int lo = 0, hi = nr - 1;   // last range starting at or before base (ranges sorted by offset)
+  SumRange rg;
+  rg.offset = rg.n = 0;
+  // warp w of the launch: neighbouring warps of a block work far apart
+  const long long wrow = ((long long)(threadIdx.x >> 5) * gridDim.x + blockIdx.x) * 32 + (threadIdx.x & 31);
+  for (long long i = wrow; i < total; i += (long long)gridDim.x * blockDim.x) {
+    if (i - rg.offset >= rg.n) {
+      int lo = 0, hi = nr - 1;   // last range starting at or before i (ranges sorted by offset)
       while (lo < hi) {
         const int mid = (lo + hi + 1) >> 1;
-        if (ranges[mid].offset <= base) lo = mid; else hi = mid - 1;
+        if (ranges[mid].offset <= i) lo = mid; else hi = mid - 1;
       }
-      s_rg = lo;
+      rg = ranges[lo];
+      if (i - rg.offset >= rg.n || i < rg.offset) {   // outside every range
+        rg.n = 0;
+        continue;
+      }
     }
-    __syncthreads();
-    const SumRange rg = ranges[s_rg];
-    long long seg_end = min(end, rg.offset + rg.n);
-    if (base < rg.offset || base >= rg.offset + rg.n) {
-      // outside every range: skip to the next range start
-      seg_end = (s_rg + 1 < nr) ? min(end, ranges[s_rg + 1].offset) : end;
-      __syncthreads();
-      base = max(seg_end, base + 1);
-      continue;
-    }
-    const bool cached = rg.count <= TERMSUM_CACHE;
-    if (cached)
-      for (int k = threadIdx.x; k < rg.count; k += blockDim.x) ss[k] = srcs[rg.first + k];
-    __syncthreads();
-    const SumSrc* sp = cached ? ss : srcs + rg.first;
+    const long long li = i - rg.offset;
+    const SumSrc* sp = all + rg.first;
+    cplx val;
     if (PREC == 1) {
-      // four elements per thread in flight: per source, four independent loads
-      const long long stride = (long long)blockDim.x;
-      for (long long i0 = base + threadIdx.x; i0 < seg_end; i0 += 4 * stride) {
-        float ar[4] = {0.f, 0.f, 0.f, 0.f}, ai[4] = {0.f, 0.f, 0.f, 0.f};
-        for (int k = 0; k < rg.count; ++k) {
-          const float cr = sp[k].cs[0] + sp[k].cs[1], ci = sp[k].cs[2] + sp[k].cs[3];
-          const cplx* src = sp[k].src;
-          const int fmt = sp[k].fmt;
-#pragma unroll
-          for (int e = 0; e < 4; ++e) {
-            const long long i = i0 + e * stride;
-            if (i >= seg_end) break;
-            const float4 x = load_split(src, i - rg.offset, fmt);
-            const float xr = x.x + x.z, xi = x.y + x.w;
-            ar[e] = fmaf(cr, xr, fmaf(-ci, xi, ar[e]));
-            ai[e] = fmaf(cr, xi, fmaf(ci, xr, ai[e]));
-          }
-        }
-#pragma unroll
-        for (int e = 0; e < 4; ++e) {
-          const long long i = i0 + e * stride;
-          if (i >= seg_end) break;
-          const cplx val = mkc(f2d_exact(ar[e]), f2d_exact(ai[e]));
-          out[i] = val;
-          if (dot.v) cfma_conj(d, dot.v[i], val);
-        }
-      }
-      __syncthreads();
-      base = seg_end;
-      continue;
-    }
-    for (long long i = base + threadIdx.x; i < seg_end; i += blockDim.x) {
-      const long long li = i - rg.offset;
-      cplx val = mkc(0, 0);
+      float ar = 0.f, ai = 0.f;
       for (int k0 = 0; k0 < rg.count; k0 += 4) {
-        cplx x[4];
+        float4 x[4];
 #pragma unroll
         for (int k = 0; k < 4; ++k)
-          x[k] = k0 + k < rg.count ? load_c(sp[k0 + k].src, li, sp[k0 + k].fmt) : mkc(0, 0);
+          if (k0 + k < rg.count) x[k] = load_split(sp[k0 + k].src, li, sp[k0 + k].fmt);
 #pragma unroll
         for (int k = 0; k < 4; ++k) {
           if (k0 + k >= rg.count) break;
-          const cplx c = sp[k0 + k].coeff;
-          const int kind = sp[k0 + k].kind;
-          if (kind == 1) {          // i c.y
-            val.x = fma(-c.y, x[k].y, val.x);
-            val.y = fma(c.y, x[k].x, val.y);
-          } else if (kind == 2) {   // c.x
-            val.x = fma(c.x, x[k].x, val.x);
-            val.y = fma(c.x, x[k].y, val.y);
-          } else {
-            cfma(val, c, x[k]);
-          }
+          const float cr = sp[k0 + k].cs[0] + sp[k0 + k].cs[1], ci = sp[k0 + k].cs[2] + sp[k0 + k].cs[3];
+          const float xr = x[k].x + x[k].z, xi = x[k].y + x[k].w;
+          ar = fmaf(cr, xr, fmaf(-ci, xi, ar));
+          ai = fmaf(cr, xi, fmaf(ci, xr, ai));
         }
       }
-      out[i] = val;
-      if (dot.v) cfma_conj(d, dot.v[i], val);
+      val = mkc(f2d_exact(ar), f2d_exact(ai));
+    } else {
+      val = mkc(0, 0);
+      termsum_run<1>(val, sp, rg.nimag, li);
+      termsum_run<2>(val, sp + rg.nimag, rg.nreal, li);
+      termsum_run<0>(val, sp + rg.nimag + rg.nreal, rg.count - rg.nimag - rg.nreal, li);
     }
-    __syncthreads();
-    base = seg_end;
+    out[i] = val;
+    if (dot.v) cfma_conj(d, dot.v[i], val);
   }
   if (dot.v) grid_sum_c(d, dot.partial, dot.counter, dot.res);
 }
@@ -1365,17 +1325,23 @@ void launch_axpy(cplx* y, const cplx* x, cplx a, long long n, cudaStream_t st) {
   axpy_kernel<<<(unsigned)((n + 255) / 256), 256, 0, st>>>(y, x, a, n);
 }
 
-__global__ void gemv_cols_kernel(cplx* out, const cplx* basis, long long ld, const cplx* coef, int ncol, long long n) {
-  long long i = (long long)blockIdx.x * blockDim.x + threadIdx.x;
-  if (i >= n) return;
-  cplx s = mkc(0, 0);
-  for (int j = 0; j < ncol; ++j) cfma(s, coef[j], basis[i + ld * j]);
-  out[i] = s;
+// out = sum_j coef_j basis_j, and the launch-wide ||out||^2
+__global__ void __launch_bounds__(256) gemv_cols_kernel(cplx* __restrict__ out, const cplx* __restrict__ basis,
+                                                        long long ld, const cplx* __restrict__ coef, int ncol,
+                                                        long long n, FusedDot nrm) {
+  double s2 = 0.0;
+  for (long long i = (long long)blockIdx.x * blockDim.x + threadIdx.x; i < n; i += (long long)gridDim.x * blockDim.x) {
+    cplx s = mkc(0, 0);
+    for (int j = 0; j < ncol; ++j) cfma(s, coef[j], basis[i + ld * j]);
+    out[i] = s;
+    s2 = fma(s.x, s.x, fma(s.y, s.y, s2));
+  }
+  grid_sum_c(mkc(s2, 0.0), nrm.partial, nrm.counter, nrm.res);
 }
 void launch_gemv_cols(cplx* out, const cplx* basis, long long ld, const cplx* coef, int ncol, long long n,
-                      cudaStream_t st) {
-  if (n <= 0) return;
-  gemv_cols_kernel<<<(unsigned)((n + 255) / 256), 256, 0, st>>>(out, basis, ld, coef, ncol, n);
+                      cudaStream_t st, FusedDot nrm) {
+  const unsigned nb = (unsigned)std::max<long long>(1, std::min<long long>((n + 255) / 256, FUSED_BLOCKS));
+  gemv_cols_kernel<<<nb, 256, 0, st>>>(out, basis, ld, coef, ncol, n, nrm);
 }
 
 // ---------------------------------------------------------------------------
@@ -1536,17 +1502,23 @@ void launch_lan_axpy(cplx* Kn, const cplx* Kj, const cplx* Kp, const cplx* dot_a
   lan_axpy_kernel<<<nb, 256, 0, st>>>(Kn, Kj, Kp, dot_alpha, beta_prev, alpha_out, n, nrm);
 }
 
-// Grid-stride: the norm and its reciprocal once per thread (FP64 square roots and
-// divisions are expensive on this GPU), then one multiply per component.
+// Grid-stride: the norm and its reciprocal once per block (an FP64 square root and a
+// division take 1,160 cycles of a sub-partition's FP64 pipe per warp), then one multiply
+// per component.
 // ... optionally also into copy (FP64) and f32 (complex FP32 rounded to nearest):
 // the input of the next H_B application, written in the same pass.
 __global__ void lan_normalize_kernel(cplx* __restrict__ out, const cplx* __restrict__ in, const cplx* __restrict__ nrm2,
                                      double* beta_out, long long n, cplx* __restrict__ copy,
                                      float2* __restrict__ f32) {
   const long long i0 = (long long)blockIdx.x * blockDim.x + threadIdx.x;
-  const double beta = sqrt(nrm2->x);
-  if (i0 == 0 && beta_out) *beta_out = beta;
-  const double s = 1.0 / beta;
+  __shared__ double s_inv;
+  if (threadIdx.x == 0) {
+    const double beta = sqrt(nrm2->x);
+    if (blockIdx.x == 0 && beta_out) *beta_out = beta;
+    s_inv = 1.0 / beta;
+  }
+  __syncthreads();
+  const double s = s_inv;
   for (long long i = i0; i < n; i += (long long)gridDim.x * blockDim.x) {
     const cplx v = in[i];
     const cplx w = mkc(v.x * s, v.y * s);

@@ -7,6 +7,7 @@
 // touched, element (l, j, r) sits at l + L*(j + n*r), with L = prod of the
 // sizes of the faster modes and R = prod of the sizes of the slower modes.
 #pragma once
+#include <algorithm>
 #include <vector>
 #include "common.cuh"
 
@@ -125,16 +126,18 @@ struct SpfStep {
 struct SumRange {
   long long offset, n;
   int first, count;
+  int nimag, nreal;        // sources first .. with an imaginary, then with a real coefficient (sort_sources)
 };
 struct SumSrc {
   const cplx* src;
   cplx coeff;
   int fmt;                 // TF_*
-  int kind;                // coeff: 0 complex, 1 imaginary, 2 real (set by split_coeffs)
-  float cs[4];             // coeff split into FP32 pairs (re hi, re lo, im hi, im lo), set by split_coeffs
+  int kind;                // coeff: 0 complex, 1 imaginary, 2 real (set by sort_sources)
+  float cs[4];             // coeff split into FP32 pairs (re hi, re lo, im hi, im lo), set by sort_sources
 };
-// Fill SumSrc::kind and SumSrc::cs from coeff (host, before upload).
-inline void split_coeffs(std::vector<SumSrc>& v) {
+// Fill SumSrc::kind and SumSrc::cs from coeff and order every range's sources by kind
+// (imaginary, real, complex; host, before either is uploaded).
+inline void sort_sources(std::vector<SumRange>& ranges, std::vector<SumSrc>& v) {
   for (auto& s : v) {
     s.kind = s.coeff.x == 0.0 ? 1 : (s.coeff.y == 0.0 ? 2 : 0);
     const float rh = (float)s.coeff.x, ih = (float)s.coeff.y;
@@ -142,6 +145,12 @@ inline void split_coeffs(std::vector<SumSrc>& v) {
     s.cs[1] = (float)(s.coeff.x - (double)rh);
     s.cs[2] = ih;
     s.cs[3] = (float)(s.coeff.y - (double)ih);
+  }
+  for (auto& r : ranges) {
+    auto b = v.begin() + r.first, e = b + r.count;
+    std::stable_sort(b, e, [](const SumSrc& x, const SumSrc& y) { return (x.kind + 2) % 3 < (y.kind + 2) % 3; });
+    r.nimag = (int)std::count_if(b, e, [](const SumSrc& x) { return x.kind == 1; });
+    r.nreal = (int)std::count_if(b, e, [](const SumSrc& x) { return x.kind == 2; });
   }
 }
 
@@ -264,6 +273,8 @@ struct FusedDot {
   unsigned* counter;
   cplx* res;
 };
+void launch_gemv_cols(cplx* out, const cplx* basis, long long ld, const cplx* coef, int ncol, long long n,
+                      cudaStream_t st, FusedDot nrm);
 // ---------------------------------------------------------------------------
 // Statistical mixtures and dissipation (gmctdh_objects.f90:481-1141,
 // derivatives.f90:70-83, 238-242).  The coefficients of every state are stored
@@ -333,10 +344,6 @@ void launch_copy_scale(cplx* out, const cplx* in, cplx s, long long n, cudaStrea
 void launch_axpy(cplx* y, const cplx* x, cplx a, long long n, cudaStream_t st);
 // out (complex FP32, TF_F32 storage) = in rounded to nearest
 void launch_to_f32(cplx* out, const cplx* in, long long n, cudaStream_t st);
-void launch_gemv_cols(cplx* out, const cplx* basis, long long ld, const cplx* coef, int ncol, long long n,
-                      cudaStream_t st);
-void launch_jacobi_tridiag(const double* alpha, const double* beta, int n, double* evals, double* evecs,
-                           int* d_status, cudaStream_t st);
 void launch_stage_modes(cplx* out, const cplx* base, const StageArgs& a, const double* dt_mode,
                         const unsigned char* elem_mode, long long off, long long n, cudaStream_t st);
 void launch_masked_copy(cplx* y, const cplx* src, const unsigned char* elem_mode, const int* accept, long long off,
