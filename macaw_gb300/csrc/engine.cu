@@ -545,6 +545,7 @@ struct Ctx {
   std::vector<GwpOvlDesc> gs_h;
   GwpOvlDesc* gs_d = nullptr;
   std::vector<RegInvDesc> gsreg_h;
+  int gsreg_maxn = 0;
   RegInvDesc* gsreg_d = nullptr;
   std::vector<GwpH1Desc> gh1_h;
   GwpH1Desc* gh1_d = nullptr;
@@ -900,6 +901,7 @@ void plan_gwp_setup(Ctx& c) {
       c.s00m1[i][s1] = c.ar.calloc_c((long long)rd.n * rd.n);
       rd.inv_out = c.s00m1[i][s1];
       c.gsreg_h.push_back(rd);
+      c.gsreg_maxn = std::max(c.gsreg_maxn, rd.n);
     }
     // h1mode of every operator of the mode
     c.hmat[m].assign(c.noper[m], nullptr);
@@ -1590,9 +1592,13 @@ void plan_gwp_derivs(Ctx& c) {
       d.rho = c.multiset[m] ? c.rho[m][s] : c.rho_ave[m];
       d.Sa0 = c.ar.calloc_c((long long)nG * n);
       d.Sa0Sm1 = c.ar.calloc_c((long long)nG * n);
-      d.M = c.ar.calloc_c(2LL * nG * (nG + 1));
-      d.R = c.ar.calloc_c((long long)nG * nG);
-      d.x = c.ar.calloc_c(nG);
+      d.M = c.ar.calloc_c((nG + 1LL) * (nG + 1));
+      d.R = c.ar.calloc_c(nG * (nG + 1LL));
+      d.rdiag = c.ar.calloc_c(nG);
+      d.x = c.ar.calloc_c(2LL * nG);
+      d.step = (int*)c.ar.alloc(sizeof(int) * 3 * (nG + 1));
+      d.perm = d.step + nG + 1;
+      d.act = d.perm + nG + 1;
       d.dxi_offset = c.naconftot + c.ipsi[m + f * s];
       c.tau[i][s] = c.ar.calloc_c((long long)n * n);
       d.tau = c.tau[i][s];
@@ -1626,7 +1632,7 @@ void plan_gwp_derivs(Ctx& c) {
   }
   c.cy_d = upload_vec(c.ar, c.cy_h);
   c.yop_d = upload_vec(c.ar, c.yop_h);
-  c.cy_part = c.ar.calloc_c((long long)c.cy_h.size() * c.cy_maxG * c.cy_maxn * std::max(c.cy_maxops, 1));
+  c.cy_part = c.ar.calloc_c(std::max(1LL, (long long)c.cy_h.size() * gwp_y_scratch(c.cy_maxG, c.cy_maxn, c.cy_maxops)));
   // dA = S^-1 (f H A) - tau A on the Gaussian modes
   c.d_adot = c.ar.calloc_c(c.naconftot);
   c.d_dA = c.ar.calloc_c(c.naconftot);
@@ -2070,7 +2076,7 @@ void run_red(Ctx& c, const RedBatch& b) {
 void gwp_setup_run(Ctx& c) {
   ProfScope ps(c, KP_GWP);
   launch_gwp_ovl(c.gs_d, (int)c.gs_h.size(), c.st);
-  launch_tikh_inv(c.gsreg_d, (int)c.gsreg_h.size(), c.st);
+  launch_tikh_inv(c.gsreg_d, (int)c.gsreg_h.size(), c.gsreg_maxn, c.st);
   launch_gwp_h1(c.gh1_d, (int)c.gh1_h.size(), c.st);
   c.count(3);
 }
@@ -2081,9 +2087,8 @@ void gwp_setup_run(Ctx& c) {
 void gwp_solve_run(Ctx& c, cplx* out) {
   RtScope rt(c, RT_CY);   // Calc_CY and the parameter solve (gmctdh_objects.f90:1198-1333)
   ProfScope ps(c, KP_GWP);
-  launch_gwp_cy(c.cy_d, (int)c.cy_h.size(), c.cy_maxG, c.cy_maxn, c.cy_maxops, c.yop_d, c.cy_part, c.st);
-  launch_gwp_solve(c.cy_d, (int)c.cy_h.size(), c.cy_maxG, c.der, out, c.d_status, c.st);
-  c.count(6 + (c.cy_maxG + GWP_QR_PW - 1) / GWP_QR_PW);
+  c.count(launch_gwp_cy(c.cy_d, (int)c.cy_h.size(), c.cy_maxG, c.cy_maxn, c.cy_maxops, c.yop_d, c.cy_part, c.st));
+  c.count(launch_gwp_solve(c.cy_d, (int)c.cy_h.size(), c.cy_maxG, c.der, out, c.d_status, c.st));
 }
 
 void gwp_derivs_run(Ctx& c, cplx* out) {

@@ -11,19 +11,18 @@
 //    coefficient correction (derivatives.f90:201-234).
 //
 // The reference solves C x = Y through the eigen-decomposition of C,
-// x = sum_j u_j w_j / (w_j^2 + eps^2) (u_j^H Y).  That is the minimiser of
-// |C x - Y|^2 + eps^2 |x|^2, which this file computes as the least-squares
-// solution of the stacked system [C; eps I] x = [Y; 0] by Householder QR: the
-// same x, with the conditioning of C/eps instead of (C/eps)^2 of the normal
-// equations, and no iterative eigen-solver.  The QR runs in panels of
-// GWP_QR_PW columns: every block of a launch factors the panel in shared memory
-// and applies its reflectors to its own trailing columns (one warp per column),
-// so no block reads what another block of the same launch writes.
+// x = sum_j u_j w_j / (w_j^2 + eps^2) (u_j^H Y).  With w / (w^2 + eps^2) =
+// (1 / (w + i eps) + 1 / (w - i eps)) / 2 this is the mean of the solutions of
+// (C + i eps) x = Y and (C + i eps)^H x = Y: one LU factorisation with partial
+// pivoting, at the condition |C| / eps of C + i eps (the normal equations would square
+// it) and without an iterative eigen-solver.  Y is carried as a column and Y^H as a row
+// of the factorisation, so only the two back-substitutions remain.
 #include <float.h>
 
 #include <algorithm>
 
 #include "kernels.cuh"
+#include "fixed.cuh"
 
 namespace {
 
@@ -162,9 +161,12 @@ __device__ cplx gau_ovl(const double* a1, const double* a2, const cplx* xi1, con
   return cscale(cexp_(cscale(c, 0.25)), sqrt(sqrt(d)));
 }
 
-__global__ void gwp_ovl_kernel(const GwpOvlDesc* __restrict__ descs) {
+// A warp per 32 entries: an entry is a serial chain of FP64 divisions (443 cycles each)
+// and exponentials, so the warps go to as many sub-partitions as there are (four
+// 32 x 32 overlaps of 12 DOFs: 509 us with a block of eight warps each, OVL_FIG).
+__global__ void __launch_bounds__(32) gwp_ovl_kernel(const GwpOvlDesc* __restrict__ descs) {
   const GwpOvlDesc& d = descs[blockIdx.x];
-  for (int e = threadIdx.x; e < d.n1 * d.n2; e += blockDim.x) {
+  for (int e = blockIdx.y * 32 + threadIdx.x; e < d.n1 * d.n2; e += 32 * gridDim.y) {
     const int j1 = e % d.n1, j2 = e / d.n1;
     cplx v;
     if (d.kind == 3) {
@@ -205,9 +207,9 @@ __device__ cplx gwp_h1_entry(const GwpH1Desc& d, int j1, int j2) {
   return cmul(d.S[j1 + d.n1 * j2], g);
 }
 
-__global__ void gwp_h1_kernel(const GwpH1Desc* __restrict__ descs) {
+__global__ void __launch_bounds__(64) gwp_h1_kernel(const GwpH1Desc* __restrict__ descs) {
   const GwpH1Desc& d = descs[blockIdx.x];
-  for (int e = threadIdx.x; e < d.n1 * d.n2; e += blockDim.x) {
+  for (int e = blockIdx.y * 64 + threadIdx.x; e < d.n1 * d.n2; e += 64 * gridDim.y) {
     const int j1 = e % d.n1, j2 = e / d.n1;
     d.out[e] = (d.same_state && j1 > j2) ? cconj(gwp_h1_entry(d, j2, j1)) : gwp_h1_entry(d, j1, j2);
   }
@@ -267,88 +269,130 @@ __device__ cplx gwp_c_entry(const GwpCYDesc& d, int r, int c) {
   return cmul(d.rho[j1 + d.n * j2], sab);
 }
 
-// The stacked least-squares system [C, Y; eps I, 0]: the Hermitian C from its
-// upper triangle, the Tikhonov block below it.
-__global__ void gwp_c_kernel(const GwpCYDesc* __restrict__ descs) {
+// C + i eps into the bordered system [C + i eps, Y; Y^H, 0], the Hermitian C from its
+// upper triangle (an element costs about 320 FP64 instructions: 64 n for the projection).
+__global__ void __launch_bounds__(64) gwp_c_kernel(const GwpCYDesc* __restrict__ descs) {
   const GwpCYDesc& d = descs[blockIdx.z];
-  const int r = blockIdx.x * blockDim.x + threadIdx.x;
-  const int c = blockIdx.y * blockDim.y + threadIdx.y;
-  if (r >= d.nG || c >= d.nG) return;
-  const long long ld = 2LL * d.nG;
-  d.M[r + ld * c] = (r <= c) ? gwp_c_entry(d, r, c) : cconj(gwp_c_entry(d, c, r));
-  d.M[d.nG + r + ld * c] = mkc(r == c ? d.eps : 0.0, 0.0);
+  const int r0 = 8 * blockIdx.x, c0 = 8 * blockIdx.y;
+  if (r0 > c0) return;
+  const int r = r0 + (threadIdx.x & 7), c = c0 + (threadIdx.x >> 3);
+  if (r > c || c >= d.nG) return;
+  const long long ld = d.nG + 1LL;
+  cplx v = gwp_c_entry(d, r, c);
+  if (r == c)
+    v.y += d.eps;
+  else
+    d.M[c + ld * r] = cconj(v);
+  d.M[r + ld * c] = v;
 }
 
-// Y (gmctdh_objects.f90:1285-1326): per entry r = j1*nmd + k,
-// sum over operators (outer) and j2 (inner) of MF(j1,j2) (Ha0 - Sa0Sm1 h)(r, j2).
-// Stage 1: one thread per (j1, j2, operator) computes the nmd one-dimensional
-// integrals of the pair once, shares them between the k entries through
-// prefix/suffix products, and writes the nmd terms to part[((o*n2 + j2)*nG + r)].
-// Stage 2: one thread per r adds its terms in the reference's order.
-__global__ void gwp_y_part_kernel(const GwpCYDesc* __restrict__ descs, const GwpYOp* __restrict__ ops,
-                                  cplx* __restrict__ part, long long part_ld, int maxn2) {
+// Y (gmctdh_objects.f90:1285-1326): per entry r = j1*nmd + k, the sum over operators and
+// j2 of MF(j1,j2) (Ha0 - Sa0Sm1 h)(r, j2).  The second part is summed over the operators
+// first, G(j, j1) = sum MF(j1, j2) h(j, j2), and multiplied by Sa0Sm1 once: n^2 products
+// per operator instead of n^2 nmd.
+// Stage 1a: a thread per (j1, j2, YOP_CHUNK operators) computes the pair's <q_k> once, the
+// integrals of each operator's acting DOFs, and the nmd sums over its operators into
+// part[(chunk*maxn2 + j2)*nG + r].
+// Stage 1b: a thread per (j, j1, operator) sums its part of G over j2.
+// Stage 2: a warp per r adds the terms in a fixed order.
+#define YOP_CHUNK 4
+__global__ void __launch_bounds__(32) gwp_y_part_kernel(const GwpCYDesc* __restrict__ descs,
+                                                        const GwpYOp* __restrict__ ops, cplx* __restrict__ part,
+                                                        long long part_ld, int maxn2) {
   const GwpCYDesc& d = descs[blockIdx.y];
   const long long e = (long long)blockIdx.x * blockDim.x + threadIdx.x;
-  if (e >= (long long)d.n * maxn2 * d.op_count) return;
+  const int nch = (d.op_count + YOP_CHUNK - 1) / YOP_CHUNK;
+  if (e >= (long long)d.n * maxn2 * nch) return;
   const int j1 = (int)(e % d.n);
   const int j2 = (int)((e / d.n) % maxn2);
-  const int o = (int)(e / ((long long)d.n * maxn2));
-  const GwpYOp& op = ops[d.op_first + o];
-  if (j2 >= op.n2) return;
+  const int ch = (int)(e / ((long long)d.n * maxn2));
   const int nmd = d.nmd;
   const double* a = d.a;
-  cplx g[GWP_MAXDOF], pre[GWP_MAXDOF + 1];
-  for (int q = 0; q < nmd; ++q)
-    g[q] = gau_int_1d(a[q + d.lda * j1], a[q + d.lda * j2], d.xi[q + d.nmd * j1], op.xi2[q + d.nmd * j2], op.ops[q]);
-  pre[0] = mkc(1.0, 0.0);
-  for (int q = 0; q < nmd; ++q) pre[q + 1] = cmul(pre[q], g[q]);
-  const cplx s12 = op.S12[j1 + d.n * j2];
-  const cplx mf = op.mf[j1 + d.n * j2];
-  cplx* out = part + (long long)blockIdx.y * part_ld + ((long long)o * maxn2 + j2) * d.nG;
-  for (int k = 0; k < nmd; ++k) {
-    cplx right = mkc(1.0, 0.0);   // prod_{q > k} g[q] in order (np.prod over gi[k+1:])
-    for (int q = k + 1; q < nmd; ++q) right = cmul(right, g[q]);
-    const cplx g10 = gau10_int_1d(a[k + d.lda * j1], a[k + d.lda * j2], d.xi[k + d.nmd * j1],
-                                  op.xi2[k + d.nmd * j2], op.ops[k]);
-    const cplx ha0 = cmul(cmul(s12, cmul(pre[k], right)), g10);
-    const int r = j1 * nmd + k;
-    cplx sh = mkc(0.0, 0.0);
-    for (int j = 0; j < d.n; ++j) cfma(sh, d.Sa0Sm1[r + d.nG * j], op.h[j + d.n * j2]);
-    out[r] = cmul(mf, csub(ha0, sh));
+  cplx q1[GWP_MAXDOF], acc[GWP_MAXDOF];
+  const cplx* xi2 = nullptr;   // q1 is of this right state
+#pragma unroll
+  for (int k = 0; k < GWP_MAXDOF; ++k) acc[k] = mkc(0.0, 0.0);
+  for (int o = ch * YOP_CHUNK; o < min(d.op_count, (ch + 1) * YOP_CHUNK); ++o) {
+    const GwpYOp& op = ops[d.op_first + o];
+    if (j2 >= op.n2) continue;
+    if (op.xi2 != xi2) {
+      xi2 = op.xi2;
+#pragma unroll
+      for (int k = 0; k < GWP_MAXDOF; ++k)
+        if (k < nmd)
+          q1[k] = gau_int_1d(a[k + d.lda * j1], a[k + d.lda * j2], d.xi[k + d.nmd * j1], xi2[k + d.nmd * j2], 1);
+    }
+    const cplx w0 = cmul(op.mf[j1 + d.n * j2], op.S12[j1 + d.n * j2]);
+    // DOFs without an operator: the product of all acting integrals times <q_k>
+    cplx w = w0;
+    for (int k = 0; k < nmd; ++k)
+      if (op.ops[k] != 0)
+        w = cmul(w, gau_int_1d(a[k + d.lda * j1], a[k + d.lda * j2], d.xi[k + d.nmd * j1], xi2[k + d.nmd * j2], op.ops[k]));
+#pragma unroll
+    for (int k = 0; k < GWP_MAXDOF; ++k) {
+      if (k >= nmd) break;
+      if (op.ops[k] == 0) {
+        cfma(acc[k], w, q1[k]);
+      } else {
+        cplx v = cmul(w0, gau10_int_1d(a[k + d.lda * j1], a[k + d.lda * j2], d.xi[k + d.nmd * j1], xi2[k + d.nmd * j2],
+                                       op.ops[k]));
+        for (int q = 0; q < nmd; ++q)
+          if (q != k && op.ops[q] != 0)
+            v = cmul(v, gau_int_1d(a[q + d.lda * j1], a[q + d.lda * j2], d.xi[q + d.nmd * j1], xi2[q + d.nmd * j2],
+                                   op.ops[q]));
+        acc[k] = cadd(acc[k], v);
+      }
+    }
   }
+  cplx* out = part + (long long)blockIdx.y * part_ld + ((long long)ch * maxn2 + j2) * d.nG + (long long)j1 * nmd;
+#pragma unroll
+  for (int k = 0; k < GWP_MAXDOF; ++k)
+    if (k < nmd) out[k] = acc[k];
 }
 
-__global__ void gwp_y_sum_kernel(const GwpCYDesc* __restrict__ descs, const GwpYOp* __restrict__ ops,
-                                 const cplx* __restrict__ part, long long part_ld, int maxn2) {
+// part of G behind the terms of stage 1a: [operator][j1][j]
+__global__ void __launch_bounds__(32) gwp_y_mf_kernel(const GwpCYDesc* __restrict__ descs,
+                                                      const GwpYOp* __restrict__ ops, cplx* __restrict__ part,
+                                                      long long part_ld, long long g_off) {
+  const GwpCYDesc& d = descs[blockIdx.z];
+  const int o = blockIdx.y;
+  if (o >= d.op_count) return;
+  const int e = blockIdx.x * 32 + threadIdx.x, j = e % d.n, j1 = e / d.n;
+  if (j1 >= d.n) return;
+  const GwpYOp& op = ops[d.op_first + o];
+  cplx v = mkc(0.0, 0.0);
+  for (int j2 = 0; j2 < op.n2; ++j2) cfma(v, op.mf[j1 + d.n * j2], op.h[j + d.n * j2]);
+  part[(long long)blockIdx.z * part_ld + g_off + ((long long)o * d.n + j1) * d.n + j] = v;
+}
+
+__device__ cplx warp_sum(cplx v);
+
+__global__ void __launch_bounds__(32) gwp_y_sum_kernel(const GwpCYDesc* __restrict__ descs,
+                                                       const cplx* __restrict__ part, long long part_ld,
+                                                       long long g_off, int maxn2) {
   const GwpCYDesc& d = descs[blockIdx.y];
-  const int r = blockIdx.x * blockDim.x + threadIdx.x;
+  const int r = blockIdx.x, lane = threadIdx.x;
   if (r >= d.nG) return;
   const cplx* base = part + (long long)blockIdx.y * part_ld;
+  const int j1 = r / d.nmd, nterm = (d.op_count + YOP_CHUNK - 1) / YOP_CHUNK * maxn2;
   cplx acc = mkc(0.0, 0.0);
-  for (int o = 0; o < d.op_count; ++o) {
-    const int n2 = ops[d.op_first + o].n2;
-    for (int j2 = 0; j2 < n2; ++j2) acc = cadd(acc, base[((long long)o * maxn2 + j2) * d.nG + r]);
+#pragma unroll 4
+  for (int t = lane; t < nterm; t += 32) acc = cadd(acc, base[(long long)t * d.nG + r]);
+  if (lane < d.n) {   // n <= 32
+    const cplx* g = base + g_off + (long long)j1 * d.n + lane;
+    cplx s = mkc(0.0, 0.0);
+#pragma unroll 4
+    for (int o = 0; o < d.op_count; ++o) s = cadd(s, g[(long long)o * d.n * d.n]);
+    acc = csub(acc, cmul(d.Sa0Sm1[r + d.nG * lane], s));
   }
-  const long long ld = 2LL * d.nG;
+  acc = warp_sum(acc);
+  if (lane) return;
+  const long long ld = d.nG + 1LL;
   d.M[r + ld * d.nG] = acc;
-  d.M[d.nG + r + ld * d.nG] = mkc(0.0, 0.0);
+  d.M[d.nG + ld * r] = cconj(acc);
+  if (r == 0) d.M[d.nG + ld * d.nG] = mkc(0.0, 0.0);
 }
 
-// Fixed-order block reduction of a double over 256 threads.
-__device__ double block_sum(double v, double* red) {
-  for (int o = 16; o > 0; o >>= 1) v += __shfl_down_sync(0xffffffffu, v, o);
-  const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
-  __syncthreads();
-  if (lane == 0) red[warp] = v;
-  __syncthreads();
-  double t = 0.0;
-  if (threadIdx.x == 0) {
-    for (int w = 0; w < (int)(blockDim.x >> 5); ++w) t += red[w];
-    red[32] = t;
-  }
-  __syncthreads();
-  return red[32];
-}
 __device__ cplx warp_sum(cplx v) {
   for (int o = 16; o > 0; o >>= 1) {
     v.x += __shfl_down_sync(0xffffffffu, v.x, o);
@@ -359,240 +403,351 @@ __device__ cplx warp_sum(cplx v) {
   return v;
 }
 
-// One panel of the Householder QR of M (2nG x (nG+1), the last column the
-// right-hand side).  Shared: the panel rows j0.. of columns j0..j0+pw-1.
-// cpb: trailing columns per block (one warp each, cpb <= 8)
-__global__ void __launch_bounds__(256) gwp_qr_panel_kernel(const GwpCYDesc* __restrict__ descs, int j0, int cpb) {
-  extern __shared__ cplx P[];
-  __shared__ double red[33];
-  __shared__ cplx s_alpha[GWP_QR_PW];
-  __shared__ double s_tau[GWP_QR_PW];
-  const GwpCYDesc& d = descs[blockIdx.y];
+// LU factorisation of the bordered system in panels of LU_PW columns, two launches per
+// panel (384 unknowns, two systems: 48 panels of LU_FIG).
+//
+// Panel: one block per system, a row of the panel per thread in registers.  Rows stay
+// where they are; perm lists them in pivot order, act the rows not yet taken (the last
+// is the border row, never a pivot).  M keeps the multipliers, R receives U in pivot
+// order.  Bound by the serial pivots and one SM's FP64 pipe (4 + 4 (PW - k) FMAs per row).
+__global__ void __launch_bounds__(LU_MAXROWS) lu_panel_kernel(const GwpCYDesc* __restrict__ descs, int j0) {
+  const GwpCYDesc& d = descs[blockIdx.x];
   const int nG = d.nG;
   if (j0 >= nG) return;
-  const int pw = min(GWP_QR_PW, nG - j0);
-  const int ncol = nG + 1;
-  const int trailing = ncol - (j0 + pw);
-  const int nblk = (trailing + cpb - 1) / cpb;
-  if ((int)blockIdx.x > 0 && (int)blockIdx.x >= nblk) return;
-  const long long ld = 2LL * nG;
-  const int rows = 2 * nG - j0;
-  for (int e = threadIdx.x; e < rows * pw; e += blockDim.x) {
-    const int rr = e % rows, jj = e / rows;
-    P[e] = d.M[(j0 + rr) + ld * (j0 + jj)];
-  }
-  __syncthreads();
-  const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
-  for (int jj = 0; jj < pw; ++jj) {
-    cplx* col = P + (long long)rows * jj;
-    // reflector j0+jj has no support below row nG + j0 + jj: the eps I block below C
-    // only fills in down to that row (panel-relative: nG + jj)
-    const int rend = min(rows, nG + jj + 1);
-    double part = 0.0;
-    for (int rr = jj + threadIdx.x; rr < rend; rr += blockDim.x) part += cabs2(col[rr]);
-    const double nrm2 = block_sum(part, red);
-    if (threadIdx.x == 0) {
-      const double nrm = sqrt(nrm2);
-      const cplx x0 = col[jj];
-      const double ax0 = sqrt(cabs2(x0));
-      if (nrm == 0.0) {
-        s_alpha[jj] = mkc(0.0, 0.0);
-        s_tau[jj] = 0.0;
-      } else {
-        const cplx ph = (ax0 > 0.0) ? cdivr(x0, ax0) : mkc(1.0, 0.0);
-        const cplx alpha = cscale(ph, -nrm);
-        col[jj] = csub(x0, alpha);
-        s_alpha[jj] = alpha;
-        s_tau[jj] = 2.0 / (2.0 * nrm2 + 2.0 * nrm * ax0);
+  const int pw = min(LU_PW, nG - j0);
+  const long long ld = nG + 1;
+  const int r = threadIdx.x, lane = r & 31, warp = r >> 5, nw = blockDim.x >> 5;
+  __shared__ cplx prow[LU_PW + 1];       // the pivot row and the pivot's reciprocal
+  __shared__ unsigned wmax[32];
+  __shared__ int wrow[32];
+  bool act = r <= nG && (j0 == 0 || d.step[r] < 0);
+  const bool start = act;
+  int step = -1;
+  cplx a[LU_PW];
+#pragma unroll
+  for (int j = 0; j < LU_PW; ++j) a[j] = act && j < pw ? d.M[r + ld * (j0 + j)] : mkc(0.0, 0.0);
+#pragma unroll
+  for (int k = 0; k < LU_PW; ++k) {
+    if (k >= pw) break;
+    // the largest remaining element of the column (by its larger component's leading word)
+    const unsigned mag = act && r < nG ? fx_mag(a[k]) + 1u : 0u;
+    const unsigned m = __reduce_max_sync(0xffffffffu, mag);
+    const unsigned who = __ballot_sync(0xffffffffu, mag == m);
+    if (lane == 0) {
+      wmax[warp] = m;
+      wrow[warp] = 32 * warp + __ffs(who) - 1;
+    }
+    __syncthreads();
+    const unsigned v = lane < nw ? wmax[lane] : 0u;
+    const int win = wrow[__ffs(__ballot_sync(0xffffffffu, v == __reduce_max_sync(0xffffffffu, v))) - 1];
+    if (r == win) {
+      act = false;
+      step = j0 + k;
+      const double q = 1.0 / (a[k].x * a[k].x + a[k].y * a[k].y);
+      prow[LU_PW] = mkc(a[k].x * q, -a[k].y * q);
+#pragma unroll
+      for (int j = k + 1; j < LU_PW; ++j) prow[j] = a[j];
+    }
+    __syncthreads();
+    if (act) {
+      const cplx w = cmul(a[k], prow[LU_PW]);
+      a[k] = w;
+#pragma unroll
+      for (int j = k + 1; j < LU_PW; ++j) {
+        const cplx u = prow[j];
+        a[j].x = fma(-w.x, u.x, fma(w.y, u.y, a[j].x));
+        a[j].y = fma(-w.x, u.y, fma(-w.y, u.x, a[j].y));
       }
     }
-    __syncthreads();
-    // apply the reflector to the later panel columns, one warp per column
-    const int c = jj + 1 + warp;
-    if (c < pw && s_tau[jj] != 0.0) {
-      cplx* y = P + (long long)rows * c;
-      cplx w = mkc(0.0, 0.0);
-      for (int rr = jj + lane; rr < rend; rr += 32) cfma_conj(w, col[rr], y[rr]);
-      w = warp_sum(w);
-      const cplx f = cscale(w, s_tau[jj]);
-      for (int rr = jj + lane; rr < rend; rr += 32) y[rr] = csub(y[rr], cmul(col[rr], f));
-    }
-    __syncthreads();
+    if (r == win) d.rdiag[j0 + k] = prow[LU_PW];
   }
-  // trailing columns of this block (the right-hand side is column nG)
-  const int c = j0 + pw + blockIdx.x * cpb + warp;
-  if (warp < cpb && c < ncol) {
-    cplx* y = d.M + ld * c;
-    for (int jj = 0; jj < pw; ++jj) {
-      if (s_tau[jj] == 0.0) continue;
-      const cplx* v = P + (long long)rows * jj;
-      cplx w = mkc(0.0, 0.0);
-      const int rend = min(rows, nG + jj + 1);
-      for (int rr = jj + lane; rr < rend; rr += 32) cfma_conj(w, v[rr], y[j0 + rr]);
-      w = warp_sum(w);
-      const cplx f = cscale(w, s_tau[jj]);
-      for (int rr = jj + lane; rr < rend; rr += 32) y[j0 + rr] = csub(y[j0 + rr], cmul(v[rr], f));
-      __syncwarp();
+  if (start) {
+    d.step[r] = step;
+    if (step >= 0) d.perm[step] = r;
+#pragma unroll
+    for (int j = 0; j < LU_PW; ++j) {
+      if (j >= pw) break;
+      d.M[r + ld * (j0 + j)] = a[j];
+      if (step >= 0 && j0 + j >= step) d.R[step + (long long)nG * (j0 + j)] = a[j];
     }
   }
-  // the R entries of the panel columns (rows j0.., above and on the diagonal)
-  if (blockIdx.x == 0) {
-    for (int e = threadIdx.x; e < pw * pw; e += blockDim.x) {
-      const int rr = e % pw, jj = e / pw;
-      if (rr > jj) continue;
-      d.R[(j0 + rr) + (long long)nG * (j0 + jj)] = (rr == jj) ? s_alpha[jj] : P[rr + (long long)rows * jj];
+  const unsigned bal = __ballot_sync(0xffffffffu, act);
+  __syncthreads();
+  if (lane == 0) wrow[warp] = __popc(bal);
+  __syncthreads();
+  if (act) {
+    int pos = __popc(bal & ((1u << lane) - 1u));
+    for (int w = 0; w < warp; ++w) pos += wrow[w];
+    d.act[pos] = r;
+  }
+}
+
+// Trailing update: a block takes 32 of the remaining rows and 32 of the remaining
+// columns (the right-hand side is the last).  It solves the panel's unit lower triangle
+// for its columns (the blocks of the first row of blocks store the result as U), then
+// subtracts the rank-8 product as exact digit products (fixed.cuh; a warp's 16 rows are
+// the MMA's rows, the (re, im) of four columns its columns, as in the mode products),
+// where FP64 would take 18 us of an SM's FP64 pipe per block.
+__global__ void __launch_bounds__(256) lu_update_kernel(const GwpCYDesc* __restrict__ descs, int j0) {
+  constexpr int NS = 8;
+  const GwpCYDesc& d = descs[blockIdx.z];
+  const int nG = d.nG;
+  if (j0 >= nG) return;
+  const int pw = min(LU_PW, nG - j0);
+  const long long ld = nG + 1;
+  const int mrows = nG - j0 - pw + 1, c0 = j0 + pw;
+  const int i0 = 32 * blockIdx.y;
+  if (i0 >= mrows || c0 + 32 * (int)blockIdx.x > nG) return;
+  __shared__ cplx Ls[LU_PW][LU_PW];
+  __shared__ cplx T[32][LU_PW + 1];
+  const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5, g = lane >> 2, q = lane & 3;
+  {
+    const int i = tid & 7, cc = tid >> 3, col = c0 + 32 * blockIdx.x + cc;
+    const int row = i < pw ? d.perm[j0 + i] : 0;
+    cplx t = i < pw && col <= nG ? d.M[row + ld * col] : mkc(0.0, 0.0);
+    if (cc < LU_PW) Ls[i][cc] = cc < i && i < pw ? d.M[row + ld * (j0 + cc)] : mkc(0.0, 0.0);
+    __syncthreads();
+#pragma unroll
+    for (int k = 0; k < LU_PW - 1; ++k) {
+      const cplx u = mkc(__shfl_sync(0xffffffffu, t.x, (lane & 24) + k), __shfl_sync(0xffffffffu, t.y, (lane & 24) + k));
+      const cplx w = Ls[i][k];
+      if (i > k) {
+        t.x = fma(-w.x, u.x, fma(w.y, u.y, t.x));
+        t.y = fma(-w.x, u.y, fma(-w.y, u.x, t.y));
+      }
+    }
+    T[cc][i] = t;
+    if (i0 == 0 && i < pw && col <= nG) d.R[j0 + i + (long long)nG * col] = t;
+  }
+  __syncthreads();
+  int row[2];
+  cplx x[2][2];
+  unsigned er[2];
+  bool bad = false;
+#pragma unroll
+  for (int f = 0; f < 2; ++f) {
+    const int i = i0 + 16 * (warp & 1) + g + 8 * f;
+    row[f] = i < mrows ? d.act[i] : -1;
+#pragma unroll
+    for (int k = 0; k < 2; ++k)
+      x[f][k] = row[f] >= 0 && 4 * k + q < pw ? d.M[row[f] + ld * (j0 + 4 * k + q)] : mkc(0.0, 0.0);
+    unsigned mag = max(fx_mag(x[f][0]), fx_mag(x[f][1]));
+    mag = max(mag, __shfl_xor_sync(0xffffffffu, mag, 1));
+    mag = max(mag, __shfl_xor_sync(0xffffffffu, mag, 2));
+    bad = bad || !fx_ok(mag);
+    er[f] = fx_ebits(mag);
+  }
+  unsigned A[NS][4];
+#pragma unroll
+  for (int f = 0; f < 2; ++f)
+#pragma unroll
+    for (int k = 0; k < 2; ++k) {
+      unsigned s[NS];
+      fx_digits<NS>(x[f][k].x, x[f][k].y, er[f], er[f], s);
+#pragma unroll
+      for (int i = 0; i < NS; ++i) A[i][2 * k + f] = s[i];
+    }
+#pragma unroll
+  for (int tt = 0; tt < 2; ++tt) {
+    const int t = 2 * (warp >> 1) + tt, jo = 4 * t + (g >> 1);
+    const cplx m0 = T[jo][q], m1 = T[jo][4 + q];
+    unsigned mag = max(fx_mag(m0), fx_mag(m1));
+    mag = max(mag, __shfl_xor_sync(0xffffffffu, mag, 1));
+    mag = max(mag, __shfl_xor_sync(0xffffffffu, mag, 2));
+    const bool slow = __any_sync(0xffffffffu, bad || !fx_ok(mag));
+    const unsigned ec = fx_ebits(mag);
+    const int es = (int)__shfl_sync(0xffffffffu, ec, 8 * q) - ((2044 + 12 + 44) << 20);
+    const int col = c0 + 32 * blockIdx.x + 4 * t + q;
+    float c[NS][4];
+    if (!slow) {
+      unsigned s0[NS], s1[NS];
+      fx_digits<NS>(m0.x, m0.y, ec, ec, s0);
+      fx_digits<NS>(m1.x, m1.y, ec, ec, s1);
+#pragma unroll
+      for (int i = 0; i < NS; ++i) {   // column re: (Mr, -Mi); column im: (Mi, Mr)
+        const unsigned w0 = (g & 1) ? __byte_perm(s0[i], s0[i], 0x1032) : s0[i] ^ 0x80000000u;
+        const unsigned w1 = (g & 1) ? __byte_perm(s1[i], s1[i], 0x1032) : s1[i] ^ 0x80000000u;
+#pragma unroll
+        for (int j = 0; j + i < NS; ++j) fx_mma16(c[i + j], A[j], w0, w1, i == 0);
+      }
+    }
+#pragma unroll
+    for (int f = 0; f < 2; ++f) {
+      if (row[f] < 0 || col > nG) continue;
+      cplx* y = d.M + row[f] + ld * col;
+      cplx v;
+      if (!slow) {
+        v = mkc(fx_double(fx_join<NS>(c, 2 * f), es + (int)er[f]), fx_double(fx_join<NS>(c, 2 * f + 1), es + (int)er[f]));
+      } else {
+        v = mkc(0.0, 0.0);
+        for (int k = 0; k < pw; ++k) cfma(v, d.M[row[f] + ld * (j0 + k)], T[4 * t + q][k]);
+      }
+      *y = csub(*y, v);
     }
   }
 }
 
-// Back substitution R x = (Q^H b)[0:nG], then dxi = der * x and tau.
-__global__ void __launch_bounds__(256) gwp_backsub_kernel(const GwpCYDesc* __restrict__ descs, cplx der,
-                                                          cplx* __restrict__ out, int* status) {
-  extern __shared__ cplx sh[];
-  const GwpCYDesc& d = descs[blockIdx.x];
-  const int nG = d.nG;
-  const long long ld = 2LL * nG;
-  cplx* b = sh;
-  cplx* xs = sh + nG;
-  for (int r = threadIdx.x; r < nG; r += blockDim.x) b[r] = d.M[r + ld * nG];
+// Back-substitutions U x = L^-1 P Y (system 0) and L^H P x = U^-H Y (system 1), a block
+// each: blocks of eight unknowns from the last, warp 0 solving the next block while the
+// other warps update the rest (one barrier per eight unknowns; the former column-wise
+// form, with a division and two barriers per unknown, took 878 us at 384 unknowns).
+__global__ void __launch_bounds__(256) lu_back_kernel(const GwpCYDesc* __restrict__ descs) {
+  extern __shared__ cplx z[];
+  const GwpCYDesc& d = descs[blockIdx.y];
+  const int nG = d.nG, sys = blockIdx.x;
+  const long long ld = nG + 1;
+  int* prm = reinterpret_cast<int*>(z + nG);
+  const int tid = threadIdx.x, lane = tid & 31;
+  for (int k = tid; k < nG; k += blockDim.x) {
+    prm[k] = d.perm[k];
+    z[k] = sys == 0 ? d.R[k + (long long)nG * nG] : cconj(d.M[nG + ld * k]);
+  }
   __syncthreads();
-  for (int c = nG - 1; c >= 0; --c) {
-    if (threadIdx.x == 0) {
-      const cplx rc = d.R[c + (long long)nG * c];
-      cplx xv = cdiv(b[c], rc);
-      if (!isfinite(xv.x) || !isfinite(xv.y)) {
-        atomicOr(status, DEVST_NONFINITE);
-        xv = mkc(0.0, 0.0);
+  // coefficient of unknown k in the equation of unknown i < k
+  auto coef = [&](int i, int k) {
+    return sys == 0 ? d.R[i + (long long)nG * k] : cconj(d.M[prm[k] + ld * i]);
+  };
+  auto less = [&](cplx& v, cplx c, cplx x) {
+    v.x = fma(-c.x, x.x, fma(c.y, x.y, v.x));
+    v.y = fma(-c.x, x.y, fma(-c.y, x.x, v.y));
+  };
+  const int nb = (nG + 7) >> 3;
+  for (int b = nb; b >= 1; --b) {
+    // unknowns 8 b .. are known; warp 0: the block's share of them, then the block before
+    const int k0 = 8 * b, kn = min(8, nG - k0);
+    if (tid < 32) {
+      const int i0 = k0 - 8, i = i0 + (lane & 7), kq = lane >> 3;
+      const bool on = i < nG;
+      cplx cd[8], cu[2], rd = mkc(1.0, 0.0);
+#pragma unroll
+      for (int k = 0; k < 8; ++k)
+        cd[k] = on && i0 + k < nG && i0 + k > i ? coef(i, i0 + k) : mkc(0.0, 0.0);
+#pragma unroll
+      for (int h = 0; h < 2; ++h) cu[h] = on && kq + 4 * h < kn ? coef(i, k0 + kq + 4 * h) : mkc(0.0, 0.0);
+      if (sys == 0 && on) rd = d.rdiag[i];
+      cplx v = kq == 0 && on ? z[i] : mkc(0.0, 0.0);
+#pragma unroll
+      for (int h = 0; h < 2; ++h)
+        if (kq + 4 * h < kn) less(v, cu[h], z[k0 + kq + 4 * h]);
+#pragma unroll
+      for (int o = 8; o < 32; o <<= 1)
+        v = cadd(v, mkc(__shfl_xor_sync(0xffffffffu, v.x, o), __shfl_xor_sync(0xffffffffu, v.y, o)));
+#pragma unroll
+      for (int k = 7; k >= 0; --k) {
+        if ((lane & 7) == k) v = cmul(v, rd);
+        const cplx x = mkc(__shfl_sync(0xffffffffu, v.x, k), __shfl_sync(0xffffffffu, v.y, k));
+        if ((lane & 7) < k) less(v, cd[k], x);
       }
-      xs[c] = xv;
-    }
-    __syncthreads();
-    const int pstart = (c / GWP_QR_PW) * GWP_QR_PW;
-    const cplx xc = xs[c];
-    for (int r = threadIdx.x; r < c; r += blockDim.x) {
-      const cplx rv = (r >= pstart) ? d.R[r + (long long)nG * c] : d.M[r + ld * c];
-      b[r] = csub(b[r], cmul(rv, xc));
+      if (kq == 0 && on) z[i] = v;
+    } else {
+      for (int r = tid - 32; r < k0 - 8; r += blockDim.x - 32) {
+        cplx v = z[r];
+        for (int k = 0; k < kn; ++k) less(v, coef(r, k0 + k), z[k0 + k]);
+        z[r] = v;
+      }
     }
     __syncthreads();
   }
+  for (int k = tid; k < nG; k += blockDim.x) d.x[sys == 0 ? k : nG + prm[k]] = z[k];
+}
+
+// x = the mean of the two solutions, dxi = der * x, and tau
+// tau(j1, j2) = sum_k conj(Sa0Sm1(j2*nmd+k, j1)) dxi(k, j2) + diagonal phase term
+__global__ void __launch_bounds__(256) gwp_tau_kernel(const GwpCYDesc* __restrict__ descs, cplx der,
+                                                      cplx* __restrict__ out, int* status) {
+  extern __shared__ cplx dx[];
+  const GwpCYDesc& d = descs[blockIdx.y];
+  const int nG = d.nG;
   for (int r = threadIdx.x; r < nG; r += blockDim.x) {
-    d.x[r] = xs[r];
-    out[d.dxi_offset + r] = cmul(der, xs[r]);
+    cplx x = cscale(cadd(d.x[r], d.x[nG + r]), 0.5);
+    if (!isfinite(x.x) || !isfinite(x.y)) {
+      if (blockIdx.x == 0) atomicOr(status, DEVST_NONFINITE);
+      x = mkc(0.0, 0.0);
+    }
+    dx[r] = cmul(der, x);
+    if (blockIdx.x == 0) out[d.dxi_offset + r] = dx[r];
   }
   __syncthreads();
-  // tau(j1, j2) = sum_k conj(Sa0Sm1(j2*nmd+k, j1)) dxi(k, j2) + diagonal phase term
   const int n = d.n, nmd = d.nmd;
-  for (int e = threadIdx.x; e < n * n; e += blockDim.x) {
+  for (int e = blockIdx.x * blockDim.x + threadIdx.x; e < n * n; e += gridDim.x * blockDim.x) {
     const int j1 = e % n, j2 = e / n;
     cplx t = mkc(0.0, 0.0);
-    for (int k = 0; k < nmd; ++k) cfma_conj(t, d.Sa0Sm1[(j2 * nmd + k) + (long long)nG * j1], cmul(der, xs[k + nmd * j2]));
+    for (int k = 0; k < nmd; ++k) cfma_conj(t, d.Sa0Sm1[(j2 * nmd + k) + (long long)nG * j1], dx[k + nmd * j2]);
     if (j1 == j2) {
       double dd = 0.0;
-      for (int k = 0; k < nmd; ++k) {
-        const cplx dx = cmul(der, xs[k + nmd * j2]);
-        dd += d.xi[k + nmd * j2].x * dx.x / d.a[k + d.lda * j2];
-      }
+      for (int k = 0; k < nmd; ++k) dd += d.xi[k + nmd * j2].x * dx[k + nmd * j2].x / d.a[k + d.lda * j2];
       t.x += dd * 0.5;
     }
     d.tau[e] = t;
   }
 }
 
-// Tikhonov-regularised inverse of a Hermitian n x n matrix (n <= 32) as the
-// least-squares solution of [A; eps I] X = [I; 0]: X = (A^2 + eps^2)^-1 A, the
-// matrix StdRegInv 'tikh' (maths.f90:8-83) builds from the eigen-decomposition
-// U w/(w^2 + eps^2) U^H.  Householder QR of the 2n x n stack in shared memory
-// with the 2n x n right-hand side carried along, one warp per column.
-__global__ void __launch_bounds__(256) tikh_inv_kernel(const RegInvDesc* __restrict__ descs) {
-  extern __shared__ cplx smq[];
+// Tikhonov-regularised inverse of a Hermitian n x n matrix (n <= 32), X = (A^2 + eps^2)^-1 A,
+// the matrix StdRegInv 'tikh' (maths.f90:8-83) builds from the eigen-decomposition
+// U w/(w^2 + eps^2) U^H: the Hermitian part of (A + i eps)^-1.  Gauss-Jordan exchanges
+// with partial pivoting, an element per thread (a warp holds a column, a lane a row),
+// one barrier per pivot: the warp of the next column updates it, finds the pivot and
+// publishes the multipliers while the others still update.  Bound by the FP64 pipe (four
+// instructions per element and pivot) and the serial pivots; two 32 x 32 inverses took
+// 710 us as a Householder QR of [A; eps I], TIKH_FIG.
+__global__ void __launch_bounds__(1024) tikh_inv_kernel(const RegInvDesc* __restrict__ descs) {
+  __shared__ cplx mult[2][MAXN_SPF];      // multipliers; the pivot row's is minus the reciprocal
+  __shared__ int s_row[MAXN_SPF];         // pivot row of each step
+  __shared__ cplx X[MAXN_SPF][MAXN_SPF + 1];
   const RegInvDesc& d = descs[blockIdx.x];
-  const int n = d.n, m = 2 * n, ld = 2 * MAXN_SPF;
-  cplx* A = smq;                       // m x n (ld)
-  cplx* B = smq + (size_t)ld * MAXN_SPF;  // m x n (ld)
-  __shared__ cplx s_alpha[MAXN_SPF];
-  __shared__ double s_tau[MAXN_SPF];
-  for (int e = threadIdx.x; e < m * n; e += blockDim.x) {
-    const int i = e % m, j = e / m;
-    cplx a, b;
-    if (i < n) {
-      // the upper triangle is authoritative (zheev 'U'): mirror it, real diagonal
-      a = (i <= j) ? d.A[i + n * j] : cconj(d.A[j + n * i]);
-      if (i == j) a.y = 0.0;
-      b = mkc(i == j ? 1.0 : 0.0, 0.0);
-    } else {
-      a = mkc((i - n) == j ? d.eps : 0.0, 0.0);
-      b = mkc(0.0, 0.0);
-    }
-    A[i + ld * j] = a;
-    B[i + ld * j] = b;
+  const int n = d.n, i = threadIdx.x & 31, j = threadIdx.x >> 5;   // a column per warp; blockDim.x = 32 max n
+  cplx a = mkc(0.0, 0.0);
+  if (i < n && j < n) {
+    // the upper triangle is authoritative (zheev 'U'): mirror it, real diagonal
+    a = (i <= j) ? d.A[i + n * j] : cconj(d.A[j + n * i]);
+    if (i == j) a.y = d.eps;
   }
+  bool taken = i >= n;                    // the lane's row has been a pivot row
+  auto pivot = [&](int k) {               // column k, by its warp
+    const unsigned mag = taken ? 0u : fx_mag(a) + 1u;
+    const int p = __ffs(__ballot_sync(0xffffffffu, mag == __reduce_max_sync(0xffffffffu, mag))) - 1;
+    const cplx v = mkc(__shfl_sync(0xffffffffu, a.x, p), __shfl_sync(0xffffffffu, a.y, p));
+    const double q = 1.0 / (v.x * v.x + v.y * v.y);
+    const cplx rc = mkc(v.x * q, -v.y * q);
+    const cplx m = i == p ? mkc(-rc.x, -rc.y) : cmul(a, rc);
+    mult[k & 1][i] = m;
+    if (i == 0) s_row[k] = p;
+    a = mkc(-m.x, -m.y);                  // the exchanged column
+  };
+  if (j == 0) pivot(0);
   __syncthreads();
-  const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
-  const int nw = blockDim.x >> 5;
-  for (int j = 0; j < n; ++j) {
-    cplx* col = A + ld * j;
-    if (warp == 0) {
-      double part = 0.0;
-      for (int r = j + lane; r < m; r += 32) part += cabs2(col[r]);
-      for (int o = 16; o > 0; o >>= 1) part += __shfl_down_sync(0xffffffffu, part, o);
-      if (lane == 0) {
-        const double nrm = sqrt(part);
-        const cplx x0 = col[j];
-        const double ax0 = sqrt(cabs2(x0));
-        if (nrm == 0.0) {
-          s_alpha[j] = mkc(0.0, 0.0);
-          s_tau[j] = 0.0;
-        } else {
-          const cplx ph = (ax0 > 0.0) ? mkc(x0.x / ax0, x0.y / ax0) : mkc(1.0, 0.0);
-          const cplx alpha = cscale(ph, -nrm);
-          col[j] = csub(x0, alpha);
-          s_alpha[j] = alpha;
-          s_tau[j] = 2.0 / (2.0 * part + 2.0 * nrm * ax0);
-        }
-      }
+  for (int k = 0; k < n; ++k) {
+    const int p = s_row[k];
+    if (j != k) {
+      const cplx m = mult[k & 1][i];
+      const cplx u = mkc(__shfl_sync(0xffffffffu, a.x, p), __shfl_sync(0xffffffffu, a.y, p));
+      if (i == p) a = mkc(0.0, 0.0);
+      a.x = fma(-m.x, u.x, fma(m.y, u.y, a.x));
+      a.y = fma(-m.x, u.y, fma(-m.y, u.x, a.y));
     }
-    __syncthreads();
-    const double tau = s_tau[j];
-    if (tau != 0.0) {
-      // columns j+1..n-1 of A, then all n columns of B
-      for (int c = warp; c < (n - j - 1) + n; c += nw) {
-        cplx* y = (c < n - j - 1) ? A + ld * (j + 1 + c) : B + ld * (c - (n - j - 1));
-        cplx w = mkc(0.0, 0.0);
-        for (int r = j + lane; r < m; r += 32) cfma_conj(w, col[r], y[r]);
-        w = warp_sum(w);
-        const cplx f = cscale(w, tau);
-        for (int r = j + lane; r < m; r += 32) y[r] = csub(y[r], cmul(col[r], f));
-      }
-    }
+    taken = taken || i == p;
+    if (j == k + 1 && j < n) pivot(k + 1);
     __syncthreads();
   }
-  // back substitution R X = (Q^H [I; 0])[0:n], one thread per right-hand side
-  for (int c = threadIdx.x; c < n; c += blockDim.x) {
-    cplx* x = B + ld * c;
-    for (int i = n - 1; i >= 0; --i) {
-      cplx v = x[i];
-      for (int k = i + 1; k < n; ++k) v = csub(v, cmul(A[i + ld * k], x[k]));
-      x[i] = cdiv(v, s_alpha[i]);
-    }
+  // row p_k holds unknown k, column m the coefficient of equation p_m
+  if (i < n && j < n) {
+    int k = 0;
+    for (int q = 0; q < n; ++q)
+      if (s_row[q] == i) k = q;
+    X[k][s_row[j]] = a;
   }
   __syncthreads();
-  for (int e = threadIdx.x; e < n * n; e += blockDim.x) {
-    const int i = e % n, j = e / n;
-    d.inv_out[i + n * j] = B[i + ld * j];
+  if (i < n && j < n) {
+    const cplx u = X[i][j], v = X[j][i];
+    d.inv_out[i + n * j] = mkc(0.5 * (u.x + v.x), 0.5 * (u.y - v.y));
   }
 }
 
 }  // namespace
 
-void launch_tikh_inv(const RegInvDesc* d, int nd, cudaStream_t st) {
+void launch_tikh_inv(const RegInvDesc* d, int nd, int maxn, cudaStream_t st) {
   if (nd <= 0) return;
-  const size_t smem = sizeof(cplx) * 2 * (size_t)(2 * MAXN_SPF) * MAXN_SPF;
-  static bool configured = false;
-  if (!configured) {
-    cudaFuncSetAttribute(tikh_inv_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
-    configured = true;
-  }
-  tikh_inv_kernel<<<nd, 256, smem, st>>>(d);
+  tikh_inv_kernel<<<nd, 32 * maxn, 0, st>>>(d);
 }
 
 // ---------------------------------------------------------------------------
@@ -846,52 +1001,47 @@ void launch_density_gwp(const DensGwpArgs& a, cudaStream_t st) { density_gwp_ker
 
 void launch_gwp_ovl(const GwpOvlDesc* d, int nd, cudaStream_t st) {
   if (nd <= 0) return;
-  gwp_ovl_kernel<<<nd, 256, 0, st>>>(d);
+  gwp_ovl_kernel<<<dim3(nd, MAXN_SPF), 32, 0, st>>>(d);
 }
 
 void launch_gwp_h1(const GwpH1Desc* d, int nd, cudaStream_t st) {
   if (nd <= 0) return;
-  gwp_h1_kernel<<<nd, 256, 0, st>>>(d);
+  gwp_h1_kernel<<<dim3(nd, MAXN_SPF / 2), 64, 0, st>>>(d);
 }
 
-void launch_gwp_cy(const GwpCYDesc* d, int nd, int maxG, int maxn, int maxops, const GwpYOp* ops, cplx* part,
-                   cudaStream_t st) {
-  if (nd <= 0) return;
+long long gwp_y_scratch(int maxG, int maxn, int maxops) {
+  return (long long)maxG * maxn * ((maxops + YOP_CHUNK - 1) / YOP_CHUNK) + (long long)maxn * maxn * maxops;
+}
+int launch_gwp_cy(const GwpCYDesc* d, int nd, int maxG, int maxn, int maxops, const GwpYOp* ops, cplx* part,
+                  cudaStream_t st) {
+  if (nd <= 0) return 0;
   const unsigned ne = (unsigned)((maxG * maxn + 255) / 256);
   gwp_sa0_kernel<<<dim3(ne, nd), 256, 0, st>>>(d);
   gwp_sa0sm1_kernel<<<dim3(ne, nd), 256, 0, st>>>(d);
-  const unsigned nt = (unsigned)((maxG + 15) / 16);
-  gwp_c_kernel<<<dim3(nt, nt, nd), dim3(16, 16), 0, st>>>(d);
-  const long long part_ld = (long long)maxG * maxn * std::max(maxops, 1);
-  const long long nthr = (long long)maxn * maxn * std::max(maxops, 1);
-  gwp_y_part_kernel<<<dim3((unsigned)((nthr + 127) / 128), nd), 128, 0, st>>>(d, ops, part, part_ld, maxn);
-  gwp_y_sum_kernel<<<dim3((maxG + 127) / 128, nd), 128, 0, st>>>(d, ops, part, part_ld, maxn);
+  const unsigned nt = (unsigned)((maxG + 7) / 8);
+  gwp_c_kernel<<<dim3(nt, nt, nd), 64, 0, st>>>(d);
+  const int nch = (maxops + YOP_CHUNK - 1) / YOP_CHUNK;
+  const long long g_off = (long long)maxG * maxn * nch, part_ld = gwp_y_scratch(maxG, maxn, maxops);
+  const long long nthr = (long long)maxn * maxn * nch;
+  if (maxops > 0) {
+    gwp_y_part_kernel<<<dim3((unsigned)((nthr + 31) / 32), nd), 32, 0, st>>>(d, ops, part, part_ld, maxn);
+    gwp_y_mf_kernel<<<dim3((unsigned)((maxn * maxn + 31) / 32), maxops, nd), 32, 0, st>>>(d, ops, part, part_ld, g_off);
+  }
+  gwp_y_sum_kernel<<<dim3(maxG, nd), 32, 0, st>>>(d, part, part_ld, g_off, maxn);
+  return maxops > 0 ? 6 : 4;
 }
 
-void launch_gwp_solve(const GwpCYDesc* d, int nd, int maxG, cplx der, cplx* out, int* status, cudaStream_t st) {
-  if (nd <= 0) return;
-  const size_t smem = sizeof(cplx) * (size_t)(2 * maxG) * GWP_QR_PW;
-  static size_t configured = 0;
-  if (smem > 48 * 1024 && smem > configured) {
-    cudaFuncSetAttribute(gwp_qr_panel_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
-    configured = smem;
+int launch_gwp_solve(const GwpCYDesc* d, int nd, int maxG, cplx der, cplx* out, int* status, cudaStream_t st) {
+  if (nd <= 0) return 0;
+  const int threads = (maxG + 1 + 31) & ~31;
+  int launches = 0;
+  for (int j0 = 0; j0 < maxG; j0 += LU_PW) {
+    lu_panel_kernel<<<nd, threads, 0, st>>>(d, j0);
+    const unsigned nt = (unsigned)((maxG + 1 - j0 + 31) / 32);
+    lu_update_kernel<<<dim3(nt, nt, nd), 256, 0, st>>>(d, j0);
+    launches += 2;
   }
-  // the trailing columns spread over at most one block per SM (every block
-  // factors the panel itself, so more blocks than SMs would share an SM's FP64
-  // pipe), at most eight per block
-  static int nsm = 0;
-  if (!nsm) {
-    int dev = 0;
-    cudaGetDevice(&dev);
-    cudaDeviceGetAttribute(&nsm, cudaDevAttrMultiProcessorCount, dev);
-    if (nsm <= 0) nsm = 152;
-  }
-  for (int j0 = 0; j0 < maxG; j0 += GWP_QR_PW) {
-    const int trailing = maxG + 1 - j0 - GWP_QR_PW;
-    const int per_desc = std::max(1, nsm / nd);
-    const int cpb = std::min(8, std::max(1, (trailing + per_desc - 1) / per_desc));
-    const unsigned nblk = (unsigned)std::max(1, (trailing + cpb - 1) / cpb);
-    gwp_qr_panel_kernel<<<dim3(nblk, nd), 256, smem, st>>>(d, j0, cpb);
-  }
-  gwp_backsub_kernel<<<nd, 256, sizeof(cplx) * 2 * maxG, st>>>(d, der, out, status);
+  lu_back_kernel<<<dim3(2, nd), 256, (sizeof(cplx) + sizeof(int)) * maxG, st>>>(d);
+  gwp_tau_kernel<<<dim3(4, nd), 256, sizeof(cplx) * maxG, st>>>(d, der, out, status);
+  return launches + 2;
 }

@@ -376,7 +376,8 @@ double measure_fp64_tflops();
 // layout a[k + lda*j]) and complex parameters xi (the psi block, xi[k + d*j]).
 // ---------------------------------------------------------------------------
 #define GWP_MAXDOF 16    // DOFs of one Gaussian mode
-#define GWP_QR_PW 8      // panel width of the regularised least-squares QR
+#define LU_PW 8          // panel width of the parameter solve's LU factorisation
+#define LU_MAXROWS 544   // rows of its bordered system (512 unknowns at most), in warps
 
 struct GwpOvlDesc {      // S(j1, j2) = <g1_j1 | g2_j2> (normalised), n1 x n2 (ld n1)
   const cplx* xi1;
@@ -416,9 +417,13 @@ struct GwpCYDesc {       // one (Gaussian mode, state) block of Calc_CY and the 
   const cplx* rho;       // density matrix of the mode (n x n)
   cplx* Sa0;             // nG x n, nG = d * n
   cplx* Sa0Sm1;          // nG x n
-  cplx* M;               // (2 nG) x (nG + 1) least-squares system [C, Y; eps I, 0], column-major
-  cplx* R;               // nG x nG: R factor entries of the panels
-  cplx* x;               // nG solution (parameter derivative before der_factor)
+  cplx* M;               // (nG + 1) x (nG + 1): [C + i eps, Y; Y^H, 0], then the multipliers of its LU
+  cplx* R;               // nG x (nG + 1): U and L^-1 P Y, rows in pivot order
+  cplx* rdiag;           // nG: 1 / U(k, k)
+  cplx* x;               // 2 nG: solutions with C + i eps and with its adjoint
+  int* step;             // nG + 1: a row's place in the pivot order, -1 before
+  int* perm;             // nG: rows in pivot order
+  int* act;              // nG + 1: rows not yet taken
   long long dxi_offset;  // where der_factor * x goes in the derivative vector
   cplx* tau;             // n x n (derivatives.f90:201-234)
   int nmd, lda, n, nG;
@@ -426,15 +431,17 @@ struct GwpCYDesc {       // one (Gaussian mode, state) block of Calc_CY and the 
   double eps;            // eps_C
 };
 void launch_gwp_ovl(const GwpOvlDesc* d, int nd, cudaStream_t st);
-// Tikhonov inverses (regtype 'tikh') of n <= 32 Hermitian matrices into inv_out, by QR
-void launch_tikh_inv(const RegInvDesc* d, int nd, cudaStream_t st);
+// Tikhonov inverses (regtype 'tikh') of n <= maxn <= 32 Hermitian matrices into inv_out
+void launch_tikh_inv(const RegInvDesc* d, int nd, int maxn, cudaStream_t st);
 void launch_gwp_h1(const GwpH1Desc* d, int nd, cudaStream_t st);
 // Calc_CY and the Tikhonov parameter solve (StdRegSol 'tikh', maths.f90:87-162)
 // for nd (mode, state) blocks; maxG = max nG.  Then dxi = der * x and tau.
-// part: scratch of nd * maxG * maxn * maxops complex (the terms of Y)
-void launch_gwp_cy(const GwpCYDesc* d, int nd, int maxG, int maxn, int maxops, const GwpYOp* ops, cplx* part,
+// part: scratch of nd * gwp_y_scratch complex (the terms of Y); returns the number of launches
+long long gwp_y_scratch(int maxG, int maxn, int maxops);
+int launch_gwp_cy(const GwpCYDesc* d, int nd, int maxG, int maxn, int maxops, const GwpYOp* ops, cplx* part,
                    cudaStream_t st);
-void launch_gwp_solve(const GwpCYDesc* d, int nd, int maxG, cplx der, cplx* out, int* status, cudaStream_t st);
+// returns the number of launches
+int launch_gwp_solve(const GwpCYDesc* d, int nd, int maxG, cplx der, cplx* out, int* status, cudaStream_t st);
 
 // CMF2 with Gaussian modes (cmf2_base.f90, cmf2_derivatives.f90)
 struct GwpIsqrtDesc {    // D = U^-1 with S = U^H U (InverseSquareRootU, maths.f90:621-644), DhS = D^H S
