@@ -443,7 +443,7 @@ __global__ void __launch_bounds__(LU_MAXROWS) lu_panel_kernel(const GwpCYDesc* _
     if (r == win) {
       act = false;
       step = j0 + k;
-      const double q = 1.0 / (a[k].x * a[k].x + a[k].y * a[k].y);
+      const double q = 1.0 / fma(a[k].x, a[k].x, a[k].y * a[k].y);
       prow[LU_PW] = mkc(a[k].x * q, -a[k].y * q);
 #pragma unroll
       for (int j = k + 1; j < LU_PW; ++j) prow[j] = a[j];
@@ -501,6 +501,16 @@ __global__ void __launch_bounds__(256) lu_update_kernel(const GwpCYDesc* __restr
   __shared__ cplx Ls[LU_PW][LU_PW];
   __shared__ cplx T[32][LU_PW + 1];
   const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5, g = lane >> 2, q = lane & 3;
+  int row[2];
+  cplx x[2][2];
+#pragma unroll
+  for (int f = 0; f < 2; ++f) {
+    const int i = i0 + 16 * (warp & 1) + g + 8 * f;
+    row[f] = i < mrows ? d.act[i] : -1;
+#pragma unroll
+    for (int k = 0; k < 2; ++k)
+      x[f][k] = row[f] >= 0 && 4 * k + q < pw ? d.M[row[f] + ld * (j0 + 4 * k + q)] : mkc(0.0, 0.0);
+  }
   {
     const int i = tid & 7, cc = tid >> 3, col = c0 + 32 * blockIdx.x + cc;
     const int row = i < pw ? d.perm[j0 + i] : 0;
@@ -520,23 +530,24 @@ __global__ void __launch_bounds__(256) lu_update_kernel(const GwpCYDesc* __restr
     if (i0 == 0 && i < pw && col <= nG) d.R[j0 + i + (long long)nG * col] = t;
   }
   __syncthreads();
-  int row[2];
-  cplx x[2][2];
   unsigned er[2];
   bool bad = false;
 #pragma unroll
   for (int f = 0; f < 2; ++f) {
-    const int i = i0 + 16 * (warp & 1) + g + 8 * f;
-    row[f] = i < mrows ? d.act[i] : -1;
-#pragma unroll
-    for (int k = 0; k < 2; ++k)
-      x[f][k] = row[f] >= 0 && 4 * k + q < pw ? d.M[row[f] + ld * (j0 + 4 * k + q)] : mkc(0.0, 0.0);
     unsigned mag = max(fx_mag(x[f][0]), fx_mag(x[f][1]));
     mag = max(mag, __shfl_xor_sync(0xffffffffu, mag, 1));
     mag = max(mag, __shfl_xor_sync(0xffffffffu, mag, 2));
     bad = bad || !fx_ok(mag);
     er[f] = fx_ebits(mag);
   }
+  cplx y[2][2];   // in flight during the products
+#pragma unroll
+  for (int tt = 0; tt < 2; ++tt)
+#pragma unroll
+    for (int f = 0; f < 2; ++f) {
+      const int col = c0 + 32 * blockIdx.x + 4 * (2 * (warp >> 1) + tt) + q;
+      y[tt][f] = row[f] >= 0 && col <= nG ? d.M[row[f] + ld * col] : mkc(0.0, 0.0);
+    }
   unsigned A[NS][4];
 #pragma unroll
   for (int f = 0; f < 2; ++f)
@@ -574,7 +585,6 @@ __global__ void __launch_bounds__(256) lu_update_kernel(const GwpCYDesc* __restr
 #pragma unroll
     for (int f = 0; f < 2; ++f) {
       if (row[f] < 0 || col > nG) continue;
-      cplx* y = d.M + row[f] + ld * col;
       cplx v;
       if (!slow) {
         v = mkc(fx_double(fx_join<NS>(c, 2 * f), es + (int)er[f]), fx_double(fx_join<NS>(c, 2 * f + 1), es + (int)er[f]));
@@ -582,7 +592,7 @@ __global__ void __launch_bounds__(256) lu_update_kernel(const GwpCYDesc* __restr
         v = mkc(0.0, 0.0);
         for (int k = 0; k < pw; ++k) cfma(v, d.M[row[f] + ld * (j0 + k)], T[4 * t + q][k]);
       }
-      *y = csub(*y, v);
+      d.M[row[f] + ld * col] = csub(y[tt][f], v);
     }
   }
 }
@@ -591,7 +601,7 @@ __global__ void __launch_bounds__(256) lu_update_kernel(const GwpCYDesc* __restr
 // each: blocks of eight unknowns from the last, warp 0 solving the next block while the
 // other warps update the rest (one barrier per eight unknowns; the former column-wise
 // form, with a division and two barriers per unknown, took 878 us at 384 unknowns).
-__global__ void __launch_bounds__(256) lu_back_kernel(const GwpCYDesc* __restrict__ descs) {
+__global__ void __launch_bounds__(512) lu_back_kernel(const GwpCYDesc* __restrict__ descs) {
   extern __shared__ cplx z[];
   const GwpCYDesc& d = descs[blockIdx.y];
   const int nG = d.nG, sys = blockIdx.x;
@@ -618,13 +628,14 @@ __global__ void __launch_bounds__(256) lu_back_kernel(const GwpCYDesc* __restric
     if (tid < 32) {
       const int i0 = k0 - 8, i = i0 + (lane & 7), kq = lane >> 3;
       const bool on = i < nG;
-      cplx cd[8], cu[2], rd = mkc(1.0, 0.0);
+      // lane (i, kq): unknowns kq, kq + 4 of either block
+      cplx cd[2], cu[2];
 #pragma unroll
-      for (int k = 0; k < 8; ++k)
-        cd[k] = on && i0 + k < nG && i0 + k > i ? coef(i, i0 + k) : mkc(0.0, 0.0);
-#pragma unroll
-      for (int h = 0; h < 2; ++h) cu[h] = on && kq + 4 * h < kn ? coef(i, k0 + kq + 4 * h) : mkc(0.0, 0.0);
-      if (sys == 0 && on) rd = d.rdiag[i];
+      for (int h = 0; h < 2; ++h) {
+        const int k = kq + 4 * h;
+        cd[h] = on && i0 + k < nG && i0 + k > i ? coef(i, i0 + k) : mkc(0.0, 0.0);
+        cu[h] = on && k < kn ? coef(i, k0 + k) : mkc(0.0, 0.0);
+      }
       cplx v = kq == 0 && on ? z[i] : mkc(0.0, 0.0);
 #pragma unroll
       for (int h = 0; h < 2; ++h)
@@ -632,17 +643,28 @@ __global__ void __launch_bounds__(256) lu_back_kernel(const GwpCYDesc* __restric
 #pragma unroll
       for (int o = 8; o < 32; o <<= 1)
         v = cadd(v, mkc(__shfl_xor_sync(0xffffffffu, v.x, o), __shfl_xor_sync(0xffffffffu, v.y, o)));
+      if (sys == 0) {   // rows divided by the diagonal ahead of the chain
+        const cplx rd = on ? d.rdiag[i] : mkc(0.0, 0.0);
+        v = cmul(v, rd);
+        cd[0] = cmul(cd[0], rd);
+        cd[1] = cmul(cd[1], rd);
+      }
 #pragma unroll
-      for (int k = 7; k >= 0; --k) {
-        if ((lane & 7) == k) v = cmul(v, rd);
+      for (int k = 7; k > 0; --k) {
+        const int src = (lane & 7) + 8 * (k & 3);
+        const cplx c = mkc(__shfl_sync(0xffffffffu, cd[k >> 2].x, src), __shfl_sync(0xffffffffu, cd[k >> 2].y, src));
         const cplx x = mkc(__shfl_sync(0xffffffffu, v.x, k), __shfl_sync(0xffffffffu, v.y, k));
-        if ((lane & 7) < k) less(v, cd[k], x);
+        less(v, c, x);   // c = 0 for unknowns k ..
       }
       if (kq == 0 && on) z[i] = v;
-    } else {
-      for (int r = tid - 32; r < k0 - 8; r += blockDim.x - 32) {
-        cplx v = z[r];
-        for (int k = 0; k < kn; ++k) less(v, coef(r, k0 + k), z[k0 + k]);
+    } else if ((tid >> 5) & 3) {   // the sub-partition of warp 0 is left to it
+      for (int r = 96 * (tid >> 7) + ((tid >> 5 & 3) - 1) * 32 + lane; r < k0 - 8; r += 96 * (blockDim.x >> 7)) {
+        cplx v = z[r], cf[8];
+#pragma unroll
+        for (int k = 0; k < 8; ++k) cf[k] = k < kn ? coef(r, k0 + k) : mkc(0.0, 0.0);
+#pragma unroll
+        for (int k = 0; k < 8; ++k)
+          if (k < kn) less(v, cf[k], z[k0 + k]);
         z[r] = v;
       }
     }
@@ -1041,7 +1063,7 @@ int launch_gwp_solve(const GwpCYDesc* d, int nd, int maxG, cplx der, cplx* out, 
     lu_update_kernel<<<dim3(nt, nt, nd), 256, 0, st>>>(d, j0);
     launches += 2;
   }
-  lu_back_kernel<<<dim3(2, nd), 256, (sizeof(cplx) + sizeof(int)) * maxG, st>>>(d);
+  lu_back_kernel<<<dim3(2, nd), 512, (sizeof(cplx) + sizeof(int)) * maxG, st>>>(d);
   gwp_tau_kernel<<<dim3(4, nd), 256, sizeof(cplx) * maxG, st>>>(d, der, out, status);
   return launches + 2;
 }
