@@ -146,7 +146,9 @@ struct ProdBatch {
 #define HOLE_NBLK_MAX 128
 inline int hole_nblk(const HoleDesc& d, int tpb, int cap) {
   const long long ntiles = (d.L * d.R + HOLE_TILE - 1) / HOLE_TILE;
-  const long long work = ntiles * ((d.n1 + 7) / 8) * ((d.n2 + 7) / 8);
+  // the wide form's blocks (two per SM) cost more to start: 283 blocks took 20.5 us
+  // where 478 took 25.8 (mixed counts of 5 to 9, 56,007 coefficients)
+  const long long work = std::max(d.n1, d.n2) <= 8 ? ntiles : ntiles * ((d.n1 + 15) / 16) * ((d.n2 + 15) / 16);
   return (int)std::min({std::max(work / tpb, 1LL), ntiles, (long long)std::min(cap, HOLE_NBLK_MAX)});
 }
 
@@ -155,6 +157,8 @@ struct HoleBatch {
   HoleDesc* d = nullptr;
   long long nblocks = 0;
   int maxn = 0;                  // largest n1, n2
+  int nnarrow = 0;               // descriptors with n1, n2 <= 8, first on the device
+  long long narrow_blocks = 0;
   bool f32 = false;              // some operand is complex FP32
   int prec = 0;                  // 1 FP32 sums, else FP64 accuracy
   double flops = 0, bytes = 0;
@@ -178,12 +182,9 @@ struct HoleBatch {
     return (int)h.size() - 1;
   }
   void finalize(DevArena& ar) {
-    nblocks = 0;
     maxn = 0;
     flops = bytes = 0;
     for (auto& hd : h) {
-      hd.block_start = nblocks;
-      nblocks += hd.nblk;
       hd.nred = prec == 1 ? hd.nblk : 1;
       maxn = std::max(maxn, std::max(hd.n1, hd.n2));
       f32 = f32 || hd.xfmt == TF_F32 || hd.yfmt == TF_F32;
@@ -196,19 +197,36 @@ struct HoleBatch {
       CK(cudaMemset(cnt, 0, sizeof(unsigned) * h.size()));
       for (size_t i = 0; i < h.size(); ++i) h[i].counter = cnt + i;
     }
-    d = upload_vec(ar, h);
+    d = upload_vec(ar, ordered());
   }
+  // block numbers, and the descriptors in their order
+  std::vector<HoleDesc> ordered() {
+    std::vector<HoleDesc> o;
+    nblocks = 0;
+    for (bool wide : {false, true}) {
+      for (auto& hd : h) {
+        if ((std::max(hd.n1, hd.n2) > 8) != wide) continue;
+        hd.block_start = nblocks;
+        nblocks += hd.nblk;
+        o.push_back(hd);
+      }
+      if (!wide) {
+        nnarrow = (int)o.size();
+        narrow_blocks = nblocks;
+      }
+    }
+    return o;
+  }
+  HoleLaunch launch() const { return HoleLaunch{d, (int)h.size(), nnarrow, nblocks, narrow_blocks, f32}; }
   // new block counts (one block per `tpb` tiles, at most `cap`), in place on the device
   void retile(int tpb, int cap, cudaStream_t st) {
     if (h.empty()) return;
-    nblocks = 0;
     for (auto& hd : h) {
       hd.nblk = hole_nblk(hd, tpb, cap);
       hd.nred = prec == 1 ? hd.nblk : 1;
-      hd.block_start = nblocks;
-      nblocks += hd.nblk;
     }
-    CK(cudaMemcpyAsync(d, h.data(), sizeof(HoleDesc) * h.size(), cudaMemcpyHostToDevice, st));
+    const std::vector<HoleDesc> o = ordered();
+    CK(cudaMemcpyAsync(d, o.data(), sizeof(HoleDesc) * o.size(), cudaMemcpyHostToDevice, st));
   }
 };
 
@@ -2062,7 +2080,7 @@ void run_prod(Ctx& c, const ProdBatch& b) {
 void run_hole(Ctx& c, const HoleBatch& b) {
   if (b.h.empty()) return;
   ProfScope ps(c, KP_HOLE, b.flops, b.bytes);
-  launch_hole(b.d, (int)b.h.size(), b.nblocks, b.maxn, b.f32, c.st, b.prec);
+  launch_hole(b.launch(), c.st, b.prec);
   c.count();
 }
 void run_red(Ctx& c, const RedBatch& b) {
@@ -2135,8 +2153,8 @@ void run_packets(Ctx& c) {
 
 // SPF derivatives into out's psi part (derivatives.f90:94-153)
 void run_spf(Ctx& c, cplx* out) {
-  launch_spf(c.spf_d, (int)c.spf_h.size(), c.spf_tiles, c.spf_holes.maxn, c.spfstep_d, c.spf_holes.d,
-             (int)c.spf_holes.h.size(), c.spf_holes.nblocks, out, c.der, c.d_status, c.st);
+  launch_spf(c.spf_d, (int)c.spf_h.size(), c.spf_tiles, c.spf_holes.maxn, c.spfstep_d,
+             c.spf_holes.launch(), out, c.der, c.d_status, c.st);
   c.count(3);
 }
 
@@ -4349,7 +4367,7 @@ void ens_run_prod(Ens& E, const ProdBatch& b) {
 }
 void ens_run_hole(Ens& E, const HoleBatch& b) {
   if (b.h.empty()) return;
-  launch_hole(b.d, (int)b.h.size(), b.nblocks, b.maxn, b.f32, E.st, b.prec, E.persist_hole);
+  launch_hole(b.launch(), E.st, b.prec, E.persist_hole);
   ++E.launches;
 }
 void ens_run_red(Ens& E, const RedBatch& b) {
@@ -4373,8 +4391,8 @@ void ens_eom(Ens& E, cplx* out) {
   ens_run_red(E, E.red);
   launch_reginv(E.reg_d, (int)E.reg_h.size(), E.mfop_d, E.status_d, E.st);
   launch_termsum(out, E.sum_d, (int)E.sum_h.size(), E.src_d, E.total, E.st, E.precision);
-  launch_spf(E.spf_d, (int)E.spf_h.size(), E.spf_tiles, E.spf_holes.maxn, E.spfstep_d, E.spf_holes.d,
-             (int)E.spf_holes.h.size(), E.spf_holes.nblocks, out, E.der, E.status_d, E.st);
+  launch_spf(E.spf_d, (int)E.spf_h.size(), E.spf_tiles, E.spf_holes.maxn, E.spfstep_d,
+             E.spf_holes.launch(), out, E.der, E.status_d, E.st);
   E.launches += 5;
   E.eom_count++;
 }

@@ -248,11 +248,11 @@ void launch_prod_fx(const ProdDesc* d, int nd, long long nblocks, int maxn, cuda
 // ---------------------------------------------------------------------------
 // Batched single-hole contraction, first stage (zher2k / zgemm('T','N') loops of
 // Calc_rho1mode and Calc_MeanField, gmctdh_objects.f90:452-457, :595-600).
-// Block b of a descriptor handles a contiguous share of the fibres.  A warp task is
-// an 8 x 8 block of (j1, j2) pairs over every FS-th group of 16 fibres: the MMA's rows
+// Block b of a descriptor handles a contiguous share of the fibres.  For n1, n2 <= 8 a
+// warp takes every fourth group of 16 fibres: the MMA's rows
 // are (re, im) of eight X columns, its columns the re, then the im of eight Y columns,
 // its inner dimension the fibres; lanes load what they hold, nothing is staged.  A
-// column has one exponent, the largest so far in the task; when it grows, the sums so
+// column has one exponent, the largest so far in the warp; when it grows, the sums so
 // far go to FP64.  Seven digits (the operands rounded at 2^-54 of the column's largest
 // element), the 34 digit products of weight above 2^-64.  The last block of a
 // descriptor to finish adds the blocks' partials in block order into the first.
@@ -260,20 +260,20 @@ void launch_prod_fx(const ProdDesc* d, int nd, long long nblocks, int maxn, cuda
 #define HOLE_NS 7        // digits per operand
 #define HOLE_ND 8        // weights kept
 #define HOLE_FLUSH 8     // groups of 16 fibres between flushes: 128 x 6 x 2^14 < 2^24
-#define HOLE_WARPS 4
-#define HOLE_MTHREADS (32 * HOLE_WARPS)
+#define HOLE_WARPS 4     // per block; twice as many where n1 or n2 is above eight
 
 // 1 x 1 contractions (inner products): every thread strides over elements with
 // coalesced loads, the block reduces in shared memory.
 static __device__ void dot_block(const HoleDesc& d, int b, cplx* red) {
+  constexpr int T = 32 * HOLE_WARPS;
   const long long n = d.L * d.R;
   const int tid = threadIdx.x;
   cplx acc = mkc(0, 0);
-  for (long long i = (long long)b * HOLE_MTHREADS + tid; i < n; i += (long long)d.nblk * HOLE_MTHREADS)
+  for (long long i = (long long)b * T + tid; i < n; i += (long long)d.nblk * T)
     cfma_conj(acc, load_c(d.X, i, d.xfmt), load_c(d.Y, i, d.yfmt));
   red[tid] = acc;
   __syncthreads();
-  for (int s = HOLE_MTHREADS / 2; s > 0; s >>= 1) {
+  for (int s = T / 2; s > 0; s >>= 1) {
     if (tid < s) red[tid] = cadd(red[tid], red[tid + s]);
     __syncthreads();
   }
@@ -299,44 +299,32 @@ static __device__ __noinline__ void hole_block_fp64(const HoleDesc& d, const cpl
 // F32: operands may be complex FP32
 template <bool F32>
 __device__ __forceinline__ void hole_fx_block(const HoleDesc& d, int b, const cplx* ybase) {
-  constexpr int NS = HOLE_NS, ND = HOLE_ND;
-  extern __shared__ cplx red[];   // [pair blocks][FS][64]
+  constexpr int NS = HOLE_NS, ND = HOLE_ND, W = HOLE_WARPS;
+  extern __shared__ cplx red[];   // [warp][64]
   __shared__ int s_slow;
   const cplx* Yp = d.Y ? d.Y : ybase + d.yoff;
   const int n1 = d.n1, n2 = d.n2, npairs = n1 * n2;
-  if (npairs == 1 && d.Y && d.L * d.R >= HOLE_MTHREADS) {
+  if (npairs == 1 && d.Y && d.L * d.R >= 32 * W) {
     dot_block(d, b, red);
     return;
   }
   const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5, g = lane >> 2, q = lane & 3;
   const int xfmt = F32 ? d.xfmt : 0, yfmt = F32 ? d.yfmt : 0;
-  // X = Y (density matrices, SPF overlaps): C is Hermitian, only the blocks on and
-  // above the diagonal are computed
+  // X = Y (density matrices, SPF overlaps): the digits serve both operands
   const bool sym = d.X == d.Y && n1 == n2 && d.xfmt == d.yfmt;
-  const int b1 = (n1 + 7) >> 3, b2 = (n2 + 7) >> 3;
-  const int nbp = sym ? b1 * (b1 + 1) / 2 : b1 * b2;
-  const int FS = (nbp & 3) == 0 ? 1 : ((nbp & 1) == 0 ? 2 : 4);   // tasks fill the warps
   const unsigned L = (unsigned)d.L, nfib = (unsigned)(d.L * d.R);
   const unsigned ngrp = (nfib + 15) / 16;
   const unsigned g0 = (unsigned)((unsigned long long)ngrp * b / d.nblk);
   const unsigned g1 = (unsigned)((unsigned long long)ngrp * (b + 1) / d.nblk);
-  const unsigned dl = (16u * FS) % L, dr = (16u * FS) / L;
+  const unsigned dl = (16u * W) % L, dr = (16u * W) / L;
   if (tid == 0) s_slow = 0;
   __syncthreads();
   bool slow = false;
-  for (int task = warp; task < nbp * FS; task += HOLE_WARPS) {
-    const int pb = task / FS, fs = task - pb * FS;
-    int c1 = pb % b1, c2 = pb / b1;
-    if (sym) {   // pb -> (c1 <= c2), c2-major
-      int rem = pb;
-      c2 = 0;
-      while (rem > c2) rem -= ++c2;
-      c1 = rem;
-    }
-    const bool same = sym && c1 == c2;
-    const int jx = 8 * c1 + g, jy = 8 * c2 + g;   // the lane's columns
+  {
+    const bool same = sym;
+    const int jx = g, jy = g;   // the lane's columns
     // the lane's fibres of a group: 2 q, 2 q + 1, 2 q + 8, 2 q + 9
-    unsigned p = 16u * (g0 + fs) + 2 * q, l[4], r[4];
+    unsigned p = 16u * (g0 + warp) + 2 * q, l[4], r[4];
 #pragma unroll
     for (int f = 0; f < 4; ++f) {
       const unsigned pf = p + (f & 1) + 8 * (f >> 1);
@@ -355,7 +343,7 @@ __device__ __forceinline__ void hole_fx_block(const HoleDesc& d, int b, const cp
         r[f] += dr;
         if (l[f] >= L) { l[f] -= L; r[f] += 1; }
       }
-      p += 16 * FS;
+      p += 16 * W;
     };
     float cr[ND][4], ci[ND][4];   // sums with Yr and Yi: rows Xr (0, 1), Xi (2, 3)
 #pragma unroll
@@ -386,7 +374,7 @@ __device__ __forceinline__ void hole_fx_block(const HoleDesc& d, int b, const cp
       pend = 0;
     };
     fetch();
-    for (unsigned gr = g0 + fs; gr < g1; gr += FS) {
+    for (unsigned gr = g0 + warp; gr < g1; gr += W) {
       unsigned mx = max(max(fx_mag(x[0]), fx_mag(x[1])), max(fx_mag(x[2]), fx_mag(x[3])));
       unsigned my = max(max(fx_mag(y[0]), fx_mag(y[1])), max(fx_mag(y[2]), fx_mag(y[3])));
       mx = max(mx, __shfl_xor_sync(0xffffffffu, mx, 1));
@@ -434,7 +422,7 @@ __device__ __forceinline__ void hole_fx_block(const HoleDesc& d, int b, const cp
           }
         }
       }
-      if (gr + FS < g1) fetch();
+      if (gr + W < g1) fetch();
 #pragma unroll
       for (int i = 0; i < NS; ++i)
 #pragma unroll
@@ -445,9 +433,9 @@ __device__ __forceinline__ void hole_fx_block(const HoleDesc& d, int b, const cp
       ++pend;
     }
     if (pend) flush();
-    // (j1, j2) = (g, 2 q), (g, 2 q + 1) of the task's block
-    red[(pb * FS + fs) * 64 + g + 8 * (2 * q)] = acc[0];
-    red[(pb * FS + fs) * 64 + g + 8 * (2 * q + 1)] = acc[1];
+    // (j1, j2) = (g, 2 q), (g, 2 q + 1)
+    red[warp * 64 + g + 8 * (2 * q)] = acc[0];
+    red[warp * 64 + g + 8 * (2 * q + 1)] = acc[1];
   }
   if (slow) s_slow = 1;
   __syncthreads();
@@ -456,21 +444,281 @@ __device__ __forceinline__ void hole_fx_block(const HoleDesc& d, int b, const cp
     return;
   }
   cplx* out = d.partial + (long long)b * npairs;
-  for (int pr = tid; pr < npairs; pr += HOLE_MTHREADS) {
-    int j1 = pr % n1, j2 = pr / n1;
-    const bool lower = sym && (j1 >> 3) > (j2 >> 3);   // conj of the transposed pair
-    if (lower) { const int tmp = j1; j1 = j2; j2 = tmp; }
-    const int c1 = j1 >> 3, c2 = j2 >> 3, pb = sym ? c2 * (c2 + 1) / 2 + c1 : c1 + b1 * c2;
-    const cplx* s = red + pb * FS * 64 + (j1 & 7) + 8 * (j2 & 7);
+  for (int pr = tid; pr < npairs; pr += 32 * W) {
+    const cplx* s = red + pr % n1 + 8 * (pr / n1);
     cplx v = s[0];
-    for (int k = 1; k < FS; ++k) v = cadd(v, s[64 * k]);
-    out[pr] = lower ? cconj(v) : v;
+    for (int k = 1; k < W; ++k) v = cadd(v, s[64 * k]);
+    out[pr] = v;
   }
+}
+
+// The same for n1 or n2 above eight.  Tiles of two by two column blocks: each operand
+// block of 32 fibres is cut once, by one warp, into shared memory in the order the MMAs
+// read it (an uint4 per lane, digit and group of 16 fibres: re, im of fibres 2 q, 2 q + 1,
+// then of 2 q + 8, 2 q + 9), and every warp takes a pair block of the tile.  Where every
+// pair block cut its own operands, cutting bound the kernel (ALU 52 %, tensor pipe 36 %).
+// A column block of at most four columns puts re and im side by side into one MMA.
+// Warps 0-3 cut the next stage while warps 4-7 multiply this one: with every warp doing
+// both in turn the phases of a block did not overlap.
+// 42 contractions of 248,832 fibres, 12 x 12 each: 3,117 -> 2,295 us.
+#define HOLEW_GRP 2      // groups of 16 fibres per stage
+#define HOLEW_FLUSH (HOLE_FLUSH / HOLEW_GRP)
+#define HOLEW_SLOTS 3    // stages of operands in flight
+struct HoleWide {
+  uint4 dig[2][4][HOLEW_GRP][HOLE_NS][32];   // [buffer][operand block][group][digit][lane]
+  cplx raw[HOLEW_SLOTS][4][4 * HOLEW_GRP][32];  // operands: [slot][block][fibre of the lane][lane]
+  cplx sum[4][64];
+  unsigned ex[2][4][8];                      // the columns' exponents
+  int grow[2][4];
+  int slow;
+};
+// both roles pass the same barriers: one before the first stage, one after each
+__device__ __forceinline__ void hole_stage_barrier() {
+  asm volatile("bar.sync 1, %0;" ::"n"(64 * HOLE_WARPS) : "memory");
+}
+template <bool F32>
+__device__ __forceinline__ void hole_cut(HoleWide& sh, const HoleDesc& d, const cplx* Yp, bool& slow, bool cut, bool isx,
+                                         int j0, unsigned nfib, unsigned g0, unsigned g1) {
+  constexpr int NS = HOLE_NS, NP = 4 * HOLEW_GRP;   // fibres per lane and stage
+  constexpr unsigned emin = (unsigned)FX_EMIN << 20;
+  const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5, g = lane >> 2, q = lane & 3;
+  const unsigned L = (unsigned)d.L, dl = (16u * HOLEW_GRP) % L, dr = (16u * HOLEW_GRP) / L;
+  const cplx* P = isx ? d.X : Yp;
+  const int np = isx ? d.n1 : d.n2, j = j0 + g;
+  const int fmt = F32 ? (isx ? d.xfmt : d.yfmt) : 0;
+  unsigned grp = g0, ec = emin, l[NP / 2], r[NP / 2];   // fibres 2 q (+ 8) of each group
+#pragma unroll
+  for (int h = 0; h < NP / 2; ++h) {
+    const unsigned p = 16 * g0 + 8 * h + 2 * q;
+    r[h] = p / L;
+    l[h] = p - L * r[h];
+  }
+  const unsigned raw0 = (unsigned)__cvta_generic_to_shared(&sh.raw[0][warp][0][lane]);
+  constexpr unsigned slot_bytes = sizeof(sh.raw[0]), point_bytes = sizeof(sh.raw[0][0][0]);
+  auto copy = [&](unsigned dst, unsigned ll, unsigned rr, bool in) {
+    const long long e = ll + (long long)L * (j + (long long)np * rr);
+    if (F32 && fmt)
+      asm volatile("cp.async.ca.shared.global [%0], [%1], 8, %2;" ::"r"(dst), "l"(reinterpret_cast<const float2*>(P) + (in ? e : 0)), "r"(in ? 8 : 0) : "memory");
+    else
+      asm volatile("cp.async.ca.shared.global [%0], [%1], 16, %2;" ::"r"(dst), "l"(P + (in ? e : 0)), "r"(in ? 16 : 0) : "memory");
+  };
+  int wslot = 0, rslot = 0;
+  auto fetch = [&]() {   // the next stage's elements, each lane its own: nothing to synchronise
+    if (cut && grp < g1) {
+#pragma unroll
+      for (int h = 0; h < NP / 2; ++h) {
+        const unsigned p = 16 * grp + 8 * h + 2 * q;
+        const bool in = j < np && grp + (h >> 1) < g1, wrap = l[h] + 1 == L;
+        const unsigned dst = raw0 + wslot * slot_bytes + 2 * h * point_bytes;
+        copy(dst, l[h], r[h], in && p < nfib);
+        copy(dst + point_bytes, wrap ? 0u : l[h] + 1, wrap ? r[h] + 1 : r[h], in && p + 1 < nfib);
+        l[h] += dl;
+        r[h] += dr;
+        if (l[h] >= L) { l[h] -= L; r[h] += 1; }
+      }
+    }
+    grp += HOLEW_GRP;
+    wslot = wslot + 1 == HOLEW_SLOTS ? 0 : wslot + 1;
+    asm volatile("cp.async.commit_group;" ::: "memory");
+  };
+  auto stage = [&](int buf) {   // cut the oldest stage in flight into buffer buf
+    asm volatile("cp.async.wait_group %0;" ::"n"(HOLEW_SLOTS - 1) : "memory");
+    cplx x[NP];
+#pragma unroll
+    for (int f = 0; f < NP; ++f) x[f] = load_c(&sh.raw[rslot][warp][f][lane], 0, fmt);
+    rslot = rslot + 1 == HOLEW_SLOTS ? 0 : rslot + 1;
+    unsigned m = 0u;
+#pragma unroll
+    for (int f = 0; f < NP; ++f) m = max(m, fx_mag(x[f]));
+    m = max(m, __shfl_xor_sync(0xffffffffu, m, 1));
+    m = max(m, __shfl_xor_sync(0xffffffffu, m, 2));
+    // out of range, or tiny with nothing larger in the column before it
+    slow = slow || (!fx_ok(m) && (m >= emin || ec == emin));
+    const bool grow = m >= ec + (1u << 20);
+    if (grow) ec = m & FX_EBITS;
+    const bool any = __any_sync(0xffffffffu, grow);
+    if (lane == 0) sh.grow[buf][warp] = any;
+    if (q == 0) sh.ex[buf][warp][g] = ec;
+#pragma unroll
+    for (int gg = 0; gg < HOLEW_GRP; ++gg) {
+      unsigned s[4][NS];
+#pragma unroll
+      for (int h = 0; h < 2; ++h) {
+        fx_digits<NS>(x[4 * gg + 2 * h].x, x[4 * gg + 2 * h + 1].x, ec, ec, s[2 * h]);
+        fx_digits<NS>(x[4 * gg + 2 * h].y, x[4 * gg + 2 * h + 1].y, ec, ec, s[2 * h + 1]);
+      }
+#pragma unroll
+      for (int k = 0; k < NS; ++k) sh.dig[buf][warp][gg][k][lane] = make_uint4(s[0][k], s[1][k], s[2][k], s[3][k]);
+    }
+  };
+  for (int k = 0; k < HOLEW_SLOTS; ++k) fetch();
+  if (cut) stage(0);
+  fetch();
+  hole_stage_barrier();
+  int buf = 1;
+  for (unsigned gr = g0; gr < g1; gr += HOLEW_GRP, buf ^= 1) {
+    if (cut && gr + HOLEW_GRP < g1) stage(buf);
+    fetch();
+    hole_stage_barrier();
+  }
+  asm volatile("cp.async.wait_group 0;" ::: "memory");
+}
+template <bool PACKED>
+__device__ __forceinline__ void hole_mul_go(HoleWide& sh, cplx* acc, bool mine, int xb, int yb, int split, int half,
+                                            unsigned g0, unsigned g1) {
+  constexpr int NS = HOLE_NS, ND = HOLE_ND;
+  constexpr unsigned emin = (unsigned)FX_EMIN << 20;
+  const int lane = threadIdx.x & 31, g = lane >> 2, q = lane & 3;
+  float cr[ND][4], ci[ND][4];   // sums with Yr and Yi (packed: all in cr): rows Xr (0, 1), Xi (2, 3)
+#pragma unroll
+  for (int k = 0; k < ND; ++k)
+#pragma unroll
+    for (int i = 0; i < 4; ++i) cr[k][i] = ci[k][i] = 0.f;
+  unsigned e1 = emin, e2[2] = {emin, emin};
+  int pend = 0;
+  auto flush = [&]() {
+#pragma unroll
+    for (int i = 0; i < 2; ++i) {
+      const int es = (int)(e1 + e2[i]) - ((2044 + 12 + 43) << 20);
+      const long long a = fx_join_wide<ND, 1>(cr, i), b = fx_join_wide<ND, 1>(cr, 2 + i);
+      if (PACKED) {
+        // conj(x) y of a column: re = Xr Yr + Xi Yi in lanes q < 2, im = Xr Yi - Xi Yr in q + 2
+        const long long o = __shfl_xor_sync(0xffffffffu, b, 2);
+        acc[i].x += fx_double(q < 2 ? a + o : a - o, es);
+      } else {
+        const long long re = a + fx_join_wide<ND, 1>(ci, 2 + i), im = fx_join_wide<ND, 1>(ci, i) - b;
+        acc[i] = cadd(acc[i], mkc(fx_double(re, es), fx_double(im, es)));
+      }
+    }
+#pragma unroll
+    for (int k = 0; k < ND; ++k)
+#pragma unroll
+      for (int i = 0; i < 4; ++i) cr[k][i] = ci[k][i] = 0.f;
+    pend = 0;
+  };
+  hole_stage_barrier();
+  int buf = 0;
+  for (unsigned gr = g0; gr < g1; gr += HOLEW_GRP, buf ^= 1) {
+    if (mine) {
+      if (sh.grow[buf][xb] || sh.grow[buf][yb] || pend == HOLEW_FLUSH) {
+        if (pend) flush();
+        e1 = sh.ex[buf][xb][g];
+        const int cy = PACKED ? 2 * (q & 1) : 2 * q;
+        e2[0] = sh.ex[buf][yb][cy];
+        e2[1] = sh.ex[buf][yb][cy + 1];
+      }
+#pragma unroll 1
+      for (int gg = split == 2 ? half : 0; gg < HOLEW_GRP; gg += split) {
+        unsigned A[NS][4];
+#pragma unroll
+        for (int k = 0; k < NS; ++k) {
+          const uint4 v = sh.dig[buf][xb][gg][k][lane];
+          A[k][0] = v.x;
+          A[k][1] = v.y;
+          A[k][2] = v.z;
+          A[k][3] = v.w;
+        }
+        // packed: columns g & 3, re for g < 4, im above
+        const uint4* yd = &sh.dig[buf][yb][gg][0][PACKED ? lane & 15 : lane];
+#pragma unroll
+        for (int j = 0; j < NS; ++j) {
+          const uint4 v = yd[32 * j];
+          if (PACKED) {
+            const unsigned w0 = g < 4 ? v.x : v.y, w1 = g < 4 ? v.z : v.w;
+#pragma unroll
+            for (int i = 0; i < NS && i + j < ND; ++i) fx_mma16(cr[i + j], A[i], w0, w1, false);
+          } else {
+#pragma unroll
+            for (int i = 0; i < NS && i + j < ND; ++i) {
+              fx_mma16(cr[i + j], A[i], v.x, v.z, false);
+              fx_mma16(ci[i + j], A[i], v.y, v.w, false);
+            }
+          }
+        }
+      }
+      ++pend;
+    }
+    hole_stage_barrier();
+  }
+  if (pend) flush();
+}
+__device__ __forceinline__ void hole_mul(HoleWide& sh, cplx* acc, bool mine, bool packed, int xb, int yb, int split,
+                                         int half, unsigned g0, unsigned g1) {
+  if (packed) hole_mul_go<true>(sh, acc, mine, xb, yb, split, half, g0, g1);
+  else hole_mul_go<false>(sh, acc, mine, xb, yb, split, half, g0, g1);
+}
+template <bool F32>
+__device__ __forceinline__ void hole_wide_block(const HoleDesc& d, int b, const cplx* ybase) {
+  constexpr int NS = HOLE_NS, ND = HOLE_ND;
+  constexpr unsigned emin = (unsigned)FX_EMIN << 20;
+  extern __shared__ cplx red[];
+  HoleWide& sh = *reinterpret_cast<HoleWide*>(red);
+  const cplx* Yp = d.Y ? d.Y : ybase + d.yoff;
+  const int n1 = d.n1, n2 = d.n2;
+  const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5, g = lane >> 2, q = lane & 3;
+  const bool sym = d.X == d.Y && n1 == n2 && d.xfmt == d.yfmt;
+  const int b1 = (n1 + 7) >> 3, b2 = (n2 + 7) >> 3;
+  const unsigned L = (unsigned)d.L, nfib = (unsigned)(d.L * d.R);
+  const unsigned ngrp = (nfib + 15) / 16;
+  const unsigned g0 = (unsigned)((unsigned long long)ngrp * b / d.nblk);
+  const unsigned g1 = (unsigned)((unsigned long long)ngrp * (b + 1) / d.nblk);
+  // the light pair blocks (short last column block) fall to other sub-partitions in
+  // every other wave of CTAs
+  const int vw = (warp + 2 * (int)((blockIdx.x / 152) & 1)) & 3;
+  cplx* out = d.partial + (long long)b * n1 * n2;
+  if (tid == 0) sh.slow = 0;
+  bool slow = false;
+  for (int s1 = 0; s1 < b1; s1 += 2)
+    for (int s2 = sym ? s1 : 0; s2 < b2; s2 += 2) {
+      const bool diag = sym && s1 == s2;
+      const int t1 = min(2, b1 - s1), t2 = min(2, b2 - s2);
+      const int njobs = diag ? t1 : t1 + t2, ntask = diag ? t1 * (t1 + 1) / 2 : t1 * t2;
+      const int split = ntask <= 2 ? 2 : 1;            // warps per pair block
+      const int task = vw / split;
+      const bool mine = warp >= 4 && task < ntask;
+      const int c1 = diag ? (task == 2 ? 1 : 0) : task % t1, c2 = diag ? (task ? 1 : 0) : task / t1;
+      const int xb = c1, yb = diag ? c2 : t1 + c2;   // operand blocks in the buffers
+      const bool packed = n2 - 8 * (s2 + c2) <= 4;
+      cplx acc[2] = {mkc(0.0, 0.0), mkc(0.0, 0.0)};   // packed: .x alone
+      __syncthreads();   // the buffers and sums of the tile before are free
+      if (warp < 4)
+        hole_cut<F32>(sh, d, Yp, slow, warp < njobs, diag || warp < t1, 8 * (diag || warp < t1 ? s1 + warp : s2 + warp - t1),
+                      nfib, g0, g1);
+      else
+        hole_mul(sh, acc, mine, packed, xb, yb, split, vw & 1, g0, g1);
+      // sums: a pair block's 8 x 8, its two halves of the fibres apart where it is split
+      if (mine) {
+#pragma unroll
+        for (int i = 0; i < 2; ++i) {
+          if (packed) {
+            double* o = reinterpret_cast<double*>(&sh.sum[vw][g + 8 * (2 * (q & 1) + i)]) + (q >> 1);
+            *o = acc[i].x;
+          } else {
+            sh.sum[vw][g + 8 * (2 * q + i)] = acc[i];
+          }
+        }
+      }
+      __syncthreads();
+      for (int e = tid; e < ntask * 64; e += 64 * HOLE_WARPS) {
+        const int tk = e >> 6, pr = e & 63;
+        const int a1 = diag ? (tk == 2 ? 1 : 0) : tk % t1, a2 = diag ? (tk ? 1 : 0) : tk / t1;
+        const int j1 = 8 * (s1 + a1) + (pr & 7), j2 = 8 * (s2 + a2) + (pr >> 3);
+        if (j1 >= n1 || j2 >= n2) continue;
+        cplx v = sh.sum[split * tk][pr];
+        if (split == 2) v = cadd(v, sh.sum[2 * tk + 1][pr]);
+        out[j1 + n1 * j2] = v;
+        if (sym && s1 + a1 != s2 + a2) out[j2 + n1 * j1] = cconj(v);
+      }
+    }
+  if (slow) sh.slow = 1;
+  __syncthreads();
+  if (sh.slow) hole_block_fp64(d, Yp, b, 16u * g0, min(16u * g1, nfib));
 }
 
 // The block that finishes last adds the descriptor's partials into the first, in
 // block order, and resets the counter for the next launch.
-static __device__ __forceinline__ void hole_sum_blocks(const HoleDesc& d) {
+template <int W>
+__device__ __forceinline__ void hole_sum_blocks(const HoleDesc& d) {
   __shared__ bool s_last;
   const int npairs = d.n1 * d.n2, nblk = d.nblk;
   if (nblk == 1) return;
@@ -481,8 +729,8 @@ static __device__ __forceinline__ void hole_sum_blocks(const HoleDesc& d) {
   if (!s_last) return;
   __threadfence();
   int sub = 1;   // neighbouring threads per pair
-  while (2 * sub * npairs <= HOLE_MTHREADS && 2 * sub <= min(nblk, 32)) sub *= 2;
-  for (int w0 = 0; w0 < npairs * sub; w0 += HOLE_MTHREADS) {
+  while (2 * sub * npairs <= 32 * W && 2 * sub <= min(nblk, 32)) sub *= 2;
+  for (int w0 = 0; w0 < npairs * sub; w0 += 32 * W) {
     const int w = w0 + threadIdx.x, pr = w / sub, k0 = w - pr * sub;
     const bool on = pr < npairs;
     cplx s = mkc(0, 0);
@@ -498,22 +746,45 @@ static __device__ __forceinline__ void hole_sum_blocks(const HoleDesc& d) {
 
 // CTA b takes the batch's blocks b, b + gridDim.x, ...: one each, or the persistent
 // form (each block writes its own partial, so the sums do not depend on the grid).
+// Descriptors with n1, n2 <= 8 and the wider ones go by launches of their own: each
+// form has the registers and the shared memory it needs.
 template <bool F32>
-__global__ void __launch_bounds__(HOLE_MTHREADS, 3)
+__global__ void __launch_bounds__(32 * HOLE_WARPS, 3)
     hole_fx_kernel(const HoleDesc* __restrict__ descs, int ndesc, long long nblocks, const cplx* ybase) {
   for (long long bb = blockIdx.x; bb < nblocks; bb += gridDim.x) {
     const HoleDesc& d = descs[warp_find_desc(descs, ndesc, bb)];
     if (bb != blockIdx.x) __syncthreads();   // the shared sums are rewritten
     hole_fx_block<F32>(d, (int)(bb - d.block_start), ybase);
-    hole_sum_blocks(d);
+    hole_sum_blocks<HOLE_WARPS>(d);
+  }
+}
+template <bool F32>
+__global__ void __launch_bounds__(64 * HOLE_WARPS, 2)
+    hole_wide_kernel(const HoleDesc* __restrict__ descs, int ndesc, long long first, long long nblocks, const cplx* ybase) {
+  for (long long bb = blockIdx.x; bb < nblocks; bb += gridDim.x) {
+    const HoleDesc& d = descs[warp_find_desc(descs, ndesc, first + bb)];
+    if (bb != blockIdx.x) __syncthreads();
+    hole_wide_block<F32>(d, (int)(first + bb - d.block_start), ybase);
+    hole_sum_blocks<2 * HOLE_WARPS>(d);
   }
 }
 
-void launch_hole_fx(const HoleDesc* d, int nd, long long nblocks, int maxn, bool f32, cudaStream_t st, int persist,
-                    const cplx* ybase) {
-  // the most tasks (pair blocks x fibre shares) of any n1, n2 <= maxn: 1 x 4, 3 x 4, 9 x 4
-  const int smem = (int)sizeof(cplx) * 64 * (maxn <= 8 ? 4 : (maxn <= 16 ? 12 : 36));
-  const unsigned grid = (unsigned)(persist > 0 ? std::min<long long>(nblocks, persist) : nblocks);
-  if (f32) hole_fx_kernel<true><<<grid, HOLE_MTHREADS, smem, st>>>(d, nd, nblocks, ybase);
-  else hole_fx_kernel<false><<<grid, HOLE_MTHREADS, smem, st>>>(d, nd, nblocks, ybase);
+template <bool F32>
+static void hole_fx_go(const HoleLaunch& b, int persist, cudaStream_t st, const cplx* ybase) {
+  static const cudaError_t configured =
+      cudaFuncSetAttribute(hole_wide_kernel<F32>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)sizeof(HoleWide));
+  (void)configured;
+  auto grid = [&](long long n) { return (unsigned)(persist > 0 ? std::min<long long>(n, persist) : n); };
+  const long long wide = b.nblocks - b.narrow_blocks;
+  if (b.narrow_blocks > 0)
+    hole_fx_kernel<F32><<<grid(b.narrow_blocks), 32 * HOLE_WARPS, sizeof(cplx) * 64 * HOLE_WARPS, st>>>(
+        b.d, b.nnarrow, b.narrow_blocks, ybase);
+  if (wide > 0)
+    hole_wide_kernel<F32><<<grid(wide), 64 * HOLE_WARPS, sizeof(HoleWide), st>>>(
+        b.d + b.nnarrow, b.ndesc - b.nnarrow, b.narrow_blocks, wide, ybase);
+}
+
+void launch_hole_fx(const HoleLaunch& b, cudaStream_t st, int persist, const cplx* ybase) {
+  if (b.f32) hole_fx_go<true>(b, persist, st, ybase);
+  else hole_fx_go<false>(b, persist, st, ybase);
 }

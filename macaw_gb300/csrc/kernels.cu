@@ -262,18 +262,17 @@ __global__ void __launch_bounds__(HOLE_THREADS, 4) hole_kernel_persistent(const 
   }
 }
 
-// maxn: the batch's largest n1, n2; f32: some operand is complex FP32; prec 1: FP32 sums, else FP64 accuracy (fixed.cu)
-void launch_hole(const HoleDesc* d_descs, int ndesc, long long nblocks, int maxn, bool f32, cudaStream_t st, int prec,
-                 int persist) {
-  if (ndesc <= 0 || nblocks <= 0) return;
+// prec 1: FP32 sums, else FP64 accuracy (fixed.cu)
+void launch_hole(const HoleLaunch& b, cudaStream_t st, int prec, int persist) {
+  if (b.ndesc <= 0 || b.nblocks <= 0) return;
   if (prec != 1) {
-    launch_hole_fx(d_descs, ndesc, nblocks, maxn, f32, st, persist);
+    launch_hole_fx(b, st, persist);
     return;
   }
-  if (persist > 0 && nblocks > persist)
-    hole_kernel_persistent<<<(unsigned)persist, HOLE_THREADS, 0, st>>>(d_descs, ndesc, nblocks);
+  if (persist > 0 && b.nblocks > persist)
+    hole_kernel_persistent<<<(unsigned)persist, HOLE_THREADS, 0, st>>>(b.d, b.ndesc, b.nblocks);
   else
-    hole_kernel<<<(unsigned)nblocks, HOLE_THREADS, 0, st>>>(d_descs, ndesc);
+    hole_kernel<<<(unsigned)b.nblocks, HOLE_THREADS, 0, st>>>(b.d, b.ndesc);
 }
 
 // ---------------------------------------------------------------------------

@@ -243,14 +243,18 @@ int tc_timeout_flag(bool clear);
 // persist > 0: at most `persist` persistent CTAs walk the batch's blocks
 void launch_prod(const ProdDesc* d_descs, int ndesc, long long nblocks, int maxn, cudaStream_t st,
                  int prec = 0, int tc = 1, int persist = 0);
-void launch_hole(const HoleDesc* d_descs, int ndesc, long long nblocks, int maxn, bool f32, cudaStream_t st,
-                 int prec = 0, int persist = 0);
+// a batch of contractions: descriptors with n1, n2 <= 8 first
+struct HoleLaunch {
+  const HoleDesc* d;
+  int ndesc, nnarrow;
+  long long nblocks, narrow_blocks;
+  bool f32;                // some operand is complex FP32
+};
+void launch_hole(const HoleLaunch& b, cudaStream_t st, int prec = 0, int persist = 0);
 // FP64 accuracy as exact digit products on the tensor cores (fixed.cu); launched by
 // launch_prod / launch_hole
 void launch_prod_fx(const ProdDesc* d_descs, int ndesc, long long nblocks, int maxn, cudaStream_t st, int persist);
-// f32: operands may be complex FP32
-void launch_hole_fx(const HoleDesc* d_descs, int ndesc, long long nblocks, int maxn, bool f32, cudaStream_t st,
-                    int persist, const cplx* ybase = nullptr);
+void launch_hole_fx(const HoleLaunch& b, cudaStream_t st, int persist, const cplx* ybase = nullptr);
 void launch_reduce(const RedTarget* d_tg, int ntg, const RedTerm* d_terms, cudaStream_t st);
 // with_h: also h1mode (second launch: the Hermitian part of same-state matrices, and
 // the operator sums `sums`); prec > 0: the operator products and phi^H (O phi) in
@@ -260,8 +264,7 @@ void launch_h1(const H1Desc* d_descs, int ndesc, int maxn2, size_t smem_bytes, b
 void launch_reginv(const RegInvDesc* d_descs, int ndesc, const MFOp* d_ops, int* d_status, cudaStream_t st);
 // holes: the contractions phi^H phi and phi^H dphi of every block (Y null: at yoff of out)
 void launch_spf(const SpfDesc* d_descs, int ndesc, long long ntiles, int maxn, const SpfStep* d_steps,
-                const HoleDesc* d_holes, int nholes, long long hole_blocks, cplx* out, cplx der_factor, int* d_status,
-                cudaStream_t st);
+                const HoleLaunch& holes, cplx* out, cplx der_factor, int* d_status, cudaStream_t st);
 // prec 1: FP32 accumulation, else FP64
 // A sum over a whole launch fused into a streaming kernel: v the vector to dot
 // with (termsum: <v|out>; Lanczos axpy: any non-null v requests ||Kn||^2), partial

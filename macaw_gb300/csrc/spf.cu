@@ -314,8 +314,7 @@ __global__ void __launch_bounds__(SPF_THREADS) spf_project_kernel(const SpfDesc*
 }
 
 void launch_spf(const SpfDesc* d_descs, int ndesc, long long ntiles, int maxn, const SpfStep* d_steps,
-                const HoleDesc* d_holes, int nholes, long long hole_blocks, cplx* out, cplx der_factor, int* d_status,
-                cudaStream_t st) {
+                const HoleLaunch& holes, cplx* out, cplx der_factor, int* d_status, cudaStream_t st) {
   if (ndesc <= 0) return;
   const int smem = (int)sizeof(RowShared), smem_x = smem + (int)sizeof(cplx) * maxn * (maxn + SPF_ROWS);
   static const cudaError_t configured = [] {
@@ -325,7 +324,7 @@ void launch_spf(const SpfDesc* d_descs, int ndesc, long long ntiles, int maxn, c
   }();
   (void)configured;
   spf_drive_kernel<<<(unsigned)ntiles, SPF_THREADS, smem, st>>>(d_descs, ndesc, d_steps, out, der_factor);
-  launch_hole_fx(d_holes, nholes, hole_blocks, maxn, false, st, 0, out);
+  launch_hole_fx(holes, st, 0, out);
   if (maxn <= 8) spf_project8_kernel<<<(unsigned)ntiles, SPF_THREADS, 0, st>>>(d_descs, ndesc, out, d_status);
   else spf_project_kernel<<<(unsigned)ntiles, SPF_THREADS, smem_x, st>>>(d_descs, ndesc, out, d_status);
 }
