@@ -257,6 +257,38 @@ void merge_holes(HoleBatch& all, const HoleBatch& a, const HoleBatch& b, DevAren
   all.finalize(ar);
 }
 
+// Operators with dense DOF matrices first (h1_kernel shares them evenly over the SMs).
+// The projections phi_l^H (O phi_r) go to the digit contractions where their FP64 form
+// (4 sum G n1 n2 instructions at 278 per cycle) would take longer than a launch more:
+// at 3.5 M terms (8-SPF QVC model) h1_kernel 59 us against 21 and 11, at 39 K (LVC, 6
+// SPFs) 8.6 us against 12 in all.
+#define H1_PROJECT_MIN 1000000
+H1Launch plan_h1(DevArena& ar, const std::vector<H1Desc>& h, HoleBatch& proj) {
+  H1Launch L;
+  memset(&L, 0, sizeof(L));
+  if (h.empty()) return L;
+  double terms = 0.0;
+  auto cost = [](const H1Desc& d) {
+    int c = 0;
+    for (int q = 0; q < d.ndof; ++q) c += d.optype[q] == 1 || d.optype[q] == 3 ? d.ng[q] : 0;
+    return (long long)c * d.G;
+  };
+  for (auto& d : h) {
+    terms += (double)d.G * d.n1 * d.n2;
+    L.maxn2 = std::max(L.maxn2, d.n2);
+    L.smem = std::max(L.smem, sizeof(cplx) * (size_t)(2 * d.G));
+  }
+  std::vector<H1Desc> o = h;
+  std::stable_sort(o.begin(), o.end(), [&](const H1Desc& a, const H1Desc& b) { return cost(a) > cost(b); });
+  L.d = upload_vec(ar, o);
+  L.n = (int)o.size();
+  if (terms >= H1_PROJECT_MIN) {
+    proj.finalize(ar);
+    L.proj = proj.launch();
+  }
+  return L;
+}
+
 struct RedBatch {
   std::vector<RedTarget> tg;
   std::vector<RedTerm> terms;
@@ -477,7 +509,6 @@ struct Ctx {
 
   // DVR operator matrices on device: (dof, code) -> pointer
   std::map<std::pair<int, int>, cplx*> dofmat;
-  std::map<std::pair<int, int>, float2*> dofmatf;   // real coefficients split into FP32 (hi, lo)
   std::map<std::pair<int, int>, int> dofkind;
 
   // per (mode, op) storage
@@ -487,9 +518,8 @@ struct Ctx {
 
   // EOM plan
   std::vector<H1Desc> h1_h;
-  H1Desc* h1_d = nullptr;
-  size_t h1_smem = 0;
-  int h1_maxn2 = 0;
+  H1Launch h1{};
+  HoleBatch h1_proj;       // their phi_l^H (O phi_r)
   std::vector<ProdBatch> chains;  // per depth
   std::vector<ProdBatch> chains_full;   // per depth: right chains needed only for dA (adjoint partners)
   HoleBatch holes;       // mean-field contractions of the general terms
@@ -536,7 +566,6 @@ struct Ctx {
   SumSrc* hbsrc_d = nullptr;
   SumRange* hbsum_d = nullptr;
   // ophi-only h1 plan (CMF2 SPF sweeps: operators on the current SPFs, mean fields frozen)
-  std::vector<std::vector<int>> h1_of_mode;  // indices into h1_h per DVR mode
   // overlap plans
   OvlPlan dpsi_plan;   // d_tmp vs d_err
   OvlPlan cmf_ovl;     // CMF2's SPF error: d_ovl1 vs d_ovl2 (own buffers: it runs beside the SPF sweep)
@@ -582,7 +611,8 @@ struct Ctx {
   std::vector<cplx> exp_ae;
   std::vector<std::vector<char>> ham_op;              // [m][k]: the operator of some Hamiltonian term
   std::vector<H1Desc> xh1_h;                          // grid-mode operators of expectation operators only
-  H1Desc* xh1_d = nullptr;
+  HoleBatch xh1_proj;
+  H1Launch xh1{};
   std::vector<GwpH1Desc> xgh1_h;                      // Gaussian-mode ones
   GwpH1Desc* xgh1_d = nullptr;
   cplx* d_adot = nullptr;                             // f * sum_t ae_t H_t A before the corrections
@@ -861,13 +891,6 @@ void load_setup(Ctx& c, const mctdh_setup_t* s) {
         }
         c.dofmat[key] = upload_vec(c.ar, v);
         c.dofkind[key] = kind;
-        std::vector<float2> vf(v.size());
-        for (size_t i = 0; i < v.size(); ++i) {
-          const double x = (kind == 3) ? v[i].y : v[i].x;
-          const float hi = (float)x;
-          vf[i] = make_float2(hi, (float)(x - (double)hi));
-        }
-        c.dofmatf[key] = upload_vec(c.ar, vf);
       }
     }
   }
@@ -1110,9 +1133,7 @@ void plan_eom(Ctx& c) {
   c.rhom1mf.assign(f, {});
   c.rho.assign(f, std::vector<cplx*>(c.nstates, nullptr));
   c.rho_ave.assign(f, nullptr);
-  c.h1_of_mode.assign(f, {});
   // h1mode / ophi descriptors
-  size_t smem = 0;
   for (int m : c.modes_dvr) {
     const int G = c.gmode[m];
     c.hmat[m].assign(c.noper[m], nullptr);
@@ -1140,8 +1161,11 @@ void plan_eom(Ctx& c) {
       hd.phi_r = c.d_in + c.naconftot + c.ipsi[m + f * r];
       hd.phi_l = c.d_in + c.naconftot + c.ipsi[m + f * l];
       hd.ophi = c.ophi[m][k];
+      HoleBatch& pb = ham ? c.h1_proj : c.xh1_proj;
+      cplx* ph = pb.h[pb.add(c.ar, hd.phi_l, hd.ophi, G, 1, n1, n2)].partial;
+      hd.X = ph;
+      if (l != r) c.hmat[m][k] = ph;   // the contraction's result itself
       hd.h = c.hmat[m][k];
-      hd.X = c.ar.calloc_c((long long)n1 * n2);
       hd.G = G;
       hd.n1 = n1;
       hd.n2 = n2;
@@ -1157,22 +1181,17 @@ void plan_eom(Ctx& c) {
           auto key = std::make_pair(d, code);
           hd.optype[q] = c.dofkind[key];
           hd.mat[q] = c.dofmat[key];
-          hd.matf[q] = c.dofmatf[key];
         }
       }
       if (ham) {
-        c.h1_of_mode[m].push_back((int)c.h1_h.size());
         c.h1_h.push_back(hd);
       } else {
         c.xh1_h.push_back(hd);
       }
-      smem = std::max(smem, sizeof(cplx) * (size_t)(2 * G));
-      c.h1_maxn2 = std::max(c.h1_maxn2, n2);
     }
   }
-  c.h1_smem = smem;
-  c.h1_d = upload_vec(c.ar, c.h1_h);
-  c.xh1_d = upload_vec(c.ar, c.xh1_h);
+  c.h1 = plan_h1(c.ar, c.h1_h, c.h1_proj);
+  c.xh1 = plan_h1(c.ar, c.xh1_h, c.xh1_proj);
   if (!c.modes_gwp.empty()) plan_gwp_setup(c);
 
   // density matrices (Calc_rho1mode, gmctdh_objects.f90:408-477)
@@ -2169,9 +2188,7 @@ void eom(Ctx& c, cplx* out, bool mf_only = false, bool reginv = true) {
   {
     RtScope rt(c, RT_H1MODE);
     ProfScope ps(c, KP_H1);
-    launch_h1(c.h1_d, (int)c.h1_h.size(), c.h1_maxn2, c.h1_smem, true, c.st, c.precision, c.msum_d, (int)c.msum_h.size(),
-              c.msum_src_d);
-    c.count(2);
+    c.count(launch_h1(c.h1, true, c.st, c.msum_d, (int)c.msum_h.size(), c.msum_src_d));
   }
   RtScope rt_mf(c, RT_MEANFIELD);   // gmctdh_objects.f90:511-1140
   // the deepest level holds only the full products H_t A of the right chains (dA)
@@ -2949,9 +2966,7 @@ void h1_only(Ctx& c, const cplx* y) {
     launch_gwp_h1(c.gh1_d, (int)c.gh1_h.size(), c.st);
     c.count(2);
   }
-  launch_h1(c.h1_d, (int)c.h1_h.size(), c.h1_maxn2, c.h1_smem, true, c.st, c.precision, c.msum_d, (int)c.msum_h.size(),
-            c.msum_src_d);
-  c.count(2);
+  c.count(launch_h1(c.h1, true, c.st, c.msum_d, (int)c.msum_h.size(), c.msum_src_d));
 }
 
 // SPF integration of all DVR modes with frozen mean fields, in lockstep: one
@@ -2964,8 +2979,6 @@ struct CmfState {
   bool planned = false;
   cplx *B0, *BHalf, *B02, *psiHalf, *psiHalf2, *AHalf;  // full-length vectors (ntot)
   cplx* ytmp;
-  std::vector<H1Desc> h1;       // operators on the current SPFs (h1mode frozen)
-  H1Desc* h1_d = nullptr;
   unsigned char* elem_mode = nullptr;   // mode of every psi element
   double* dt_mode = nullptr;            // device, per mode
   int* accept = nullptr;                // device, per mode
@@ -3061,7 +3074,7 @@ void spf_eval_all(Ctx& c, CmfState& S, cplx* out, cplx* Dout) {
     RtScope rt(c, RT_SPF_DVR);   // Calc_Der_SPF (cmf2_derivatives.f90:84-235), h1 refresh included
     {
       ProfScope ps(c, KP_H1);
-      launch_h1(S.h1_d, (int)S.h1.size(), c.h1_maxn2, c.h1_smem, false, c.st, c.precision);
+      launch_h1(c.h1, false, c.st);   // mean fields and h1mode stay frozen; only ophi is refreshed
     }
     {
       ProfScope ps(c, KP_SPF);
@@ -3202,11 +3215,6 @@ void plan_cmf(Ctx& c, CmfState& S) {
   S.psiHalf2 = c.ar.calloc_c(c.ntot);
   S.AHalf = c.ar.calloc_c(c.ntot);
   S.ytmp = c.ar.calloc_c(c.ntot);
-  for (auto hd : c.h1_h) {
-    hd.h = nullptr;   // mean fields and h1mode stay frozen; only ophi is refreshed
-    S.h1.push_back(hd);
-  }
-  S.h1_d = upload_vec(c.ar, S.h1);
   std::vector<unsigned char> em((size_t)std::max<long long>(c.dimpsi, 1), 0);
   std::vector<HoleRef> hrefs;
   for (int m : c.modes_dvr) {
@@ -4106,9 +4114,8 @@ struct Ens {
   HoleBatch rho_holes, holes, all_holes;
   RedBatch red;
   std::vector<H1Desc> h1_h;
-  H1Desc* h1_d = nullptr;
-  int h1_maxn2 = 0;
-  size_t h1_smem = 0;
+  H1Launch h1{};
+  HoleBatch h1_proj;
   std::vector<MatSumDesc> msum_h;
   std::vector<MatSumSrc> msum_src_h;
   MatSumDesc* msum_d = nullptr;
@@ -4261,8 +4268,7 @@ Ens* ens_create(const mctdh_setup_t* setups, int n) {
       merge_hole(E->holes, c->holes);
       merge_red(E->red, c->red);
       E->h1_h.insert(E->h1_h.end(), c->h1_h.begin(), c->h1_h.end());
-      E->h1_maxn2 = std::max(E->h1_maxn2, c->h1_maxn2);
-      E->h1_smem = std::max(E->h1_smem, c->h1_smem);
+      merge_hole(E->h1_proj, c->h1_proj);
       for (MatSumDesc md : c->msum_h) {
         md.first += (int)E->msum_src_h.size();
         E->msum_h.push_back(md);
@@ -4316,7 +4322,7 @@ Ens* ens_create(const mctdh_setup_t* setups, int n) {
     merge_full(E->full, E->chains, E->chains_full, E->gprods, E->ar);
     merge_holes(E->all_holes, E->rho_holes, E->holes, E->ar);
     E->red.finalize(E->ar);
-    E->h1_d = upload_vec(E->ar, E->h1_h);
+    E->h1 = plan_h1(E->ar, E->h1_h, E->h1_proj);
     E->msum_d = upload_vec(E->ar, E->msum_h);
     E->msum_src_d = upload_vec(E->ar, E->msum_src_h);
     E->reg_d = upload_vec(E->ar, E->reg_h);
@@ -4336,7 +4342,7 @@ Ens* ens_create(const mctdh_setup_t* setups, int n) {
     E->acc_d = (int*)E->ar.alloc(sizeof(int) * n);
     E->status_d = (int*)E->ar.alloc(64);
     CK(cudaMemset(E->status_d, 0, 64));
-    if (E->h1_smem > 48 * 1024) throw StatusError(MCTDH_EUNSUPPORTED, "grid of a mode too large for the h1 kernel");
+    if (E->h1.smem > 48 * 1024) throw StatusError(MCTDH_EUNSUPPORTED, "grid of a mode too large for the h1 kernel");
     CK(cudaDeviceSynchronize());
   } catch (...) {
     for (Ctx* c : E->m) delete c;
@@ -4378,9 +4384,7 @@ void ens_run_red(Ens& E, const RedBatch& b) {
 
 // EOM of every member: IN -> out (same layout as the ensemble vectors).
 void ens_eom(Ens& E, cplx* out) {
-  launch_h1(E.h1_d, (int)E.h1_h.size(), E.h1_maxn2, E.h1_smem, true, E.st, E.precision, E.msum_d, (int)E.msum_h.size(),
-            E.msum_src_d);
-  E.launches += 2;
+  E.launches += launch_h1(E.h1, true, E.st, E.msum_d, (int)E.msum_h.size(), E.msum_src_d);
   for (size_t i = 1; i < E.full.size(); ++i) ens_run_prod(E, E.full[i]);
   if (E.all_holes.h.empty()) {
     ens_run_hole(E, E.rho_holes);
@@ -4761,9 +4765,7 @@ void expectation(Ctx& c, cplx* values) {
     launch_gwp_h1(c.xgh1_d, (int)c.xgh1_h.size(), c.st);
     c.count(3);
   }
-  launch_h1(c.h1_d, (int)c.h1_h.size(), c.h1_maxn2, c.h1_smem, true, c.st, 0);
-  launch_h1(c.xh1_d, (int)c.xh1_h.size(), c.h1_maxn2, c.h1_smem, true, c.st, 0);
-  c.count(2);
+  c.count(launch_h1(c.h1, true, c.st) + launch_h1(c.xh1, true, c.st));
   for (size_t i = 1; i < W.chain.size(); ++i) run_prod(c, W.chain[i]);
   run_hole(c, W.dots);
   run_red(c, W.red);

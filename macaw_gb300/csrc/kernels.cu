@@ -34,20 +34,6 @@ __device__ __forceinline__ int find_desc(const D* descs, int ndesc) {
 // One thread owns one fibre (l, :, r): it reads the nin inputs once into
 // registers and writes the nout outputs.
 // ---------------------------------------------------------------------------
-// acc (hi, lo) += a * b for FP32 pairs a = ah + al, b = bh + bl: the leading
-// product is split exactly with an FMA, the sum keeps its rounding error in lo.
-__device__ __forceinline__ void df_fma(float& sh, float& sl, float ah, float al, float bh, float bl) {
-  const float p = ah * bh;
-  float e = fmaf(ah, bh, -p);
-  e = fmaf(ah, bl, e);
-  e = fmaf(al, bh, e);
-  const float s = sh + p;
-  const float bp = s - sh;
-  const float t = (sh - (s - bp)) + (p - bp);
-  sh = s;
-  sl += t + e;
-}
-
 // FP32 products: the FP32-rounded x and M are multiplied and accumulated in FP32
 // (~1e-7 relative; the split's correction products would sit at the accumulation's
 // own rounding level), outputs complex FP32 (TF_F32) or FP64.
@@ -346,12 +332,15 @@ void launch_reduce(const RedTarget* d_tg, int ntg, const RedTerm* d_terms, cudaS
 // One block per (operator, SPF column j2): the primitive DOF operators act
 // within each SPF, so a column is transformed in shared memory on its own
 // (MultTens / MultTensDiag, hamilton.f90:577-629).  The DVR matrices of p, qp
-// (i x real) and d^2/dq^2 (real) are applied with real arithmetic.  Then, when
-// h1mode is wanted, the column j2 of phi_l^H (O phi_r), one warp per row j1.
-__global__ void __launch_bounds__(256) h1_kernel(const H1Desc* __restrict__ descs) {
+// (i x real) and d^2/dq^2 (real) are applied with real arithmetic.  The operators with
+// such matrices cost 2 ng FP64 instructions per element and come first in the list, the
+// columns of an operator as neighbouring blocks, so that the SMs share them evenly.
+// project: also the column j2 of phi_l^H (O phi_r), one warp per row j1 (small models;
+// H1_PROJECT_MIN).
+__global__ void __launch_bounds__(256) h1_kernel(const H1Desc* __restrict__ descs, int maxn2, bool project) {
   extern __shared__ cplx sm[];
-  const H1Desc& d = descs[blockIdx.x];
-  const int j2 = blockIdx.y;
+  const H1Desc& d = descs[blockIdx.x / maxn2];
+  const int j2 = blockIdx.x % maxn2;
   if (j2 >= d.n2) return;
   const int G = d.G, n1 = d.n1;
   cplx* bufA = sm;
@@ -402,99 +391,12 @@ __global__ void __launch_bounds__(256) h1_kernel(const H1Desc* __restrict__ desc
   }
   cplx* dst = d.ophi + (long long)G * j2;
   for (int e = threadIdx.x; e < G; e += blockDim.x) dst[e] = bufA[e];
-  if (d.h == nullptr) return;
+  if (!project) return;
   const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
   for (int j1 = warp; j1 < n1; j1 += (int)(blockDim.x >> 5)) {
     const cplx* pl = d.phi_l + (long long)G * j1;
     cplx s = mkc(0, 0);
     for (int gg = lane; gg < G; gg += 32) cfma_conj(s, pl[gg], bufA[gg]);
-    for (int o = 16; o > 0; o >>= 1) {
-      s.x += __shfl_down_sync(0xffffffffu, s.x, o);
-      s.y += __shfl_down_sync(0xffffffffu, s.y, o);
-    }
-    if (lane == 0) {
-      if (d.same_state) d.X[j1 + n1 * j2] = s;
-      else d.h[j1 + n1 * j2] = s;
-    }
-  }
-}
-
-// Split-FP32 variant of h1_kernel (precision modes 1 and 2): the column is held
-// as FP32 (hi, lo) pairs, the DOF matrices come pre-split, every product is
-// accumulated as a compensated FP32 pair (df_fma, ~1e-13 relative).
-__global__ void __launch_bounds__(256) h1_split_kernel(const H1Desc* __restrict__ descs) {
-  extern __shared__ float4 smf[];
-  const H1Desc& d = descs[blockIdx.x];
-  const int j2 = blockIdx.y;
-  if (j2 >= d.n2) return;
-  const int G = d.G, n1 = d.n1;
-  float4* bufA = smf;
-  float4* bufB = smf + G;
-  const cplx* src = d.phi_r + (long long)G * j2;
-  for (int e = threadIdx.x; e < G; e += blockDim.x) {
-    const cplx v = src[e];
-    float hx, lx, hy, ly;
-    split_d2f(v.x, hx, lx);
-    split_d2f(v.y, hy, ly);
-    bufA[e] = make_float4(hx, hy, lx, ly);
-  }
-  __syncthreads();
-  int ll = 1;
-  for (int k = 0; k < d.ndof; ++k) {
-    const int ng = d.ng[k];
-    const int ot = d.optype[k];
-    if (ot != 0) {
-      const float2* Mf = d.matf[k];
-      for (int e = threadIdx.x; e < G; e += blockDim.x) {
-        const int a = e % ll;
-        const int gg = (e / ll) % ng;
-        const int bidx = e / (ll * ng);
-        float rh = 0.f, rl = 0.f, ih = 0.f, il = 0.f;
-        if (ot == 2) {
-          const float4 x = bufA[e];
-          const float2 m = Mf[gg];
-          df_fma(rh, rl, m.x, m.y, x.x, x.z);
-          df_fma(ih, il, m.x, m.y, x.y, x.w);
-        } else {
-          const float4* in = bufA + a + (long long)ll * ng * bidx;
-          const float2* mc = Mf + (long long)ng * gg;
-          for (int gp = 0; gp < ng; ++gp) {
-            const float4 x = in[(long long)ll * gp];
-            const float2 m = mc[gp];
-            df_fma(rh, rl, m.x, m.y, x.x, x.z);
-            df_fma(ih, il, m.x, m.y, x.y, x.w);
-          }
-        }
-        bufB[e] = (ot == 3) ? make_float4(-ih, rh, -il, rl) : make_float4(rh, ih, rl, il);
-      }
-      __syncthreads();
-      float4* t = bufA; bufA = bufB; bufB = t;
-    }
-    ll *= ng;
-  }
-  cplx* dst = d.ophi + (long long)G * j2;
-  for (int e = threadIdx.x; e < G; e += blockDim.x) {
-    const float4 x = bufA[e];
-    dst[e] = mkc(f2d_exact(x.x) + f2d_exact(x.z), f2d_exact(x.y) + f2d_exact(x.w));
-  }
-  if (d.h == nullptr) return;
-  const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
-  for (int j1 = warp; j1 < n1; j1 += (int)(blockDim.x >> 5)) {
-    const cplx* pl = d.phi_l + (long long)G * j1;
-    float rh = 0.f, rl = 0.f, ih = 0.f, il = 0.f;
-    for (int gg = lane; gg < G; gg += 32) {
-      const cplx p = pl[gg];
-      float phx, plx, phy, ply;
-      split_d2f(p.x, phx, plx);
-      split_d2f(p.y, phy, ply);
-      const float4 x = bufA[gg];
-      // conj(p) * x
-      df_fma(rh, rl, phx, plx, x.x, x.z);
-      df_fma(rh, rl, phy, ply, x.y, x.w);
-      df_fma(ih, il, phx, plx, x.y, x.w);
-      df_fma(ih, il, -phy, -ply, x.x, x.z);
-    }
-    cplx s = mkc(f2d_exact(rh) + f2d_exact(rl), f2d_exact(ih) + f2d_exact(il));
     for (int o = 16; o > 0; o >>= 1) {
       s.x += __shfl_down_sync(0xffffffffu, s.x, o);
       s.y += __shfl_down_sync(0xffffffffu, s.y, o);
@@ -527,7 +429,7 @@ __global__ void h1_finish_kernel(const H1Desc* __restrict__ descs, int nh, const
     return;
   }
   const H1Desc& d = descs[blockIdx.x];
-  if (d.h == nullptr || !d.same_state) return;
+  if (!d.same_state) return;
   const int n1 = d.n1;
   for (int pr = threadIdx.x; pr < n1 * d.n2; pr += blockDim.x) {
     const int j1 = pr % n1, j2 = pr / n1;
@@ -535,20 +437,29 @@ __global__ void h1_finish_kernel(const H1Desc* __restrict__ descs, int nh, const
   }
 }
 
-void launch_h1(const H1Desc* d_descs, int ndesc, int maxn2, size_t smem_bytes, bool with_h, cudaStream_t st,
-               int prec, const MatSumDesc* sums, int nsums, const MatSumSrc* srcs) {
-  if (ndesc > 0) {
+int launch_h1(const H1Launch& b, bool with_h, cudaStream_t st, const MatSumDesc* sums, int nsums,
+              const MatSumSrc* srcs) {
+  int launches = 0;
+  const bool proj = with_h && b.proj.ndesc > 0;
+  if (b.n > 0) {
     static size_t configured = 0;
-    if (smem_bytes > 48 * 1024 && smem_bytes > configured) {
-      cudaFuncSetAttribute(h1_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem_bytes);
-      cudaFuncSetAttribute(h1_split_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem_bytes);
-      configured = smem_bytes;
+    if (b.smem > 48 * 1024 && b.smem > configured) {
+      cudaFuncSetAttribute(h1_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)b.smem);
+      configured = b.smem;
     }
-    if (prec > 0) h1_split_kernel<<<dim3(ndesc, maxn2), 256, smem_bytes, st>>>(d_descs);
-    else h1_kernel<<<dim3(ndesc, maxn2), 256, smem_bytes, st>>>(d_descs);
+    h1_kernel<<<(unsigned)(b.n * b.maxn2), 256, b.smem, st>>>(b.d, b.maxn2, with_h && !proj);
+    ++launches;
   }
-  const int nh = with_h ? ndesc : 0;
-  if (nh + nsums > 0) h1_finish_kernel<<<nh + nsums, 128, 0, st>>>(d_descs, nh, sums, srcs);
+  if (proj) {
+    launch_hole(b.proj, st);
+    ++launches;
+  }
+  const int nh = with_h ? b.n : 0;
+  if (nh + nsums > 0) {
+    h1_finish_kernel<<<nh + nsums, 128, 0, st>>>(b.d, nh, sums, srcs);
+    ++launches;
+  }
+  return launches;
 }
 
 // ---------------------------------------------------------------------------

@@ -79,7 +79,6 @@ struct H1Desc {
   int ng[MAXDOF_MODE];
   int optype[MAXDOF_MODE]; // 0 none, 1 dense real, 2 diagonal, 3 dense imaginary (i x real)
   const cplx* mat[MAXDOF_MODE];
-  const float2* matf[MAXDOF_MODE];  // the real coefficients split into FP32 (hi, lo)
 };
 
 // Regularised inverse of a Hermitian n x n matrix by Jacobi rotations
@@ -256,11 +255,17 @@ void launch_hole(const HoleLaunch& b, cudaStream_t st, int prec = 0, int persist
 void launch_prod_fx(const ProdDesc* d_descs, int ndesc, long long nblocks, int maxn, cudaStream_t st, int persist);
 void launch_hole_fx(const HoleLaunch& b, cudaStream_t st, int persist, const cplx* ybase = nullptr);
 void launch_reduce(const RedTarget* d_tg, int ntg, const RedTerm* d_terms, cudaStream_t st);
-// with_h: also h1mode (second launch: the Hermitian part of same-state matrices, and
-// the operator sums `sums`); prec > 0: the operator products and phi^H (O phi) in
-// compensated split FP32
-void launch_h1(const H1Desc* d_descs, int ndesc, int maxn2, size_t smem_bytes, bool with_h, cudaStream_t st,
-               int prec, const MatSumDesc* sums = nullptr, int nsums = 0, const MatSumSrc* srcs = nullptr);
+// with_h: also h1mode, by `proj` (phi_l^H (O phi_r) of every operator into X or h) or, where
+// that is empty, in the first launch; then the Hermitian part of same-state matrices and
+// the operator sums `sums`.  Returns the number of launches.
+struct H1Launch {
+  const H1Desc* d;
+  int n, maxn2;
+  size_t smem;
+  HoleLaunch proj;
+};
+int launch_h1(const H1Launch& b, bool with_h, cudaStream_t st, const MatSumDesc* sums = nullptr, int nsums = 0,
+              const MatSumSrc* srcs = nullptr);
 void launch_reginv(const RegInvDesc* d_descs, int ndesc, const MFOp* d_ops, int* d_status, cudaStream_t st);
 // holes: the contractions phi^H phi and phi^H dphi of every block (Y null: at yoff of out)
 void launch_spf(const SpfDesc* d_descs, int ndesc, long long ntiles, int maxn, const SpfStep* d_steps,
