@@ -535,6 +535,7 @@ struct Ctx {
   SpfStep* spfstep_d = nullptr;
   HoleBatch spf_holes;     // phi^H phi and phi^H dphi of every SPF derivative block
   long long spf_tiles = 0;
+  cplx* spf_part = nullptr;   // contractions of the tiles
   std::vector<SumRange> sum_h;
   std::vector<SumSrc> src_h;
   SumRange* sum_d = nullptr;
@@ -1587,6 +1588,7 @@ void plan_eom(Ctx& c) {
   }
   c.spf_d = upload_vec(c.ar, c.spf_h);
   c.spfstep_d = upload_vec(c.ar, c.spfstep_h);
+  if (c.spf_tiles) c.spf_part = c.ar.calloc_c(128 * c.spf_tiles);
 
   // dA = f * sum_t ae_t * (H_t A)   (conjugate of Adot_tmp, gmctdh_objects.f90:578; derivatives.f90:155-156)
   for (int s = 0; s < c.nstates; ++s) {
@@ -2171,10 +2173,9 @@ void run_packets(Ctx& c) {
 }
 
 // SPF derivatives into out's psi part (derivatives.f90:94-153)
-void run_spf(Ctx& c, cplx* out) {
-  launch_spf(c.spf_d, (int)c.spf_h.size(), c.spf_tiles, c.spf_holes.maxn, c.spfstep_d,
-             c.spf_holes.launch(), out, c.der, c.d_status, c.st);
-  c.count(3);
+void run_spf(Ctx& c, cplx* out, const SpfStage& next = SpfStage{}) {
+  c.count(launch_spf(c.spf_d, (int)c.spf_h.size(), c.spf_tiles, c.spf_holes.maxn, c.spfstep_d,
+                     c.spf_holes.launch(), c.spf_part, out, c.der, c.d_status, c.st, next));
 }
 
 void eom(Ctx& c, cplx* out, bool mf_only = false, bool reginv = true) {
@@ -3030,19 +3031,20 @@ struct CmfState {
 };
 std::map<const Ctx*, CmfState*> g_cmf;
 
-void stage_modes(Ctx& c, CmfState& S, cplx* out, const cplx* base, const double* coef, int nk) {
+StageArgs stage_args(Ctx& c, const double* coef, int nk) {
   StageArgs a;
   memset(&a, 0, sizeof(a));
-  int n = 0;
   for (int j = 0; j < nk; ++j) {
     if (coef[j] == 0.0) continue;
-    a.k[n] = c.d_k[j];
-    a.c[n] = coef[j];
-    ++n;
+    a.k[a.nk] = c.d_k[j];
+    a.c[a.nk] = coef[j];
+    ++a.nk;
   }
-  a.nk = n;
+  return a;
+}
+void stage_modes(Ctx& c, CmfState& S, cplx* out, const cplx* base, const double* coef, int nk) {
   ProfScope ps(c, KP_ELEM);
-  launch_stage_modes(out, base, a, S.dt_mode, S.elem_mode, c.naconftot, c.dimpsi, c.st);
+  launch_stage_modes(out, base, stage_args(c, coef, nk), S.dt_mode, S.elem_mode, c.naconftot, c.dimpsi, c.st);
   c.count();
 }
 
@@ -3069,7 +3071,8 @@ void stage_D(Ctx& c, CmfState& S, cplx* out, const cplx* base, const double* coe
 // h1 and SPF-tile kernels; Gaussian modes through S00, its Tikhonov inverse,
 // h1mode, C and Y with the frozen density matrices and mean fields, the
 // Tikhonov solve (der_factor * x into out) and dD = -tau D into Dout.
-void spf_eval_all(Ctx& c, CmfState& S, cplx* out, cplx* Dout) {
+// next: the following stage's input, written along (grid modes only).
+void spf_eval_all(Ctx& c, CmfState& S, cplx* out, cplx* Dout, const SpfStage& next = SpfStage{}) {
   if (!c.modes_dvr.empty()) {
     RtScope rt(c, RT_SPF_DVR);   // Calc_Der_SPF (cmf2_derivatives.f90:84-235), h1 refresh included
     {
@@ -3078,7 +3081,7 @@ void spf_eval_all(Ctx& c, CmfState& S, cplx* out, cplx* Dout) {
     }
     {
       ProfScope ps(c, KP_SPF);
-      run_spf(c, out);
+      run_spf(c, out, next);
     }
     c.count();
   }
@@ -3335,31 +3338,45 @@ void spf_issue(Ctx& c, CmfState& S, SpfRun& R) {
   run_graphed(c, 1, y, [&] {
     copy_dev(c, c.d_in + nA, y + nA, c.dimpsi);
     if (S.gwp) copy_dev(c, S.Din, Dy, S.nD);
-    spf_eval_all(c, S, c.d_k[0], S.Dk[0]);
-    for (int st = 1; st < 6; ++st) {
-      stage_modes(c, S, c.d_in, y, dp ? DP_B[st] : CK_B[st], st);
-      stage_D(c, S, S.Din, Dy, dp ? DP_B[st] : CK_B[st], st);
-      spf_eval_all(c, S, c.d_k[st], S.Dk[st]);
+    // stage st (6: the derivative at the 5th-order solution, :386-393) starts from
+    // y + dt sum_k coef_k k_k
+    const int nst = dp ? 7 : 6;
+    const double* const c5 = dp ? DP_C : CK_C;
+    auto coefs = [&](int st) { return st == 6 ? c5 : (dp ? DP_B[st] : CK_B[st]); };
+    const bool fused = !S.gwp && c.spf_holes.maxn <= 8;   // launch_spf writes the next stage's input
+    for (int st = 0; st < nst; ++st) {
+      if (st && !fused) stage_modes(c, S, c.d_in, y, coefs(st), st);
+      if (st) stage_D(c, S, S.Din, Dy, coefs(st), st);
+      SpfStage next{};
+      if (fused && st + 1 < nst)
+        next = SpfStage{1,         c.d_in,      y, stage_args(c, coefs(st + 1), st), coefs(st + 1)[st],
+                        S.dt_mode, S.elem_mode, nA};
+      spf_eval_all(c, S, c.d_k[st], S.Dk[st], next);
     }
-    if (dp) {
-      // the 7th stage is the derivative at the 5th-order solution (:386-393)
-      stage_modes(c, S, c.d_in, y, DP_C, 6);
-      stage_D(c, S, S.Din, Dy, DP_C, 6);
-      spf_eval_all(c, S, c.d_k[6], S.Dk[6]);
-      stage_modes(c, S, c.d_tmp, y, DP_C, 6);
-      stage_D(c, S, S.Dtmp, Dy, DP_C, 6);
-      stage_modes(c, S, c.d_err, y, DP_D, 7);
+    stage_D(c, S, S.Dtmp, Dy, c5, 6);
+    const double* const c4 = dp ? DP_D : CK_D;
+    if (S.gwp) {   // the Gaussian modes' errors need the 4th-order solution itself
+      stage_modes(c, S, c.d_tmp, y, c5, 6);
+      stage_modes(c, S, c.d_err, y, c4, nst);
+      StageArgs a;
+      memset(&a, 0, sizeof(a));
+      a.k[0] = c.d_err + nA;
+      a.c[0] = -1.0;
+      a.nk = 1;
+      launch_stage(S.ytmp + nA, c.d_tmp + nA, a, 1.0, c.dimpsi, c.st);
     } else {
-      stage_modes(c, S, c.d_tmp, y, CK_C, 6);
-      stage_D(c, S, S.Dtmp, Dy, CK_C, 6);
-      stage_modes(c, S, c.d_err, y, CK_D, 6);
+      StageArgs a;
+      memset(&a, 0, sizeof(a));
+      double d4[7];
+      for (int j = 0; j < nst; ++j) {
+        const double w5 = j < 6 ? c5[j] : 0.0;
+        if (w5 == 0.0 && c4[j] == 0.0) continue;
+        a.k[a.nk] = c.d_k[j];
+        a.c[a.nk] = w5;
+        d4[a.nk++] = c4[j];
+      }
+      launch_rk_end(c.d_tmp, S.ytmp, y, a, d4, S.dt_mode, S.elem_mode, nA, c.dimpsi, c.st);
     }
-    StageArgs a;
-    memset(&a, 0, sizeof(a));
-    a.k[0] = c.d_err + nA;
-    a.c[0] = -1.0;
-    a.nk = 1;
-    launch_stage(S.ytmp + nA, c.d_tmp + nA, a, 1.0, c.dimpsi, c.st);
     c.count();
     run_hole(c, S.err_holes);
     run_red(c, S.err_red);
@@ -4130,6 +4147,7 @@ struct Ens {
   SpfStep* spfstep_d = nullptr;
   HoleBatch spf_holes;
   long long spf_tiles = 0;
+  cplx* spf_part = nullptr;   // contractions of the tiles
   std::vector<SumRange> sum_h;
   std::vector<SumSrc> src_h;
   SumRange* sum_d = nullptr;
@@ -4329,6 +4347,7 @@ Ens* ens_create(const mctdh_setup_t* setups, int n) {
     E->mfop_d = upload_vec(E->ar, E->mfop_h);
     E->spf_d = upload_vec(E->ar, E->spf_h);
     E->spfstep_d = upload_vec(E->ar, E->spfstep_h);
+    if (E->spf_tiles) E->spf_part = E->ar.calloc_c(128 * E->spf_tiles);
     E->spf_holes.finalize(E->ar);
     E->sum_d = upload_vec(E->ar, E->sum_h);
     E->src_d = upload_vec(E->ar, E->src_h);
@@ -4395,9 +4414,9 @@ void ens_eom(Ens& E, cplx* out) {
   ens_run_red(E, E.red);
   launch_reginv(E.reg_d, (int)E.reg_h.size(), E.mfop_d, E.status_d, E.st);
   launch_termsum(out, E.sum_d, (int)E.sum_h.size(), E.src_d, E.total, E.st, E.precision);
-  launch_spf(E.spf_d, (int)E.spf_h.size(), E.spf_tiles, E.spf_holes.maxn, E.spfstep_d,
-             E.spf_holes.launch(), out, E.der, E.status_d, E.st);
-  E.launches += 5;
+  E.launches += launch_spf(E.spf_d, (int)E.spf_h.size(), E.spf_tiles, E.spf_holes.maxn, E.spfstep_d,
+                           E.spf_holes.launch(), E.spf_part, out, E.der, E.status_d, E.st);
+  E.launches += 2;
   E.eom_count++;
 }
 

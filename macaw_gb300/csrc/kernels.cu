@@ -1324,6 +1324,34 @@ void launch_stage_modes(cplx* out, const cplx* base, const StageArgs& a, const d
   stage_modes_kernel<<<(unsigned)((n + 255) / 256), 256, 0, st>>>(out, base, a, dt_mode, elem_mode, off, n);
 }
 
+__global__ void rk_end_kernel(cplx* __restrict__ y5, cplx* __restrict__ diff, const cplx* __restrict__ base, StageArgs a,
+                              StageArgs a4, const double* __restrict__ dt_mode,
+                              const unsigned char* __restrict__ elem_mode, long long off, long long n) {
+  const long long i = (long long)blockIdx.x * blockDim.x + threadIdx.x;
+  if (i >= n) return;
+  const long long g = off + i;
+  const double dt = dt_mode[elem_mode[i]];
+  cplx s = mkc(0, 0), r = mkc(0, 0);
+  for (int k = 0; k < a.nk; ++k) {
+    const cplx v = a.k[k][g];
+    s.x = fma(a.c[k], v.x, s.x);
+    s.y = fma(a.c[k], v.y, s.y);
+    r.x = fma(a4.c[k], v.x, r.x);
+    r.y = fma(a4.c[k], v.y, r.y);
+  }
+  const cplx b = base[g];
+  const cplx u = mkc(fma(dt, s.x, b.x), fma(dt, s.y, b.y)), w = mkc(fma(dt, r.x, b.x), fma(dt, r.y, b.y));
+  y5[g] = u;
+  diff[g] = csub(u, w);
+}
+void launch_rk_end(cplx* y5, cplx* diff, const cplx* base, const StageArgs& a, const double* c4, const double* dt_mode,
+                   const unsigned char* elem_mode, long long off, long long n, cudaStream_t st) {
+  if (n <= 0) return;
+  StageArgs a4 = a;
+  for (int k = 0; k < a.nk; ++k) a4.c[k] = c4[k];
+  rk_end_kernel<<<(unsigned)((n + 255) / 256), 256, 0, st>>>(y5, diff, base, a, a4, dt_mode, elem_mode, off, n);
+}
+
 // y <- src on the elements of accepted modes
 __global__ void masked_copy_kernel(cplx* __restrict__ y, const cplx* __restrict__ src,
                                    const unsigned char* __restrict__ elem_mode, const int* __restrict__ accept,

@@ -250,6 +250,27 @@ struct HoleLaunch {
   bool f32;                // some operand is complex FP32
 };
 void launch_hole(const HoleLaunch& b, cudaStream_t st, int prec = 0, int persist = 0);
+// The input of the next Runge-Kutta stage, written along with SPF derivatives (v) by
+// launch_spf for at most eight SPFs: out = base + dt_mode (sum_k a.c[k] a.k[k] + last v) on
+// the elements from off on, dt_mode by the element's mode.  Not wanted with on = 0.
+struct SpfStage {
+  int on;
+  cplx* out;
+  const cplx* base;
+  StageArgs a;
+  double last;
+  const double* dt_mode;
+  const unsigned char* elem_mode;
+  long long off;
+};
+// part: 128 complex per tile (scratch); returns the number of launches
+int launch_spf(const SpfDesc* d_descs, int ndesc, long long ntiles, int maxn, const SpfStep* d_steps,
+               const HoleLaunch& holes, cplx* part, cplx* out, cplx der_factor, int* d_status, cudaStream_t st,
+               const SpfStage& stage = SpfStage{});
+// SPF Cash-Karp or Dormand-Prince ends: y5 = base + dt_mode sum_k c5_k k_k, y4 likewise, and
+// diff = y5 - y4
+void launch_rk_end(cplx* y5, cplx* diff, const cplx* base, const StageArgs& a, const double* c4, const double* dt_mode,
+                   const unsigned char* elem_mode, long long off, long long n, cudaStream_t st);
 // FP64 accuracy as exact digit products on the tensor cores (fixed.cu); launched by
 // launch_prod / launch_hole
 void launch_prod_fx(const ProdDesc* d_descs, int ndesc, long long nblocks, int maxn, cudaStream_t st, int persist);
@@ -268,8 +289,6 @@ int launch_h1(const H1Launch& b, bool with_h, cudaStream_t st, const MatSumDesc*
               const MatSumSrc* srcs = nullptr);
 void launch_reginv(const RegInvDesc* d_descs, int ndesc, const MFOp* d_ops, int* d_status, cudaStream_t st);
 // holes: the contractions phi^H phi and phi^H dphi of every block (Y null: at yoff of out)
-void launch_spf(const SpfDesc* d_descs, int ndesc, long long ntiles, int maxn, const SpfStep* d_steps,
-                const HoleLaunch& holes, cplx* out, cplx der_factor, int* d_status, cudaStream_t st);
 // prec 1: FP32 accumulation, else FP64
 // A sum over a whole launch fused into a streaming kernel: v the vector to dot
 // with (termsum: <v|out>; Lanczos axpy: any non-null v requests ||Kn||^2), partial

@@ -1,9 +1,13 @@
 // SPF derivatives of the grid modes (derivatives.f90:94-153) for sm_103a: exact digit
-// products on the tensor cores (fixed.cuh) for the operator sum and the projection,
-// FP64 for the small solve.  Three launches over all (mode, state) blocks:
-//  (1) spf_drive_kernel: dphi = f sum_k ophi_k rhom1MF_k^T, 64 grid rows per CTA;
-//  (2) the contractions phi^H phi and phi^H dphi (fixed.cu);
-//  (3) spf_project_kernel: solve (phi^H phi) X = phi^H dphi (zposv 'U'), dphi -= phi X.
+// products on the tensor cores (fixed.cuh) for the operator sum and the contractions,
+// FP64 for the small solve:
+//  (1) dphi = f sum_k ophi_k rhom1MF_k^T, 64 grid rows per CTA;
+//  (2) the contractions phi^H phi and phi^H dphi;
+//  (3) solve (phi^H phi) X = phi^H dphi (zposv 'U'), dphi -= phi X.
+// Up to eight SPFs a CTA contracts its own rows after (1), from shared memory; modes of
+// at most 64 grid points then go through (3) in the same CTA, one launch in all, larger
+// ones through a second launch that adds the CTAs' contractions.  More SPFs: (2) is the
+// contraction kernel (fixed.cu), three launches.
 #include "kernels.cuh"
 #include "fixed.cuh"
 
@@ -206,13 +210,12 @@ __device__ __forceinline__ double newton_rcp(double d) {
 
 // (phi^H phi) X = phi^H dphi by Gauss-Jordan elimination of [S | O] without pivoting,
 // which is stable for the Hermitian positive definite S.  Pivots are real; a thread
-// holds EPT elements in registers, and per pivot one column and one row pass through
+// holds EPT elements of get(row, column) in registers, and per pivot one column and one row pass through
 // shared memory (two buffers, one barrier).  X transposed into Xt[j + n k] = X(k, j).
 // Returns false at a pivot that is not positive.
-template <int EPT>
-__device__ __forceinline__ bool solve_elimination(const SpfDesc& d, cplx (*colb)[MAXN_SPF], cplx (*rowb)[2 * MAXN_SPF],
+template <int EPT, typename Get>
+__device__ __forceinline__ bool solve_elimination(int n, Get&& get, cplx (*colb)[MAXN_SPF], cplx (*rowb)[2 * MAXN_SPF],
                                                   cplx* Xt) {
-  const int n = d.n;
   cplx a[EPT];
   int ei[EPT], ec[EPT];   // the element's row and column (column -1: none)
 #pragma unroll
@@ -224,7 +227,7 @@ __device__ __forceinline__ bool solve_elimination(const SpfDesc& d, cplx (*colb)
     ec[q] = c < 2 * n ? c : -1;
     if (ec[q] < 0) continue;
     // the contraction's upper triangle is authoritative
-    a[q] = c < n ? (i <= c ? d.S[i + n * c] : cconj(d.S[c + n * i])) : d.O[i + n * (c - n)];
+    a[q] = c < n ? (i <= c ? get(i, c) : cconj(get(c, i))) : get(i, c);
     if (c == 0) colb[0][i] = a[q];
     if (i == 0) rowb[0][c] = a[q];
   }
@@ -258,36 +261,227 @@ __device__ __forceinline__ bool solve_elimination(const SpfDesc& d, cplx (*colb)
   return ok;
 }
 
-// Every CTA solves for itself (64 rows each: one or two CTAs per (mode, state) and SM
-// at the sizes met), then subtracts its rows of phi X; its rows of phi and dphi are
-// copied meanwhile.  Up to eight SPFs the product is 8 n FP64 instructions a row and
-// column pair of warps, less than cutting and joining digits.
-__global__ void __launch_bounds__(SPF_THREADS) spf_project8_kernel(const SpfDesc* __restrict__ descs, int ndesc,
-                                                                   cplx* __restrict__ out, int* status) {
-  __shared__ cplx colb[2][MAXN_SPF], rowb[2][2 * MAXN_SPF], Xt[64], phs[8 * SPF_ROWS], dph[8 * SPF_ROWS];
-  const SpfDesc& d = descs[warp_find_desc(descs, ndesc, (long long)blockIdx.x)];
-  const int n = d.n, G = d.G, tile = (int)(blockIdx.x - d.block_start), row0 = tile * SPF_ROWS;
-  const int row = threadIdx.x & (SPF_ROWS - 1);
-  const bool in = row0 + row < G;
-  cplx* o = out + d.out_offset + row0 + row;
-  const cplx* phi = d.phi + row0 + row;
-  for (int j = threadIdx.x / SPF_ROWS; j < n && in; j += SPF_THREADS / SPF_ROWS) {
-    copy_async16(phs + row + SPF_ROWS * j, phi + (long long)G * j);
-    copy_async16(dph + row + SPF_ROWS * j, o + (long long)G * j);
+// Shared memory of the forms for n <= 8; in the first launch it takes the place of the
+// matrix digits once these are read.
+struct SpfSmall {
+  cplx phs[8][SPF_PITCH], dph[8][SPF_PITCH];   // the CTA's rows of phi and dphi, zeros beyond G and n
+  cplx red[4][128];                            // the warps' phi^H phi, then phi^H dphi ([j1 + 8 j2] each)
+  cplx so[128];
+  cplx colb[2][MAXN_SPF], rowb[2][2 * MAXN_SPF], Xt[64];
+};
+static_assert(sizeof(SpfSmall) <= sizeof(RowShared::W), "fits in the place of the digits");
+
+// so = (phi^H phi, phi^H dphi) of the CTA's 64 rows: a warp takes 16 rows as in the
+// contraction kernel for n <= 8 (seven digits, weights above 2^-64), the four warps'
+// sums are added in order.
+__device__ __forceinline__ void contract_rows(SpfSmall& T) {
+  constexpr int NS = 7, ND = 8;
+  const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5, g = lane >> 2, q = lane & 3;
+  const int r0 = 16 * warp + 2 * q;
+  cplx x[4], y[4];
+  unsigned mx = 0u, my = 0u;
+#pragma unroll
+  for (int f = 0; f < 4; ++f) {
+    x[f] = T.phs[g][r0 + (f & 1) + 8 * (f >> 1)];
+    y[f] = T.dph[g][r0 + (f & 1) + 8 * (f >> 1)];
+    mx = max(mx, fx_mag(x[f]));
+    my = max(my, fx_mag(y[f]));
   }
-  const bool ok = solve_elimination<1>(d, colb, rowb, Xt);
-  if (threadIdx.x == 0 && tile == 0 && !ok) atomicOr(status, DEVST_CHOL_FAIL);
-  copy_async_wait();
+#pragma unroll
+  for (int o = 1; o < 4; o <<= 1) {
+    mx = max(mx, __shfl_xor_sync(0xffffffffu, mx, o));
+    my = max(my, __shfl_xor_sync(0xffffffffu, my, o));
+  }
+  const unsigned ex = fx_ebits(mx), ey = fx_ebits(my);
+  unsigned A[NS][4];   // (re, im) of fibres 2 q, 2 q + 1, then of 2 q + 8, 2 q + 9
+#pragma unroll
+  for (int h = 0; h < 2; ++h) {
+    unsigned s[NS];
+    fx_digits<NS>(x[2 * h].x, x[2 * h + 1].x, ex, ex, s);
+#pragma unroll
+    for (int k = 0; k < NS; ++k) A[k][2 * h] = s[k];
+    fx_digits<NS>(x[2 * h].y, x[2 * h + 1].y, ex, ex, s);
+#pragma unroll
+    for (int k = 0; k < NS; ++k) A[k][2 * h + 1] = s[k];
+  }
+#pragma unroll
+  for (int which = 0; which < 2; ++which) {
+    unsigned B[NS][4];
+    const unsigned eb = which ? ey : ex;
+    if (which) {
+#pragma unroll
+      for (int h = 0; h < 2; ++h) {
+        unsigned s[NS];
+        fx_digits<NS>(y[2 * h].x, y[2 * h + 1].x, ey, ey, s);
+#pragma unroll
+        for (int k = 0; k < NS; ++k) B[k][2 * h] = s[k];
+        fx_digits<NS>(y[2 * h].y, y[2 * h + 1].y, ey, ey, s);
+#pragma unroll
+        for (int k = 0; k < NS; ++k) B[k][2 * h + 1] = s[k];
+      }
+    } else {
+#pragma unroll
+      for (int k = 0; k < NS; ++k)
+#pragma unroll
+        for (int h = 0; h < 4; ++h) B[k][h] = A[k][h];
+    }
+    float cr[ND][4], ci[ND][4];
+#pragma unroll
+    for (int i = 0; i < NS; ++i)
+#pragma unroll
+      for (int j = 0; j < NS && j + i < ND; ++j) {
+        const bool first = i == 0 || (i == 1 && j == NS - 1);   // the first product of weight i + j
+        fx_mma16(cr[i + j], A[i], B[j][0], B[j][2], first);
+        fx_mma16(ci[i + j], A[i], B[j][1], B[j][3], first);
+      }
+    const unsigned e2[2] = {__shfl_sync(0xffffffffu, eb, 8 * q), __shfl_sync(0xffffffffu, eb, 8 * q + 4)};
+#pragma unroll
+    for (int i = 0; i < 2; ++i) {
+      const long long re = fx_join_wide<ND, 1>(cr, i) + fx_join_wide<ND, 1>(ci, 2 + i);
+      const long long im = fx_join_wide<ND, 1>(ci, i) - fx_join_wide<ND, 1>(cr, 2 + i);
+      const int es = (int)(ex + e2[i]) - ((2044 + 12 + 43) << 20);
+      T.red[warp][64 * which + g + 8 * (2 * q + i)] = mkc(fx_double(re, es), fx_double(im, es));
+    }
+  }
+  const bool slow = __syncthreads_or(!fx_ok(mx) || !fx_ok(my));
+  cplx v = mkc(0.0, 0.0);
+  if (slow) {
+    const cplx* a = T.phs[tid & 7];
+    const cplx* b = tid < 64 ? T.phs[tid >> 3] : T.dph[(tid - 64) >> 3];
+    for (int r = 0; r < SPF_ROWS; ++r) cfma_conj(v, a[r], b[r]);
+  } else {
+#pragma unroll
+    for (int w = 0; w < 4; ++w) v = cadd(v, T.red[w][tid]);
+  }
+  T.so[tid] = v;
+}
+
+// The next Runge-Kutta stage's input at element e: base + dt (sum_k c_k k_k + last v);
+// stage_sum is the part that does not need v.
+__device__ __forceinline__ cplx stage_sum(const SpfStage& g, long long e) {
+  cplx s = mkc(0, 0);
+  for (int k = 0; k < g.a.nk; ++k) {
+    const cplx v = g.a.k[k][e];
+    s.x = fma(g.a.c[k], v.x, s.x);
+    s.y = fma(g.a.c[k], v.y, s.y);
+  }
+  return s;
+}
+
+// Solve from T.so and subtract the CTA's rows of phi X; with g.on also the next stage's
+// input (the CTA's rows of phi are in shared memory by now, so it may replace them).  A
+// thread has row threadIdx.x % 64 of columns threadIdx.x / 64, + 2, ...  Eight FP64
+// instructions a row and column pair of warps, less than cutting and joining digits.
+__device__ __forceinline__ bool solve_project(SpfSmall& T, const SpfDesc& d, int row0, cplx* o, const SpfStage& g) {
+  const int n = d.n, G = d.G, row = threadIdx.x & (SPF_ROWS - 1), jr = threadIdx.x / SPF_ROWS;
+  const bool in = row0 + row < G;
+  cplx ss[4], bs[4];
+  double dt = 0.0;
+  if (g.on) {
+    dt = g.dt_mode[g.elem_mode[d.out_offset - g.off]];
+#pragma unroll
+    for (int i = 0; i < 4; ++i) {
+      ss[i] = bs[i] = mkc(0.0, 0.0);
+      if (in && jr + 2 * i < n) {
+        const long long e = d.out_offset + row0 + row + (long long)G * (jr + 2 * i);
+        ss[i] = stage_sum(g, e);
+        bs[i] = g.base[e];
+      }
+    }
+  }
+  const bool ok = solve_elimination<1>(
+      n, [&](int i, int c) { return c < n ? T.so[i + 8 * c] : T.so[64 + i + 8 * (c - n)]; }, T.colb, T.rowb, T.Xt);
   __syncthreads();
-  for (int j = threadIdx.x / SPF_ROWS; j < n && in; j += SPF_THREADS / SPF_ROWS) {
-    cplx v = dph[row + SPF_ROWS * j];
+#pragma unroll
+  for (int i = 0; i < 4; ++i) {
+    const int j = jr + 2 * i;
+    if (!in || j >= n) break;
+    cplx v = T.dph[j][row];
     for (int k = 0; k < n; ++k) {
-      const cplx x = phs[row + SPF_ROWS * k], c = Xt[j + n * k];
+      const cplx x = T.phs[k][row], c = T.Xt[j + n * k];
       v.x = fma(-x.x, c.x, fma(x.y, c.y, v.x));
       v.y = fma(-x.x, c.y, fma(-x.y, c.x, v.y));
     }
-    o[(long long)G * j] = v;
+    const long long e = row0 + row + (long long)G * j;
+    o[e] = v;
+    if (g.on) {
+      const cplx s = mkc(fma(g.last, v.x, ss[i].x), fma(g.last, v.y, ss[i].y));
+      g.out[d.out_offset + e] = mkc(fma(dt, s.x, bs[i].x), fma(dt, s.y, bs[i].y));
+    }
   }
+  return ok;
+}
+
+// n <= 8.  ONE: every mode has at most 64 grid points, the CTA goes on to the solve.
+// Otherwise dphi goes to out and the contractions of the CTA's rows to part.
+template <bool ONE>
+__global__ void __launch_bounds__(SPF_THREADS) spf_drive8_kernel(const SpfDesc* __restrict__ descs, int ndesc,
+                                                                 const SpfStep* __restrict__ steps, cplx* out, cplx der,
+                                                                 cplx* __restrict__ part, int* status, SpfStage g) {
+  extern __shared__ __align__(16) unsigned char spf_sm[];
+  RowShared& S = *reinterpret_cast<RowShared*>(spf_sm);
+  SpfSmall& T = *reinterpret_cast<SpfSmall*>(&S.W);
+  __shared__ SpfStep st[SPF_CHUNK];
+  const SpfDesc& d = descs[warp_find_desc(descs, ndesc, (long long)blockIdx.x)];
+  const SpfStep* gst = steps + d.step_first;
+  const int nsteps = d.step_count, n = d.n;
+  // one chunk's steps in shared memory; longer lists are read where they are
+  const bool local = nsteps <= SPF_CHUNK;
+  if (local && (int)threadIdx.x < nsteps) st[threadIdx.x] = gst[threadIdx.x];
+  __syncthreads();
+  cplx* o = out + d.out_offset;
+  const int G = d.G, row0 = (int)(blockIdx.x - d.block_start) * SPF_ROWS;
+  const int row = threadIdx.x & (SPF_ROWS - 1), jr = threadIdx.x / SPF_ROWS;
+  const bool rot = der.x == 0.0 && der.y == -1.0, neg = der.x == -1.0 && der.y == 0.0;
+  auto step = [&](int s) { return local ? st[s] : gst[s]; };
+  stage_rows(S, 0, min(SPF_CHUNK, nsteps), step, G, row0);
+  cplx ph[4];
+#pragma unroll
+  for (int i = 0; i < 4; ++i)
+    ph[i] = row0 + row < G && jr + 2 * i < n ? d.phi[row0 + row + (long long)G * (jr + 2 * i)] : mkc(0.0, 0.0);
+  row_products(S, nsteps, step, n, G, row0, [&](int r, int j1, cplx v) {
+    const cplx w = rot ? mkc(v.y, -v.x) : (neg ? mkc(-v.x, -v.y) : cmul(der, v));
+    T.dph[j1][r - row0] = w;
+    if (!ONE) o[r + (long long)G * j1] = w;
+  });
+#pragma unroll
+  for (int i = 0; i < 4; ++i) {
+    T.phs[jr + 2 * i][row] = ph[i];
+    if (row0 + row >= G || jr + 2 * i >= n) T.dph[jr + 2 * i][row] = mkc(0.0, 0.0);
+  }
+  __syncthreads();
+  contract_rows(T);
+  if (!ONE) {
+    part[128LL * blockIdx.x + threadIdx.x] = T.so[threadIdx.x];
+    return;
+  }
+  __syncthreads();
+  if (!solve_project(T, d, row0, o, g) && threadIdx.x == 0) atomicOr(status, DEVST_CHOL_FAIL);
+}
+
+// n <= 8, several CTAs per mode: every CTA adds its mode's contractions and solves for
+// itself; its rows of phi and dphi are copied meanwhile.
+__global__ void __launch_bounds__(SPF_THREADS) spf_project8_kernel(const SpfDesc* __restrict__ descs, int ndesc,
+                                                                   cplx* out, const cplx* __restrict__ part,
+                                                                   int* status, SpfStage g) {
+  __shared__ SpfSmall T;
+  const SpfDesc& d = descs[warp_find_desc(descs, ndesc, (long long)blockIdx.x)];
+  const int n = d.n, G = d.G, tile = (int)(blockIdx.x - d.block_start), row0 = tile * SPF_ROWS;
+  const int row = threadIdx.x & (SPF_ROWS - 1);
+  cplx* o = out + d.out_offset;
+  for (int j = threadIdx.x / SPF_ROWS; j < n && row0 + row < G; j += SPF_THREADS / SPF_ROWS) {
+    copy_async16(&T.phs[j][row], d.phi + row0 + row + (long long)G * j);
+    copy_async16(&T.dph[j][row], o + row0 + row + (long long)G * j);
+  }
+  cplx v = mkc(0.0, 0.0);
+  const cplx* p = part + 128LL * d.block_start + threadIdx.x;
+  const int ntile = (G + SPF_ROWS - 1) / SPF_ROWS;
+#pragma unroll 4
+  for (int t = 0; t < ntile; ++t) v = cadd(v, p[128LL * t]);
+  T.so[threadIdx.x] = v;
+  copy_async_wait();
+  __syncthreads();
+  if (!solve_project(T, d, row0, o, g) && threadIdx.x == 0 && tile == 0) atomicOr(status, DEVST_CHOL_FAIL);
 }
 __global__ void __launch_bounds__(SPF_THREADS) spf_project_kernel(const SpfDesc* __restrict__ descs, int ndesc,
                                                                   cplx* __restrict__ out, int* status) {
@@ -304,8 +498,9 @@ __global__ void __launch_bounds__(SPF_THREADS) spf_project_kernel(const SpfDesc*
   stage_rows(S, 0, (n + 7) / 8, step, G, row0);
   for (int e = threadIdx.x; e < n * SPF_ROWS; e += SPF_THREADS)
     if (row0 + (e & (SPF_ROWS - 1)) < G) copy_async16(dph + e, o + row0 + (e & (SPF_ROWS - 1)) + (long long)G * (e / SPF_ROWS));
-  const bool ok = n <= 8 ? solve_elimination<1>(d, colb, rowb, Xt)
-                         : (n <= 16 ? solve_elimination<4>(d, colb, rowb, Xt) : solve_elimination<16>(d, colb, rowb, Xt));
+  auto get = [&](int i, int c) { return c < n ? d.S[i + n * c] : d.O[i + n * (c - n)]; };
+  const bool ok = n <= 8 ? solve_elimination<1>(n, get, colb, rowb, Xt)
+                         : (n <= 16 ? solve_elimination<4>(n, get, colb, rowb, Xt) : solve_elimination<16>(n, get, colb, rowb, Xt));
   if (threadIdx.x == 0 && tile == 0 && !ok) atomicOr(status, DEVST_CHOL_FAIL);
   __syncthreads();
   row_products(S, (n + 7) / 8, step, n, G, row0, [&](int row, int j1, cplx v) {
@@ -313,18 +508,31 @@ __global__ void __launch_bounds__(SPF_THREADS) spf_project_kernel(const SpfDesc*
   });
 }
 
-void launch_spf(const SpfDesc* d_descs, int ndesc, long long ntiles, int maxn, const SpfStep* d_steps,
-                const HoleLaunch& holes, cplx* out, cplx der_factor, int* d_status, cudaStream_t st) {
-  if (ndesc <= 0) return;
+int launch_spf(const SpfDesc* d_descs, int ndesc, long long ntiles, int maxn, const SpfStep* d_steps,
+               const HoleLaunch& holes, cplx* part, cplx* out, cplx der_factor, int* d_status, cudaStream_t st,
+               const SpfStage& stage) {
+  if (ndesc <= 0) return 0;
   const int smem = (int)sizeof(RowShared), smem_x = smem + (int)sizeof(cplx) * maxn * (maxn + SPF_ROWS);
   static const cudaError_t configured = [] {
     constexpr int most = (int)(sizeof(RowShared) + sizeof(cplx) * MAXN_SPF * (MAXN_SPF + SPF_ROWS));
     cudaFuncSetAttribute(spf_drive_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, most);
+    cudaFuncSetAttribute(spf_drive8_kernel<true>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)sizeof(RowShared));
+    cudaFuncSetAttribute(spf_drive8_kernel<false>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)sizeof(RowShared));
     return cudaFuncSetAttribute(spf_project_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, most);
   }();
   (void)configured;
-  spf_drive_kernel<<<(unsigned)ntiles, SPF_THREADS, smem, st>>>(d_descs, ndesc, d_steps, out, der_factor);
+  const unsigned nb = (unsigned)ntiles;
+  if (maxn <= 8 && ntiles == ndesc) {
+    spf_drive8_kernel<true><<<nb, SPF_THREADS, smem, st>>>(d_descs, ndesc, d_steps, out, der_factor, part, d_status, stage);
+    return 1;
+  }
+  if (maxn <= 8) {
+    spf_drive8_kernel<false><<<nb, SPF_THREADS, smem, st>>>(d_descs, ndesc, d_steps, out, der_factor, part, d_status, stage);
+    spf_project8_kernel<<<nb, SPF_THREADS, 0, st>>>(d_descs, ndesc, out, part, d_status, stage);
+    return 2;
+  }
+  spf_drive_kernel<<<nb, SPF_THREADS, smem, st>>>(d_descs, ndesc, d_steps, out, der_factor);
   launch_hole_fx(holes, st, 0, out);
-  if (maxn <= 8) spf_project8_kernel<<<(unsigned)ntiles, SPF_THREADS, 0, st>>>(d_descs, ndesc, out, d_status);
-  else spf_project_kernel<<<(unsigned)ntiles, SPF_THREADS, smem_x, st>>>(d_descs, ndesc, out, d_status);
+  spf_project_kernel<<<nb, SPF_THREADS, smem_x, st>>>(d_descs, ndesc, out, d_status);
+  return 3;
 }
