@@ -11,7 +11,7 @@
 #include "kernels.cuh"
 #include "fixed.cuh"
 
-#define SPF_THREADS 128
+#define SPF_THREADS 256
 #define SPF_NS 8
 #define SPF_CHUNK 9      // steps of eight j2 between flushes: 9 x 16 x 7 x 2^14 < 2^24
 
@@ -20,7 +20,13 @@
 // Shared operands of row_products.
 struct RowShared {
   cplx x[SPF_CHUNK][8][SPF_PITCH];         // the CTA's rows of a chunk of steps
-  uint2 W[SPF_CHUNK][2][SPF_NS][32];       // digits of eight columns of the matrix (j2 = q and q + 4)
+  union {
+    uint2 W[SPF_CHUNK][2][SPF_NS][32];     // digits of eight columns of the matrix (j2 = q and q + 4)
+    struct {
+      unsigned char small[sizeof(uint2) * SPF_CHUNK * 2 * SPF_NS * 32 - 8192];
+      cplx other[4][2][2][32];             // the second warps' sums, once W is read
+    };
+  };
   unsigned colmag[MAXN_SPF];
 };
 
@@ -47,16 +53,19 @@ __device__ __forceinline__ void stage_rows(RowShared& S, int s0, int ns, Step&& 
 }
 
 // The CTA's rows row0 .. row0 + 63 of sum_steps sum_j x(row, j) rm(j1, j) for all
-// j1 < n: a warp owns 16 rows (the MMA's rows), its columns the (re, im) of four j1; a row
+// j1 < n: warps w and w + 4 own 16 rows (the MMA's rows) and every second step, the
+// columns are the (re, im) of four j1; a row
 // has one exponent per chunk of steps, a column j1 of the matrices another.  step(s)
 // returns the s-th step (up to eight j); the first chunk is staged already.
-// put(row, j1, value) takes the results; rows from G on are skipped.  Operands outside
+// put(row, j1, value) takes the results (warps 0 - 3); rows from G on are skipped.  The
+// matrices are cut while the rows are on their way.  Operands outside
 // the exponent range are multiplied in FP64.
 template <typename Step, typename Put>
 __device__ __forceinline__ void row_products(RowShared& S, int nsteps, Step&& step, int n, int G, int row0, Put&& put) {
   constexpr int NS = SPF_NS;
   const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5, g = lane >> 2, q = lane & 3;
-  const int lr = 16 * warp + g;   // the lane's rows: lr, lr + 8
+  const int half = warp >> 2, lr = 16 * (warp & 3) + g;   // the lane's rows: lr, lr + 8
+  auto& other = S.other;
   for (int j0 = 0; j0 < n; j0 += 8) {   // eight outputs per pass
     cplx sum[2][2];                     // [group of four j1][row]
     for (int s0 = 0; s0 < nsteps; s0 += SPF_CHUNK) {
@@ -66,21 +75,7 @@ __device__ __forceinline__ void row_products(RowShared& S, int nsteps, Step&& st
         stage_rows(S, s0, ns, step, G, row0);
       }
       if (tid < 8) S.colmag[tid] = 0u;
-      copy_async_wait();
       __syncthreads();
-      unsigned mag[2] = {0u, 0u};
-      for (int s = 0; s < ns; ++s)
-#pragma unroll
-        for (int f = 0; f < 2; ++f)
-          mag[f] = max(mag[f], max(fx_mag(S.x[s][q][lr + 8 * f]), fx_mag(S.x[s][q + 4][lr + 8 * f])));
-      bool bad = false;
-#pragma unroll
-      for (int f = 0; f < 2; ++f) {
-        mag[f] = max(mag[f], __shfl_xor_sync(0xffffffffu, mag[f], 1));
-        mag[f] = max(mag[f], __shfl_xor_sync(0xffffffffu, mag[f], 2));
-        bad = bad || !fx_ok(mag[f]);
-      }
-      const unsigned eb[2] = {fx_ebits(mag[0]), fx_ebits(mag[1])};
       const int nc = min(8, n - j0);
       for (int e = tid; e < 64 * ns; e += SPF_THREADS) {   // (step, j, j1)
         const int j1 = e & 7, j = (e >> 3) & 7;
@@ -88,8 +83,8 @@ __device__ __forceinline__ void row_products(RowShared& S, int nsteps, Step&& st
         if (j1 < nc && j < st.nj) atomicMax(&S.colmag[j1], fx_mag(st.rm[j0 + j1 + n * j]));
       }
       __syncthreads();
-      if (tid < nc) bad = bad || !fx_ok(S.colmag[tid]);
-      for (int w = warp; w < 2 * ns; w += 4) {
+      bool bad = tid < nc && !fx_ok(S.colmag[tid]);
+      for (int w = warp; w < 2 * ns; w += SPF_THREADS / 32) {
         const int t = w & 1, s = w >> 1, j1 = 4 * t + (g >> 1);
         if (4 * t >= nc) continue;
         const SpfStep st = step(s0 + s);
@@ -106,6 +101,20 @@ __device__ __forceinline__ void row_products(RowShared& S, int nsteps, Step&& st
           S.W[s][t][i][lane] = make_uint2(w0, w1);
         }
       }
+      copy_async_wait();
+      __syncthreads();
+      unsigned mag[2] = {0u, 0u};
+      for (int s = 0; s < ns; ++s)
+#pragma unroll
+        for (int f = 0; f < 2; ++f)
+          mag[f] = max(mag[f], max(fx_mag(S.x[s][q][lr + 8 * f]), fx_mag(S.x[s][q + 4][lr + 8 * f])));
+#pragma unroll
+      for (int f = 0; f < 2; ++f) {
+        mag[f] = max(mag[f], __shfl_xor_sync(0xffffffffu, mag[f], 1));
+        mag[f] = max(mag[f], __shfl_xor_sync(0xffffffffu, mag[f], 2));
+        bad = bad || !fx_ok(mag[f]);
+      }
+      const unsigned eb[2] = {fx_ebits(mag[0]), fx_ebits(mag[1])};
       if (__syncthreads_or(bad)) {   // the pass in FP64
         for (int e = tid; e < SPF_ROWS * nc; e += SPF_THREADS) {
           const int row = row0 + (e & (SPF_ROWS - 1)), j1 = j0 + e / SPF_ROWS;
@@ -127,7 +136,7 @@ __device__ __forceinline__ void row_products(RowShared& S, int nsteps, Step&& st
           for (int i = 0; i < NS; ++i)
 #pragma unroll
             for (int k = 0; k < 4; ++k) c[t][i][k] = 0.f;
-        for (int s = 0; s < ns; ++s) {
+        for (int s = half; s < ns; s += 2) {
           unsigned A[NS][4];
 #pragma unroll
           for (int f = 0; f < 2; ++f)
@@ -167,12 +176,19 @@ __device__ __forceinline__ void row_products(RowShared& S, int nsteps, Step&& st
       }
       __syncthreads();   // colmag and W are read
     }
+    if (half)
 #pragma unroll
-    for (int t = 0; t < 2; ++t)
+      for (int t = 0; t < 2; ++t)
 #pragma unroll
-      for (int f = 0; f < 2; ++f)
-        if (j0 + 4 * t + q < n && row0 + lr + 8 * f < G)
-          put(row0 + lr + 8 * f, j0 + 4 * t + q, nsteps ? sum[t][f] : mkc(0, 0));
+        for (int f = 0; f < 2; ++f) other[warp & 3][t][f][lane] = nsteps ? sum[t][f] : mkc(0, 0);
+    __syncthreads();
+    if (!half)
+#pragma unroll
+      for (int t = 0; t < 2; ++t)
+#pragma unroll
+        for (int f = 0; f < 2; ++f)
+          if (j0 + 4 * t + q < n && row0 + lr + 8 * f < G)
+            put(row0 + lr + 8 * f, j0 + 4 * t + q, nsteps ? cadd(sum[t][f], other[warp & 3][t][f][lane]) : mkc(0, 0));
   next_pass:;
   }
 }
@@ -265,25 +281,27 @@ __device__ __forceinline__ bool solve_elimination(int n, Get&& get, cplx (*colb)
 // matrix digits once these are read.
 struct SpfSmall {
   cplx phs[8][SPF_PITCH], dph[8][SPF_PITCH];   // the CTA's rows of phi and dphi, zeros beyond G and n
-  cplx red[4][128];                            // the warps' phi^H phi, then phi^H dphi ([j1 + 8 j2] each)
-  cplx so[128];
+  cplx so[128];                                // phi^H phi, then phi^H dphi ([j1 + 8 j2] each)
   cplx colb[2][MAXN_SPF], rowb[2][2 * MAXN_SPF], Xt[64];
+  cplx red[4][128];                            // the warps' share of so
 };
-static_assert(sizeof(SpfSmall) <= sizeof(RowShared::W), "fits in the place of the digits");
+static_assert(sizeof(SpfSmall) <= sizeof(RowShared::W) && offsetof(SpfSmall, red) <= sizeof(RowShared::small),
+              "takes the place of the digits, red alone that of the second warps' sums");
 
-// so = (phi^H phi, phi^H dphi) of the CTA's 64 rows: a warp takes 16 rows as in the
-// contraction kernel for n <= 8 (seven digits, weights above 2^-64), the four warps'
-// sums are added in order.
+// so = (phi^H phi, phi^H dphi) of the CTA's 64 rows: warp w takes 16 rows of the first
+// as in the contraction kernel for n <= 8 (seven digits, weights above 2^-64), warp w + 4
+// of the second; the four warps' sums are added in order.
 __device__ __forceinline__ void contract_rows(SpfSmall& T) {
   constexpr int NS = 7, ND = 8;
   const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5, g = lane >> 2, q = lane & 3;
-  const int r0 = 16 * warp + 2 * q;
-  cplx x[4], y[4];
+  const int which = warp >> 2, r0 = 16 * (warp & 3) + 2 * q;
+  const cplx (*Y)[SPF_PITCH] = which ? T.dph : T.phs;
   unsigned mx = 0u, my = 0u;
+  cplx x[4], y[4];
 #pragma unroll
   for (int f = 0; f < 4; ++f) {
     x[f] = T.phs[g][r0 + (f & 1) + 8 * (f >> 1)];
-    y[f] = T.dph[g][r0 + (f & 1) + 8 * (f >> 1)];
+    y[f] = Y[g][r0 + (f & 1) + 8 * (f >> 1)];
     mx = max(mx, fx_mag(x[f]));
     my = max(my, fx_mag(y[f]));
   }
@@ -293,7 +311,7 @@ __device__ __forceinline__ void contract_rows(SpfSmall& T) {
     my = max(my, __shfl_xor_sync(0xffffffffu, my, o));
   }
   const unsigned ex = fx_ebits(mx), ey = fx_ebits(my);
-  unsigned A[NS][4];   // (re, im) of fibres 2 q, 2 q + 1, then of 2 q + 8, 2 q + 9
+  unsigned A[NS][4], B[NS][4];   // (re, im) of fibres 2 q, 2 q + 1, then of 2 q + 8, 2 q + 9
 #pragma unroll
   for (int h = 0; h < 2; ++h) {
     unsigned s[NS];
@@ -303,47 +321,32 @@ __device__ __forceinline__ void contract_rows(SpfSmall& T) {
     fx_digits<NS>(x[2 * h].y, x[2 * h + 1].y, ex, ex, s);
 #pragma unroll
     for (int k = 0; k < NS; ++k) A[k][2 * h + 1] = s[k];
+    fx_digits<NS>(y[2 * h].x, y[2 * h + 1].x, ey, ey, s);
+#pragma unroll
+    for (int k = 0; k < NS; ++k) B[k][2 * h] = s[k];
+    fx_digits<NS>(y[2 * h].y, y[2 * h + 1].y, ey, ey, s);
+#pragma unroll
+    for (int k = 0; k < NS; ++k) B[k][2 * h + 1] = s[k];
   }
+  float cr[ND][4], ci[ND][4];
 #pragma unroll
-  for (int which = 0; which < 2; ++which) {
-    unsigned B[NS][4];
-    const unsigned eb = which ? ey : ex;
-    if (which) {
+  for (int i = 0; i < NS; ++i)
 #pragma unroll
-      for (int h = 0; h < 2; ++h) {
-        unsigned s[NS];
-        fx_digits<NS>(y[2 * h].x, y[2 * h + 1].x, ey, ey, s);
-#pragma unroll
-        for (int k = 0; k < NS; ++k) B[k][2 * h] = s[k];
-        fx_digits<NS>(y[2 * h].y, y[2 * h + 1].y, ey, ey, s);
-#pragma unroll
-        for (int k = 0; k < NS; ++k) B[k][2 * h + 1] = s[k];
-      }
-    } else {
-#pragma unroll
-      for (int k = 0; k < NS; ++k)
-#pragma unroll
-        for (int h = 0; h < 4; ++h) B[k][h] = A[k][h];
+    for (int j = 0; j < NS && j + i < ND; ++j) {
+      const bool first = i == 0 || (i == 1 && j == NS - 1);   // the first product of weight i + j
+      fx_mma16(cr[i + j], A[i], B[j][0], B[j][2], first);
+      fx_mma16(ci[i + j], A[i], B[j][1], B[j][3], first);
     }
-    float cr[ND][4], ci[ND][4];
+  const unsigned e2[2] = {__shfl_sync(0xffffffffu, ey, 8 * q), __shfl_sync(0xffffffffu, ey, 8 * q + 4)};
 #pragma unroll
-    for (int i = 0; i < NS; ++i)
-#pragma unroll
-      for (int j = 0; j < NS && j + i < ND; ++j) {
-        const bool first = i == 0 || (i == 1 && j == NS - 1);   // the first product of weight i + j
-        fx_mma16(cr[i + j], A[i], B[j][0], B[j][2], first);
-        fx_mma16(ci[i + j], A[i], B[j][1], B[j][3], first);
-      }
-    const unsigned e2[2] = {__shfl_sync(0xffffffffu, eb, 8 * q), __shfl_sync(0xffffffffu, eb, 8 * q + 4)};
-#pragma unroll
-    for (int i = 0; i < 2; ++i) {
-      const long long re = fx_join_wide<ND, 1>(cr, i) + fx_join_wide<ND, 1>(ci, 2 + i);
-      const long long im = fx_join_wide<ND, 1>(ci, i) - fx_join_wide<ND, 1>(cr, 2 + i);
-      const int es = (int)(ex + e2[i]) - ((2044 + 12 + 43) << 20);
-      T.red[warp][64 * which + g + 8 * (2 * q + i)] = mkc(fx_double(re, es), fx_double(im, es));
-    }
+  for (int i = 0; i < 2; ++i) {
+    const long long re = fx_join_wide<ND, 1>(cr, i) + fx_join_wide<ND, 1>(ci, 2 + i);
+    const long long im = fx_join_wide<ND, 1>(ci, i) - fx_join_wide<ND, 1>(cr, 2 + i);
+    const int es = (int)(ex + e2[i]) - ((2044 + 12 + 43) << 20);
+    T.red[warp & 3][64 * which + g + 8 * (2 * q + i)] = mkc(fx_double(re, es), fx_double(im, es));
   }
   const bool slow = __syncthreads_or(!fx_ok(mx) || !fx_ok(my));
+  if (tid >= 128) return;
   cplx v = mkc(0.0, 0.0);
   if (slow) {
     const cplx* a = T.phs[tid & 7];
@@ -370,20 +373,20 @@ __device__ __forceinline__ cplx stage_sum(const SpfStage& g, long long e) {
 
 // Solve from T.so and subtract the CTA's rows of phi X; with g.on also the next stage's
 // input (the CTA's rows of phi are in shared memory by now, so it may replace them).  A
-// thread has row threadIdx.x % 64 of columns threadIdx.x / 64, + 2, ...  Eight FP64
+// thread has row threadIdx.x % 64 of columns threadIdx.x / 64 and + 4.  Eight FP64
 // instructions a row and column pair of warps, less than cutting and joining digits.
 __device__ __forceinline__ bool solve_project(SpfSmall& T, const SpfDesc& d, int row0, cplx* o, const SpfStage& g) {
   const int n = d.n, G = d.G, row = threadIdx.x & (SPF_ROWS - 1), jr = threadIdx.x / SPF_ROWS;
   const bool in = row0 + row < G;
-  cplx ss[4], bs[4];
+  cplx ss[2], bs[2];
   double dt = 0.0;
   if (g.on) {
     dt = g.dt_mode[g.elem_mode[d.out_offset - g.off]];
 #pragma unroll
-    for (int i = 0; i < 4; ++i) {
+    for (int i = 0; i < 2; ++i) {
       ss[i] = bs[i] = mkc(0.0, 0.0);
-      if (in && jr + 2 * i < n) {
-        const long long e = d.out_offset + row0 + row + (long long)G * (jr + 2 * i);
+      if (in && jr + 4 * i < n) {
+        const long long e = d.out_offset + row0 + row + (long long)G * (jr + 4 * i);
         ss[i] = stage_sum(g, e);
         bs[i] = g.base[e];
       }
@@ -393,8 +396,8 @@ __device__ __forceinline__ bool solve_project(SpfSmall& T, const SpfDesc& d, int
       n, [&](int i, int c) { return c < n ? T.so[i + 8 * c] : T.so[64 + i + 8 * (c - n)]; }, T.colb, T.rowb, T.Xt);
   __syncthreads();
 #pragma unroll
-  for (int i = 0; i < 4; ++i) {
-    const int j = jr + 2 * i;
+  for (int i = 0; i < 2; ++i) {
+    const int j = jr + 4 * i;
     if (!in || j >= n) break;
     cplx v = T.dph[j][row];
     for (int k = 0; k < n; ++k) {
@@ -435,24 +438,24 @@ __global__ void __launch_bounds__(SPF_THREADS) spf_drive8_kernel(const SpfDesc* 
   const bool rot = der.x == 0.0 && der.y == -1.0, neg = der.x == -1.0 && der.y == 0.0;
   auto step = [&](int s) { return local ? st[s] : gst[s]; };
   stage_rows(S, 0, min(SPF_CHUNK, nsteps), step, G, row0);
-  cplx ph[4];
+  cplx ph[2];
 #pragma unroll
-  for (int i = 0; i < 4; ++i)
-    ph[i] = row0 + row < G && jr + 2 * i < n ? d.phi[row0 + row + (long long)G * (jr + 2 * i)] : mkc(0.0, 0.0);
+  for (int i = 0; i < 2; ++i)
+    ph[i] = row0 + row < G && jr + 4 * i < n ? d.phi[row0 + row + (long long)G * (jr + 4 * i)] : mkc(0.0, 0.0);
   row_products(S, nsteps, step, n, G, row0, [&](int r, int j1, cplx v) {
     const cplx w = rot ? mkc(v.y, -v.x) : (neg ? mkc(-v.x, -v.y) : cmul(der, v));
     T.dph[j1][r - row0] = w;
     if (!ONE) o[r + (long long)G * j1] = w;
   });
 #pragma unroll
-  for (int i = 0; i < 4; ++i) {
-    T.phs[jr + 2 * i][row] = ph[i];
-    if (row0 + row >= G || jr + 2 * i >= n) T.dph[jr + 2 * i][row] = mkc(0.0, 0.0);
+  for (int i = 0; i < 2; ++i) {
+    T.phs[jr + 4 * i][row] = ph[i];
+    if (row0 + row >= G || jr + 4 * i >= n) T.dph[jr + 4 * i][row] = mkc(0.0, 0.0);
   }
   __syncthreads();
   contract_rows(T);
   if (!ONE) {
-    part[128LL * blockIdx.x + threadIdx.x] = T.so[threadIdx.x];
+    if (threadIdx.x < 128) part[128LL * blockIdx.x + threadIdx.x] = T.so[threadIdx.x];   // the thread's own
     return;
   }
   __syncthreads();
@@ -473,12 +476,14 @@ __global__ void __launch_bounds__(SPF_THREADS) spf_project8_kernel(const SpfDesc
     copy_async16(&T.phs[j][row], d.phi + row0 + row + (long long)G * j);
     copy_async16(&T.dph[j][row], o + row0 + row + (long long)G * j);
   }
-  cplx v = mkc(0.0, 0.0);
-  const cplx* p = part + 128LL * d.block_start + threadIdx.x;
-  const int ntile = (G + SPF_ROWS - 1) / SPF_ROWS;
+  if (threadIdx.x < 128) {
+    cplx v = mkc(0.0, 0.0);
+    const cplx* p = part + 128LL * d.block_start + threadIdx.x;
+    const int ntile = (G + SPF_ROWS - 1) / SPF_ROWS;
 #pragma unroll 4
-  for (int t = 0; t < ntile; ++t) v = cadd(v, p[128LL * t]);
-  T.so[threadIdx.x] = v;
+    for (int t = 0; t < ntile; ++t) v = cadd(v, p[128LL * t]);
+    T.so[threadIdx.x] = v;
+  }
   copy_async_wait();
   __syncthreads();
   if (!solve_project(T, d, row0, o, g) && threadIdx.x == 0 && tile == 0) atomicOr(status, DEVST_CHOL_FAIL);
@@ -500,7 +505,7 @@ __global__ void __launch_bounds__(SPF_THREADS) spf_project_kernel(const SpfDesc*
     if (row0 + (e & (SPF_ROWS - 1)) < G) copy_async16(dph + e, o + row0 + (e & (SPF_ROWS - 1)) + (long long)G * (e / SPF_ROWS));
   auto get = [&](int i, int c) { return c < n ? d.S[i + n * c] : d.O[i + n * (c - n)]; };
   const bool ok = n <= 8 ? solve_elimination<1>(n, get, colb, rowb, Xt)
-                         : (n <= 16 ? solve_elimination<4>(n, get, colb, rowb, Xt) : solve_elimination<16>(n, get, colb, rowb, Xt));
+                         : (n <= 16 ? solve_elimination<2>(n, get, colb, rowb, Xt) : solve_elimination<8>(n, get, colb, rowb, Xt));
   if (threadIdx.x == 0 && tile == 0 && !ok) atomicOr(status, DEVST_CHOL_FAIL);
   __syncthreads();
   row_products(S, (n + 7) / 8, step, n, G, row0, [&](int row, int j1, cplx v) {
