@@ -530,9 +530,9 @@ struct Ctx {
   RegInvDesc* reg_d = nullptr;
   MFOp* mfop_d = nullptr;
   std::vector<SpfDesc> spf_h;
-  std::vector<SpfStep> spfstep_h;
+  std::vector<SpfCol> spfcol_h;
   SpfDesc* spf_d = nullptr;
-  SpfStep* spfstep_d = nullptr;
+  SpfCol* spfcol_d = nullptr;
   HoleBatch spf_holes;     // phi^H phi and phi^H dphi of every SPF derivative block
   long long spf_tiles = 0;
   cplx* spf_part = nullptr;   // contractions of the tiles
@@ -1563,16 +1563,15 @@ void plan_eom(Ctx& c) {
       sd.out_offset = c.naconftot + c.ipsi[m + f * s];
       sd.G = c.gmode[m];
       sd.n = c.m_of(m, s);
-      sd.step_first = (int)c.spfstep_h.size();
+      sd.col_first = (int)c.spfcol_h.size();
       for (int k = 0; k < c.noper[m]; ++k) {
         if (c.is_identity[m + f * k] || !c.ham_op[m][k]) continue;
         if (c.multiset[m] && c.oper[m][k][0] != s) continue;
         const int n2 = c.m_of(m, c.oper[m][k][1]);
-        for (int j = 0; j < n2; j += 8)
-          c.spfstep_h.push_back(SpfStep{c.ophi[m][k] + (long long)sd.G * j, c.rhom1mf[m][k] + (long long)sd.n * j,
-                                        std::min(8, n2 - j), 0});
+        for (int j = 0; j < n2; ++j)
+          c.spfcol_h.push_back(SpfCol{c.ophi[m][k] + (long long)sd.G * j, c.rhom1mf[m][k] + (long long)sd.n * j});
       }
-      sd.step_count = (int)c.spfstep_h.size() - sd.step_first;
+      sd.col_count = (int)c.spfcol_h.size() - sd.col_first;
       sd.block_start = c.spf_tiles;
       c.spf_tiles += (sd.G + SPF_ROWS - 1) / SPF_ROWS;
       c.spf_h.push_back(sd);
@@ -1587,7 +1586,7 @@ void plan_eom(Ctx& c) {
     c.spf_h[i].O = c.spf_holes.h[2 * i + 1].partial;
   }
   c.spf_d = upload_vec(c.ar, c.spf_h);
-  c.spfstep_d = upload_vec(c.ar, c.spfstep_h);
+  c.spfcol_d = upload_vec(c.ar, c.spfcol_h);
   if (c.spf_tiles) c.spf_part = c.ar.calloc_c(128 * c.spf_tiles);
 
   // dA = f * sum_t ae_t * (H_t A)   (conjugate of Adot_tmp, gmctdh_objects.f90:578; derivatives.f90:155-156)
@@ -2174,7 +2173,7 @@ void run_packets(Ctx& c) {
 
 // SPF derivatives into out's psi part (derivatives.f90:94-153)
 void run_spf(Ctx& c, cplx* out, const SpfStage& next = SpfStage{}) {
-  c.count(launch_spf(c.spf_d, (int)c.spf_h.size(), c.spf_tiles, c.spf_holes.maxn, c.spfstep_d,
+  c.count(launch_spf(c.spf_d, (int)c.spf_h.size(), c.spf_tiles, c.spf_holes.maxn, c.spfcol_d,
                      c.spf_holes.launch(), c.spf_part, out, c.der, c.d_status, c.st, next));
 }
 
@@ -4142,9 +4141,9 @@ struct Ens {
   RegInvDesc* reg_d = nullptr;
   MFOp* mfop_d = nullptr;
   std::vector<SpfDesc> spf_h;
-  std::vector<SpfStep> spfstep_h;
+  std::vector<SpfCol> spfcol_h;
   SpfDesc* spf_d = nullptr;
-  SpfStep* spfstep_d = nullptr;
+  SpfCol* spfcol_d = nullptr;
   HoleBatch spf_holes;
   long long spf_tiles = 0;
   cplx* spf_part = nullptr;   // contractions of the tiles
@@ -4303,13 +4302,13 @@ Ens* ens_create(const mctdh_setup_t* setups, int n) {
       }
       E->mfop_h.insert(E->mfop_h.end(), c->mfop_h.begin(), c->mfop_h.end());
       for (SpfDesc sd : c->spf_h) {
-        sd.step_first += (int)E->spfstep_h.size();
+        sd.col_first += (int)E->spfcol_h.size();
         sd.out_offset += o;
         sd.block_start += E->spf_tiles;
         E->spf_h.push_back(sd);
       }
       E->spf_tiles += c->spf_tiles;
-      E->spfstep_h.insert(E->spfstep_h.end(), c->spfstep_h.begin(), c->spfstep_h.end());
+      E->spfcol_h.insert(E->spfcol_h.end(), c->spfcol_h.begin(), c->spfcol_h.end());
       for (HoleDesc hd : c->spf_holes.h) {
         if (!hd.Y) hd.yoff += o;
         E->spf_holes.h.push_back(hd);
@@ -4346,7 +4345,7 @@ Ens* ens_create(const mctdh_setup_t* setups, int n) {
     E->reg_d = upload_vec(E->ar, E->reg_h);
     E->mfop_d = upload_vec(E->ar, E->mfop_h);
     E->spf_d = upload_vec(E->ar, E->spf_h);
-    E->spfstep_d = upload_vec(E->ar, E->spfstep_h);
+    E->spfcol_d = upload_vec(E->ar, E->spfcol_h);
     if (E->spf_tiles) E->spf_part = E->ar.calloc_c(128 * E->spf_tiles);
     E->spf_holes.finalize(E->ar);
     E->sum_d = upload_vec(E->ar, E->sum_h);
@@ -4414,7 +4413,7 @@ void ens_eom(Ens& E, cplx* out) {
   ens_run_red(E, E.red);
   launch_reginv(E.reg_d, (int)E.reg_h.size(), E.mfop_d, E.status_d, E.st);
   launch_termsum(out, E.sum_d, (int)E.sum_h.size(), E.src_d, E.total, E.st, E.precision);
-  E.launches += launch_spf(E.spf_d, (int)E.spf_h.size(), E.spf_tiles, E.spf_holes.maxn, E.spfstep_d,
+  E.launches += launch_spf(E.spf_d, (int)E.spf_h.size(), E.spf_tiles, E.spf_holes.maxn, E.spfcol_d,
                            E.spf_holes.launch(), E.spf_part, out, E.der, E.status_d, E.st);
   E.launches += 2;
   E.eom_count++;

@@ -109,16 +109,15 @@ struct SpfDesc {
   const cplx* phi;         // G x n
   long long out_offset;    // offset of the block in the output vector
   int G, n;
-  int step_first, step_count;
+  int col_first, col_count;
   const cplx* S;           // phi^H phi, phi^H dphi: the contractions' sums (n x n)
   const cplx* O;
   long long block_start;   // first row block of this descriptor
 };
-// up to eight columns j2 of one operator: x = ophi(:, j2) (G x nj), rm = rhom1MF(:, j2) (n x nj)
-struct SpfStep {
+// a column j2 of an operator: x = ophi(:, j2) (G), rm = rhom1MF(:, j2) (n)
+struct SpfCol {
   const cplx* x;
   const cplx* rm;
-  int nj, pad;
 };
 
 // Elementwise weighted sum of source tensors into a range of the output vector.
@@ -264,7 +263,7 @@ struct SpfStage {
   long long off;
 };
 // part: 128 complex per tile (scratch); returns the number of launches
-int launch_spf(const SpfDesc* d_descs, int ndesc, long long ntiles, int maxn, const SpfStep* d_steps,
+int launch_spf(const SpfDesc* d_descs, int ndesc, long long ntiles, int maxn, const SpfCol* d_cols,
                const HoleLaunch& holes, cplx* part, cplx* out, cplx der_factor, int* d_status, cudaStream_t st,
                const SpfStage& stage = SpfStage{});
 // SPF Cash-Karp or Dormand-Prince ends: y5 = base + dt_mode sum_k c5_k k_k, y4 likewise, and

@@ -13,7 +13,8 @@
 
 #define SPF_THREADS 256
 #define SPF_NS 8
-#define SPF_CHUNK 9      // steps of eight j2 between flushes: 9 x 16 x 7 x 2^14 < 2^24
+#define SPF_CHUNK 9      // steps of eight columns between flushes: 9 x 16 x 7 x 2^14 < 2^24
+#define SPF_COLS (8 * SPF_CHUNK)
 
 #define SPF_PITCH (SPF_ROWS + 2)   // staged rows of a column: the lanes' 16-byte reads meet no bank twice
 
@@ -36,33 +37,32 @@ __device__ __forceinline__ void copy_async16(void* dst, const void* src) {
 }
 __device__ __forceinline__ void copy_async_wait() { asm volatile("cp.async.wait_all;" ::: "memory"); }
 
-// Rows row0 .. row0 + 63 of the steps [s0, s0 + ns) on their way into S.x (zeros beyond
-// G and nj); copy_async_wait and a barrier complete it.
-template <typename Step>
-__device__ __forceinline__ void stage_rows(RowShared& S, int s0, int ns, Step&& step, int G, int row0) {
-  const int row = threadIdx.x & (SPF_ROWS - 1), jr = threadIdx.x / SPF_ROWS;
-  for (int s = 0; s < ns; ++s) {
-    const SpfStep st = step(s0 + s);
-#pragma unroll
-    for (int j = 0; j < 8; j += SPF_THREADS / SPF_ROWS) {
-      cplx* to = &S.x[s][j + jr][row];
-      if (row0 + row < G && j + jr < st.nj) copy_async16(to, st.x + row0 + row + (long long)G * (j + jr));
-      else *to = mkc(0.0, 0.0);
-    }
+// Rows row0 .. row0 + 63 of the columns 8 s0 .. 8 (s0 + ns) - 1 on their way into S.x
+// (zeros beyond G and ncols); copy_async_wait and a barrier complete it.
+template <typename Col>
+__device__ __forceinline__ void stage_rows(RowShared& S, int s0, int ns, Col&& col, int ncols, int G, int row0) {
+  const int row = threadIdx.x & (SPF_ROWS - 1);
+#pragma unroll 2
+  for (int j = threadIdx.x / SPF_ROWS; j < 8 * ns; j += SPF_THREADS / SPF_ROWS) {
+    cplx* to = &S.x[j >> 3][j & 7][row];
+    if (row0 + row < G && 8 * s0 + j < ncols) copy_async16(to, col(8 * s0 + j).x + row0 + row);
+    else *to = mkc(0.0, 0.0);
   }
 }
 
-// The CTA's rows row0 .. row0 + 63 of sum_steps sum_j x(row, j) rm(j1, j) for all
+// The CTA's rows row0 .. row0 + 63 of sum_j x(row, j) rm(j1, j) over ncols columns for all
 // j1 < n: warps w and w + 4 own 16 rows (the MMA's rows) and every second step, the
 // columns are the (re, im) of four j1; a row
-// has one exponent per chunk of steps, a column j1 of the matrices another.  step(s)
-// returns the s-th step (up to eight j); the first chunk is staged already.
+// has one exponent per chunk of steps, a column j1 of the matrices another.  col(j)
+// returns the j-th column of x and of rm, a step is eight of them (whatever operators
+// they belong to); the first chunk is staged already.
 // put(row, j1, value) takes the results (warps 0 - 3); rows from G on are skipped.  The
 // matrices are cut while the rows are on their way.  Operands outside
 // the exponent range are multiplied in FP64.
-template <typename Step, typename Put>
-__device__ __forceinline__ void row_products(RowShared& S, int nsteps, Step&& step, int n, int G, int row0, Put&& put) {
+template <typename Col, typename Put>
+__device__ __forceinline__ void row_products(RowShared& S, int ncols, Col&& col, int n, int G, int row0, Put&& put) {
   constexpr int NS = SPF_NS;
+  const int nsteps = (ncols + 7) / 8;
   const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5, g = lane >> 2, q = lane & 3;
   const int half = warp >> 2, lr = 16 * (warp & 3) + g;   // the lane's rows: lr, lr + 8
   auto& other = S.other;
@@ -72,25 +72,30 @@ __device__ __forceinline__ void row_products(RowShared& S, int nsteps, Step&& st
       const int ns = min(SPF_CHUNK, nsteps - s0);
       if (s0 || (j0 && nsteps > SPF_CHUNK)) {
         __syncthreads();   // the previous chunk is read
-        stage_rows(S, s0, ns, step, G, row0);
+        stage_rows(S, s0, ns, col, ncols, G, row0);
       }
       if (tid < 8) S.colmag[tid] = 0u;
       __syncthreads();
       const int nc = min(8, n - j0);
-      for (int e = tid; e < 64 * ns; e += SPF_THREADS) {   // (step, j, j1)
-        const int j1 = e & 7, j = (e >> 3) & 7;
-        const SpfStep st = step(s0 + (e >> 6));
-        if (j1 < nc && j < st.nj) atomicMax(&S.colmag[j1], fx_mag(st.rm[j0 + j1 + n * j]));
+      for (int e0 = tid; e0 < 64 * ns; e0 += 3 * SPF_THREADS) {   // (j, j1), three loads in flight
+        unsigned m[3];
+#pragma unroll
+        for (int i = 0; i < 3; ++i) {
+          const int e = e0 + i * SPF_THREADS, j = 8 * s0 + (e >> 3);
+          m[i] = e < 64 * ns && j < ncols && (e & 7) < nc ? fx_mag(col(j).rm[j0 + (e & 7)]) : 0u;
+        }
+        const unsigned all = max(m[0], max(m[1], m[2]));
+        if (all) atomicMax(&S.colmag[e0 & 7], all);
       }
       __syncthreads();
       bool bad = tid < nc && !fx_ok(S.colmag[tid]);
       for (int w = warp; w < 2 * ns; w += SPF_THREADS / 32) {
         const int t = w & 1, s = w >> 1, j1 = 4 * t + (g >> 1);
         if (4 * t >= nc) continue;
-        const SpfStep st = step(s0 + s);
+        const int jc = 8 * (s0 + s) + q;
         unsigned d0[NS], d1[NS];
-        const cplx m0 = (j1 < nc && q < st.nj) ? st.rm[j0 + j1 + n * q] : mkc(0, 0);
-        const cplx m1 = (j1 < nc && q + 4 < st.nj) ? st.rm[j0 + j1 + n * (q + 4)] : mkc(0, 0);
+        const cplx m0 = (j1 < nc && jc < ncols) ? col(jc).rm[j0 + j1] : mkc(0, 0);
+        const cplx m1 = (j1 < nc && jc + 4 < ncols) ? col(jc + 4).rm[j0 + j1] : mkc(0, 0);
         const unsigned em = fx_ebits(S.colmag[j1]);
         fx_digits<NS>(m0.x, m0.y, em, em, d0);
         fx_digits<NS>(m1.x, m1.y, em, em, d1);
@@ -104,6 +109,7 @@ __device__ __forceinline__ void row_products(RowShared& S, int nsteps, Step&& st
       copy_async_wait();
       __syncthreads();
       unsigned mag[2] = {0u, 0u};
+#pragma unroll 3
       for (int s = 0; s < ns; ++s)
 #pragma unroll
         for (int f = 0; f < 2; ++f)
@@ -120,10 +126,7 @@ __device__ __forceinline__ void row_products(RowShared& S, int nsteps, Step&& st
           const int row = row0 + (e & (SPF_ROWS - 1)), j1 = j0 + e / SPF_ROWS;
           if (row >= G) continue;
           cplx acc = mkc(0, 0);
-          for (int s = 0; s < nsteps; ++s) {
-            const SpfStep st = step(s);
-            for (int j = 0; j < st.nj; ++j) cfma(acc, st.x[row + (long long)G * j], st.rm[j1 + n * j]);
-          }
+          for (int j = 0; j < ncols; ++j) cfma(acc, col(j).x[row], col(j).rm[j1]);
           put(row, j1, acc);
         }
         goto next_pass;
@@ -194,24 +197,24 @@ __device__ __forceinline__ void row_products(RowShared& S, int nsteps, Step&& st
 }
 
 __global__ void __launch_bounds__(SPF_THREADS) spf_drive_kernel(const SpfDesc* __restrict__ descs, int ndesc,
-                                                                const SpfStep* __restrict__ steps,
+                                                                const SpfCol* __restrict__ cols,
                                                                 cplx* __restrict__ out, cplx der) {
   extern __shared__ __align__(16) unsigned char spf_sm[];
   RowShared& S = *reinterpret_cast<RowShared*>(spf_sm);
-  __shared__ SpfStep st[SPF_CHUNK];
+  __shared__ SpfCol st[SPF_COLS];
   const SpfDesc& d = descs[warp_find_desc(descs, ndesc, (long long)blockIdx.x)];
-  const SpfStep* gst = steps + d.step_first;
-  const int nsteps = d.step_count;
-  // one chunk's steps in shared memory; longer lists are read where they are
-  const bool local = nsteps <= SPF_CHUNK;
-  if (local && (int)threadIdx.x < nsteps) st[threadIdx.x] = gst[threadIdx.x];
+  const SpfCol* gst = cols + d.col_first;
+  const int ncols = d.col_count;
+  // one chunk's columns in shared memory; longer lists are read where they are
+  const bool local = ncols <= SPF_COLS;
+  if (local && (int)threadIdx.x < ncols) st[threadIdx.x] = gst[threadIdx.x];
   __syncthreads();
   cplx* o = out + d.out_offset;
   const int G = d.G, row0 = (int)(blockIdx.x - d.block_start) * SPF_ROWS;
   const bool rot = der.x == 0.0 && der.y == -1.0, neg = der.x == -1.0 && der.y == 0.0;
-  auto step = [&](int s) { return local ? st[s] : gst[s]; };
-  stage_rows(S, 0, min(SPF_CHUNK, nsteps), step, G, row0);
-  row_products(S, nsteps, step, d.n, G, row0, [&](int row, int j1, cplx v) {
+  auto col = [&](int j) { return local ? st[j] : gst[j]; };
+  stage_rows(S, 0, min(SPF_CHUNK, (ncols + 7) / 8), col, ncols, G, row0);
+  row_products(S, ncols, col, d.n, G, row0, [&](int row, int j1, cplx v) {
     o[row + (long long)G * j1] = rot ? mkc(v.y, -v.x) : (neg ? mkc(-v.x, -v.y) : cmul(der, v));
   });
 }
@@ -419,30 +422,30 @@ __device__ __forceinline__ bool solve_project(SpfSmall& T, const SpfDesc& d, int
 // Otherwise dphi goes to out and the contractions of the CTA's rows to part.
 template <bool ONE>
 __global__ void __launch_bounds__(SPF_THREADS) spf_drive8_kernel(const SpfDesc* __restrict__ descs, int ndesc,
-                                                                 const SpfStep* __restrict__ steps, cplx* out, cplx der,
+                                                                 const SpfCol* __restrict__ cols, cplx* out, cplx der,
                                                                  cplx* __restrict__ part, int* status, SpfStage g) {
   extern __shared__ __align__(16) unsigned char spf_sm[];
   RowShared& S = *reinterpret_cast<RowShared*>(spf_sm);
   SpfSmall& T = *reinterpret_cast<SpfSmall*>(&S.W);
-  __shared__ SpfStep st[SPF_CHUNK];
+  __shared__ SpfCol st[SPF_COLS];
   const SpfDesc& d = descs[warp_find_desc(descs, ndesc, (long long)blockIdx.x)];
-  const SpfStep* gst = steps + d.step_first;
-  const int nsteps = d.step_count, n = d.n;
-  // one chunk's steps in shared memory; longer lists are read where they are
-  const bool local = nsteps <= SPF_CHUNK;
-  if (local && (int)threadIdx.x < nsteps) st[threadIdx.x] = gst[threadIdx.x];
+  const SpfCol* gst = cols + d.col_first;
+  const int ncols = d.col_count, n = d.n;
+  // one chunk's columns in shared memory; longer lists are read where they are
+  const bool local = ncols <= SPF_COLS;
+  if (local && (int)threadIdx.x < ncols) st[threadIdx.x] = gst[threadIdx.x];
   __syncthreads();
   cplx* o = out + d.out_offset;
   const int G = d.G, row0 = (int)(blockIdx.x - d.block_start) * SPF_ROWS;
   const int row = threadIdx.x & (SPF_ROWS - 1), jr = threadIdx.x / SPF_ROWS;
   const bool rot = der.x == 0.0 && der.y == -1.0, neg = der.x == -1.0 && der.y == 0.0;
-  auto step = [&](int s) { return local ? st[s] : gst[s]; };
-  stage_rows(S, 0, min(SPF_CHUNK, nsteps), step, G, row0);
+  auto col = [&](int j) { return local ? st[j] : gst[j]; };
+  stage_rows(S, 0, min(SPF_CHUNK, (ncols + 7) / 8), col, ncols, G, row0);
   cplx ph[2];
 #pragma unroll
   for (int i = 0; i < 2; ++i)
     ph[i] = row0 + row < G && jr + 4 * i < n ? d.phi[row0 + row + (long long)G * (jr + 4 * i)] : mkc(0.0, 0.0);
-  row_products(S, nsteps, step, n, G, row0, [&](int r, int j1, cplx v) {
+  row_products(S, ncols, col, n, G, row0, [&](int r, int j1, cplx v) {
     const cplx w = rot ? mkc(v.y, -v.x) : (neg ? mkc(-v.x, -v.y) : cmul(der, v));
     T.dph[j1][r - row0] = w;
     if (!ONE) o[r + (long long)G * j1] = w;
@@ -499,8 +502,8 @@ __global__ void __launch_bounds__(SPF_THREADS) spf_project_kernel(const SpfDesc*
   cplx* dph = Xt + n * n;                                           // [n][SPF_ROWS]
   cplx* o = out + d.out_offset;
   const cplx* phi = d.phi;
-  auto step = [&](int s) { return SpfStep{phi + (long long)G * 8 * s, Xt + n * 8 * s, min(8, n - 8 * s), 0}; };
-  stage_rows(S, 0, (n + 7) / 8, step, G, row0);
+  auto col = [&](int j) { return SpfCol{phi + (long long)G * j, Xt + n * j}; };
+  stage_rows(S, 0, (n + 7) / 8, col, n, G, row0);
   for (int e = threadIdx.x; e < n * SPF_ROWS; e += SPF_THREADS)
     if (row0 + (e & (SPF_ROWS - 1)) < G) copy_async16(dph + e, o + row0 + (e & (SPF_ROWS - 1)) + (long long)G * (e / SPF_ROWS));
   auto get = [&](int i, int c) { return c < n ? d.S[i + n * c] : d.O[i + n * (c - n)]; };
@@ -508,12 +511,12 @@ __global__ void __launch_bounds__(SPF_THREADS) spf_project_kernel(const SpfDesc*
                          : (n <= 16 ? solve_elimination<2>(n, get, colb, rowb, Xt) : solve_elimination<8>(n, get, colb, rowb, Xt));
   if (threadIdx.x == 0 && tile == 0 && !ok) atomicOr(status, DEVST_CHOL_FAIL);
   __syncthreads();
-  row_products(S, (n + 7) / 8, step, n, G, row0, [&](int row, int j1, cplx v) {
+  row_products(S, n, col, n, G, row0, [&](int row, int j1, cplx v) {
     o[row + (long long)G * j1] = csub(dph[row - row0 + SPF_ROWS * j1], v);
   });
 }
 
-int launch_spf(const SpfDesc* d_descs, int ndesc, long long ntiles, int maxn, const SpfStep* d_steps,
+int launch_spf(const SpfDesc* d_descs, int ndesc, long long ntiles, int maxn, const SpfCol* d_cols,
                const HoleLaunch& holes, cplx* part, cplx* out, cplx der_factor, int* d_status, cudaStream_t st,
                const SpfStage& stage) {
   if (ndesc <= 0) return 0;
@@ -528,15 +531,15 @@ int launch_spf(const SpfDesc* d_descs, int ndesc, long long ntiles, int maxn, co
   (void)configured;
   const unsigned nb = (unsigned)ntiles;
   if (maxn <= 8 && ntiles == ndesc) {
-    spf_drive8_kernel<true><<<nb, SPF_THREADS, smem, st>>>(d_descs, ndesc, d_steps, out, der_factor, part, d_status, stage);
+    spf_drive8_kernel<true><<<nb, SPF_THREADS, smem, st>>>(d_descs, ndesc, d_cols, out, der_factor, part, d_status, stage);
     return 1;
   }
   if (maxn <= 8) {
-    spf_drive8_kernel<false><<<nb, SPF_THREADS, smem, st>>>(d_descs, ndesc, d_steps, out, der_factor, part, d_status, stage);
+    spf_drive8_kernel<false><<<nb, SPF_THREADS, smem, st>>>(d_descs, ndesc, d_cols, out, der_factor, part, d_status, stage);
     spf_project8_kernel<<<nb, SPF_THREADS, 0, st>>>(d_descs, ndesc, out, part, d_status, stage);
     return 2;
   }
-  spf_drive_kernel<<<nb, SPF_THREADS, smem, st>>>(d_descs, ndesc, d_steps, out, der_factor);
+  spf_drive_kernel<<<nb, SPF_THREADS, smem, st>>>(d_descs, ndesc, d_cols, out, der_factor);
   launch_hole_fx(holes, st, 0, out);
   spf_project_kernel<<<nb, SPF_THREADS, smem_x, st>>>(d_descs, ndesc, out, d_status);
   return 3;
