@@ -1311,6 +1311,59 @@ void plan_eom(Ctx& c) {
       }
     }
   }
+  // The mode order of a state pair's chains: R runs from the back, L from the front.
+  // Modes on which the pair's terms carry the same matrix (SPF overlaps, mostly) go to
+  // the two ends, so that the terms share the chains' beginnings; products with the same
+  // input and matrix are computed once (8-SPF QVC model, eight general
+  // terms: 68 -> 57 products, 260 -> 226 us).
+  // The order changes only the rounding; FP32 products, whose rounding shows, and pairs
+  // with one term keep the reference order.
+  std::map<std::tuple<int, int, int>, std::vector<int>> pair_order;
+  {
+    std::map<std::tuple<int, int, int>, std::vector<int>> pair_terms;
+    for (int t = 0; t < c.nham; ++t)
+      if (is_general[t] && c.kind[t] != 1) pair_terms[std::make_tuple(c.kind[t], c.lhs[t], c.rhs[t])].push_back(t);
+    for (auto& pt : pair_terms) {
+      std::vector<int> by(f), order(f), distinct(f);
+      for (int m = 0; m < f; ++m) {
+        by[m] = order[m] = m;
+        std::set<int> ops;
+        for (int t : pt.second) ops.insert(c.skip_term[m + f * t] ? -1 : c.ioper[m + f * t]);
+        distinct[m] = (int)ops.size();
+      }
+      if (pt.second.size() > 1 && c.precision != 1) {
+        std::stable_sort(by.begin(), by.end(), [&](int a, int b) { return distinct[a] < distinct[b]; });
+        for (int i = 0; i < f; ++i) order[i & 1 ? i / 2 : f - 1 - i / 2] = by[i];
+      }
+      pair_order[pt.first] = order;
+    }
+  }
+  // one product of a chain, or the earlier one of the same input and matrix; products of
+  // c.chains serve both chain sets (c.chains_full is skipped where only mean fields are wanted)
+  struct Link {
+    TRef ref;
+    int depth;
+  };
+  std::map<std::tuple<const cplx*, int, const cplx*, int>, Link> links[2];
+  auto extend = [&](const Link& in, const cplx* raw_in, int raw_fmt, int mode, const cplx* mat, int ldm, int conj, int nout,
+                    bool full) {
+    const auto key = std::make_tuple((const cplx*)in.ref.p, mode, mat, conj);
+    for (int set = 0; set <= (full ? 1 : 0); ++set) {
+      auto it = links[set].find(key);
+      if (it != links[set].end()) return it->second;
+    }
+    Link out;
+    out.depth = in.depth + 1;
+    out.ref.shape = in.ref.shape;
+    out.ref.shape[mode] = nout;
+    out.ref.p = c.ar.calloc_c(prod_range(out.ref.shape, 0, (int)out.ref.shape.size()));
+    out.ref.fmt = chain_fmt;
+    (full ? c.chains_full : c.chains)[out.depth].add(raw_in, out.ref.p, mat, ldm, conj, in.ref.shape, mode, nout,
+                                                     mkc(1, 0), 0, raw_fmt, chain_fmt);
+    links[full ? 1 : 0][key] = out;
+    return out;
+  };
+  std::map<std::tuple<const cplx*, const cplx*, int>, int> hole_of;   // (X, Y, mode) -> contraction
   std::map<std::pair<int, int>, int> term_hole;   // (leader term, mode) -> contraction
   for (int t = 0; t < c.nham; ++t) {
     const int s1 = c.lhs[t], s2 = c.rhs[t];
@@ -1334,45 +1387,41 @@ void plan_eom(Ctx& c) {
     const int leader = leader_of[t];
     // type-1 terms: the right chain on A serves V A only (gmctdh_objects.f90:628-649);
     // their mean fields contract the left chain with a right chain on AuxA (below)
-    std::vector<ProdBatch>& rchains = (leader >= 0 || c.kind[t] == 1) ? c.chains_full : c.chains;
+    const bool rfull = leader >= 0 || c.kind[t] == 1;
+    std::vector<int> order(f);   // order[i]: the i-th mode of L, the (f - 1 - i)-th of R
+    for (int m = 0; m < f; ++m) order[m] = m;
+    if (c.kind[t] != 1) order = pair_order.at(std::make_tuple(c.kind[t], s1, s2));
     int lmax = 0;
-    for (int im = 0; im < f; ++im)
-      if (!c.is_identity[im + f * c.ioper[im + f * t]]) lmax = im;
-    if (leader >= 0 || c.kind[t] == 1) lmax = 0;
+    for (int i = 0; i < f; ++i)
+      if (!c.is_identity[order[i] + f * c.ioper[order[i] + f * t]]) lmax = i;
+    if (rfull) lmax = 0;
     std::vector<TRef> R(f + 1), L(f);
-    R[0].p = c.d_in + c.aoff[s2];
-    R[0].shape = c.shape_of(s2);
+    Link cur;
+    cur.depth = 0;
+    cur.ref.p = c.d_in + c.aoff[s2];
+    cur.ref.shape = c.shape_of(s2);
+    R[0] = cur.ref;
     for (int i = 1; i <= f; ++i) {
-      const int jm = f - i;
-      if (c.skip_term[jm + f * t]) { R[i] = R[i - 1]; continue; }
-      const int k = c.ioper[jm + f * t];
-      const int n1 = c.m_of(jm, s1);
-      std::vector<int> ns = R[i - 1].shape;
-      ns[jm] = n1;
-      cplx* out = c.ar.calloc_c(prod_range(ns, 0, (int)ns.size()));
-      const auto in = prod_in(R[i - 1], s2);
-      rchains[i].add(in.first, out, c.hmat[jm][k], n1, 0, R[i - 1].shape, jm, n1, mkc(1, 0), 0, in.second,
-                     chain_fmt);
-      R[i].p = out;
-      R[i].shape = ns;
-      R[i].fmt = chain_fmt;
+      const int jm = order[f - i];
+      if (!c.skip_term[jm + f * t]) {
+        const int n1 = c.m_of(jm, s1);
+        const auto in = prod_in(cur.ref, s2);
+        cur = extend(cur, in.first, in.second, jm, c.hmat[jm][c.ioper[jm + f * t]], n1, 0, n1, rfull);
+      }
+      R[i] = cur.ref;
     }
-    L[0].p = c.d_in + c.aoff[s1];
-    L[0].shape = c.shape_of(s1);
+    cur = Link();
+    cur.depth = 0;
+    cur.ref.p = c.d_in + c.aoff[s1];
+    cur.ref.shape = c.shape_of(s1);
+    L[0] = cur.ref;
     for (int i = 1; i <= lmax; ++i) {
-      const int im = i - 1;
-      if (c.skip_term[im + f * t]) { L[i] = L[i - 1]; continue; }
-      const int k = c.ioper[im + f * t];
-      const int n1 = c.m_of(im, s1), n2 = c.m_of(im, s2);
-      std::vector<int> ns = L[i - 1].shape;
-      ns[im] = n2;
-      cplx* out = c.ar.calloc_c(prod_range(ns, 0, (int)ns.size()));
-      const auto in = prod_in(L[i - 1], s1);
-      c.chains[i].add(in.first, out, c.hmat[im][k], n1, 1, L[i - 1].shape, im, n2, mkc(1, 0), 0, in.second,
-                      chain_fmt);
-      L[i].p = out;
-      L[i].shape = ns;
-      L[i].fmt = chain_fmt;
+      const int im = order[i - 1];
+      if (!c.skip_term[im + f * t]) {
+        const auto in = prod_in(cur.ref, s1);
+        cur = extend(cur, in.first, in.second, im, c.hmat[im][c.ioper[im + f * t]], c.m_of(im, s1), 1, c.m_of(im, s2), false);
+      }
+      L[i] = cur.ref;
     }
     if (c.kind[t] == 1) {
       // V_k A = sum_t ae_t V_t A (no der_factor), and the mean fields of
@@ -1436,17 +1485,19 @@ void plan_eom(Ctx& c) {
     }
     srcs_of(t)[s1].push_back(SumSrc{R[f].p, cmul(c.der, c.ae[t]), R[f].fmt});
     c.general_terms.push_back(t);
-    for (int im = 0; im < f; ++im) {
-      const int k = c.ioper[im + f * t];
+    for (int pos = 0; pos < f; ++pos) {
+      const int im = order[pos], k = c.ioper[im + f * t];
       if (c.is_identity[im + f * k]) continue;
       if (leader >= 0) {
         hrefs.push_back(HoleRef{term_hole.at(std::make_pair(leader, im)), mf_tg(im, k), c.ae[t], 1});
         continue;
       }
-      const TRef& X = L[im];
-      const TRef& Y = R[f - 1 - im];
+      const TRef& X = L[pos];
+      const TRef& Y = R[f - 1 - pos];
       long long Ll = prod_range(X.shape, 0, im), Rr = prod_range(X.shape, im + 1, (int)X.shape.size());
-      int hidx = c.holes.add(c.ar, X.p, Y.p, Ll, Rr, X.shape[im], Y.shape[im], X.fmt, Y.fmt);
+      const auto hkey = std::make_tuple((const cplx*)X.p, (const cplx*)Y.p, im);
+      if (!hole_of.count(hkey)) hole_of[hkey] = c.holes.add(c.ar, X.p, Y.p, Ll, Rr, X.shape[im], Y.shape[im], X.fmt, Y.fmt);
+      const int hidx = hole_of[hkey];
       term_hole[std::make_pair(t, im)] = hidx;
       hrefs.push_back(HoleRef{hidx, mf_tg(im, k), c.ae[t]});
     }
