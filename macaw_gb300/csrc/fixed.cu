@@ -27,21 +27,6 @@ static int sm_count() {
 // by the MMAs.
 // ---------------------------------------------------------------------------
 
-// The same product in FP64, for fibres or matrices outside the exponent range.
-static __device__ __noinline__ void prod_fibre_fp64(const ProdDesc& d, long long l, long long r) {
-  const long long L = d.L;
-  for (int jo = 0; jo < d.nout; ++jo) {
-    cplx acc = mkc(0.0, 0.0);
-    for (int j = 0; j < d.nin; ++j) {
-      const cplx m = d.conjT ? cconj(d.M[j + (long long)d.ldm * jo]) : d.M[jo + (long long)d.ldm * j];
-      cfma(acc, m, load_c(d.X, l + L * (j + (long long)d.nin * r), d.xfmt));
-    }
-    cplx v = cmul(d.alpha, acc);
-    cplx* y = d.Y + l + L * (jo + (long long)d.nout * r);
-    if (d.accumulate) v = cadd(v, *y);
-    *y = v;
-  }
-}
 #define PROD_THREADS 128
 #define PROD_NS 8
 // resident CTAs per SM the register budget is set for
@@ -236,7 +221,13 @@ static void prod_fx_go(const ProdDesc* d, int nd, long long nblocks, int persist
   prod_fx_kernel<NJ><<<(unsigned)std::min((split ? 8 : 2) * nblocks, most), PROD_THREADS, smem, st>>>(d, nd, nblocks, split);
 }
 
+// The tcgen05 form (tc.cu) takes batches of 5 to 16 SPFs that give every one of its CTAs
+// a tile; T5_RULE.
 void launch_prod_fx(const ProdDesc* d, int nd, long long nblocks, int maxn, cudaStream_t st, int persist) {
+  if (persist <= 0 && maxn > 4 && maxn <= 16 && nblocks >= (maxn <= 8 ? 4 : 2) * (long long)sm_count()) {
+    launch_prod_digits_tc(d, nd, nblocks, maxn, sm_count(), st);
+    return;
+  }
   if (maxn <= 4) prod_fx_go<1>(d, nd, nblocks, persist, st);
   else if (maxn <= 8) prod_fx_go<2>(d, nd, nblocks, persist, st);
   else if (maxn <= 12) prod_fx_go<3>(d, nd, nblocks, persist, st);
@@ -649,8 +640,6 @@ __device__ __forceinline__ void hole_mul(HoleWide& sh, cplx* acc, bool mine, boo
 }
 template <bool F32>
 __device__ __forceinline__ void hole_wide_block(const HoleDesc& d, int b, const cplx* ybase) {
-  constexpr int NS = HOLE_NS, ND = HOLE_ND;
-  constexpr unsigned emin = (unsigned)FX_EMIN << 20;
   extern __shared__ cplx red[];
   HoleWide& sh = *reinterpret_cast<HoleWide*>(red);
   const cplx* Yp = d.Y ? d.Y : ybase + d.yoff;
@@ -658,7 +647,7 @@ __device__ __forceinline__ void hole_wide_block(const HoleDesc& d, int b, const 
   const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5, g = lane >> 2, q = lane & 3;
   const bool sym = d.X == d.Y && n1 == n2 && d.xfmt == d.yfmt;
   const int b1 = (n1 + 7) >> 3, b2 = (n2 + 7) >> 3;
-  const unsigned L = (unsigned)d.L, nfib = (unsigned)(d.L * d.R);
+  const unsigned nfib = (unsigned)(d.L * d.R);
   const unsigned ngrp = (nfib + 15) / 16;
   const unsigned g0 = (unsigned)((unsigned long long)ngrp * b / d.nblk);
   const unsigned g1 = (unsigned)((unsigned long long)ngrp * (b + 1) / d.nblk);

@@ -14,6 +14,7 @@
 // of 8 x 8 complex products).
 #pragma once
 #include "common.cuh"
+#include "kernels.cuh"
 
 // Exponent fields (biased) within which no intermediate leaves the normal range;
 // vectors outside (and non-finite ones) take the FP64 code.
@@ -92,8 +93,8 @@ __device__ __forceinline__ void fx_mma8(float* c, const unsigned* a, unsigned b0
 
 // sum_k D_k 2^(-8 k) 2^44 as an integer, |D_k| < 2^22, |D_0 2^44| < 2^62: the integer of D
 // appears in the low bits of D + 1.5 2^23; the biases are taken out as constants.
-template <int NS>
-__device__ __forceinline__ long long fx_join(const float (*c)[4], int i) {
+template <int NS, int W>
+__device__ __forceinline__ long long fx_join(const float (*c)[W], int i) {
   constexpr float mg = 12582912.f;
   constexpr unsigned z = 0x4B400000u, zz = (z << 8) + z;
   const float f6 = NS > 7 ? fmaf(c[NS > 7 ? 7 : 0][i], 1.f / 256.f, c[6][i]) : c[6][i];
@@ -125,6 +126,22 @@ __device__ __forceinline__ double fx_double(long long v, int es) {
   const double d = (double)v;
   const int hi = __double2hiint(d);
   return __hiloint2double(hi ? hi + es : hi, __double2loint(d));
+}
+
+// A mode product's fibre (l, :, r) in FP64, for fibres or matrices outside the exponent range.
+static __device__ __noinline__ void prod_fibre_fp64(const ProdDesc& d, long long l, long long r) {
+  const long long L = d.L;
+  for (int jo = 0; jo < d.nout; ++jo) {
+    cplx acc = mkc(0.0, 0.0);
+    for (int j = 0; j < d.nin; ++j) {
+      const cplx m = d.conjT ? cconj(d.M[j + (long long)d.ldm * jo]) : d.M[jo + (long long)d.ldm * j];
+      cfma(acc, m, load_c(d.X, l + L * (j + (long long)d.nin * r), d.xfmt));
+    }
+    cplx v = cmul(d.alpha, acc);
+    cplx* y = d.Y + l + L * (jo + (long long)d.nout * r);
+    if (d.accumulate) v = cadd(v, *y);
+    *y = v;
+  }
 }
 
 // Descriptor of block b, found by every warp for itself: 32 candidates per round

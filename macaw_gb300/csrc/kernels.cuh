@@ -273,6 +273,8 @@ void launch_rk_end(cplx* y5, cplx* diff, const cplx* base, const StageArgs& a, c
 // FP64 accuracy as exact digit products on the tensor cores (fixed.cu); launched by
 // launch_prod / launch_hole
 void launch_prod_fx(const ProdDesc* d_descs, int ndesc, long long nblocks, int maxn, cudaStream_t st, int persist);
+// ... with tcgen05 MMAs, nin and nout <= 16 (tc.cu)
+void launch_prod_digits_tc(const ProdDesc* d_descs, int ndesc, long long nblocks, int maxn, int nsm, cudaStream_t st);
 void launch_hole_fx(const HoleLaunch& b, cudaStream_t st, int persist, const cplx* ybase = nullptr);
 void launch_reduce(const RedTarget* d_tg, int ntg, const RedTerm* d_terms, cudaStream_t st);
 // with_h: also h1mode, by `proj` (phi_l^H (O phi_r) of every operator into X or h) or, where

@@ -28,6 +28,7 @@
 #include "../../include/macaw_gb300.h"
 #include "kernels.cuh"
 #include "tc.cuh"
+#include "fixed.cuh"
 
 #define TC_ROWS 128
 #define TC_MAXN 16          // largest nin / nout of the tensor-core mode product
@@ -210,6 +211,188 @@ __global__ void __launch_bounds__(TC_ROWS) prod_tc_kernel(const ProdDesc* __rest
     tc_fence_after();
     tc_dealloc(tmem, 64);
   }
+}
+
+// ---------------------------------------------------------------------------
+// Mode products of FP64 accuracy as exact digit products (fixed.cuh) with tcgen05.  A
+// tile is 128 fibres, one per thread and MMA row; the thread cuts its fibre into eight
+// FP16 digits of one exponent, digit i of all fibres being operand A_i (128 x 2 nin).
+// The matrix's digits lie side by side as columns, B = [B_0 B_1 .. B_7] (WC columns
+// each: the (re, im) of the outputs), and D = [D_0 .. D_7] holds the sums of equal weight
+// in TMEM: A_i times the first 8 - i blocks adds into D_i .. D_7, so a K step of a tile
+// takes eight MMAs of N = WC (8 - i).  A thread reads its fibre's sums back, joins and
+// rounds them: no shuffles, no fragments in registers.  Bound by the instructions that
+// cut and join (about 30 per real number on either side) and by the conversions on the
+// FP64 pipe (62 cycles per warp and real number): 262,144 fibres of 8 x 8 products T5_FIG.
+// ---------------------------------------------------------------------------
+template <int NG>   // groups of four j
+struct DigitTile {
+  static constexpr int K = NG <= 2 ? 16 : 32;    // halfs per row
+  static constexpr int WC = NG <= 2 ? 16 : 32;   // columns per weight
+  static constexpr uint32_t SBO = K / 8 * 128, A = 128 * K * 2, B = 8 * WC * K * 2;
+  static constexpr uint32_t COLS = 8 * WC;       // TMEM columns
+};
+template <int NG>
+__global__ void __launch_bounds__(128, NG <= 2 ? 4 : 2)
+    prod_digits_kernel(const ProdDesc* __restrict__ descs, int ndesc, long long ntiles) {
+  using T = DigitTile<NG>;
+  extern __shared__ __align__(128) unsigned char tc_smem[];   // A_0 .. A_7, B
+  __shared__ __align__(8) uint64_t bar;
+  __shared__ uint32_t s_tmem;
+  __shared__ unsigned rowexp[4 * NG];
+  __shared__ int s_bad;
+  const int tid = threadIdx.x, warp = tid >> 5;
+  long long t0 = ntiles * blockIdx.x / gridDim.x;
+  const long long tend = ntiles * (blockIdx.x + 1) / gridDim.x;
+  if (tid == 0) tc_bar_init(&bar, 1);
+  if (warp == 0) tc_alloc(&s_tmem, T::COLS);
+  if (NG == 3)   // the last K group of A stays zero
+    for (int i = 0; i < 8; ++i)
+      *reinterpret_cast<uint4*>(tc_smem + i * T::A + (tid >> 3) * T::SBO + 3 * 128 + (tid & 7) * 16) = make_uint4(0, 0, 0, 0);
+  tc_fence_before();
+  __syncthreads();
+  tc_fence_after();
+  const uint32_t tmem = s_tmem, base = tc_smem_addr(tc_smem);
+  uint32_t parity = 0;
+  bool ok = true;
+  int di = t0 < tend ? warp_find_desc(descs, ndesc, t0) : 0;
+  for (; t0 < tend && ok; ++di) {
+    const ProdDesc& d = descs[di];
+    const int nin = d.nin, nout = d.nout;
+    const unsigned L = (unsigned)d.L, nfib = (unsigned)(d.L * d.R);
+    const long long dend = min(tend, d.block_start + (long long)((nfib + 127) / 128));
+    const long long Lx = d.L * (nin - 1), Ly = d.L * (nout - 1);
+    unsigned p = (unsigned)(t0 - d.block_start) * 128 + tid, r = p / L;
+    cplx x[4 * NG];
+    auto fetch = [&]() {   // element j of fibre (l, r): l + L (j + nin r) = p + Lx r + L j
+      const cplx* xp = d.X + ((long long)p + Lx * r);
+      const bool act = p < nfib;
+#pragma unroll
+      for (int j = 0; j < 4 * NG; ++j) {
+        x[j] = mkc(0.0, 0.0);
+        if (act && j < nin) x[j] = *xp;
+        xp += L;
+      }
+    };
+    fetch();
+    // the matrix: a row's exponent, then its digits
+    __syncthreads();   // B of the descriptor before is read (its MMAs are complete)
+    if (tid < 4 * NG) rowexp[tid] = 0u;
+    if (tid == 0) s_bad = 0;
+    __syncthreads();
+    for (int e = tid; e < T::WC / 2 * 4 * NG; e += 128) {
+      const int jo = e / (4 * NG), ji = e % (4 * NG);
+      if (jo < nout && ji < nin)
+        atomicMax(&rowexp[jo], fx_mag(d.conjT ? d.M[ji + (long long)d.ldm * jo] : d.M[jo + (long long)d.ldm * ji]));
+    }
+    __syncthreads();
+    if (tid < nout && !fx_ok(rowexp[tid])) s_bad = 1;
+    for (int e = tid; e < T::WC / 2 * (T::K / 2); e += 128) {
+      const int jo = e / (T::K / 2), ji = e % (T::K / 2);
+      cplx m = mkc(0.0, 0.0);
+      if (jo < nout && ji < nin) m = d.conjT ? cconj(d.M[ji + (long long)d.ldm * jo]) : d.M[jo + (long long)d.ldm * ji];
+      const unsigned eb = jo < nout ? fx_ebits(rowexp[jo]) : fx_ebits(0u);
+      unsigned s[8];
+      fx_digits<8>(m.x, m.y, eb, eb, s);
+      unsigned char* b = tc_smem + 8 * T::A + (ji >> 2) * 128 + (ji & 3) * 4;
+#pragma unroll
+      for (int i = 0; i < 8; ++i) {   // columns re: (Mr, -Mi), im: (Mi, Mr)
+        const int n = i * T::WC + 2 * jo;
+        *reinterpret_cast<unsigned*>(b + (n >> 3) * T::SBO + (n & 7) * 16) = s[i] ^ 0x80000000u;
+        *reinterpret_cast<unsigned*>(b + (n >> 3) * T::SBO + ((n & 7) + 1) * 16) = __byte_perm(s[i], s[i], 0x1032);
+      }
+    }
+    const bool plain = !d.accumulate && d.alpha.x == 1.0 && d.alpha.y == 0.0;
+    for (; t0 < dend; ++t0) {
+      unsigned mag = 0u;
+#pragma unroll
+      for (int j = 0; j < 4 * NG; ++j) mag = max(mag, fx_mag(x[j]));
+      const unsigned eb = fx_ebits(mag);
+      const int ef = (int)eb - ((2044 + 12 + 44) << 20);
+      bool bad = !fx_ok(mag);
+#pragma unroll
+      for (int k = 0; k < NG; ++k) {
+        unsigned s[4][8];
+#pragma unroll
+        for (int j = 0; j < 4; ++j) fx_digits<8>(x[4 * k + j].x, x[4 * k + j].y, eb, eb, s[j]);
+        unsigned char* a = tc_smem + (tid >> 3) * T::SBO + k * 128 + (tid & 7) * 16;
+#pragma unroll
+        for (int i = 0; i < 8; ++i)
+          *reinterpret_cast<uint4*>(a + i * T::A) = make_uint4(s[0][i], s[1][i], s[2][i], s[3][i]);
+      }
+      tc_fence_smem();
+      tc_fence_before();
+      __syncthreads();
+      bad = bad || s_bad;
+      if (tid == 0) {
+        tc_fence_after();
+#pragma unroll
+        for (int ks = 0; ks < T::K / 16; ++ks)
+#pragma unroll
+          for (int i = 0; i < 8; ++i)
+            tc_mma_f16(tmem + i * T::WC, tc_smem_desc(base + i * T::A + ks * 256, 128, T::SBO),
+                       tc_smem_desc(base + 8 * T::A + ks * 256, 128, T::SBO), tc_idesc_f16(128, T::WC * (8 - i)),
+                       ks || i);
+        tc_commit(&bar);
+      }
+      const unsigned pc = p, rc = r;
+      if (t0 + 1 < dend) {
+        p += 128;
+        r = p / L;
+        fetch();
+      }
+      // every thread polls; the verdict is made uniform so that all leave together
+      ok = __syncthreads_and(tc_wait(&bar, parity));
+      parity ^= 1;
+      tc_fence_after();
+      if (!ok) break;
+      const bool act = pc < nfib;
+      cplx* y = d.Y + ((long long)pc + Ly * rc);
+#pragma unroll
+      for (int h = 0; h < NG; ++h) {
+        if (4 * h >= nout) break;
+        float c[8][8];
+        tc_ld8x8(tmem + ((uint32_t)(warp * 32) << 16) + 8 * h, T::WC, c);
+#pragma unroll
+        for (int o = 0; o < 4; ++o) {
+          if (4 * h + o < nout) {
+            const int es = (int)fx_ebits(rowexp[4 * h + o]) + ef;
+            cplx v = mkc(fx_double(fx_join<8>(c, 2 * o), es), fx_double(fx_join<8>(c, 2 * o + 1), es));
+            if (!plain) {
+              v = cmul(d.alpha, v);
+              if (d.accumulate && act) v = cadd(v, y[(long long)L * (4 * h + o)]);
+            }
+            if (act && !bad) y[(long long)L * (4 * h + o)] = v;
+          }
+        }
+      }
+      if (act && bad) prod_fibre_fp64(d, pc - L * rc, rc);
+    }
+    t0 = dend;
+  }
+  if (!ok && tid == 0) atomicExch(&g_tc_timeout, 1);
+  tc_fence_before();
+  __syncthreads();
+  if (warp == 0) {
+    tc_fence_after();
+    tc_dealloc(tmem, T::COLS);
+  }
+}
+
+template <int NG>
+static void prod_digits_go(const ProdDesc* d, int nd, long long nblocks, int nsm, cudaStream_t st) {
+  using T = DigitTile<NG>;
+  constexpr int smem = (int)(8 * T::A + T::B);
+  static const cudaError_t configured =
+      cudaFuncSetAttribute(prod_digits_kernel<NG>, cudaFuncAttributeMaxDynamicSharedMemorySize, smem);
+  (void)configured;
+  const long long grid = std::min<long long>(nblocks, (NG <= 2 ? 4LL : 2LL) * nsm);
+  prod_digits_kernel<NG><<<(unsigned)grid, 128, smem, st>>>(d, nd, nblocks);
+}
+void launch_prod_digits_tc(const ProdDesc* d, int nd, long long nblocks, int maxn, int nsm, cudaStream_t st) {
+  if (maxn <= 8) prod_digits_go<2>(d, nd, nblocks, nsm, st);
+  else if (maxn <= 12) prod_digits_go<3>(d, nd, nblocks, nsm, st);
+  else prod_digits_go<4>(d, nd, nblocks, nsm, st);
 }
 
 static int g_tc_nsm = 0;

@@ -35,6 +35,12 @@ __host__ __device__ __forceinline__ uint32_t tc_idesc_tf32(int M, int N) {
   return (1u << 4) | (2u << 7) | (2u << 10) | ((uint32_t)(N >> 3) << 17) | ((uint32_t)(M >> 4) << 24);
 }
 
+// kind::f16, FP16 operands (formats 0), FP32 accumulation; K-major tiles as above with
+// 8 elements per 16 bytes, an MMA step of K = 16
+__host__ __device__ __forceinline__ uint32_t tc_idesc_f16(int M, int N) {
+  return (1u << 4) | ((uint32_t)(N >> 3) << 17) | ((uint32_t)(M >> 4) << 24);
+}
+
 __device__ __forceinline__ float tc_tf32(float x) {
   uint32_t r;
   asm("cvt.rna.tf32.f32 %0, %1;" : "=r"(r) : "f"(x));
@@ -76,6 +82,13 @@ __device__ __forceinline__ void tc_mma_tf32(uint32_t dtmem, uint64_t adesc, uint
       "tcgen05.mma.cta_group::1.kind::tf32 [%0], %1, %2, %3, p;\n\t}"
       :: "r"(dtmem), "l"(adesc), "l"(bdesc), "r"(idesc), "r"(accumulate));
 }
+__device__ __forceinline__ void tc_mma_f16(uint32_t dtmem, uint64_t adesc, uint64_t bdesc, uint32_t idesc,
+                                           uint32_t accumulate) {
+  asm volatile(
+      "{\n\t.reg .pred p;\n\tsetp.ne.b32 p, %4, 0;\n\t"
+      "tcgen05.mma.cta_group::1.kind::f16 [%0], %1, %2, %3, p;\n\t}"
+      :: "r"(dtmem), "l"(adesc), "l"(bdesc), "r"(idesc), "r"(accumulate));
+}
 // the mbarrier completes one phase when every MMA this thread issued before has finished
 __device__ __forceinline__ void tc_commit(uint64_t* bar) {
   asm volatile("tcgen05.commit.cta_group::1.mbarrier::arrive::one.shared::cluster.b64 [%0];"
@@ -107,6 +120,23 @@ __device__ __forceinline__ void tc_ld16(uint32_t taddr, float* v) {
   asm volatile("tcgen05.wait::ld.sync.aligned;" ::: "memory");
 #pragma unroll
   for (int i = 0; i < 16; ++i) v[i] = __uint_as_float(r[i]);
+}
+
+// Columns taddr + w * stride .. + 7 for w = 0 .. 7 of this warp's 32 lanes into v[w][0 .. 7]
+__device__ __forceinline__ void tc_ld8x8(uint32_t taddr, uint32_t stride, float (*v)[8]) {
+#define TC_LD8(W)                                                                                                  \
+  asm volatile("tcgen05.ld.sync.aligned.32x32b.x8.b32 {%0,%1,%2,%3,%4,%5,%6,%7}, [%8];"                            \
+               : "=f"(v[W][0]), "=f"(v[W][1]), "=f"(v[W][2]), "=f"(v[W][3]), "=f"(v[W][4]), "=f"(v[W][5]),         \
+                 "=f"(v[W][6]), "=f"(v[W][7])                                                                      \
+               : "r"(taddr + W * stride))
+  TC_LD8(0); TC_LD8(1); TC_LD8(2); TC_LD8(3); TC_LD8(4); TC_LD8(5); TC_LD8(6); TC_LD8(7);
+#undef TC_LD8
+  asm volatile("tcgen05.wait::ld.sync.aligned;" ::: "memory");
+  // no use of the values above the wait
+#pragma unroll
+  for (int w = 0; w < 8; ++w)
+    asm volatile("" : "+f"(v[w][0]), "+f"(v[w][1]), "+f"(v[w][2]), "+f"(v[w][3]), "+f"(v[w][4]), "+f"(v[w][5]),
+                      "+f"(v[w][6]), "+f"(v[w][7]));
 }
 
 // byte offset of element (row, k) in a K-major tile with K (multiple of 8) columns
