@@ -222,8 +222,9 @@ __global__ void __launch_bounds__(TC_ROWS) prod_tc_kernel(const ProdDesc* __rest
 // in TMEM: A_i times the first 8 - i blocks adds into D_i .. D_7, so a K step of a tile
 // takes eight MMAs of N = WC (8 - i).  A thread reads its fibre's sums back, joins and
 // rounds them: no shuffles, no fragments in registers.  Bound by the instructions that
-// cut and join (about 30 per real number on either side) and by the conversions on the
-// FP64 pipe (62 cycles per warp and real number): 262,144 fibres of 8 x 8 products T5_FIG.
+// cut and join (about 50 per complex number on either side; issue 48 %, FP64 pipe 42 % for
+// the conversions) at the occupancy that registers and TMEM leave: the products of the
+// 8-SPF QVC model's EOM 226 -> 191 us, with 12 SPFs 2,900 -> 2,206.
 // ---------------------------------------------------------------------------
 template <int NG>   // groups of four j
 struct DigitTile {
