@@ -492,6 +492,9 @@ struct Ctx {
   // a second stream for CMF2 work that runs beside the Lanczos build (own contexts only)
   cudaStream_t st2 = nullptr;
   cudaEvent_t ev_fork = nullptr, ev_join = nullptr;
+  // copies of host coefficients beside the EOM (calc_derivs_overlapped)
+  cudaStream_t st_copy = nullptr;
+  cudaEvent_t ev_copy[2] = {nullptr, nullptr};
   bool member = false;      // ensemble member: RK only, state vectors owned by the ensemble
   DevArena ar;
   int* d_status = nullptr;
@@ -627,6 +630,9 @@ struct Ctx {
     if (ev_fork) cudaEventDestroy(ev_fork);
     if (ev_join) cudaEventDestroy(ev_join);
     if (st2) cudaStreamDestroy(st2);
+    for (cudaEvent_t e : ev_copy)
+      if (e) cudaEventDestroy(e);
+    if (st_copy) cudaStreamDestroy(st_copy);
   }
   int m_of(int m, int s) const { return nspf[m + nmodes * s]; }
   // tensor shape of state s; a mixture adds the packet index as the slowest dimension
@@ -2228,54 +2234,73 @@ void run_spf(Ctx& c, cplx* out, const SpfStage& next = SpfStage{}) {
                      c.spf_holes.launch(), c.spf_part, out, c.der, c.d_status, c.st, next));
 }
 
-void eom(Ctx& c, cplx* out, bool mf_only = false, bool reginv = true) {
-  RtScope rt_all(c, RT_CALCDERIVS, true, !mf_only);   // derivatives.f90:92-476
-  const bool gwp = !c.modes_gwp.empty();
-  if (gwp) gwp_setup_run(c);
+// The EOM in three parts: what needs the SPFs only; the products of A and, from them, dA
+// of a wave packet in grid modes (early_sum); the mean fields and the SPF derivatives.
+void eom_operators(Ctx& c) {
+  if (!c.modes_gwp.empty()) gwp_setup_run(c);
+  RtScope rt(c, RT_H1MODE);
+  ProfScope ps(c, KP_H1);
+  c.count(launch_h1(c.h1, true, c.st, c.msum_d, (int)c.msum_h.size(), c.msum_src_d));
+}
+
+bool early_sum(const Ctx& c) { return !c.pk_on; }   // packets' terms come with run_packets
+
+void eom_sum(Ctx& c, cplx* out) {
+  ProfScope ps(c, KP_TERMSUM, 0.0, 16.0 * (double)c.src_h.size() * (double)c.naconftot / std::max(1, c.nstates));
+  launch_termsum(c.modes_gwp.empty() ? out : c.d_adot, c.sum_d, (int)c.sum_h.size(), c.src_d, c.naconftot, c.st,
+                 c.precision);
+  c.count();
+}
+
+void eom_products(Ctx& c, cplx* out, bool mf_only) {
   if (c.d_in32) {
     launch_to_f32(c.d_in32, c.d_in, c.naconftot, c.st);
     c.count();
   }
   {
-    RtScope rt(c, RT_H1MODE);
-    ProfScope ps(c, KP_H1);
-    c.count(launch_h1(c.h1, true, c.st, c.msum_d, (int)c.msum_h.size(), c.msum_src_d));
+    RtScope rt_mf(c, RT_MEANFIELD);   // gmctdh_objects.f90:511-1140
+    // the deepest level holds only the full products H_t A of the right chains (dA)
+    const size_t depth_end = mf_only ? c.chains.size() - 1 : c.chains.size();
+    for (size_t i = 1; i < depth_end; ++i) run_prod(c, mf_only ? c.chains[i] : c.full[i]);
+    for (auto& b : c.gwp_rho_chain) run_prod(c, b);
   }
-  RtScope rt_mf(c, RT_MEANFIELD);   // gmctdh_objects.f90:511-1140
-  // the deepest level holds only the full products H_t A of the right chains (dA)
-  const size_t depth_end = mf_only ? c.chains.size() - 1 : c.chains.size();
-  for (size_t i = 1; i < depth_end; ++i) run_prod(c, mf_only ? c.chains[i] : c.full[i]);
-  for (auto& b : c.gwp_rho_chain) run_prod(c, b);
-  if (c.all_holes.h.empty()) {
-    run_hole(c, c.rho_holes);
-    run_hole(c, c.holes);
-  } else {
-    run_hole(c, c.all_holes);
-  }
-  run_red(c, c.red);
-  if (c.pk_on) run_packets(c);
-  if (reginv || !mf_only) run_reginv(c);
-  if (mf_only) {
-    c.eom_count++;
-    return;
-  }
+  if (!mf_only && early_sum(c)) eom_sum(c, out);
+}
+
+void eom_fields(Ctx& c, cplx* out, bool mf_only, bool reginv) {
   {
-    ProfScope ps(c, KP_TERMSUM, 0.0, 16.0 * (double)c.src_h.size() * (double)c.naconftot / std::max(1, c.nstates));
-    launch_termsum(gwp ? c.d_adot : out, c.sum_d, (int)c.sum_h.size(), c.src_d, c.naconftot, c.st, c.precision);
-    c.count();
+    RtScope rt_mf(c, RT_MEANFIELD, false);
+    if (c.all_holes.h.empty()) {
+      run_hole(c, c.rho_holes);
+      run_hole(c, c.holes);
+    } else {
+      run_hole(c, c.all_holes);
+    }
+    run_red(c, c.red);
+    if (c.pk_on) run_packets(c);
+    if (reginv || !mf_only) run_reginv(c);
   }
+  c.eom_count++;
+  if (mf_only) return;
+  if (!early_sum(c)) eom_sum(c, out);
   {
     RtScope rt(c, RT_SPF_DVR);
     ProfScope ps(c, KP_SPF);
     run_spf(c, out);
   }
-  if (gwp) gwp_derivs_run(c, out);
+  if (!c.modes_gwp.empty()) gwp_derivs_run(c, out);
   // Lagrange multipliers: dA += A (multLagDiag I + i multLag) (derivatives.f90:238-242)
   if (c.pk_mult && !c.skip_mult) {
     launch_pk_mix(c.pk_mult, 1, c.pk_st, c.nstates, c.n1tot, c.npk, out, c.st);
     c.count();
   }
-  c.eom_count++;
+}
+
+void eom(Ctx& c, cplx* out, bool mf_only = false, bool reginv = true) {
+  RtScope rt_all(c, RT_CALCDERIVS, true, !mf_only);   // derivatives.f90:92-476
+  eom_operators(c);
+  eom_products(c, out, mf_only);
+  eom_fields(c, out, mf_only, reginv);
 }
 
 void eom_from(Ctx& c, const cplx* y, cplx* out) {
@@ -4149,6 +4174,48 @@ void download(Ctx& c, const cplx* src, double* A, double* psi) {
 }
 
 
+// Calc_Derivs on host arrays with the coefficients copied beside the parts of the EOM that
+// do not touch them: in while the operators act on the SPFs, out while the mean fields
+// and the SPF derivatives are computed.  From OVERLAP_MIN coefficients (0.5 MB, about
+// 10 us either way; at 56,007 coefficients 225 -> 222 us, at 786,432 625 -> 537); not for
+// packets and Gaussian modes, whose dA is complete at the end only.
+#define OVERLAP_MIN 32768
+bool overlapped_copies(const Ctx& c) {
+  return c.naconftot >= OVERLAP_MIN && c.npk == 1 && !c.pk_on && !c.pk_mult && c.modes_gwp.empty() && !c.profiling &&
+         !c.timing;
+}
+void calc_derivs_overlapped(Ctx& c, const double* A, const double* psi, double* dA, double* dpsi) {
+  if (!c.st_copy) {
+    CK(cudaStreamCreateWithFlags(&c.st_copy, cudaStreamNonBlocking));
+    CK(cudaEventCreateWithFlags(&c.ev_copy[0], cudaEventDisableTiming));
+    CK(cudaEventCreateWithFlags(&c.ev_copy[1], cudaEventDisableTiming));
+  }
+  struct Finish {   // the caller's arrays are not touched any more once this returns or throws
+    Ctx& c;
+    ~Finish() {
+      cudaStreamSynchronize(c.st_copy);
+      cudaStreamSynchronize(c.st);
+    }
+  } finish{c};
+  const size_t nA = sizeof(cplx) * c.naconftot, nP = sizeof(cplx) * c.dimpsi;
+  CK(cudaEventRecord(c.ev_copy[0], c.st));
+  CK(cudaStreamWaitEvent(c.st_copy, c.ev_copy[0], 0));   // d_in and d_out are free
+  if (nP) CK(cudaMemcpyAsync(c.d_in + c.naconftot, psi, nP, cudaMemcpyHostToDevice, c.st));
+  run_graphed(c, 21, nullptr, [&] { eom_operators(c); });
+  CK(cudaMemcpyAsync(c.d_in, A, nA, cudaMemcpyHostToDevice, c.st_copy));
+  CK(cudaEventRecord(c.ev_copy[0], c.st_copy));
+  CK(cudaStreamWaitEvent(c.st, c.ev_copy[0], 0));
+  run_graphed(c, 22, nullptr, [&] { eom_products(c, c.d_out, false); });
+  CK(cudaEventRecord(c.ev_copy[1], c.st));
+  run_graphed(c, 23, nullptr, [&] { eom_fields(c, c.d_out, false, true); });
+  CK(cudaStreamWaitEvent(c.st_copy, c.ev_copy[1], 0));
+  CK(cudaMemcpyAsync(dA, c.d_out, nA, cudaMemcpyDeviceToHost, c.st_copy));
+  check_status(c);
+  if (nP) CK(cudaMemcpyAsync(dpsi, c.d_out + c.naconftot, nP, cudaMemcpyDeviceToHost, c.st));
+  CK(cudaStreamSynchronize(c.st_copy));
+  CK(cudaStreamSynchronize(c.st));
+}
+
 // ---------------------------------------------------------------------------
 // Ensembles of independent wavepackets of uneven shape (different state, mode,
 // SPF and grid counts).  Every member is planned like a single context, on
@@ -5054,6 +5121,10 @@ int64_t mctdh_calc_derivs(mctdh_ctx_t* ctx, const double* A, const double* psi, 
   Ctx* c = ctx->c;
   return guarded(c, [&] {
     (void)t;
+    if (overlapped_copies(*c)) {
+      calc_derivs_overlapped(*c, A, psi, dA, dpsi);
+      return;
+    }
     upload(*c, c->d_in, A, psi);
     run_graphed(*c, 20, nullptr, [&] { eom(*c, c->d_out); });
     check_status(*c);
