@@ -1322,8 +1322,9 @@ void plan_eom(Ctx& c) {
   // the two ends, so that the terms share the chains' beginnings; products with the same
   // input and matrix are computed once (8-SPF QVC model, eight general
   // terms: 68 -> 57 products, 260 -> 226 us).
-  // The order changes only the rounding; FP32 products, whose rounding shows, and pairs
-  // with one term keep the reference order.
+  // The order changes only the rounding; FP32 products, whose rounding shows, pairs
+  // with one term, and pairs whose tensors would grow by it (states of different SPF
+  // counts) keep the reference order.
   std::map<std::tuple<int, int, int>, std::vector<int>> pair_order;
   {
     std::map<std::tuple<int, int, int>, std::vector<int>> pair_terms;
@@ -1339,7 +1340,41 @@ void plan_eom(Ctx& c) {
       }
       if (pt.second.size() > 1 && c.precision != 1) {
         std::stable_sort(by.begin(), by.end(), [&](int a, int b) { return distinct[a] < distinct[b]; });
-        for (int i = 0; i < f; ++i) order[i & 1 ? i / 2 : f - 1 - i / 2] = by[i];
+        std::vector<int> shared(f);
+        for (int i = 0; i < f; ++i) shared[i & 1 ? i / 2 : f - 1 - i / 2] = by[i];
+        // elements read and written by the pair's distinct products and contractions
+        auto cost = [&](const std::vector<int>& ord) {
+          const int s1 = std::get<1>(pt.first), s2 = std::get<2>(pt.first);
+          std::set<std::vector<int>> seen;
+          double sum = 0.0;
+          for (int t : pt.second) {
+            std::vector<double> size[2] = {std::vector<double>(f + 1), std::vector<double>(f + 1)};
+            for (int side = 0; side < 2; ++side) {   // R from the back, L from the front
+              if (side && leader_of[t] >= 0) continue;
+              const int from = side ? s1 : s2, to = side ? s2 : s1;
+              std::vector<int> key(1, side);
+              double n = 1.0;
+              for (int m = 0; m < f; ++m) n *= c.m_of(m, from);
+              size[side][0] = n;
+              for (int i = 0; i < f - side; ++i) {
+                const int m = ord[side ? i : f - 1 - i];
+                if (!c.skip_term[m + f * t]) {
+                  const double in = n;
+                  n = n / c.m_of(m, from) * c.m_of(m, to);
+                  key.push_back(m);
+                  key.push_back(c.ioper[m + f * t]);
+                  if (seen.insert(key).second) sum += in + n;
+                }
+                size[side][i + 1] = n;
+              }
+            }
+            if (leader_of[t] < 0)
+              for (int i = 0; i < f; ++i)
+                if (!c.is_identity[ord[i] + f * c.ioper[ord[i] + f * t]]) sum += size[1][i] + size[0][f - 1 - i];
+          }
+          return sum;
+        };
+        if (cost(shared) < cost(order)) order = shared;
       }
       pair_order[pt.first] = order;
     }
