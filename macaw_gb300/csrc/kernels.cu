@@ -1011,7 +1011,8 @@ __device__ void grid_sum_c(cplx v, cplx* partial, unsigned* counter, cplx* out) 
 // The sources come sorted by kind; told apart inside the loop they were issued under
 // predicates and all paid for (8-SPF QVC model, about ten sources a state: 107 -> 51 us with the inner product, 48 -> 43 without).
 // PREC 1: FP32 coefficients times FP32-rounded sources accumulated in FP32 (the
-// sources are FP32 products there).
+// sources are FP32 products there); two elements per thread, bound by the loads in flight
+// (8-SPF QVC model, about ten sources a state: 39 -> 28 us).
 #define TERMSUM_CACHE 64
 // KIND 0 complex, 1 imaginary, 2 real
 template <int KIND>
@@ -1037,6 +1038,37 @@ __device__ __forceinline__ void termsum_run(cplx& val, const SumSrc* sp, int n, 
     }
   }
 }
+// FP32: N (1 or 2) neighbouring elements from li on into a (re, im each)
+template <int N>
+__device__ __forceinline__ void termsum_f32(float* a, const SumSrc* sp, int n, long long li) {
+  for (int k0 = 0; k0 < n; k0 += 4) {
+    float4 x[4][N];
+#pragma unroll
+    for (int k = 0; k < 4; ++k)
+      if (k0 + k < n) {
+        const SumSrc& s = sp[k0 + k];
+        if (N == 2 && s.fmt) {   // 16 bytes hold both
+          const float4 v = *reinterpret_cast<const float4*>(reinterpret_cast<const float2*>(s.src) + li);
+          x[k][0] = make_float4(v.x, v.y, 0.f, 0.f);
+          x[k][N - 1] = make_float4(v.z, v.w, 0.f, 0.f);
+        } else {
+#pragma unroll
+          for (int e = 0; e < N; ++e) x[k][e] = load_split(s.src, li + e, s.fmt);
+        }
+      }
+#pragma unroll
+    for (int k = 0; k < 4; ++k) {
+      if (k0 + k >= n) break;
+      const float cr = sp[k0 + k].cs[0] + sp[k0 + k].cs[1], ci = sp[k0 + k].cs[2] + sp[k0 + k].cs[3];
+#pragma unroll
+      for (int e = 0; e < N; ++e) {
+        const float xr = x[k][e].x + x[k][e].z, xi = x[k][e].y + x[k][e].w;
+        a[2 * e] = fmaf(cr, xr, fmaf(-ci, xi, a[2 * e]));
+        a[2 * e + 1] = fmaf(cr, xi, fmaf(ci, xr, a[2 * e + 1]));
+      }
+    }
+  }
+}
 template <int PREC>
 __global__ void __launch_bounds__(256, 4) termsum_kernel(cplx* __restrict__ out, const SumRange* __restrict__ ranges,
                                                       int nr, const SumSrc* __restrict__ srcs, long long total,
@@ -1052,8 +1084,10 @@ __global__ void __launch_bounds__(256, 4) termsum_kernel(cplx* __restrict__ out,
   SumRange rg;
   rg.offset = rg.n = 0;
   // warp w of the launch: neighbouring warps of a block work far apart
+  constexpr int N = PREC == 1 ? 2 : 1;   // elements per thread and row
   const long long wrow = ((long long)(threadIdx.x >> 5) * gridDim.x + blockIdx.x) * 32 + (threadIdx.x & 31);
-  for (long long i = wrow; i < total; i += (long long)gridDim.x * blockDim.x) {
+  const long long stride = (long long)N * gridDim.x * blockDim.x;
+  for (long long i0 = N * wrow, i = i0; i < total; i = i + 1 < min(total, i0 + N) ? i + 1 : (i0 += stride)) {
     if (i - rg.offset >= rg.n) {
       int lo = 0, hi = nr - 1;   // last range starting at or before i (ranges sorted by offset)
       while (lo < hi) {
@@ -1068,24 +1102,24 @@ __global__ void __launch_bounds__(256, 4) termsum_kernel(cplx* __restrict__ out,
     }
     const long long li = i - rg.offset;
     const SumSrc* sp = all + rg.first;
+    // both of a pair: the FP32 sources are whole allocations, 16-byte aligned at even li
+    if (PREC == 1 && i == i0 && !(li & 1) && li + 1 < rg.n) {
+      float a[4] = {0.f, 0.f, 0.f, 0.f};
+      termsum_f32<2>(a, sp, rg.count, li);
+#pragma unroll
+      for (int e = 0; e < 2; ++e) {
+        const cplx v = mkc(f2d_exact(a[2 * e]), f2d_exact(a[2 * e + 1]));
+        out[i + e] = v;
+        if (dot.v) cfma_conj(d, dot.v[i + e], v);
+      }
+      ++i;
+      continue;
+    }
     cplx val;
     if (PREC == 1) {
-      float ar = 0.f, ai = 0.f;
-      for (int k0 = 0; k0 < rg.count; k0 += 4) {
-        float4 x[4];
-#pragma unroll
-        for (int k = 0; k < 4; ++k)
-          if (k0 + k < rg.count) x[k] = load_split(sp[k0 + k].src, li, sp[k0 + k].fmt);
-#pragma unroll
-        for (int k = 0; k < 4; ++k) {
-          if (k0 + k >= rg.count) break;
-          const float cr = sp[k0 + k].cs[0] + sp[k0 + k].cs[1], ci = sp[k0 + k].cs[2] + sp[k0 + k].cs[3];
-          const float xr = x[k].x + x[k].z, xi = x[k].y + x[k].w;
-          ar = fmaf(cr, xr, fmaf(-ci, xi, ar));
-          ai = fmaf(cr, xi, fmaf(ci, xr, ai));
-        }
-      }
-      val = mkc(f2d_exact(ar), f2d_exact(ai));
+      float a[2] = {0.f, 0.f};
+      termsum_f32<1>(a, sp, rg.count, li);
+      val = mkc(f2d_exact(a[0]), f2d_exact(a[1]));
     } else {
       val = mkc(0, 0);
       termsum_run<1>(val, sp, rg.nimag, li);
