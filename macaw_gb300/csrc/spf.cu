@@ -376,43 +376,92 @@ __device__ __forceinline__ cplx stage_sum(const SpfStage& g, long long e) {
 
 // Solve from T.so and subtract the CTA's rows of phi X; with g.on also the next stage's
 // input (the CTA's rows of phi are in shared memory by now, so it may replace them).  A
-// thread has row threadIdx.x % 64 of columns threadIdx.x / 64 and + 4.  Eight FP64
-// instructions a row and column pair of warps, less than cutting and joining digits.
+// warp has 16 rows and four columns of phi X, one set of digit products (in FP64 the 8 n
+// instructions a row and column pair took 4.7 us at n = 8).
 __device__ __forceinline__ bool solve_project(SpfSmall& T, const SpfDesc& d, int row0, cplx* o, const SpfStage& g) {
-  const int n = d.n, G = d.G, row = threadIdx.x & (SPF_ROWS - 1), jr = threadIdx.x / SPF_ROWS;
-  const bool in = row0 + row < G;
+  constexpr int NS = SPF_NS;
+  const int n = d.n, G = d.G, lane = threadIdx.x & 31, warp = threadIdx.x >> 5, gl = lane >> 2, q = lane & 3;
+  const int lr = 16 * (warp & 3) + gl, j0 = 4 * (warp >> 2), j = j0 + q;   // elements (lr, j), (lr + 8, j)
   cplx ss[2], bs[2];
   double dt = 0.0;
   if (g.on) {
     dt = g.dt_mode[g.elem_mode[d.out_offset - g.off]];
 #pragma unroll
-    for (int i = 0; i < 2; ++i) {
-      ss[i] = bs[i] = mkc(0.0, 0.0);
-      if (in && jr + 4 * i < n) {
-        const long long e = d.out_offset + row0 + row + (long long)G * (jr + 4 * i);
-        ss[i] = stage_sum(g, e);
-        bs[i] = g.base[e];
+    for (int f = 0; f < 2; ++f) {
+      ss[f] = bs[f] = mkc(0.0, 0.0);
+      if (row0 + lr + 8 * f < G && j < n) {
+        const long long e = d.out_offset + row0 + lr + 8 * f + (long long)G * j;
+        ss[f] = stage_sum(g, e);
+        bs[f] = g.base[e];
       }
     }
+  }
+  // the rows of phi, cut ahead of the solve
+  unsigned A[NS][4], er[2];
+  bool bad = false;
+#pragma unroll
+  for (int f = 0; f < 2; ++f) {
+    const cplx x0 = T.phs[q][lr + 8 * f], x1 = T.phs[q + 4][lr + 8 * f];
+    const cplx y0 = q < n ? x0 : mkc(0.0, 0.0), y1 = q + 4 < n ? x1 : mkc(0.0, 0.0);
+    unsigned mag = row0 + lr + 8 * f < G ? max(fx_mag(y0), fx_mag(y1)) : 0u;
+    mag = max(mag, __shfl_xor_sync(0xffffffffu, mag, 1));
+    mag = max(mag, __shfl_xor_sync(0xffffffffu, mag, 2));
+    bad = bad || !fx_ok(mag);
+    er[f] = fx_ebits(mag);
+    unsigned s[NS];
+    fx_digits<NS>(y0.x, y0.y, er[f], er[f], s);
+#pragma unroll
+    for (int i = 0; i < NS; ++i) A[i][f] = s[i];
+    fx_digits<NS>(y1.x, y1.y, er[f], er[f], s);
+#pragma unroll
+    for (int i = 0; i < NS; ++i) A[i][2 + f] = s[i];
   }
   const bool ok = solve_elimination<1>(
       n, [&](int i, int c) { return c < n ? T.so[i + 8 * c] : T.so[64 + i + 8 * (c - n)]; }, T.colb, T.rowb, T.Xt);
   __syncthreads();
+  if (j0 >= n) return ok;   // whole warps
+  cplx v[2];
+  const int jo = j0 + (gl >> 1);
+  const cplx m0 = jo < n && q < n ? T.Xt[jo + n * q] : mkc(0.0, 0.0);
+  const cplx m1 = jo < n && q + 4 < n ? T.Xt[jo + n * (q + 4)] : mkc(0.0, 0.0);
+  unsigned mag = max(fx_mag(m0), fx_mag(m1));
+  mag = max(mag, __shfl_xor_sync(0xffffffffu, mag, 1));
+  mag = max(mag, __shfl_xor_sync(0xffffffffu, mag, 2));
+  if (__any_sync(0xffffffffu, bad || !fx_ok(mag))) {
 #pragma unroll
-  for (int i = 0; i < 2; ++i) {
-    const int j = jr + 4 * i;
-    if (!in || j >= n) break;
-    cplx v = T.dph[j][row];
-    for (int k = 0; k < n; ++k) {
-      const cplx x = T.phs[k][row], c = T.Xt[j + n * k];
-      v.x = fma(-x.x, c.x, fma(x.y, c.y, v.x));
-      v.y = fma(-x.x, c.y, fma(-x.y, c.x, v.y));
+    for (int f = 0; f < 2; ++f) {
+      v[f] = mkc(0.0, 0.0);
+      if (j < n)
+        for (int k = 0; k < n; ++k) cfma(v[f], T.phs[k][lr + 8 * f], T.Xt[j + n * k]);
     }
+  } else {
+    const unsigned ec = fx_ebits(mag);
+    const int es = (int)__shfl_sync(0xffffffffu, ec, 8 * q) - ((2044 + 12 + 44) << 20);
+    unsigned s0[NS], s1[NS];
+    fx_digits<NS>(m0.x, m0.y, ec, ec, s0);
+    fx_digits<NS>(m1.x, m1.y, ec, ec, s1);
+    float c[NS][4];
+#pragma unroll
+    for (int i = 0; i < NS; ++i) {   // column re: (Mr, -Mi); column im: (Mi, Mr)
+      const unsigned w0 = (gl & 1) ? __byte_perm(s0[i], s0[i], 0x1032) : s0[i] ^ 0x80000000u;
+      const unsigned w1 = (gl & 1) ? __byte_perm(s1[i], s1[i], 0x1032) : s1[i] ^ 0x80000000u;
+#pragma unroll
+      for (int k = 0; k + i < NS; ++k) fx_mma16(c[i + k], A[k], w0, w1, i == 0);
+    }
+#pragma unroll
+    for (int f = 0; f < 2; ++f)
+      v[f] = mkc(fx_double(fx_join<NS>(c, 2 * f), es + (int)er[f]), fx_double(fx_join<NS>(c, 2 * f + 1), es + (int)er[f]));
+  }
+#pragma unroll
+  for (int f = 0; f < 2; ++f) {
+    const int row = lr + 8 * f;
+    if (row0 + row >= G || j >= n) continue;
+    const cplx w = csub(T.dph[j][row], v[f]);
     const long long e = row0 + row + (long long)G * j;
-    o[e] = v;
+    o[e] = w;
     if (g.on) {
-      const cplx s = mkc(fma(g.last, v.x, ss[i].x), fma(g.last, v.y, ss[i].y));
-      g.out[d.out_offset + e] = mkc(fma(dt, s.x, bs[i].x), fma(dt, s.y, bs[i].y));
+      const cplx s = mkc(fma(g.last, w.x, ss[f].x), fma(g.last, w.y, ss[f].y));
+      g.out[d.out_offset + e] = mkc(fma(dt, s.x, bs[f].x), fma(dt, s.y, bs[f].y));
     }
   }
   return ok;
