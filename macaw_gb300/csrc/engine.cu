@@ -263,9 +263,11 @@ void merge_holes(HoleBatch& all, const HoleBatch& a, const HoleBatch& b, DevAren
 // at 3.5 M terms (8-SPF QVC model) h1_kernel 59 us against 21 and 11, at 39 K (LVC, 6
 // SPFs) 8.6 us against 12 in all.
 #define H1_PROJECT_MIN 1000000
-H1Launch plan_h1(DevArena& ar, const std::vector<H1Desc>& h, HoleBatch& proj) {
+// split: the context has FP32 mode products.
+H1Launch plan_h1(DevArena& ar, const std::vector<H1Desc>& h, HoleBatch& proj, bool split) {
   H1Launch L;
   memset(&L, 0, sizeof(L));
+  L.split = split;
   if (h.empty()) return L;
   double terms = 0.0;
   auto cost = [](const H1Desc& d) {
@@ -282,7 +284,7 @@ H1Launch plan_h1(DevArena& ar, const std::vector<H1Desc>& h, HoleBatch& proj) {
   std::stable_sort(o.begin(), o.end(), [&](const H1Desc& a, const H1Desc& b) { return cost(a) > cost(b); });
   L.d = upload_vec(ar, o);
   L.n = (int)o.size();
-  if (terms >= H1_PROJECT_MIN) {
+  if (terms >= H1_PROJECT_MIN && !split) {
     proj.finalize(ar);
     L.proj = proj.launch();
   }
@@ -512,6 +514,7 @@ struct Ctx {
 
   // DVR operator matrices on device: (dof, code) -> pointer
   std::map<std::pair<int, int>, cplx*> dofmat;
+  std::map<std::pair<int, int>, float2*> dofmatf;   // real coefficients split into FP32 (hi, lo)
   std::map<std::pair<int, int>, int> dofkind;
 
   // per (mode, op) storage
@@ -521,7 +524,7 @@ struct Ctx {
 
   // EOM plan
   std::vector<H1Desc> h1_h;
-  H1Launch h1{};
+  H1Launch h1{}, h1x{};    // in the context's arithmetic; in FP64 (expectation values)
   HoleBatch h1_proj;       // their phi_l^H (O phi_r)
   std::vector<ProdBatch> chains;  // per depth
   std::vector<ProdBatch> chains_full;   // per depth: right chains needed only for dA (adjoint partners)
@@ -581,7 +584,7 @@ struct Ctx {
   OvlPlan io_plan;     // d_in vs d_out (host API norm/ovl)
   // CMF2 / Lanczos
   cplx* d_krylov = nullptr;  // [ntotA x 21]
-  double* d_lan = nullptr;   // alpha[20], beta[20]
+  double* d_lan = nullptr;   // alpha[20], beta[20], evals[20], evecs[400]
   int lan_nk = 0;
   std::vector<double> lan_evals, lan_evecs;
   cplx* d_coef = nullptr;
@@ -898,6 +901,13 @@ void load_setup(Ctx& c, const mctdh_setup_t* s) {
         }
         c.dofmat[key] = upload_vec(c.ar, v);
         c.dofkind[key] = kind;
+        std::vector<float2> vf(v.size());
+        for (size_t i = 0; i < v.size(); ++i) {
+          const double x = (kind == 3) ? v[i].y : v[i].x;
+          const float hi = (float)x;
+          vf[i] = make_float2(hi, (float)(x - (double)hi));
+        }
+        c.dofmatf[key] = upload_vec(c.ar, vf);
       }
     }
   }
@@ -1188,6 +1198,7 @@ void plan_eom(Ctx& c) {
           auto key = std::make_pair(d, code);
           hd.optype[q] = c.dofkind[key];
           hd.mat[q] = c.dofmat[key];
+          hd.matf[q] = c.dofmatf[key];
         }
       }
       if (ham) {
@@ -1197,8 +1208,10 @@ void plan_eom(Ctx& c) {
       }
     }
   }
-  c.h1 = plan_h1(c.ar, c.h1_h, c.h1_proj);
-  c.xh1 = plan_h1(c.ar, c.xh1_h, c.xh1_proj);
+  const bool fp32 = c.precision == 1 || c.hb_prec == 1;
+  c.h1 = plan_h1(c.ar, c.h1_h, c.h1_proj, fp32);
+  c.h1x = fp32 ? plan_h1(c.ar, c.h1_h, c.h1_proj, false) : c.h1;
+  c.xh1 = plan_h1(c.ar, c.xh1_h, c.xh1_proj, false);
   if (!c.modes_gwp.empty()) plan_gwp_setup(c);
 
   // density matrices (Calc_rho1mode, gmctdh_objects.f90:408-477)
@@ -3006,6 +3019,19 @@ void tridiag_eig(int n, double* d, double* e, double* z) {
 void lan_finish(Ctx& c, LanRun& R) {
   RtScope rt(c, RT_LANCZOS);   // one call per Lanczos run
   const int nk = R.nk;
+  if (c.hb_prec == 1) {   // on the device, in the arithmetic these runs keep
+    launch_jacobi_tridiag(c.d_lan, c.d_lan + NKRYLOV_MAX, nk, c.d_lan + 2 * NKRYLOV_MAX,
+                          c.d_lan + 3 * NKRYLOV_MAX, c.d_status, c.st);
+    c.count();
+    c.lan_evals.assign(nk, 0.0);
+    c.lan_evecs.assign(nk * nk, 0.0);
+    CK(cudaMemcpyAsync(c.lan_evals.data(), c.d_lan + 2 * NKRYLOV_MAX, sizeof(double) * nk, cudaMemcpyDeviceToHost, c.st));
+    CK(cudaMemcpyAsync(c.lan_evecs.data(), c.d_lan + 3 * NKRYLOV_MAX, sizeof(double) * nk * nk,
+                       cudaMemcpyDeviceToHost, c.st));
+    check_status(c);
+    c.lan_nk = nk;
+    return;
+  }
   double* ab = c.h_scal + 128;   // pinned: alpha, beta
   CK(cudaMemcpyAsync(ab, c.d_lan, sizeof(double) * 2 * NKRYLOV_MAX, cudaMemcpyDeviceToHost, c.st));
   check_status(c);               // waits for the stream
@@ -3032,8 +3058,9 @@ void lan_combine(Ctx& c, cplx* BT, double dt) {
     }
   }
   CK(cudaMemcpyAsync(c.d_coef, coef.data(), sizeof(cplx) * nk, cudaMemcpyHostToDevice, c.st));
-  launch_gemv_cols(BT, c.d_krylov, n, c.d_coef, nk, n, c.st, c.lan_nrm);
-  launch_lan_normalize(BT, BT, c.lan_nrm.res, nullptr, n, c.st);
+  const bool fused = c.hb_prec != 1;   // the norm along with the combination
+  launch_gemv_cols(BT, c.d_krylov, n, c.d_coef, nk, n, c.st, fused ? c.lan_nrm : FusedDot{nullptr, nullptr, nullptr, nullptr});
+  launch_lan_normalize(BT, BT, fused ? c.lan_nrm.res : dot_dev(c, BT, BT, n), nullptr, n, c.st);
   c.count(2);
 }
 
@@ -3374,7 +3401,7 @@ void plan_cmf(Ctx& c, CmfState& S) {
       S.opsave = c.ar.calloc_c(off);
     }
     S.krylov0 = c.ar.calloc_c(c.naconftot * (NKRYLOV_MAX + 1));
-    S.lan0 = (double*)c.ar.alloc(sizeof(double) * (2 * NKRYLOV_MAX));
+    S.lan0 = (double*)c.ar.alloc(sizeof(double) * (3 * NKRYLOV_MAX + NKRYLOV_MAX * NKRYLOV_MAX));
   }
   S.elem_mode = upload_vec(c.ar, em);
   // the SPF error norms: compensated split FP32 (~1e-13) in the split modes
@@ -4144,7 +4171,7 @@ Ctx* create(const mctdh_setup_t* s, const MemberBufs* mb = nullptr) {
       }
       c->d_hb = c->ar.calloc_c(c->naconftot);
       c->d_krylov = c->ar.calloc_c(c->naconftot * (NKRYLOV_MAX + 1));
-      c->d_lan = (double*)c->ar.alloc(sizeof(double) * (2 * NKRYLOV_MAX));
+      c->d_lan = (double*)c->ar.alloc(sizeof(double) * (3 * NKRYLOV_MAX + NKRYLOV_MAX * NKRYLOV_MAX));
       c->d_coef = c->ar.calloc_c(NKRYLOV_MAX);
       plan_hb(*c);
       c->d_ovl1 = c->ar.calloc_c(c->ntot);
@@ -4492,7 +4519,7 @@ Ens* ens_create(const mctdh_setup_t* setups, int n) {
     merge_full(E->full, E->chains, E->chains_full, E->gprods, E->ar);
     merge_holes(E->all_holes, E->rho_holes, E->holes, E->ar);
     E->red.finalize(E->ar);
-    E->h1 = plan_h1(E->ar, E->h1_h, E->h1_proj);
+    E->h1 = plan_h1(E->ar, E->h1_h, E->h1_proj, E->precision == 1);
     E->msum_d = upload_vec(E->ar, E->msum_h);
     E->msum_src_d = upload_vec(E->ar, E->msum_src_h);
     E->reg_d = upload_vec(E->ar, E->reg_h);
@@ -4936,7 +4963,7 @@ void expectation(Ctx& c, cplx* values) {
     launch_gwp_h1(c.xgh1_d, (int)c.xgh1_h.size(), c.st);
     c.count(3);
   }
-  c.count(launch_h1(c.h1, true, c.st) + launch_h1(c.xh1, true, c.st));
+  c.count(launch_h1(c.h1x, true, c.st) + launch_h1(c.xh1, true, c.st));
   for (size_t i = 1; i < W.chain.size(); ++i) run_prod(c, W.chain[i]);
   run_hole(c, W.dots);
   run_red(c, W.red);

@@ -414,6 +414,110 @@ __global__ void __launch_bounds__(256) h1_kernel(const H1Desc* __restrict__ desc
   }
 }
 
+// acc (hi, lo) += a * b for FP32 pairs a = ah + al, b = bh + bl: the leading
+// product is split exactly with an FMA, the sum keeps its rounding error in lo.
+__device__ __forceinline__ void df_fma(float& sh, float& sl, float ah, float al, float bh, float bl) {
+  const float p = ah * bh;
+  float e = fmaf(ah, bh, -p);
+  e = fmaf(ah, bl, e);
+  e = fmaf(al, bh, e);
+  const float s = sh + p;
+  const float bp = s - sh;
+  const float t = (sh - (s - bp)) + (p - bp);
+  sh = s;
+  sl += t + e;
+}
+
+// Split-FP32 variant of h1_kernel, for contexts with FP32 mode products: the column is held
+// as FP32 (hi, lo) pairs, the DOF matrices come pre-split, every product is
+// accumulated as a compensated FP32 pair (df_fma, ~1e-13 relative).  FP32 products round
+// the operators' matrices to FP32: another 1e-13 in them now and then rounds an element the
+// other way, 6e-8 of it, so these contexts keep one arithmetic for them (the FP64 forms
+// are as fast: 62 us for 12 SPFs against 26 and 33).
+__global__ void __launch_bounds__(256) h1_split_kernel(const H1Desc* __restrict__ descs, int maxn2, bool project) {
+  extern __shared__ float4 smf[];
+  const H1Desc& d = descs[blockIdx.x / maxn2];
+  const int j2 = blockIdx.x % maxn2;
+  if (j2 >= d.n2) return;
+  const int G = d.G, n1 = d.n1;
+  float4* bufA = smf;
+  float4* bufB = smf + G;
+  const cplx* src = d.phi_r + (long long)G * j2;
+  for (int e = threadIdx.x; e < G; e += blockDim.x) {
+    const cplx v = src[e];
+    float hx, lx, hy, ly;
+    split_d2f(v.x, hx, lx);
+    split_d2f(v.y, hy, ly);
+    bufA[e] = make_float4(hx, hy, lx, ly);
+  }
+  __syncthreads();
+  int ll = 1;
+  for (int k = 0; k < d.ndof; ++k) {
+    const int ng = d.ng[k];
+    const int ot = d.optype[k];
+    if (ot != 0) {
+      const float2* Mf = d.matf[k];
+      for (int e = threadIdx.x; e < G; e += blockDim.x) {
+        const int a = e % ll;
+        const int gg = (e / ll) % ng;
+        const int bidx = e / (ll * ng);
+        float rh = 0.f, rl = 0.f, ih = 0.f, il = 0.f;
+        if (ot == 2) {
+          const float4 x = bufA[e];
+          const float2 m = Mf[gg];
+          df_fma(rh, rl, m.x, m.y, x.x, x.z);
+          df_fma(ih, il, m.x, m.y, x.y, x.w);
+        } else {
+          const float4* in = bufA + a + (long long)ll * ng * bidx;
+          const float2* mc = Mf + (long long)ng * gg;
+          for (int gp = 0; gp < ng; ++gp) {
+            const float4 x = in[(long long)ll * gp];
+            const float2 m = mc[gp];
+            df_fma(rh, rl, m.x, m.y, x.x, x.z);
+            df_fma(ih, il, m.x, m.y, x.y, x.w);
+          }
+        }
+        bufB[e] = (ot == 3) ? make_float4(-ih, rh, -il, rl) : make_float4(rh, ih, rl, il);
+      }
+      __syncthreads();
+      float4* t = bufA; bufA = bufB; bufB = t;
+    }
+    ll *= ng;
+  }
+  cplx* dst = d.ophi + (long long)G * j2;
+  for (int e = threadIdx.x; e < G; e += blockDim.x) {
+    const float4 x = bufA[e];
+    dst[e] = mkc(f2d_exact(x.x) + f2d_exact(x.z), f2d_exact(x.y) + f2d_exact(x.w));
+  }
+  if (!project) return;
+  const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
+  for (int j1 = warp; j1 < n1; j1 += (int)(blockDim.x >> 5)) {
+    const cplx* pl = d.phi_l + (long long)G * j1;
+    float rh = 0.f, rl = 0.f, ih = 0.f, il = 0.f;
+    for (int gg = lane; gg < G; gg += 32) {
+      const cplx p = pl[gg];
+      float phx, plx, phy, ply;
+      split_d2f(p.x, phx, plx);
+      split_d2f(p.y, phy, ply);
+      const float4 x = bufA[gg];
+      // conj(p) * x
+      df_fma(rh, rl, phx, plx, x.x, x.z);
+      df_fma(rh, rl, phy, ply, x.y, x.w);
+      df_fma(ih, il, phx, plx, x.y, x.w);
+      df_fma(ih, il, -phy, -ply, x.x, x.z);
+    }
+    cplx s = mkc(f2d_exact(rh) + f2d_exact(rl), f2d_exact(ih) + f2d_exact(il));
+    for (int o = 16; o > 0; o >>= 1) {
+      s.x += __shfl_down_sync(0xffffffffu, s.x, o);
+      s.y += __shfl_down_sync(0xffffffffu, s.y, o);
+    }
+    if (lane == 0) {
+      if (d.same_state) d.X[j1 + n1 * j2] = s;
+      else d.h[j1 + n1 * j2] = s;
+    }
+  }
+}
+
 // Blocks 0 .. nh - 1: same-state h1mode = (X + X^H) / 2 (the zher2k form,
 // hamilton.f90:500-506).  The others: operators pre-summed per state and mode,
 // out = sum_k coeff_k src_k, from the same X.
@@ -451,9 +555,11 @@ int launch_h1(const H1Launch& b, bool with_h, cudaStream_t st, const MatSumDesc*
     static size_t configured = 0;
     if (b.smem > 48 * 1024 && b.smem > configured) {
       cudaFuncSetAttribute(h1_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)b.smem);
+      cudaFuncSetAttribute(h1_split_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)b.smem);
       configured = b.smem;
     }
-    h1_kernel<<<(unsigned)(b.n * b.maxn2), 256, b.smem, st>>>(b.d, b.maxn2, with_h && !proj);
+    if (b.split) h1_split_kernel<<<(unsigned)(b.n * b.maxn2), 256, b.smem, st>>>(b.d, b.maxn2, with_h);
+    else h1_kernel<<<(unsigned)(b.n * b.maxn2), 256, b.smem, st>>>(b.d, b.maxn2, with_h && !proj);
     ++launches;
   }
   if (proj) {
@@ -952,6 +1058,38 @@ void launch_dot(const cplx* a, const cplx* b, long long n, cplx* partial, unsign
   dot_kernel<<<DOT_BLOCKS, 256, 0, st>>>(a, b, n, partial, counter, out);
 }
 
+// Tridiagonal eigenproblem of the Lanczos matrix (dstev, cmf2_integration.f90:85), for
+// Lanczos runs on FP32 products (see grid_sum_tree).
+__global__ void tridiag_kernel(const double* alpha, const double* beta, int n, double* evals, double* evecs,
+                               int* status) {
+  __shared__ cplx A[MAXN_SPF * MAXN_SPF];
+  __shared__ cplx V[MAXN_SPF * MAXN_SPF];
+  __shared__ JacRot R[MAXN_SPF / 2];
+  const int ld = MAXN_SPF;
+  for (int e = threadIdx.x; e < n * n; e += blockDim.x) {
+    int i = e % n, j = e / n;
+    double v = 0.0;
+    if (i == j) v = alpha[i];
+    else if (j == i + 1) v = beta[i];
+    else if (i == j + 1) v = beta[j];
+    A[i + ld * j] = mkc(v, 0.0);
+  }
+  __syncthreads();
+  bool ok;
+  jacobi_herm(A, V, n, ld, R, &ok);
+  if (!ok && threadIdx.x == 0) atomicOr(status, DEVST_EIG_NOCONV);
+  for (int e = threadIdx.x; e < n * n; e += blockDim.x) {
+    int i = e % n, j = e / n;
+    evecs[i + n * j] = V[i + ld * j].x;   // real symmetric input keeps V real
+  }
+  if (threadIdx.x < n) evals[threadIdx.x] = A[threadIdx.x + ld * threadIdx.x].x;
+}
+
+void launch_jacobi_tridiag(const double* alpha, const double* beta, int n, double* evals, double* evecs,
+                           int* d_status, cudaStream_t st) {
+  tridiag_kernel<<<1, 32, 0, st>>>(alpha, beta, n, evals, evecs, d_status);
+}
+
 // ---------------------------------------------------------------------------
 // Elementwise helpers
 // ---------------------------------------------------------------------------
@@ -996,6 +1134,49 @@ __device__ void grid_sum_c(cplx v, cplx* partial, unsigned* counter, cplx* out) 
   for (int q = tid; q < (int)gridDim.x; q += GRID_SUM_THREADS) t = cadd(t, mkc(pv[2 * q], pv[2 * q + 1]));
   block_sum_c(t, sv, &r);
   if (tid == 0) {
+    *out = r;
+    *counter = 0u;
+  }
+}
+
+// The same with a tree in every warp, the order of Lanczos runs on FP32 products: these
+// round every Krylov vector to FP32, so that a last-bit change of a sum (or of the
+// eigenvectors above) is carried to FP32 level within a few steps; these runs keep one
+// arithmetic, which costs about 300 us a CMF2 step of the 8-SPF QVC model.
+__device__ __forceinline__ cplx warp_sum_cd(cplx v) {
+  for (int off = 16; off > 0; off >>= 1) {
+    v.x += __shfl_down_sync(0xffffffffu, v.x, off);
+    v.y += __shfl_down_sync(0xffffffffu, v.y, off);
+  }
+  return v;
+}
+__device__ void grid_sum_tree(cplx v, cplx* partial, unsigned* counter, cplx* out) {
+  __shared__ cplx ws[32];
+  __shared__ bool last;
+  const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5, nw = (blockDim.x + 31) >> 5;
+  v = warp_sum_cd(v);
+  if (lane == 0) ws[warp] = v;
+  __syncthreads();
+  if (tid == 0) {
+    cplx t = ws[0];
+    for (int w = 1; w < nw; ++w) t = cadd(t, ws[w]);
+    partial[blockIdx.x] = t;
+    __threadfence();
+    last = (atomicAdd(counter, 1u) == gridDim.x - 1);
+  }
+  __syncthreads();
+  if (!last) return;
+  __threadfence();
+  const volatile double* pv = (const volatile double*)partial;
+  cplx t = mkc(0.0, 0.0);
+  for (int q = tid; q < (int)gridDim.x; q += blockDim.x) t = cadd(t, mkc(pv[2 * q], pv[2 * q + 1]));
+  t = warp_sum_cd(t);
+  __syncthreads();
+  if (lane == 0) ws[warp] = t;
+  __syncthreads();
+  if (tid == 0) {
+    cplx r = ws[0];
+    for (int w = 1; w < nw; ++w) r = cadd(r, ws[w]);
     *out = r;
     *counter = 0u;
   }
@@ -1132,11 +1313,83 @@ __global__ void __launch_bounds__(256, 4) termsum_kernel(cplx* __restrict__ out,
   if (dot.v) grid_sum_c(d, dot.partial, dot.counter, dot.res);
 }
 
+// FP32 term sum with the launch-wide <dot.v|out> in the order of grid_sum_tree: contiguous
+// shares per block, four elements per thread in flight.
+__global__ void __launch_bounds__(256) termsum_f32_dot_kernel(cplx* __restrict__ out, const SumRange* __restrict__ ranges,
+                                                      int nr, const SumSrc* __restrict__ srcs, long long total,
+                                                      FusedDot dot) {
+  __shared__ SumSrc ss[TERMSUM_CACHE];
+  __shared__ int s_rg;
+  const long long chunk = (total + gridDim.x - 1) / gridDim.x;
+  const long long start = (long long)blockIdx.x * chunk, end = min(total, start + chunk);
+  cplx d = mkc(0, 0);
+  long long base = start;
+  while (base < end) {
+    if (threadIdx.x == 0) {
+      int lo = 0, hi = nr - 1;   // last range starting at or before base (ranges sorted by offset)
+      while (lo < hi) {
+        const int mid = (lo + hi + 1) >> 1;
+        if (ranges[mid].offset <= base) lo = mid; else hi = mid - 1;
+      }
+      s_rg = lo;
+    }
+    __syncthreads();
+    const SumRange rg = ranges[s_rg];
+    long long seg_end = min(end, rg.offset + rg.n);
+    if (base < rg.offset || base >= rg.offset + rg.n) {
+      // outside every range: skip to the next range start
+      seg_end = (s_rg + 1 < nr) ? min(end, ranges[s_rg + 1].offset) : end;
+      __syncthreads();
+      base = max(seg_end, base + 1);
+      continue;
+    }
+    const bool cached = rg.count <= TERMSUM_CACHE;
+    if (cached)
+      for (int k = threadIdx.x; k < rg.count; k += blockDim.x) ss[k] = srcs[rg.first + k];
+    __syncthreads();
+    const SumSrc* sp = cached ? ss : srcs + rg.first;
+    {
+      // four elements per thread in flight: per source, four independent loads
+      const long long stride = (long long)blockDim.x;
+      for (long long i0 = base + threadIdx.x; i0 < seg_end; i0 += 4 * stride) {
+        float ar[4] = {0.f, 0.f, 0.f, 0.f}, ai[4] = {0.f, 0.f, 0.f, 0.f};
+        for (int k = 0; k < rg.count; ++k) {
+          const float cr = sp[k].cs[0] + sp[k].cs[1], ci = sp[k].cs[2] + sp[k].cs[3];
+          const cplx* src = sp[k].src;
+          const int fmt = sp[k].fmt;
+#pragma unroll
+          for (int e = 0; e < 4; ++e) {
+            const long long i = i0 + e * stride;
+            if (i >= seg_end) break;
+            const float4 x = load_split(src, i - rg.offset, fmt);
+            const float xr = x.x + x.z, xi = x.y + x.w;
+            ar[e] = fmaf(cr, xr, fmaf(-ci, xi, ar[e]));
+            ai[e] = fmaf(cr, xi, fmaf(ci, xr, ai[e]));
+          }
+        }
+#pragma unroll
+        for (int e = 0; e < 4; ++e) {
+          const long long i = i0 + e * stride;
+          if (i >= seg_end) break;
+          const cplx val = mkc(f2d_exact(ar[e]), f2d_exact(ai[e]));
+          out[i] = val;
+          cfma_conj(d, dot.v[i], val);
+        }
+      }
+      __syncthreads();
+      base = seg_end;
+    }
+  }
+  grid_sum_tree(d, dot.partial, dot.counter, dot.res);
+}
+
 void launch_termsum(cplx* out, const SumRange* d_ranges, int nranges, const SumSrc* d_srcs, long long total,
                     cudaStream_t st, int prec, FusedDot dot) {
   if (total <= 0) return;
   const unsigned nb = (unsigned)std::min<long long>((total + 255) / 256, FUSED_BLOCKS);
-  if (prec == 1)
+  if (prec == 1 && dot.v)
+    termsum_f32_dot_kernel<<<nb, 256, 0, st>>>(out, d_ranges, nranges, d_srcs, total, dot);
+  else if (prec == 1)
     termsum_kernel<1><<<nb, 256, 0, st>>>(out, d_ranges, nranges, d_srcs, total, dot);
   else
     termsum_kernel<0><<<nb, 256, 0, st>>>(out, d_ranges, nranges, d_srcs, total, dot);
@@ -1275,7 +1528,7 @@ void launch_axpy(cplx* y, const cplx* x, cplx a, long long n, cudaStream_t st) {
   axpy_kernel<<<(unsigned)((n + 255) / 256), 256, 0, st>>>(y, x, a, n);
 }
 
-// out = sum_j coef_j basis_j, and the launch-wide ||out||^2
+// out = sum_j coef_j basis_j, and with nrm.res the launch-wide ||out||^2
 __global__ void __launch_bounds__(256) gemv_cols_kernel(cplx* __restrict__ out, const cplx* __restrict__ basis,
                                                         long long ld, const cplx* __restrict__ coef, int ncol,
                                                         long long n, FusedDot nrm) {
@@ -1287,7 +1540,7 @@ __global__ void __launch_bounds__(256) gemv_cols_kernel(cplx* __restrict__ out, 
     out[i] = s;
     s2 = fma(s.x, s.x, fma(s.y, s.y, s2));
   }
-  grid_sum_c(mkc(s2, 0.0), nrm.partial, nrm.counter, nrm.res);
+  if (nrm.res) grid_sum_c(mkc(s2, 0.0), nrm.partial, nrm.counter, nrm.res);
 }
 void launch_gemv_cols(cplx* out, const cplx* basis, long long ld, const cplx* coef, int ncol, long long n,
                       cudaStream_t st, FusedDot nrm) {
@@ -1473,7 +1726,7 @@ __global__ void lan_axpy_kernel(cplx* __restrict__ Kn, const cplx* __restrict__ 
     Kn[i] = w;
     s2 = fma(w.x, w.x, fma(w.y, w.y, s2));
   }
-  if (nrm.res) grid_sum_c(mkc(s2, 0.0), nrm.partial, nrm.counter, nrm.res);
+  if (nrm.res) grid_sum_tree(mkc(s2, 0.0), nrm.partial, nrm.counter, nrm.res);
 }
 void launch_lan_axpy(cplx* Kn, const cplx* Kj, const cplx* Kp, const cplx* dot_alpha, const double* beta_prev,
                      double* alpha_out, long long n, cudaStream_t st, FusedDot nrm) {

@@ -79,6 +79,7 @@ struct H1Desc {
   int ng[MAXDOF_MODE];
   int optype[MAXDOF_MODE]; // 0 none, 1 dense real, 2 diagonal, 3 dense imaginary (i x real)
   const cplx* mat[MAXDOF_MODE];
+  const float2* matf[MAXDOF_MODE];  // the real coefficients split into FP32 (hi, lo)
 };
 
 // Regularised inverse of a Hermitian n x n matrix by Jacobi rotations
@@ -285,6 +286,7 @@ struct H1Launch {
   int n, maxn2;
   size_t smem;
   HoleLaunch proj;
+  bool split;              // split FP32 (no proj)
 };
 int launch_h1(const H1Launch& b, bool with_h, cudaStream_t st, const MatSumDesc* sums = nullptr, int nsums = 0,
               const MatSumSrc* srcs = nullptr);
@@ -377,6 +379,8 @@ void launch_stage_modes(cplx* out, const cplx* base, const StageArgs& a, const d
 void launch_masked_copy(cplx* y, const cplx* src, const unsigned char* elem_mode, const int* accept, long long off,
                         long long n, cudaStream_t st);
 void launch_spf_err(const SpfErrDesc* d, int nd, double* err_mode, int nmodes, cudaStream_t st);
+void launch_jacobi_tridiag(const double* alpha, const double* beta, int n, double* evals, double* evecs,
+                           int* d_status, cudaStream_t st);
 void launch_lan_axpy(cplx* Kn, const cplx* Kj, const cplx* Kp, const cplx* dot_alpha, const double* beta_prev,
                      double* alpha_out, long long n, cudaStream_t st,
                      FusedDot nrm = FusedDot{nullptr, nullptr, nullptr, nullptr});
