@@ -59,11 +59,11 @@ typedef struct mctdh_setup {
   double min_stepsize, writetime;
   double der_factor_re, der_factor_im;  /* -i for propagation, -1 for relaxation */
   int64_t int_type_psi;                 /* 1 = Cash-Karp for the CMF2 SPF sweeps  */
-  int64_t precision;                    /* 0 FP64; 1 FP32 products, compensated contractions;
-                                           2 compensated products and contractions; 3 FP32 products
-                                           and contractions; 4 as 1 with compensated H_B products of the
-                                           Lanczos steps; 5 as 2 with FP32 H_B products; 6 as 1 with
-                                           FP32-summed mean-field contractions (densities compensated) */
+  int64_t precision;                    /* 0 FP64; 1 FP32 products, contractions of FP64 accuracy;
+                                           2 as 0; 3 FP32 products and contractions; 4 as 1 with H_B
+                                           products of the Lanczos steps of FP64 accuracy; 5 as 2 with
+                                           FP32 H_B products; 6 as 1 with FP32-summed mean-field
+                                           contractions (densities of FP64 accuracy) */
   int64_t int_order, int_par1;          /* Adams PECE order and extra EC iterations (abm<order><par1>) */
   /* Operators whose expectation values are written (the 'expect' keyword,
    * input.f90:196-216, terms read by Read_Operators, input.f90:516-748).  Their

@@ -96,7 +96,7 @@ struct ProdBatch {
   ProdDesc* d = nullptr;
   long long nblocks = 0;
   int maxn = 0;
-  int prec = 0;                  // 0 FP64, 1 split FP32, 2 split FP32 compensated
+  int prec = 0;                  // 1 FP32, else FP64 accuracy (digit products)
   double flops = 0, bytes = 0;   // algorithmic work of one launch
   void add(const cplx* X, cplx* Y, const cplx* M, int ldm, int conjT, const std::vector<int>& shape, int mode,
            int nout, cplx alpha, int accumulate, int xfmt = TF_C64, int yfmt = TF_C64) {
@@ -481,9 +481,9 @@ struct Ctx {
   cplx der = mkc(0, -1);
   int int_type_psi = 1;
   int precision = 0;
-  int hole_prec = 0;   // single-hole contractions: 0 FP64, 1 FP32 sums, 2 compensated FP32
+  int hole_prec = 0;   // single-hole contractions: 1 FP32 sums, 0 and 2 FP64 accuracy
   int mf_hole_prec = 0;   // the mean-field ones (densities keep hole_prec)
-  int hb_prec = 0;     // H_B * B products of the Lanczos steps: 0 FP64, 1 FP32, 2 compensated FP32
+  int hb_prec = 0;     // H_B * B products of the Lanczos steps: 1 FP32, 0 and 2 FP64 accuracy
   bool reginv_cold = false;   // regularised inverses without the Jacobi warm start
   std::string last_error;
   long long launches = 0;
@@ -818,9 +818,9 @@ void load_setup(Ctx& c, const mctdh_setup_t* s) {
   c.precision = (int)s->precision;
   if (c.precision < 0 || c.precision > 6) throw StatusError(MCTDH_EARG, "precision must be 0 .. 6");
   // precision 3: the products of precision 1 with FP32-accumulated contractions;
-  // 4: FP32 mean-field and A-derivative products, compensated H_B products;
-  // 5: compensated mean-field and A-derivative products, FP32 H_B products;
-  // 6: precision 1 with FP32-accumulated mean-field contractions (densities compensated)
+  // 4: FP32 mean-field and A-derivative products, FP64-accurate H_B products;
+  // 5: FP64-accurate mean-field and A-derivative products, FP32 H_B products;
+  // 6: precision 1 with FP32-accumulated mean-field contractions (densities FP64-accurate)
   c.hole_prec = c.precision == 3 ? 1 : (c.precision ? 2 : 0);
   c.mf_hole_prec = (c.precision == 6) ? 1 : c.hole_prec;
   c.hb_prec = c.precision == 4 ? 2 : (c.precision == 5 || c.precision == 3 || c.precision == 6 ? 1 : c.precision);
@@ -1598,7 +1598,7 @@ void plan_eom(Ctx& c) {
   c.msum_src_d = upload_vec(c.ar, c.msum_src_h);
   // Precision: the chain products run in the context's precision (FP32 in
   // precision 1).  The contractions of the mean fields and density matrices use
-  // the compensated split (about 1e-13 relative) whenever a split mode is chosen:
+  // FP64-accurate digit products except in precisions 3 and 6:
   // the regularised inverse of rho scales mean-field errors by up to 1/eps_rho.
   for (auto& b : c.chains_full) {
     b.prec = c.precision;
@@ -1612,7 +1612,7 @@ void plan_eom(Ctx& c) {
   c.gprods.finalize(c.ar);
   c.holes.prec = c.mf_hole_prec;
   c.holes.finalize(c.ar);
-  // density matrices: compensated split FP32 (~1e-13 relative) in the split modes
+  // density matrices: FP64 accuracy except in precision 3
   c.rho_holes.prec = c.hole_prec;
   c.rho_holes.finalize(c.ar);
   merge_full(c.full, c.chains, c.chains_full, c.gprods, c.ar);
@@ -1919,9 +1919,8 @@ void plan_hb(Ctx& c) {
 
 // Overlap plan between states y1 and y2: o11 = <1|1>, o22 = <2|2>, o12 = <1|2>
 // (norm_wf / WF_Ovl / DeltaPsi, gmctdh_objects.f90:21-226).  prec 2: the mode
-// products of the chains in compensated split FP32 (~1e-13 relative); used for
-// the step-error norm DeltaPsi of split-precision contexts, where 1 - Re<1|2>/..
-// is of order eps_int^2 / 2 >> 1e-13.  Norms and C(t) keep prec 0.
+// products of the chains may take FP32 operands' storage; like prec 0 they have FP64
+// accuracy.
 void plan_ovl(Ctx& c, OvlPlan& P, cplx* y1, cplx* y2, int prec, bool norm_only, bool shared) {
   const int f = c.nmodes;
   P.npk = c.npk;
@@ -1985,8 +1984,7 @@ void plan_ovl(Ctx& c, OvlPlan& P, cplx* y1, cplx* y2, int prec, bool norm_only, 
     }
   }
   P.gwp_d = upload_vec(c.ar, P.gwp_h);
-  // the SPF overlaps over the grid: compensated split FP32 (~1e-13) where the
-  // plan's chains are (the step-error overlaps of the split paths), else FP64
+  // the SPF overlaps over the grid, FP64 accuracy in either
   P.spf_holes.prec = prec;
   P.spf_holes.finalize(c.ar);
   for (auto& hr : hrefs) P.spf_red.add_term(hr.target, P.spf_holes.h[hr.hole], hr.alpha);
@@ -3404,7 +3402,7 @@ void plan_cmf(Ctx& c, CmfState& S) {
     S.lan0 = (double*)c.ar.alloc(sizeof(double) * (3 * NKRYLOV_MAX + NKRYLOV_MAX * NKRYLOV_MAX));
   }
   S.elem_mode = upload_vec(c.ar, em);
-  // the SPF error norms: compensated split FP32 (~1e-13) in the split modes
+  // the SPF error norms, FP64 accuracy in every mode
   S.err_holes.prec = c.precision ? 2 : 0;
   S.err_holes.finalize(c.ar);
   for (auto& hr : hrefs) S.err_red.add_term(hr.target, S.err_holes.h[hr.hole], hr.alpha);
@@ -4178,8 +4176,7 @@ Ctx* create(const mctdh_setup_t* s, const MemberBufs* mb = nullptr) {
       c->d_ovl2 = c->ar.calloc_c(c->ntot);
       plan_ovl(*c, c->cmf_ovl, c->d_ovl1, c->d_ovl2, (c->precision && c->eps_int >= 1e-5) ? 2 : 0, false, false);
     }
-    // the compensated products of DeltaPsi (~1e-13) resolve 1 - Re<1|2>/.. ~ eps_int^2 / 2
-    // only for loose tolerances; tight ones keep FP64
+    // prec 0 and 2 are the same arithmetic by now
     plan_ovl(*c, c->dpsi_plan, c->d_tmp, c->d_err, (c->precision && c->eps_int >= 1e-5) ? 2 : 0);
     plan_ovl(*c, c->auto_plan, c->d_y0, c->d_y, 0);
     plan_ovl(*c, c->io_plan, c->d_in, c->d_out, 0);
