@@ -53,10 +53,10 @@ MFX_GATE = 0.5
 # H_B*B launches)
 TRAFFIC_PER_ALG_BYTE = {"mode_product": 0.385}
 ROOF_BOUND = {"mode_product": "hbm", "hole_contract": "hbm", "spf_derivative": "hbm"}
-ROOF_NOTE = {"mode_product": "not HBM: the compensated mean-field products are FMA-issue bound (55 % of the FMA "
-                             "pipe), the FP32 H_B products load-latency bound; operands mostly L2-resident "
-                             "(12.6 MB state)",
-             "hole_contract": "compensated FP32 sums: FP32 issue",
+ROOF_NOTE = {"mode_product": "not HBM: the mean-field products of FP64 accuracy are bound by instruction issue "
+                             "(cutting and joining digits), the FP32 H_B products by load latency; operands "
+                             "mostly L2-resident (12.6 MB state)",
+             "hole_contract": "cutting operands into digits: ALU",
              "spf_derivative": "small per-mode problems: latency and occupancy"}
 ACC_FS = 0.5   # short comparison interval of the size scan
 REF_BUDGET_S = 150.0   # timed seconds after which the reference arm stops early
@@ -162,11 +162,11 @@ def flush_l2(buf):
     buf.add_(1.0)
 
 
-PRECISION_LABEL = {0: "fp64", 1: "fp32 products, compensated fp32 contractions",
-                   2: "compensated fp32 products and contractions", 3: "fp32 products and contractions",
-                   4: "fp32 mean-field products, compensated H_B products and contractions",
-                   5: "compensated mean-field products and contractions, fp32 H_B products",
-                   6: "fp32 products and mean-field contractions, compensated densities"}
+PRECISION_LABEL = {0: "fp64", 1: "fp32 products, contractions of fp64 accuracy",
+                   2: "products and contractions of fp64 accuracy", 3: "fp32 products and contractions",
+                   4: "fp32 mean-field products, H_B products and contractions of fp64 accuracy",
+                   5: "mean-field products and contractions of fp64 accuracy, fp32 H_B products",
+                   6: "fp32 products and mean-field contractions, densities of fp64 accuracy"}
 
 
 def precision_label(prec):
@@ -870,7 +870,7 @@ def main():
                     help="extrapolator: seeded initial-state variants recorded besides the start state")
     ap.add_argument("--pre-fs", type=float, default=0.3, help="qvc24: untimed FP64 propagation before the steps")
     ap.add_argument("--precision", type=int, default=5, choices=[0, 1, 2, 3, 4, 5, 6],
-                    help="arm timed against the FP64 path (mode of mctdh_setup_t.precision; 5: compensated "
+                    help="arm timed against the FP64 path (mode of mctdh_setup_t.precision; 5: FP64-accurate "
                          "mean-field products and contractions, FP32 Lanczos H_B products)")
     ap.add_argument("--workload", default="qvc12",
                     choices=["qvc12", "qvc12n", "qvc24", "ensemble", "lvc5", "gmctdh16", "lvc5mix", "accuracy"],
