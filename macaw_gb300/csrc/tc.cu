@@ -257,7 +257,7 @@ __global__ void __launch_bounds__(128, NG <= 2 ? 4 : 2)
   uint32_t parity = 0;
   bool ok = true;
   int di = t0 < tend ? warp_find_desc(descs, ndesc, t0) : 0;
-  for (; t0 < tend && ok; ++di) {
+  for (; t0 < tend; ++di) {
     const ProdDesc& d = descs[di];
     const int nin = d.nin, nout = d.nout;
     const unsigned L = (unsigned)d.L, nfib = (unsigned)(d.L * d.R);
@@ -305,6 +305,11 @@ __global__ void __launch_bounds__(128, NG <= 2 ? 4 : 2)
     }
     const bool plain = !d.accumulate && d.alpha.x == 1.0 && d.alpha.y == 0.0;
     for (; t0 < dend; ++t0) {
+      if (!ok) {   // a wait ran out (never expected): the rest of the tiles in FP64
+        if (p < nfib) prod_fibre_fp64(d, p % L, p / L);
+        p += 128;
+        continue;
+      }
       unsigned mag = 0u;
 #pragma unroll
       for (int j = 0; j < 4 * NG; ++j) mag = max(mag, fx_mag(x[j]));
@@ -342,16 +347,15 @@ __global__ void __launch_bounds__(128, NG <= 2 ? 4 : 2)
         r = p / L;
         fetch();
       }
-      // every thread polls; the verdict is made uniform so that all leave together
+      // every thread polls; the verdict is made uniform
       ok = __syncthreads_and(tc_wait(&bar, parity));
       parity ^= 1;
       tc_fence_after();
-      if (!ok) break;
       const bool act = pc < nfib;
       cplx* y = d.Y + ((long long)pc + Ly * rc);
 #pragma unroll
       for (int h = 0; h < NG; ++h) {
-        if (4 * h >= nout) break;
+        if (4 * h >= nout || !ok) break;
         float c[8][8];
         tc_ld8x8(tmem + ((uint32_t)(warp * 32) << 16) + 8 * h, T::WC, c);
 #pragma unroll
@@ -367,7 +371,7 @@ __global__ void __launch_bounds__(128, NG <= 2 ? 4 : 2)
           }
         }
       }
-      if (act && bad) prod_fibre_fp64(d, pc - L * rc, rc);
+      if (act && (bad || !ok)) prod_fibre_fp64(d, pc - L * rc, rc);
     }
     t0 = dend;
   }
