@@ -4110,6 +4110,7 @@ Ctx* create(const mctdh_setup_t* s, const MemberBufs* mb = nullptr) {
     throw StatusError(MCTDH_ECUDA, "no CUDA device available (this core has no CPU fallback)");
   Ctx* c = new Ctx();
   try {
+    if (!mb) CK(prepare_device());
     if (mb) {
       c->st = mb->st;
       c->own_stream = false;
@@ -4406,6 +4407,7 @@ Ens* ens_create(const mctdh_setup_t* setups, int n) {
   if (n < 1) throw StatusError(MCTDH_EARG, "empty ensemble");
   Ens* E = new Ens();
   try {
+    CK(prepare_device());
     CK(cudaStreamCreateWithFlags(&E->st, cudaStreamNonBlocking));
     // sizes first: the member layout fixes the ensemble vectors
     E->off.assign(n + 1, 0);

@@ -6,16 +6,6 @@
 #include "kernels.cuh"
 #include "fixed.cuh"
 
-static int sm_count() {
-  static const int n = [] {
-    int dev = 0, v = 0;
-    cudaGetDevice(&dev);
-    cudaDeviceGetAttribute(&v, cudaDevAttrMultiProcessorCount, dev);
-    return v > 0 ? v : 152;
-  }();
-  return n;
-}
-
 // ---------------------------------------------------------------------------
 // Batched mode product (Mult_HeM_MatV / Mult_GM_MatV, gmctdh_objects.f90:1407-1468)
 // A warp owns 16 fibres (l, :, r) (the rows of the MMA), the columns are the (re, im)
@@ -209,16 +199,16 @@ __global__ void __launch_bounds__(PROD_THREADS, prod_ctas<NJ>())
 }
 
 template <int NJ>
+constexpr int prod_smem() {
+  return NJ * ((NJ + 1) / 2) * PROD_NS * 32 * (int)sizeof(uint2);
+}
+template <int NJ>
 static void prod_fx_go(const ProdDesc* d, int nd, long long nblocks, int persist, cudaStream_t st) {
-  constexpr int smem = NJ * ((NJ + 1) / 2) * PROD_NS * 32 * (int)sizeof(uint2);
-  static const cudaError_t configured =
-      cudaFuncSetAttribute(prod_fx_kernel<NJ>, cudaFuncAttributeMaxDynamicSharedMemorySize, smem);
-  (void)configured;
   long long most = (long long)sm_count() * prod_ctas<NJ>();
   // below one 64-fibre unit per SM the latency of a unit counts, not its cost
   const int split = 2 * nblocks < sm_count();
   if (persist > 0) most = std::min<long long>(most, persist);
-  prod_fx_kernel<NJ><<<(unsigned)std::min((split ? 8 : 2) * nblocks, most), PROD_THREADS, smem, st>>>(d, nd, nblocks, split);
+  prod_fx_kernel<NJ><<<(unsigned)std::min((split ? 8 : 2) * nblocks, most), PROD_THREADS, prod_smem<NJ>(), st>>>(d, nd, nblocks, split);
 }
 
 // The tcgen05 form (tc.cu) takes batches of 5 to 16 SPFs that give every one of its CTAs
@@ -763,9 +753,6 @@ __global__ void __launch_bounds__(64 * HOLE_WARPS, 2)
 
 template <bool F32>
 static void hole_fx_go(const HoleLaunch& b, int persist, cudaStream_t st, const cplx* ybase) {
-  static const cudaError_t configured =
-      cudaFuncSetAttribute(hole_wide_kernel<F32>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)sizeof(HoleWide));
-  (void)configured;
   auto grid = [&](long long n) { return (unsigned)(persist > 0 ? std::min<long long>(n, persist) : n); };
   const long long wide = b.nblocks - b.narrow_blocks;
   if (b.narrow_blocks > 0)
@@ -779,4 +766,12 @@ static void hole_fx_go(const HoleLaunch& b, int persist, cudaStream_t st, const 
 void launch_hole_fx(const HoleLaunch& b, cudaStream_t st, int persist, const cplx* ybase) {
   if (b.f32) hole_fx_go<true>(b, persist, st, ybase);
   else hole_fx_go<false>(b, persist, st, ybase);
+}
+
+cudaError_t configure_fx() {
+  cudaError_t e = allow_smem(prod_fx_kernel<8>, prod_smem<8>());   // the others' is below 48 KB
+  static_assert(prod_smem<6>() <= 48 * 1024, "needs the opt-in");
+  if (e == cudaSuccess) e = allow_smem(hole_wide_kernel<false>, sizeof(HoleWide));
+  if (e == cudaSuccess) e = allow_smem(hole_wide_kernel<true>, sizeof(HoleWide));
+  return e;
 }

@@ -6,6 +6,7 @@
 // are staged in shared memory for the single-hole contractions, and reductions
 // are two-stage with a fixed summation order so reruns are bitwise identical.
 #include <algorithm>
+#include <atomic>
 
 #include "kernels.cuh"
 #include "fixed.cuh"
@@ -117,6 +118,18 @@ bool tc_enabled() {
     on = (e && e[0] == '0') ? 0 : 1;
   }
   return on == 1;
+}
+
+int sm_count() {
+  static std::atomic<int> known[64];
+  int dev = 0;
+  if (cudaGetDevice(&dev) != cudaSuccess || dev < 0 || dev >= 64) return 152;
+  int n = known[dev].load(std::memory_order_relaxed);
+  if (n == 0) {
+    if (cudaDeviceGetAttribute(&n, cudaDevAttrMultiProcessorCount, dev) != cudaSuccess || n <= 0) n = 152;
+    known[dev].store(n, std::memory_order_relaxed);
+  }
+  return n;
 }
 
 // prec 0 and 2: FP64 accuracy (fixed.cu); prec 1: FP32 products.
@@ -547,17 +560,20 @@ __global__ void h1_finish_kernel(const H1Desc* __restrict__ descs, int nh, const
   }
 }
 
+cudaError_t prepare_device() {
+  cudaError_t e = allow_smem(h1_kernel, 227 * 1024);
+  if (e == cudaSuccess) e = allow_smem(h1_split_kernel, 227 * 1024);
+  if (e == cudaSuccess) e = configure_fx();
+  if (e == cudaSuccess) e = configure_spf();
+  if (e == cudaSuccess) e = configure_tc();
+  return e;
+}
+
 int launch_h1(const H1Launch& b, bool with_h, cudaStream_t st, const MatSumDesc* sums, int nsums,
               const MatSumSrc* srcs) {
   int launches = 0;
   const bool proj = with_h && b.proj.ndesc > 0;
   if (b.n > 0) {
-    static size_t configured = 0;
-    if (b.smem > 48 * 1024 && b.smem > configured) {
-      cudaFuncSetAttribute(h1_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)b.smem);
-      cudaFuncSetAttribute(h1_split_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)b.smem);
-      configured = b.smem;
-    }
     if (b.split) h1_split_kernel<<<(unsigned)(b.n * b.maxn2), 256, b.smem, st>>>(b.d, b.maxn2, with_h);
     else h1_kernel<<<(unsigned)(b.n * b.maxn2), 256, b.smem, st>>>(b.d, b.maxn2, with_h && !proj);
     ++launches;

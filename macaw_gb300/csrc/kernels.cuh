@@ -235,6 +235,18 @@ struct StageArgs {
 };
 
 // Launch helpers (kernels.cu)
+// SMs of the current device
+int sm_count();
+// Lets the kernels have the dynamic shared memory they need on the current device: the
+// limit belongs to a device, so every context creation sets it on its own.
+cudaError_t prepare_device();
+cudaError_t configure_fx();
+cudaError_t configure_spf();
+cudaError_t configure_tc();
+template <typename K>
+cudaError_t allow_smem(K* kernel, size_t bytes) {
+  return cudaFuncSetAttribute((const void*)kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)bytes);
+}
 bool tc_enabled();
 void tc_prepare();
 bool launch_prod_tc(const ProdDesc* d_descs, int ndesc, long long nblocks, int maxn, cudaStream_t st, bool force);

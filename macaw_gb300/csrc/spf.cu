@@ -570,14 +570,6 @@ int launch_spf(const SpfDesc* d_descs, int ndesc, long long ntiles, int maxn, co
                const SpfStage& stage) {
   if (ndesc <= 0) return 0;
   const int smem = (int)sizeof(RowShared), smem_x = smem + (int)sizeof(cplx) * maxn * (maxn + SPF_ROWS);
-  static const cudaError_t configured = [] {
-    constexpr int most = (int)(sizeof(RowShared) + sizeof(cplx) * MAXN_SPF * (MAXN_SPF + SPF_ROWS));
-    cudaFuncSetAttribute(spf_drive_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, most);
-    cudaFuncSetAttribute(spf_drive8_kernel<true>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)sizeof(RowShared));
-    cudaFuncSetAttribute(spf_drive8_kernel<false>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)sizeof(RowShared));
-    return cudaFuncSetAttribute(spf_project_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, most);
-  }();
-  (void)configured;
   const unsigned nb = (unsigned)ntiles;
   if (maxn <= 8 && ntiles == ndesc) {
     spf_drive8_kernel<true><<<nb, SPF_THREADS, smem, st>>>(d_descs, ndesc, d_cols, out, der_factor, part, d_status, stage);
@@ -592,4 +584,13 @@ int launch_spf(const SpfDesc* d_descs, int ndesc, long long ntiles, int maxn, co
   launch_hole_fx(holes, st, 0, out);
   spf_project_kernel<<<nb, SPF_THREADS, smem_x, st>>>(d_descs, ndesc, out, d_status);
   return 3;
+}
+
+cudaError_t configure_spf() {
+  cudaError_t e = allow_smem(spf_drive_kernel, sizeof(RowShared));
+  if (e == cudaSuccess) e = allow_smem(spf_drive8_kernel<true>, sizeof(RowShared));
+  if (e == cudaSuccess) e = allow_smem(spf_drive8_kernel<false>, sizeof(RowShared));
+  if (e == cudaSuccess)
+    e = allow_smem(spf_project_kernel, sizeof(RowShared) + sizeof(cplx) * MAXN_SPF * (MAXN_SPF + SPF_ROWS));
+  return e;
 }

@@ -23,6 +23,7 @@
 // stage a CTA drains each tile before loading the next, and twice as many CTAs
 // share an SM.
 #include <algorithm>
+#include <mutex>
 #include <stdlib.h>
 
 #include "../../include/macaw_gb300.h"
@@ -232,6 +233,7 @@ struct DigitTile {
   static constexpr int WC = NG <= 2 ? 16 : 32;   // columns per weight
   static constexpr uint32_t SBO = K / 8 * 128, A = 128 * K * 2, B = 8 * WC * K * 2;
   static constexpr uint32_t COLS = 8 * WC;       // TMEM columns
+  static constexpr uint32_t SMEM = 8 * A + B;
 };
 template <int NG>
 __global__ void __launch_bounds__(128, NG <= 2 ? 4 : 2)
@@ -387,12 +389,8 @@ __global__ void __launch_bounds__(128, NG <= 2 ? 4 : 2)
 template <int NG>
 static void prod_digits_go(const ProdDesc* d, int nd, long long nblocks, int nsm, cudaStream_t st) {
   using T = DigitTile<NG>;
-  constexpr int smem = (int)(8 * T::A + T::B);
-  static const cudaError_t configured =
-      cudaFuncSetAttribute(prod_digits_kernel<NG>, cudaFuncAttributeMaxDynamicSharedMemorySize, smem);
-  (void)configured;
   const long long grid = std::min<long long>(nblocks, (NG <= 2 ? 4LL : 2LL) * nsm);
-  prod_digits_kernel<NG><<<(unsigned)grid, 128, smem, st>>>(d, nd, nblocks);
+  prod_digits_kernel<NG><<<(unsigned)grid, 128, T::SMEM, st>>>(d, nd, nblocks);
 }
 void launch_prod_digits_tc(const ProdDesc* d, int nd, long long nblocks, int maxn, int nsm, cudaStream_t st) {
   if (maxn <= 8) prod_digits_go<2>(d, nd, nblocks, nsm, st);
@@ -400,7 +398,6 @@ void launch_prod_digits_tc(const ProdDesc* d, int nd, long long nblocks, int max
   else prod_digits_go<4>(d, nd, nblocks, nsm, st);
 }
 
-static int g_tc_nsm = 0;
 // pipeline stages of the tensor-core mode product (MACAW_GB300_TC_STAGES=1 or 2)
 static int g_tc_stages = 1;
 // smallest largest-SPF-count of a batch that single contexts send to the tensor
@@ -409,33 +406,35 @@ static int g_tc_stages = 1;
 // 12 SPFs and its round-to-nearest sums drift less over long propagations.
 static int g_tc_min_n = 17;
 
-// Once per process, outside any stream capture (context creation calls it): the
-// SM count and the dynamic shared-memory limit of the tensor-core kernel.
+// Once per process (context creation calls it): the settings from the environment.
 void tc_prepare() {
-  if (g_tc_nsm) return;
-  int dev = 0, nsm = 0;
-  cudaGetDevice(&dev);
-  cudaDeviceGetAttribute(&nsm, cudaDevAttrMultiProcessorCount, dev);
-  cudaFuncSetAttribute(prod_tc_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize,
-                       2 * TC_NPART * (TC_ROWS * 2 * TC_MAXN * 4 + 2 * TC_MAXN * 2 * TC_MAXN * 4));
-  const char* e = getenv("MACAW_GB300_TC_STAGES");
-  g_tc_stages = (e && e[0] == '2') ? 2 : 1;
-  const char* m = getenv("MACAW_GB300_TC_MIN_N");
-  if (m && atoi(m) > 0) g_tc_min_n = atoi(m);
-  g_tc_nsm = nsm > 0 ? nsm : 152;
+  static std::once_flag once;
+  std::call_once(once, [] {
+    const char* e = getenv("MACAW_GB300_TC_STAGES");
+    g_tc_stages = (e && e[0] == '2') ? 2 : 1;
+    const char* m = getenv("MACAW_GB300_TC_MIN_N");
+    if (m && atoi(m) > 0) g_tc_min_n = atoi(m);
+  });
+}
+cudaError_t configure_tc() {
+  cudaError_t e = allow_smem(prod_tc_kernel, 2 * TC_NPART * (TC_ROWS * 2 * TC_MAXN * 4 + 2 * TC_MAXN * 2 * TC_MAXN * 4));
+  if (e == cudaSuccess) e = allow_smem(prod_digits_kernel<2>, DigitTile<2>::SMEM);
+  if (e == cudaSuccess) e = allow_smem(prod_digits_kernel<3>, DigitTile<3>::SMEM);
+  if (e == cudaSuccess) e = allow_smem(prod_digits_kernel<4>, DigitTile<4>::SMEM);
+  return e;
 }
 
 // Tensor-core path for FP32 products of nin, nout <= 16, from the threshold on
 // (force: any size up to 16); false: not taken
 bool launch_prod_tc(const ProdDesc* d_descs, int ndesc, long long nblocks, int maxn, cudaStream_t st, bool force) {
-  if (maxn > TC_MAXN || (!force && maxn < g_tc_min_n) || ndesc <= 0 || nblocks <= 0 || !g_tc_nsm) return false;
+  if (maxn > TC_MAXN || (!force && maxn < g_tc_min_n) || ndesc <= 0 || nblocks <= 0) return false;
   const int K = ((2 * maxn + 7) / 8) * 8;
   const int N = 2 * maxn <= 16 ? 16 : 32;
   const size_t stage = (size_t)TC_NPART * ((size_t)TC_ROWS * K * 4 + (size_t)N * K * 4);
   const int nstage = g_tc_stages;
   const size_t smem = stage * nstage;
   const int per_sm = std::max(1, std::min(8, (int)((220 * 1024) / smem)));
-  const long long grid = std::min<long long>(nblocks, (long long)g_tc_nsm * per_sm);
+  const long long grid = std::min<long long>(nblocks, (long long)sm_count() * per_sm);
   prod_tc_kernel<<<(unsigned)grid, TC_ROWS, smem, st>>>(d_descs, ndesc, nblocks, K, N, nstage);
   return true;
 }
