@@ -38,6 +38,16 @@ struct StatusError : std::runtime_error {
 
 std::string g_create_error;
 
+// A refused launch shows in the runtime's last error only.  An error that was pending
+// before the entry point (t_pending) is its owner's and stays.
+thread_local cudaError_t t_pending = cudaSuccess;
+void check_launches() {
+  const cudaError_t e = cudaPeekAtLastError();
+  if (e == t_pending) return;
+  cudaGetLastError();
+  if (e != cudaSuccess) throw CudaError(std::string("kernel launch: ") + cudaGetErrorString(e));
+}
+
 // Bump allocator over large device chunks; buffers live as long as the context.
 struct DevArena {
   std::vector<void*> chunks;
@@ -2159,6 +2169,7 @@ void run_graphed(Ctx& c, int kind, const void* key, F&& body) {
     bool ok = true;
     try {
       body();
+      check_launches();   // a refused launch is no node: the graph would lack it for good
     } catch (...) {
       ok = false;
     }
@@ -2368,6 +2379,7 @@ void run_ovl(Ctx& c, OvlPlan& P) {
 }
 
 void check_status(Ctx& c) {
+  check_launches();
   int* pinned = reinterpret_cast<int*>(c.h_scal + 32);
   CK(cudaMemcpyAsync(pinned, c.d_status, sizeof(int), cudaMemcpyDeviceToHost, c.st));
   CK(cudaStreamSynchronize(c.st));
@@ -4192,8 +4204,10 @@ Ctx* create(const mctdh_setup_t* s, const MemberBufs* mb = nullptr) {
 
 template <typename F>
 int64_t guarded(Ctx* c, F&& fn) {
+  t_pending = cudaPeekAtLastError();
   try {
     fn();
+    check_launches();
     return MCTDH_OK;
   } catch (const StatusError& e) {
     if (c) c->last_error = e.what();
@@ -4374,6 +4388,7 @@ void ens_graph(Ens& E, int k, F body) {
     bool ok = true;
     try {
       body();
+      check_launches();   // a refused launch is no node: the graph would lack it for good
     } catch (...) {
       ok = false;
     }
@@ -4706,6 +4721,7 @@ void ens_stage(Ens& E, cplx* out, const cplx* base, const double* coef, int nk) 
 }
 
 void ens_check_status(Ens& E) {
+  check_launches();
   int st = 0;
   CK(cudaMemcpyAsync(&st, E.status_d, sizeof(int), cudaMemcpyDeviceToHost, E.st));
   CK(cudaStreamSynchronize(E.st));
@@ -5104,8 +5120,10 @@ struct mctdh_ens {
 
 template <typename F>
 int64_t ens_guarded(mctdh_ens* h, F&& fn) {
+  t_pending = cudaPeekAtLastError();
   try {
     fn();
+    check_launches();
     return MCTDH_OK;
   } catch (const StatusError& e) {
     h->e->last_error = e.what();
