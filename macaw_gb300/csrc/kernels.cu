@@ -766,7 +766,7 @@ __device__ __forceinline__ bool sweep_inverse(cplx* A, int n, int ld, cplx (*v)[
 }
 
 // Where every eigenvalue of rho is at least eps the 'poly' regularisation is the plain
-// inverse, 1 / w; the inverse itself shows it: positive pivots, and |rho^-1|_F <= 1 / eps
+// inverse, 1 / w; the inverse itself shows it: positive pivots, and eps |rho^-1|_F <= 1
 // bounds its largest eigenvalue.  Then no eigen-decomposition is needed (8 x 8: 63 -> 9 us
 // a launch of 18 matrices); otherwise the Jacobi path below.  blockIdx.y: the blocks
 // of a matrix share its rho^-1 MF products, one warp per operator at a time, each
@@ -801,14 +801,13 @@ __global__ void __launch_bounds__(128) reginv_kernel(const RegInvDesc* __restric
     float f2 = 0.f;
     for (int e = threadIdx.x; e < n * n; e += blockDim.x) {
       const cplx v = Inv[e % n + ld * (e / n)];
-      const float x = (float)v.x, y = (float)v.y;
+      const float x = (float)(v.x * d.eps), y = (float)(v.y * d.eps);   // about one at most, whatever eps
       f2 = fmaf(x, x, fmaf(y, y, f2));
     }
     for (int o = 16; o > 0; o >>= 1) f2 += __shfl_down_sync(0xffffffffu, f2, o);
     if ((threadIdx.x & 31) == 0) fro[threadIdx.x >> 5] = f2;
     __syncthreads();
-    const float lim = 0.999f / (float)d.eps;
-    if (pos && fro[0] + fro[1] + fro[2] + fro[3] <= lim * lim) {
+    if (pos && fro[0] + fro[1] + fro[2] + fro[3] <= 0.998f) {
       if (d.inv_out && blockIdx.y == 0)
         for (int e = threadIdx.x; e < n * n; e += blockDim.x) d.inv_out[e] = Inv[e % n + ld * (e / n)];
       const int lane = threadIdx.x & 31;
