@@ -126,7 +126,8 @@ int64_t mctdh_destroy(mctdh_ctx_t *ctx);
  * integrator.f90:244-380), 4 Bulirsch-Stoer (bsstep, integrator.f90:418-608), 10 CMF2. */
 
 /* Equation of motion (A, psi, t) -> (dA, dpsi) on host buffers.
- * Replaces Calc_Derivs(A0, psi0, dA, dpsi, tt) -- derivatives.f90:39. */
+ * Replaces Calc_Derivs(A0, psi0, dA, dpsi, tt) -- derivatives.f90:39.  dA and dpsi are
+ * written on success only. */
 int64_t mctdh_calc_derivs(mctdh_ctx_t *ctx, const double *A, const double *psi,
                           double *dA, double *dpsi, double t);
 

@@ -506,7 +506,7 @@ struct Ctx {
   cudaEvent_t ev_fork = nullptr, ev_join = nullptr;
   // copies of host coefficients beside the EOM (calc_derivs_overlapped)
   cudaStream_t st_copy = nullptr;
-  cudaEvent_t ev_copy[2] = {nullptr, nullptr};
+  cudaEvent_t ev_copy = nullptr;
   bool member = false;      // ensemble member: RK only, state vectors owned by the ensemble
   DevArena ar;
   int* d_status = nullptr;
@@ -643,8 +643,7 @@ struct Ctx {
     if (ev_fork) cudaEventDestroy(ev_fork);
     if (ev_join) cudaEventDestroy(ev_join);
     if (st2) cudaStreamDestroy(st2);
-    for (cudaEvent_t e : ev_copy)
-      if (e) cudaEventDestroy(e);
+    if (ev_copy) cudaEventDestroy(ev_copy);
     if (st_copy) cudaStreamDestroy(st_copy);
   }
   int m_of(int m, int s) const { return nspf[m + nmodes * s]; }
@@ -4248,22 +4247,18 @@ void download(Ctx& c, const cplx* src, double* A, double* psi) {
 }
 
 
-// Calc_Derivs on host arrays with the coefficients copied beside the parts of the EOM that
-// do not touch them: in while the operators act on the SPFs, out while the mean fields
-// and the SPF derivatives are computed.  From OVERLAP_MIN coefficients (0.5 MB, about
-// 10 us either way; at 56,007 coefficients 225 -> 222 us, at 786,432 625 -> 537); not for
-// packets and Gaussian modes, whose dA is complete at the end only.
+// Calc_Derivs on host arrays with the coefficients copied in while the operators act on
+// the SPFs, which do not need them.  The results leave once the status is known: a call
+// that fails leaves the caller's arrays alone.  From OVERLAP_MIN coefficients (0.5 MB,
+// about 10 us); not for packets, whose host arrays are gathered by state.
 #define OVERLAP_MIN 32768
 bool overlapped_copies(const Ctx& c) {
   return c.naconftot >= OVERLAP_MIN && c.npk == 1 && !c.pk_on && !c.pk_mult && c.modes_gwp.empty() && !c.profiling &&
          !c.timing;
 }
 void calc_derivs_overlapped(Ctx& c, const double* A, const double* psi, double* dA, double* dpsi) {
-  if (!c.st_copy) {
-    CK(cudaStreamCreateWithFlags(&c.st_copy, cudaStreamNonBlocking));
-    CK(cudaEventCreateWithFlags(&c.ev_copy[0], cudaEventDisableTiming));
-    CK(cudaEventCreateWithFlags(&c.ev_copy[1], cudaEventDisableTiming));
-  }
+  if (!c.st_copy) CK(cudaStreamCreateWithFlags(&c.st_copy, cudaStreamNonBlocking));
+  if (!c.ev_copy) CK(cudaEventCreateWithFlags(&c.ev_copy, cudaEventDisableTiming));
   struct Finish {   // the caller's arrays are not touched any more once this returns or throws
     Ctx& c;
     ~Finish() {
@@ -4272,22 +4267,19 @@ void calc_derivs_overlapped(Ctx& c, const double* A, const double* psi, double* 
     }
   } finish{c};
   const size_t nA = sizeof(cplx) * c.naconftot, nP = sizeof(cplx) * c.dimpsi;
-  CK(cudaEventRecord(c.ev_copy[0], c.st));
-  CK(cudaStreamWaitEvent(c.st_copy, c.ev_copy[0], 0));   // d_in and d_out are free
+  CK(cudaEventRecord(c.ev_copy, c.st));
+  CK(cudaStreamWaitEvent(c.st_copy, c.ev_copy, 0));   // d_in is free
   if (nP) CK(cudaMemcpyAsync(c.d_in + c.naconftot, psi, nP, cudaMemcpyHostToDevice, c.st));
   run_graphed(c, 21, nullptr, [&] { eom_operators(c); });
   CK(cudaMemcpyAsync(c.d_in, A, nA, cudaMemcpyHostToDevice, c.st_copy));
-  CK(cudaEventRecord(c.ev_copy[0], c.st_copy));
-  CK(cudaStreamWaitEvent(c.st, c.ev_copy[0], 0));
-  run_graphed(c, 22, nullptr, [&] { eom_products(c, c.d_out, false); });
-  CK(cudaEventRecord(c.ev_copy[1], c.st));
-  run_graphed(c, 23, nullptr, [&] { eom_fields(c, c.d_out, false, true); });
-  CK(cudaStreamWaitEvent(c.st_copy, c.ev_copy[1], 0));
-  CK(cudaMemcpyAsync(dA, c.d_out, nA, cudaMemcpyDeviceToHost, c.st_copy));
+  CK(cudaEventRecord(c.ev_copy, c.st_copy));
+  CK(cudaStreamWaitEvent(c.st, c.ev_copy, 0));
+  run_graphed(c, 22, nullptr, [&] {
+    eom_products(c, c.d_out, false);
+    eom_fields(c, c.d_out, false, true);
+  });
   check_status(c);
-  if (nP) CK(cudaMemcpyAsync(dpsi, c.d_out + c.naconftot, nP, cudaMemcpyDeviceToHost, c.st));
-  CK(cudaStreamSynchronize(c.st_copy));
-  CK(cudaStreamSynchronize(c.st));
+  download(c, c.d_out, dA, dpsi);
 }
 
 // ---------------------------------------------------------------------------
