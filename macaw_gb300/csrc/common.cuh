@@ -115,6 +115,6 @@ enum {
 };
 
 // Device status word bits written by kernels whose iteration caps ran out.
-enum { DEVST_EIG_NOCONV = 1, DEVST_CHOL_FAIL = 2, DEVST_NONFINITE = 4 };
+enum { DEVST_EIG_NOCONV = 1, DEVST_CHOL_FAIL = 2, DEVST_NONFINITE = 4, DEVST_TC_WAIT = 8 };
 
 #define MAXN_SPF 32   // largest SPF count per mode handled by the small dense kernels

@@ -2207,7 +2207,7 @@ struct StreamSwap {
 void run_prod(Ctx& c, const ProdBatch& b) {
   if (b.h.empty()) return;
   ProfScope ps(c, KP_PROD, b.flops, b.bytes);
-  launch_prod(b.d, (int)b.h.size(), b.nblocks, b.maxn, c.st, b.prec);
+  launch_prod(b.d, (int)b.h.size(), b.nblocks, b.maxn, c.d_status, c.st, b.prec);
   c.count();
 }
 void run_hole(Ctx& c, const HoleBatch& b) {
@@ -2387,6 +2387,7 @@ void check_status(Ctx& c) {
     CK(cudaMemsetAsync(c.d_status, 0, sizeof(int), c.st));
     if (st & DEVST_EIG_NOCONV) throw StatusError(MCTDH_EEIG, "Jacobi eigensolver did not converge");
     if (st & DEVST_CHOL_FAIL) throw StatusError(MCTDH_EEIG, "SPF overlap matrix is not positive definite");
+    if (st & DEVST_TC_WAIT) throw StatusError(MCTDH_ECUDA, "a tensor-core kernel gave up waiting for its MMAs");
     throw StatusError(MCTDH_ENONFINITE, "device status " + std::to_string(st));
   }
 }
@@ -4572,7 +4573,7 @@ void ens_destroy(Ens* E) {
 
 void ens_run_prod(Ens& E, const ProdBatch& b) {
   if (b.h.empty()) return;
-  launch_prod(b.d, (int)b.h.size(), b.nblocks, b.maxn, E.st, b.prec, E.tune_tc ? 2 : 0, E.persist_prod);
+  launch_prod(b.d, (int)b.h.size(), b.nblocks, b.maxn, E.status_d, E.st, b.prec, E.tune_tc ? 2 : 0, E.persist_prod);
   ++E.launches;
 }
 void ens_run_hole(Ens& E, const HoleBatch& b) {
@@ -4721,6 +4722,7 @@ void ens_check_status(Ens& E) {
     CK(cudaMemsetAsync(E.status_d, 0, sizeof(int), E.st));
     if (st & DEVST_EIG_NOCONV) throw StatusError(MCTDH_EEIG, "Jacobi eigensolver did not converge");
     if (st & DEVST_CHOL_FAIL) throw StatusError(MCTDH_EEIG, "SPF overlap matrix is not positive definite");
+    if (st & DEVST_TC_WAIT) throw StatusError(MCTDH_ECUDA, "a tensor-core kernel gave up waiting for its MMAs");
     throw StatusError(MCTDH_ENONFINITE, "device status " + std::to_string(st));
   }
 }

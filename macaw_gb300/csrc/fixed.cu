@@ -216,9 +216,9 @@ static void prod_fx_go(const ProdDesc* d, int nd, long long nblocks, int persist
 // matrix digits and the pipeline's start are paid for: 57 products of 32,768 fibres of 8
 // took 191 us against 226, of 248,832 fibres of 12 2,206 against 2,900; a batch of 700
 // tiles of 5 to 9 took 19 against 17.
-void launch_prod_fx(const ProdDesc* d, int nd, long long nblocks, int maxn, cudaStream_t st, int persist) {
+void launch_prod_fx(const ProdDesc* d, int nd, long long nblocks, int maxn, int* status, cudaStream_t st, int persist) {
   if (persist <= 0 && maxn > 4 && maxn <= 16 && nblocks >= (maxn <= 8 ? 8 : 4) * (long long)sm_count()) {
-    launch_prod_digits_tc(d, nd, nblocks, maxn, sm_count(), st);
+    launch_prod_digits_tc(d, nd, nblocks, maxn, status, st);
     return;
   }
   if (maxn <= 4) prod_fx_go<1>(d, nd, nblocks, persist, st);

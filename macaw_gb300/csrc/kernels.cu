@@ -136,14 +136,14 @@ int sm_count() {
 // tc: 0 CUDA-core kernel, 1 tensor cores from the configured SPF count on,
 // 2 tensor cores for every size they take (the ensemble autotuner's candidate).
 // persist > 0: at most that many persistent CTAs walk the blocks.
-void launch_prod(const ProdDesc* d_descs, int ndesc, long long nblocks, int maxn, cudaStream_t st, int prec,
-                 int tc, int persist) {
+void launch_prod(const ProdDesc* d_descs, int ndesc, long long nblocks, int maxn, int* status, cudaStream_t st,
+                 int prec, int tc, int persist) {
   if (ndesc <= 0 || nblocks <= 0) return;
   if (prec != 1) {
-    launch_prod_fx(d_descs, ndesc, nblocks, maxn, st, persist);
+    launch_prod_fx(d_descs, ndesc, nblocks, maxn, status, st, persist);
     return;
   }
-  if (tc && tc_enabled() && launch_prod_tc(d_descs, ndesc, nblocks, maxn, st, tc == 2)) return;
+  if (tc && tc_enabled() && launch_prod_tc(d_descs, ndesc, nblocks, maxn, status, st, tc == 2)) return;
   // register arrays sized for the batch's largest SPF count: no dead unrolled
   // iterations and fewer registers (more resident warps) at 8 SPFs and below
   if (persist > 0 && nblocks > persist) {

@@ -35,8 +35,17 @@
 #define TC_MAXN 16          // largest nin / nout of the tensor-core mode product
 #define TC_NPART 3          // hi, mid, lo
 
-// set when a tensor-core kernel gave up waiting for its MMAs (never expected)
+// set when a tensor-core kernel gave up waiting for its MMAs (never expected); the call
+// that launched it fails by its own status word
 __device__ int g_tc_timeout = 0;
+
+// A wait ran out: results are missing, and the MMAs in flight may still write TMEM.  Wait
+// once more before the caller gives TMEM back.
+__device__ __forceinline__ void tc_gave_up(uint64_t* bar, uint32_t parity, int* status) {
+  tc_wait(bar, parity);
+  atomicExch(&g_tc_timeout, 1);
+  atomicOr(status, DEVST_TC_WAIT);
+}
 
 __device__ __forceinline__ int tc_find_tile(const ProdDesc* descs, int ndesc, long long b) {
   int lo = 0, hi = ndesc - 1;
@@ -48,7 +57,7 @@ __device__ __forceinline__ int tc_find_tile(const ProdDesc* descs, int ndesc, lo
 }
 
 __global__ void __launch_bounds__(TC_ROWS) prod_tc_kernel(const ProdDesc* __restrict__ descs, int ndesc,
-                                                          long long ntiles, int K, int N, int nstage) {
+                                                          long long ntiles, int K, int N, int nstage, int* status) {
   extern __shared__ __align__(128) unsigned char tc_smem[];
   __shared__ __align__(8) uint64_t bar[2];
   __shared__ uint32_t s_tmem;
@@ -69,6 +78,7 @@ __global__ void __launch_bounds__(TC_ROWS) prod_tc_kernel(const ProdDesc* __rest
   const uint32_t idesc = tc_idesc_tf32(TC_ROWS, N);
   const uint32_t sbo = (uint32_t)K * 32;
   bool ok = true;
+  uint32_t late = 0;         // where a wait ran out: 2 stage + parity of the last commit
   int prev_di = -1;          // the tile loaded in the previous iteration
   long long prev_p = 0;
   int it = 0;
@@ -169,6 +179,7 @@ __global__ void __launch_bounds__(TC_ROWS) prod_tc_kernel(const ProdDesc* __rest
       tc_fence_after();
       if (!w) {
         ok = false;
+        late = nstage == 2 && have ? 2 * s + ((uint32_t)(it >> 1) & 1u) : 2 * ps + parity;
       } else {
         const ProdDesc& d = descs[dd];
         const int nout = d.nout;
@@ -205,7 +216,7 @@ __global__ void __launch_bounds__(TC_ROWS) prod_tc_kernel(const ProdDesc* __rest
     prev_di = di;
     prev_p = p;
   }
-  if (!ok && tid == 0) atomicExch(&g_tc_timeout, 1);
+  if (!ok && tid == 0) tc_gave_up(&bar[late >> 1], late & 1, status);
   tc_fence_before();
   __syncthreads();
   if (warp == 0) {
@@ -237,7 +248,7 @@ struct DigitTile {
 };
 template <int NG>
 __global__ void __launch_bounds__(128, NG <= 2 ? 4 : 2)
-    prod_digits_kernel(const ProdDesc* __restrict__ descs, int ndesc, long long ntiles) {
+    prod_digits_kernel(const ProdDesc* __restrict__ descs, int ndesc, long long ntiles, int* status) {
   using T = DigitTile<NG>;
   extern __shared__ __align__(128) unsigned char tc_smem[];   // A_0 .. A_7, B
   __shared__ __align__(8) uint64_t bar;
@@ -259,7 +270,7 @@ __global__ void __launch_bounds__(128, NG <= 2 ? 4 : 2)
   uint32_t parity = 0;
   bool ok = true;
   int di = t0 < tend ? warp_find_desc(descs, ndesc, t0) : 0;
-  for (; t0 < tend; ++di) {
+  for (; ok && t0 < tend; ++di) {
     const ProdDesc& d = descs[di];
     const int nin = d.nin, nout = d.nout;
     const unsigned L = (unsigned)d.L, nfib = (unsigned)(d.L * d.R);
@@ -307,11 +318,6 @@ __global__ void __launch_bounds__(128, NG <= 2 ? 4 : 2)
     }
     const bool plain = !d.accumulate && d.alpha.x == 1.0 && d.alpha.y == 0.0;
     for (; t0 < dend; ++t0) {
-      if (!ok) {   // a wait ran out (never expected): the rest of the tiles in FP64
-        if (p < nfib) prod_fibre_fp64(d, p % L, p / L);
-        p += 128;
-        continue;
-      }
       unsigned mag = 0u;
 #pragma unroll
       for (int j = 0; j < 4 * NG; ++j) mag = max(mag, fx_mag(x[j]));
@@ -351,13 +357,14 @@ __global__ void __launch_bounds__(128, NG <= 2 ? 4 : 2)
       }
       // every thread polls; the verdict is made uniform
       ok = __syncthreads_and(tc_wait(&bar, parity));
+      if (!ok) break;
       parity ^= 1;
       tc_fence_after();
       const bool act = pc < nfib;
       cplx* y = d.Y + ((long long)pc + Ly * rc);
 #pragma unroll
       for (int h = 0; h < NG; ++h) {
-        if (4 * h >= nout || !ok) break;
+        if (4 * h >= nout) break;
         float c[8][8];
         tc_ld8x8(tmem + ((uint32_t)(warp * 32) << 16) + 8 * h, T::WC, c);
 #pragma unroll
@@ -373,11 +380,11 @@ __global__ void __launch_bounds__(128, NG <= 2 ? 4 : 2)
           }
         }
       }
-      if (act && (bad || !ok)) prod_fibre_fp64(d, pc - L * rc, rc);
+      if (act && bad) prod_fibre_fp64(d, pc - L * rc, rc);
     }
     t0 = dend;
   }
-  if (!ok && tid == 0) atomicExch(&g_tc_timeout, 1);
+  if (!ok && tid == 0) tc_gave_up(&bar, parity, status);
   tc_fence_before();
   __syncthreads();
   if (warp == 0) {
@@ -387,15 +394,16 @@ __global__ void __launch_bounds__(128, NG <= 2 ? 4 : 2)
 }
 
 template <int NG>
-static void prod_digits_go(const ProdDesc* d, int nd, long long nblocks, int nsm, cudaStream_t st) {
+static void prod_digits_go(const ProdDesc* d, int nd, long long nblocks, int nsm, int* status, cudaStream_t st) {
   using T = DigitTile<NG>;
   const long long grid = std::min<long long>(nblocks, (NG <= 2 ? 4LL : 2LL) * nsm);
-  prod_digits_kernel<NG><<<(unsigned)grid, 128, T::SMEM, st>>>(d, nd, nblocks);
+  prod_digits_kernel<NG><<<(unsigned)grid, 128, T::SMEM, st>>>(d, nd, nblocks, status);
 }
-void launch_prod_digits_tc(const ProdDesc* d, int nd, long long nblocks, int maxn, int nsm, cudaStream_t st) {
-  if (maxn <= 8) prod_digits_go<2>(d, nd, nblocks, nsm, st);
-  else if (maxn <= 12) prod_digits_go<3>(d, nd, nblocks, nsm, st);
-  else prod_digits_go<4>(d, nd, nblocks, nsm, st);
+void launch_prod_digits_tc(const ProdDesc* d, int nd, long long nblocks, int maxn, int* status, cudaStream_t st) {
+  const int nsm = sm_count();
+  if (maxn <= 8) prod_digits_go<2>(d, nd, nblocks, nsm, status, st);
+  else if (maxn <= 12) prod_digits_go<3>(d, nd, nblocks, nsm, status, st);
+  else prod_digits_go<4>(d, nd, nblocks, nsm, status, st);
 }
 
 // pipeline stages of the tensor-core mode product (MACAW_GB300_TC_STAGES=1 or 2)
@@ -426,7 +434,8 @@ cudaError_t configure_tc() {
 
 // Tensor-core path for FP32 products of nin, nout <= 16, from the threshold on
 // (force: any size up to 16); false: not taken
-bool launch_prod_tc(const ProdDesc* d_descs, int ndesc, long long nblocks, int maxn, cudaStream_t st, bool force) {
+bool launch_prod_tc(const ProdDesc* d_descs, int ndesc, long long nblocks, int maxn, int* status, cudaStream_t st,
+                    bool force) {
   if (maxn > TC_MAXN || (!force && maxn < g_tc_min_n) || ndesc <= 0 || nblocks <= 0) return false;
   const int K = ((2 * maxn + 7) / 8) * 8;
   const int N = 2 * maxn <= 16 ? 16 : 32;
@@ -435,7 +444,7 @@ bool launch_prod_tc(const ProdDesc* d_descs, int ndesc, long long nblocks, int m
   const size_t smem = stage * nstage;
   const int per_sm = std::max(1, std::min(8, (int)((220 * 1024) / smem)));
   const long long grid = std::min<long long>(nblocks, (long long)sm_count() * per_sm);
-  prod_tc_kernel<<<(unsigned)grid, TC_ROWS, smem, st>>>(d_descs, ndesc, nblocks, K, N, nstage);
+  prod_tc_kernel<<<(unsigned)grid, TC_ROWS, smem, st>>>(d_descs, ndesc, nblocks, K, N, nstage, status);
   return true;
 }
 

@@ -15,7 +15,7 @@ def library(tmp_path_factory):
     return fake.fake_runtime(tmp_path_factory.mktemp("fake"))
 
 
-@pytest.mark.parametrize("status, code", [(1, -2), (2, -2), (4, -5)])
+@pytest.mark.parametrize("status, code", [(1, -2), (2, -2), (4, -5), (8, -6)])
 @pytest.mark.parametrize("modes", [3, 5])
 def test_outputs_stay(library, monkeypatch, modes, status, code):
     rt = fake.use(monkeypatch, library)
