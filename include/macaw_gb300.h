@@ -405,9 +405,10 @@ const char *mctdh_ens_last_error(mctdh_ens_t *ens);
  * one- or two-stage pipeline (default 1).  Single contexts default to min_n = 17
  * (the CUDA-core kernel, faster on the measured models); ensembles let their
  * autotuner choose.  status: *enabled is 1 unless the environment variable
- * MACAW_GB300_TC=0 selected the CUDA-core kernels for this process; *timeouts is
- * 1 when a tensor-core kernel gave up waiting for its MMAs since the previous
- * call (the flag is cleared).  config: 0 keeps a setting; it applies to launches
+ * MACAW_GB300_TC=0 keeps every tcgen05 kernel out of this process (the large
+ * batches of FP64-accurate products then use mma.sync); *timeouts is 1 when a
+ * tensor-core kernel gave up waiting for its MMAs since the previous call (the
+ * flag is cleared).  config: 0 keeps a setting; it applies to launches
  * issued afterwards (CUDA graphs captured earlier keep their kernels). */
 int64_t mctdh_tensor_core_status(int64_t *enabled, int64_t *timeouts);
 int64_t mctdh_tensor_core_config(int64_t min_n, int64_t stages);

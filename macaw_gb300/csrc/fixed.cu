@@ -217,7 +217,7 @@ static void prod_fx_go(const ProdDesc* d, int nd, long long nblocks, int persist
 // took 191 us against 226, of 248,832 fibres of 12 2,206 against 2,900; a batch of 700
 // tiles of 5 to 9 took 19 against 17.
 void launch_prod_fx(const ProdDesc* d, int nd, long long nblocks, int maxn, int* status, cudaStream_t st, int persist) {
-  if (persist <= 0 && maxn > 4 && maxn <= 16 && nblocks >= (maxn <= 8 ? 8 : 4) * (long long)sm_count()) {
+  if (persist <= 0 && tc_enabled() && maxn > 4 && maxn <= 16 && nblocks >= (maxn <= 8 ? 8 : 4) * (long long)sm_count()) {
     launch_prod_digits_tc(d, nd, nblocks, maxn, status, st);
     return;
   }

@@ -109,8 +109,8 @@ __global__ void __launch_bounds__(128) prod_kernel_persistent(const ProdDesc* __
   }
 }
 
-// Tensor-core kernels (tc.cu) may serve the FP32 products unless
-// MACAW_GB300_TC=0 selects the CUDA-core kernels (read once per process).
+// tcgen05 kernels (tc.cu) may serve the mode products unless MACAW_GB300_TC=0 keeps
+// them out (read once per process).
 bool tc_enabled() {
   static int on = -1;
   if (on < 0) {

@@ -1,0 +1,24 @@
+"""MACAW_GB300_TC=0 keeps every tcgen05 kernel out.  On the stand-in runtime, by the names of the launched kernels."""
+import pytest
+
+from macaw_gb300 import capi
+from macaw_gb300.generate import qvc
+from tests import fake
+from tests.helpers import random_state
+
+
+def _model(modes):
+    return qvc(2, modes, 18, 8, 2, 5, (200.0, 3500.0), (0.05, 0.2), (0.0, 0.4), "settings", dofs_per_mode=1)
+
+
+# 262,144 coefficients and fewer than 152 x 8 tiles
+@pytest.mark.parametrize("value, modes, digits", [("1", 6, True), ("0", 6, False), ("1", 3, False)])
+def test_switch_covers_the_digit_products(tmp_path, monkeypatch, value, modes, digits):
+    monkeypatch.setenv("MACAW_GB300_TC", value)
+    rt = fake.use(monkeypatch, fake.fake_runtime(tmp_path))
+    model = _model(modes)
+    core = capi.GpuCore(model)
+    A, psi = random_state(model)
+    core.calc_derivs(A, psi)
+    assert any("prod_digits_kernel" in k for k in rt.kernels()) == digits
+    assert capi.tensor_core_status()["enabled"] == int(value)
