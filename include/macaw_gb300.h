@@ -408,8 +408,8 @@ const char *mctdh_ens_last_error(mctdh_ens_t *ens);
  * MACAW_GB300_TC=0 keeps every tcgen05 kernel out of this process (the large
  * batches of FP64-accurate products then use mma.sync); *timeouts is 1 when a
  * tensor-core kernel gave up waiting for its MMAs since the previous call (the
- * flag is cleared).  config: 0 keeps a setting; it applies to launches
- * issued afterwards (CUDA graphs captured earlier keep their kernels). */
+ * flag is cleared).  config: 0 keeps a setting; it applies to the calls made
+ * afterwards (ensembles that are propagated keep the kernels they captured). */
 int64_t mctdh_tensor_core_status(int64_t *enabled, int64_t *timeouts);
 int64_t mctdh_tensor_core_config(int64_t min_n, int64_t stages);
 

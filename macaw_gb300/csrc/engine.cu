@@ -410,7 +410,7 @@ struct Ctx {
     cudaGraphExec_t exec;
     long long launches, eoms, hbs;   // what one replay accounts for
   };
-  std::map<std::pair<int, const void*>, GraphRec> graphs;
+  std::map<std::pair<int, const void*>, GraphRec> graphs;   // (kind + 100 tensor-core settings, key)
   std::set<std::pair<int, const void*>> graph_seen;   // run once directly before capture
   bool graphs_off = false;
   KProf prof[KP_N];
@@ -2148,7 +2148,7 @@ void run_graphed(Ctx& c, int kind, const void* key, F&& body) {
     body();
     return;
   }
-  auto k = std::make_pair(kind, key);
+  auto k = std::make_pair(kind + 100 * tc_config(), key);
   auto it = c.graphs.find(k);
   if (it == c.graphs.end()) {
     if (!c.graph_seen.count(k)) {

@@ -252,6 +252,8 @@ void tc_prepare();
 bool launch_prod_tc(const ProdDesc* d_descs, int ndesc, long long nblocks, int maxn, int* status, cudaStream_t st,
                     bool force);
 int tc_timeout_flag(bool clear);
+// the settings that choose the captured kernels, as one number
+int tc_config();
 // persist > 0: at most `persist` persistent CTAs walk the batch's blocks; status: the
 // word that takes DEVST_TC_WAIT
 void launch_prod(const ProdDesc* d_descs, int ndesc, long long nblocks, int maxn, int* status, cudaStream_t st,

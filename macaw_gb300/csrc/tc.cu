@@ -469,6 +469,8 @@ extern "C" int64_t mctdh_tensor_core_status(int64_t* enabled, int64_t* timeouts)
   return MCTDH_OK;
 }
 
+int tc_config() { return 4 * std::min(g_tc_min_n, TC_MAXN + 1) + g_tc_stages; }
+
 extern "C" int64_t mctdh_tensor_core_config(int64_t min_n, int64_t stages) {
   if (min_n < 0 || stages < 0 || stages > 2) return MCTDH_EARG;
   if (min_n > 0) g_tc_min_n = (int)min_n;

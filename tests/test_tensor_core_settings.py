@@ -1,4 +1,6 @@
-"""MACAW_GB300_TC=0 keeps every tcgen05 kernel out.  On the stand-in runtime, by the names of the launched kernels."""
+"""The tensor-core settings choose the kernels of the calls made after them, also where
+an EOM evaluation is replayed from a graph; MACAW_GB300_TC=0 keeps every tcgen05 kernel
+out.  On the stand-in runtime, by the names of the launched kernels."""
 import pytest
 
 from macaw_gb300 import capi
@@ -9,6 +11,20 @@ from tests.helpers import random_state
 
 def _model(modes):
     return qvc(2, modes, 18, 8, 2, 5, (200.0, 3500.0), (0.05, 0.2), (0.0, 0.4), "settings", dofs_per_mode=1)
+
+
+@pytest.mark.parametrize("modes", [3, 5])   # one graph; copies beside the operators
+def test_settings_reach_replayed_calls(tmp_path, monkeypatch, modes):
+    rt = fake.use(monkeypatch, fake.fake_runtime(tmp_path))
+    model = _model(modes)
+    core = capi.GpuCore(model, precision=1)
+    A, psi = random_state(model)
+    for min_n, name in ((17, "prod_kernel"), (4, "prod_tc_kernel"), (17, "prod_kernel")):
+        capi.tensor_core_config(min_n=min_n)
+        for _ in range(3):
+            core.calc_derivs(A, psi)
+            launched = [k for k in rt.kernels() if "prod" in k]
+            assert launched and all(name in k for k in launched)
 
 
 # 262,144 coefficients and fewer than 152 x 8 tiles
