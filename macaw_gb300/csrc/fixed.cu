@@ -118,7 +118,7 @@ __global__ void __launch_bounds__(PROD_THREADS, prod_ctas<NJ>())
                        (__double2hiint(d.alpha.y) << 1 | __double2loint(d.alpha.y)) == 0;   // alpha = 1
     for (; left; --left) {
       if (p - g >= nfib) break;
-      int ef[2];
+      unsigned ef[2];
       bool bad = badM;
       unsigned A[NK][NS][4];   // digits: (fibre g, j), (fibre g + 8, j), (g, j + 4), (g + 8, j + 4)
 #pragma unroll
@@ -130,7 +130,7 @@ __global__ void __launch_bounds__(PROD_THREADS, prod_ctas<NJ>())
         mag = max(mag, __shfl_xor_sync(0xffffffffu, mag, 2));
         bad = bad || !fx_ok(mag);
         const unsigned eb = fx_ebits(mag);
-        ef[f] = (int)eb - ((2044 + 12 + 44) << 20);
+        ef[f] = fx_exp(eb, 0u, 44);
 #pragma unroll
         for (int k = 0; k < NJ; ++k) {
           unsigned s[NS];
@@ -177,11 +177,11 @@ __global__ void __launch_bounds__(PROD_THREADS, prod_ctas<NJ>())
               }
             }
           }
-          const int em = (int)rowexp[4 * t + q];
+          const unsigned em = rowexp[4 * t + q];
           if (4 * t + q < nout) {
 #pragma unroll
             for (int f = 0; f < 2; ++f) {
-              const int es = em + ef[f];
+              const unsigned es = em + ef[f];
               cplx v = mkc(fx_double(BIG ? fx_join_wide<NS, 0>(c, 2 * f) : fx_join<NS>(c, 2 * f), es),
                            fx_double(BIG ? fx_join_wide<NS, 0>(c, 2 * f + 1) : fx_join<NS>(c, 2 * f + 1), es));
               if (!plain) {
@@ -346,7 +346,7 @@ __device__ __forceinline__ void hole_fx_block(const HoleDesc& d, int b, const cp
       for (int i = 0; i < 2; ++i) {
         const long long re = fx_join_wide<ND, 1>(cr, i) + fx_join_wide<ND, 1>(ci, 2 + i);
         const long long im = fx_join_wide<ND, 1>(ci, i) - fx_join_wide<ND, 1>(cr, 2 + i);
-        const int es = (int)(ex + e2[i]) - ((2044 + 12 + 43) << 20);
+        const unsigned es = fx_exp(ex, e2[i], 43);
         const cplx v = mkc(fx_double(re, es), fx_double(im, es));
         acc[i] = fresh ? v : cadd(acc[i], v);
       }
@@ -563,7 +563,7 @@ __device__ __forceinline__ void hole_mul_go(HoleWide& sh, cplx* acc, bool mine, 
   auto flush = [&]() {
 #pragma unroll
     for (int i = 0; i < 2; ++i) {
-      const int es = (int)(e1 + e2[i]) - ((2044 + 12 + 43) << 20);
+      const unsigned es = fx_exp(e1, e2[i], 43);
       const long long a = fx_join_wide<ND, 1>(cr, i), b = fx_join_wide<ND, 1>(cr, 2 + i);
       if (PACKED) {
         // conj(x) y of a column: re = Xr Yr + Xi Yi in lanes q < 2, im = Xr Yi - Xi Yr in q + 2

@@ -119,13 +119,18 @@ __device__ __forceinline__ long long fx_join_wide(const float (*c)[4], int i) {
          (DN ? (lo + ((1 << DN) >> 1)) >> DN : lo);
 }
 
-// v 2^(es / 2^20) as FP64, rounded to nearest (es: the exponent in the exponent field's
-// place; the result is a normal number or zero).  The conversion is one instruction of
-// the otherwise idle FP64 pipe.
-__device__ __forceinline__ double fx_double(long long v, int es) {
+// The exponent, in the exponent field's place, of an integer joined to 2^bits times the
+// digits' product: ea, eb the exponent words the operands were cut with.  Exponents
+// below zero wrap, as unsigned words do.
+__host__ __device__ __forceinline__ unsigned fx_exp(unsigned ea, unsigned eb, unsigned bits) {
+  return ea + eb - ((2044u + 12u + bits) << 20);
+}
+__host__ __device__ __forceinline__ unsigned fx_add_exp(unsigned hi, unsigned es) { return hi ? hi + es : hi; }
+// v 2^(es / 2^20) as FP64, rounded to nearest (the result is a normal number or zero).
+// The conversion is one instruction of the otherwise idle FP64 pipe.
+__device__ __forceinline__ double fx_double(long long v, unsigned es) {
   const double d = (double)v;
-  const int hi = __double2hiint(d);
-  return __hiloint2double(hi ? hi + es : hi, __double2loint(d));
+  return __hiloint2double((int)fx_add_exp((unsigned)__double2hiint(d), es), __double2loint(d));
 }
 
 // A mode product's fibre (l, :, r) in FP64, for fibres or matrices outside the exponent range.

@@ -568,7 +568,7 @@ __global__ void __launch_bounds__(256) lu_update_kernel(const GwpCYDesc* __restr
     mag = max(mag, __shfl_xor_sync(0xffffffffu, mag, 2));
     const bool slow = __any_sync(0xffffffffu, bad || !fx_ok(mag));
     const unsigned ec = fx_ebits(mag);
-    const int es = (int)__shfl_sync(0xffffffffu, ec, 8 * q) - ((2044 + 12 + 44) << 20);
+    const unsigned es = fx_exp(__shfl_sync(0xffffffffu, ec, 8 * q), 0u, 44);
     const int col = c0 + 32 * blockIdx.x + 4 * t + q;
     float c[NS][4];
     if (!slow) {
@@ -588,7 +588,7 @@ __global__ void __launch_bounds__(256) lu_update_kernel(const GwpCYDesc* __restr
       if (row[f] < 0 || col > nG) continue;
       cplx v;
       if (!slow) {
-        v = mkc(fx_double(fx_join<NS>(c, 2 * f), es + (int)er[f]), fx_double(fx_join<NS>(c, 2 * f + 1), es + (int)er[f]));
+        v = mkc(fx_double(fx_join<NS>(c, 2 * f), es + er[f]), fx_double(fx_join<NS>(c, 2 * f + 1), es + er[f]));
       } else {
         v = mkc(0.0, 0.0);
         for (int k = 0; k < pw; ++k) cfma(v, d.M[row[f] + ld * (j0 + k)], T[4 * t + q][k]);

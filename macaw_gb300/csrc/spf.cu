@@ -166,10 +166,10 @@ __device__ __forceinline__ void row_products(RowShared& S, int ncols, Col&& col,
 #pragma unroll
         for (int t = 0; t < 2; ++t) {
           if (4 * t < nc) {
-            const int em = (int)fx_ebits(S.colmag[4 * t + q]);
+            const unsigned em = fx_ebits(S.colmag[4 * t + q]);
 #pragma unroll
             for (int f = 0; f < 2; ++f) {
-              const int es = em + (int)eb[f] - ((2044 + 12 + 43) << 20);
+              const unsigned es = fx_exp(em, eb[f], 43);
               const cplx v =
                   mkc(fx_double(fx_join_wide<NS, 1>(c[t], 2 * f), es), fx_double(fx_join_wide<NS, 1>(c[t], 2 * f + 1), es));
               sum[t][f] = s0 ? cadd(sum[t][f], v) : v;
@@ -345,7 +345,7 @@ __device__ __forceinline__ void contract_rows(SpfSmall& T) {
   for (int i = 0; i < 2; ++i) {
     const long long re = fx_join_wide<ND, 1>(cr, i) + fx_join_wide<ND, 1>(ci, 2 + i);
     const long long im = fx_join_wide<ND, 1>(ci, i) - fx_join_wide<ND, 1>(cr, 2 + i);
-    const int es = (int)(ex + e2[i]) - ((2044 + 12 + 43) << 20);
+    const unsigned es = fx_exp(ex, e2[i], 43);
     T.red[warp & 3][64 * which + g + 8 * (2 * q + i)] = mkc(fx_double(re, es), fx_double(im, es));
   }
   const bool slow = __syncthreads_or(!fx_ok(mx) || !fx_ok(my));
@@ -436,7 +436,7 @@ __device__ __forceinline__ bool solve_project(SpfSmall& T, const SpfDesc& d, int
     }
   } else {
     const unsigned ec = fx_ebits(mag);
-    const int es = (int)__shfl_sync(0xffffffffu, ec, 8 * q) - ((2044 + 12 + 44) << 20);
+    const unsigned es = fx_exp(__shfl_sync(0xffffffffu, ec, 8 * q), 0u, 44);
     unsigned s0[NS], s1[NS];
     fx_digits<NS>(m0.x, m0.y, ec, ec, s0);
     fx_digits<NS>(m1.x, m1.y, ec, ec, s1);
@@ -450,7 +450,7 @@ __device__ __forceinline__ bool solve_project(SpfSmall& T, const SpfDesc& d, int
     }
 #pragma unroll
     for (int f = 0; f < 2; ++f)
-      v[f] = mkc(fx_double(fx_join<NS>(c, 2 * f), es + (int)er[f]), fx_double(fx_join<NS>(c, 2 * f + 1), es + (int)er[f]));
+      v[f] = mkc(fx_double(fx_join<NS>(c, 2 * f), es + er[f]), fx_double(fx_join<NS>(c, 2 * f + 1), es + er[f]));
   }
 #pragma unroll
   for (int f = 0; f < 2; ++f) {

@@ -322,7 +322,7 @@ __global__ void __launch_bounds__(128, NG <= 2 ? 4 : 2)
 #pragma unroll
       for (int j = 0; j < 4 * NG; ++j) mag = max(mag, fx_mag(x[j]));
       const unsigned eb = fx_ebits(mag);
-      const int ef = (int)eb - ((2044 + 12 + 44) << 20);
+      const unsigned ef = fx_exp(eb, 0u, 44);
       bool bad = !fx_ok(mag);
 #pragma unroll
       for (int k = 0; k < NG; ++k) {
@@ -370,7 +370,7 @@ __global__ void __launch_bounds__(128, NG <= 2 ? 4 : 2)
 #pragma unroll
         for (int o = 0; o < 4; ++o) {
           if (4 * h + o < nout) {
-            const int es = (int)fx_ebits(rowexp[4 * h + o]) + ef;
+            const unsigned es = fx_ebits(rowexp[4 * h + o]) + ef;
             cplx v = mkc(fx_double(fx_join<8>(c, 2 * o), es), fx_double(fx_join<8>(c, 2 * o + 1), es));
             if (!plain) {
               v = cmul(d.alpha, v);
