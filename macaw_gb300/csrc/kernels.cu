@@ -695,15 +695,6 @@ __device__ void jacobi_herm(cplx* A, cplx* V, int n, int ld, JacRot* R, bool* ok
   *ok = converged;
 }
 
-// 1 / d for d > 0 by Newton's iteration on the hardware's approximate reciprocal:
-// four dependent FP64 instructions instead of a full division (443 cycles of latency).
-__device__ __forceinline__ double newton_rcp(double d) {
-  double y;
-  asm("rcp.approx.ftz.f64 %0, %1;" : "=d"(y) : "d"(d));
-  y = fma(y, fma(-d, y, 1.0), y);
-  return fma(y, fma(-d, y, 1.0), y);
-}
-
 // Inverse of a Hermitian positive definite n x n matrix (n <= 32) by n symmetric sweeps
 // (Gauss-Jordan elimination of the upper triangle, whose every intermediate is
 // Hermitian): A -> A^-1 in place, A[i + ld j], both triangles filled.  A thread holds EPT

@@ -219,14 +219,6 @@ __global__ void __launch_bounds__(SPF_THREADS) spf_drive_kernel(const SpfDesc* _
   });
 }
 
-// 1 / d for d > 0 by Newton's iteration on the hardware's approximate reciprocal
-__device__ __forceinline__ double newton_rcp(double d) {
-  double y;
-  asm("rcp.approx.ftz.f64 %0, %1;" : "=d"(y) : "d"(d));
-  y = fma(y, fma(-d, y, 1.0), y);
-  return fma(y, fma(-d, y, 1.0), y);
-}
-
 // (phi^H phi) X = phi^H dphi by Gauss-Jordan elimination of [S | O] without pivoting,
 // which is stable for the Hermitian positive definite S.  Pivots are real; a thread
 // holds EPT elements of get(row, column) in registers, and per pivot one column and one row pass through
