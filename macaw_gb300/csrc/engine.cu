@@ -1029,7 +1029,7 @@ const cplx* plan_s_weighted(Ctx& c, int s, int skip) {
 // ---------------------------------------------------------------------------
 void plan_gwp_derivs(Ctx& c);
 
-void plan_ovl(Ctx& c, OvlPlan& P, cplx* y1, cplx* y2, int prec, bool norm_only = false, bool shared = true);
+void plan_ovl(Ctx& c, OvlPlan& P, cplx* y1, cplx* y2, bool norm_only = false, bool shared = true);
 void run_ovl(Ctx& c, OvlPlan& P);
 
 // type-1 mean-field contribution: contraction of L_im(A) with the right chain on AuxA
@@ -1075,7 +1075,7 @@ void plan_packets(Ctx& c, std::vector<std::vector<SumSrc>>& srcs, std::vector<st
   std::vector<PkGramPair> pairs;
   // WPpop = norm_wf(A_W, psi) with the SPF overlaps (derivatives.f90:70-76): the
   // intermediate states of an integrator step have non-orthonormal SPFs
-  if (P > 1) plan_ovl(c, c.pk_norm, c.d_in, c.d_in, 0, true);
+  if (P > 1) plan_ovl(c, c.pk_norm, c.d_in, c.d_in, true);
   if (has2) {
     c.pk_xa = c.ar.calloc_c(c.naconftot);
     sum_plan(srcs2, c.pk_sum2);
@@ -1927,10 +1927,8 @@ void plan_hb(Ctx& c) {
 }
 
 // Overlap plan between states y1 and y2: o11 = <1|1>, o22 = <2|2>, o12 = <1|2>
-// (norm_wf / WF_Ovl / DeltaPsi, gmctdh_objects.f90:21-226).  prec 2: the mode
-// products of the chains may take FP32 operands' storage; like prec 0 they have FP64
-// accuracy.
-void plan_ovl(Ctx& c, OvlPlan& P, cplx* y1, cplx* y2, int prec, bool norm_only, bool shared) {
+// (norm_wf / WF_Ovl / DeltaPsi, gmctdh_objects.f90:21-226), FP64 accuracy in every mode.
+void plan_ovl(Ctx& c, OvlPlan& P, cplx* y1, cplx* y2, bool norm_only, bool shared) {
   const int f = c.nmodes;
   P.npk = c.npk;
   P.d_result = c.ar.calloc_c(3 * c.npk);
@@ -1993,8 +1991,6 @@ void plan_ovl(Ctx& c, OvlPlan& P, cplx* y1, cplx* y2, int prec, bool norm_only, 
     }
   }
   P.gwp_d = upload_vec(c.ar, P.gwp_h);
-  // the SPF overlaps over the grid, FP64 accuracy in either
-  P.spf_holes.prec = prec;
   P.spf_holes.finalize(c.ar);
   for (auto& hr : hrefs) P.spf_red.add_term(hr.target, P.spf_holes.h[hr.hole], hr.alpha);
   P.spf_red.finalize(c.ar);
@@ -2045,10 +2041,7 @@ void plan_ovl(Ctx& c, OvlPlan& P, cplx* y1, cplx* y2, int prec, bool norm_only, 
                               mkc(1, 0)});
     }
   }
-  for (auto& b : P.chain) {
-    b.prec = prec;
-    b.finalize(c.ar);
-  }
+  for (auto& b : P.chain) b.finalize(c.ar);
   P.dots.finalize(c.ar);
   for (auto& hr : drefs) P.dot_red.add_term(hr.target, P.dots.h[hr.hole], hr.alpha);
   P.dot_red.finalize(c.ar);
@@ -2523,7 +2516,7 @@ void adams_plan(Ctx& c) {
   c.ad_new1 = c.ar.calloc_c(c.ntot);
   c.ad_dnew = c.ar.calloc_c(c.ntot);
   c.ad_d1 = c.ar.calloc_c(c.ntot);
-  plan_ovl(c, c.ad_plan, c.ad_new, c.ad_new1, (c.precision && c.eps_int >= 1e-5) ? 2 : 0);
+  plan_ovl(c, c.ad_plan, c.ad_new, c.ad_new1);
   c.ad_planned = true;
 }
 
@@ -2714,7 +2707,7 @@ void bs_plan(Ctx& c) {
   cplx** bufs[] = {&c.bs_save, &c.bs_d0, &c.bs_am, &c.bs_an, &c.bs_sw, &c.bs_d, &c.bs_seq, &c.bs_a0, &c.bs_a1};
   for (cplx** b : bufs) *b = c.ar.calloc_c(c.ntot);
   for (int q = 1; q <= BS_KMAXX + 1; ++q) c.bs_q[q] = c.ar.calloc_c(c.ntot);
-  plan_ovl(c, c.bs_plan, c.bs_a0, c.bs_a1, (c.precision && c.eps_int >= 1e-5) ? 2 : 0);
+  plan_ovl(c, c.bs_plan, c.bs_a0, c.bs_a1);
   c.bs_planned = true;
 }
 
@@ -3414,8 +3407,6 @@ void plan_cmf(Ctx& c, CmfState& S) {
     S.lan0 = (double*)c.ar.alloc(sizeof(double) * (3 * NKRYLOV_MAX + NKRYLOV_MAX * NKRYLOV_MAX));
   }
   S.elem_mode = upload_vec(c.ar, em);
-  // the SPF error norms, FP64 accuracy in every mode
-  S.err_holes.prec = c.precision ? 2 : 0;
   S.err_holes.finalize(c.ar);
   for (auto& hr : hrefs) S.err_red.add_term(hr.target, S.err_holes.h[hr.hole], hr.alpha);
   S.err_red.finalize(c.ar);
@@ -4187,12 +4178,11 @@ Ctx* create(const mctdh_setup_t* s, const MemberBufs* mb = nullptr) {
       plan_hb(*c);
       c->d_ovl1 = c->ar.calloc_c(c->ntot);
       c->d_ovl2 = c->ar.calloc_c(c->ntot);
-      plan_ovl(*c, c->cmf_ovl, c->d_ovl1, c->d_ovl2, (c->precision && c->eps_int >= 1e-5) ? 2 : 0, false, false);
+      plan_ovl(*c, c->cmf_ovl, c->d_ovl1, c->d_ovl2, false, false);
     }
-    // prec 0 and 2 are the same arithmetic by now
-    plan_ovl(*c, c->dpsi_plan, c->d_tmp, c->d_err, (c->precision && c->eps_int >= 1e-5) ? 2 : 0);
-    plan_ovl(*c, c->auto_plan, c->d_y0, c->d_y, 0);
-    plan_ovl(*c, c->io_plan, c->d_in, c->d_out, 0);
+    plan_ovl(*c, c->dpsi_plan, c->d_tmp, c->d_err);
+    plan_ovl(*c, c->auto_plan, c->d_y0, c->d_y);
+    plan_ovl(*c, c->io_plan, c->d_in, c->d_out);
     CK(cudaDeviceSynchronize());
   } catch (...) {
     if (c->st && c->own_stream) cudaStreamDestroy(c->st);
@@ -4349,7 +4339,7 @@ struct Ens {
   long long graph_launches[3] = {0, 0, 0}, graph_eoms[3] = {0, 0, 0};
   bool graphs_off = false;
   // autotuned launch shapes (ens_autotune): fibre tiles per contraction block,
-  // block cap per contraction, tensor-core mode products (split path)
+  // block cap per contraction, tensor-core mode products (precision 1)
   bool tuned = false;
   int tune_tpb = HOLE_TPB, tune_cap = HOLE_CAP;
   bool tune_tc = true;
@@ -4617,7 +4607,7 @@ void ens_retile(Ens& E, int tpb, int cap) {
 // Autotuner of the ensemble's launch shapes, run once on the members' states
 // before the first propagation (and before any graph is captured): each
 // candidate (fibre tiles per contraction block, block cap per contraction, and
-// in the split path tensor-core or CUDA-core mode products) is timed with CUDA
+// in precision 1 tensor-core or CUDA-core mode products) is timed with CUDA
 // events over two EOM evaluations of all members after one untimed one, and the
 // fastest is kept.  The merged EOM and the error-norm contractions share the
 // tiling.  Block counts change the order of the partial sums, not the

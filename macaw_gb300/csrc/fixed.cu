@@ -1,6 +1,6 @@
 // Mode products and single-hole contractions of FP64 accuracy as exact digit
 // products on the tensor cores (fixed.cuh) for sm_103a: precision 0, and the
-// compensated products and contractions of the split modes.
+// FP64-accurate products and contractions of the mixed modes.
 #include <algorithm>
 
 #include "kernels.cuh"
