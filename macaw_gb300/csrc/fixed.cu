@@ -632,7 +632,7 @@ __device__ __forceinline__ void hole_mul(HoleWide& sh, cplx* acc, bool mine, boo
   else hole_mul_go<false>(sh, acc, mine, xb, yb, split, half, g0, g1);
 }
 template <bool F32>
-__device__ __forceinline__ void hole_wide_block(const HoleDesc& d, int b, const cplx* ybase) {
+__device__ __forceinline__ void hole_wide_block(const HoleDesc& d, int b, const cplx* ybase, int nsm) {
   extern __shared__ cplx red[];
   HoleWide& sh = *reinterpret_cast<HoleWide*>(red);
   const cplx* Yp = d.Y ? d.Y : ybase + d.yoff;
@@ -646,7 +646,7 @@ __device__ __forceinline__ void hole_wide_block(const HoleDesc& d, int b, const 
   const unsigned g1 = (unsigned)((unsigned long long)ngrp * (b + 1) / d.nblk);
   // the light pair blocks (short last column block) fall to other sub-partitions in
   // every other wave of CTAs
-  const int vw = (warp + 2 * (int)((blockIdx.x / 152) & 1)) & 3;
+  const int vw = (warp + 2 * (int)((blockIdx.x / nsm) & 1)) & 3;
   cplx* out = d.partial + (long long)b * n1 * n2;
   if (tid == 0) sh.slow = 0;
   bool slow = false;
@@ -742,11 +742,12 @@ __global__ void __launch_bounds__(32 * HOLE_WARPS, 3)
 }
 template <bool F32>
 __global__ void __launch_bounds__(64 * HOLE_WARPS, 2)
-    hole_wide_kernel(const HoleDesc* __restrict__ descs, int ndesc, long long first, long long nblocks, const cplx* ybase) {
+    hole_wide_kernel(const HoleDesc* __restrict__ descs, int ndesc, long long first, long long nblocks, const cplx* ybase,
+                     int nsm) {
   for (long long bb = blockIdx.x; bb < nblocks; bb += gridDim.x) {
     const HoleDesc& d = descs[warp_find_desc(descs, ndesc, first + bb)];
     if (bb != blockIdx.x) __syncthreads();
-    hole_wide_block<F32>(d, (int)(first + bb - d.block_start), ybase);
+    hole_wide_block<F32>(d, (int)(first + bb - d.block_start), ybase, nsm);
     hole_sum_blocks<2 * HOLE_WARPS>(d);
   }
 }
@@ -760,7 +761,7 @@ static void hole_fx_go(const HoleLaunch& b, int persist, cudaStream_t st, const 
         b.d, b.nnarrow, b.narrow_blocks, ybase);
   if (wide > 0)
     hole_wide_kernel<F32><<<grid(wide), 64 * HOLE_WARPS, sizeof(HoleWide), st>>>(
-        b.d + b.nnarrow, b.ndesc - b.nnarrow, b.narrow_blocks, wide, ybase);
+        b.d + b.nnarrow, b.ndesc - b.nnarrow, b.narrow_blocks, wide, ybase, sm_count());
 }
 
 void launch_hole_fx(const HoleLaunch& b, cudaStream_t st, int persist, const cplx* ybase) {

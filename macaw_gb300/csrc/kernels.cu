@@ -903,7 +903,7 @@ __global__ void __launch_bounds__(128) reginv_kernel(const RegInvDesc* __restric
 void launch_reginv(const RegInvDesc* d_descs, int ndesc, const MFOp* d_ops, int* d_status, cudaStream_t st) {
   if (ndesc <= 0) return;
   // up to four blocks per matrix while the GPU has SMs for them
-  const unsigned split = (unsigned)std::max(1, std::min(4, 152 / ndesc));
+  const unsigned split = (unsigned)std::max(1, std::min(4, sm_count() / ndesc));
   reginv_kernel<<<dim3(ndesc, split), 128, 0, st>>>(d_descs, d_ops, d_status);
 }
 
@@ -1773,7 +1773,7 @@ __global__ void lan_normalize_kernel(cplx* __restrict__ out, const cplx* __restr
 void launch_lan_normalize(cplx* out, const cplx* in, const cplx* nrm2, double* beta_out, long long n, cudaStream_t st,
                           cplx* copy, cplx* f32) {
   const long long want = (n + 255) / 256;
-  const unsigned nb = (unsigned)std::max<long long>(1, std::min<long long>(want, 152 * 4));
+  const unsigned nb = (unsigned)std::max<long long>(1, std::min<long long>(want, 4LL * sm_count()));
   lan_normalize_kernel<<<nb, 256, 0, st>>>(out, in, nrm2, beta_out, n, copy, reinterpret_cast<float2*>(f32));
 }
 

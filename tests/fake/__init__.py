@@ -36,11 +36,14 @@ class Fake:
         self.lib.fake_status(0)
         self.lib.fake_clear()
 
-    def kernels(self):
-        """Names of the kernels launched since the last reset or call of this."""
-        names = self.lib.fake_log().decode().split()
+    def launches(self):
+        """(kernel, grid x, grid y) of the launches since the last reset or call of this."""
+        lines = [x.split("@") for x in self.lib.fake_log().decode().split()]
         self.lib.fake_clear()
-        return names
+        return [(name, *map(int, grid.split(","))) for name, grid in lines]
+
+    def kernels(self):
+        return [x[0] for x in self.launches()]
 
 
 def use(monkeypatch, path):

@@ -13,7 +13,7 @@
 
 namespace {
 constexpr int DEVICES = 2;
-int g_dev = 0;
+int g_dev = 0, g_sms[DEVICES] = {152, 152};
 cudaError_t g_last = cudaSuccess;
 std::map<const void*, std::string> g_name;               // host stub -> kernel
 std::map<std::pair<int, const void*>, int> g_optin;      // (device, kernel) -> dynamic shared memory
@@ -37,11 +37,12 @@ cudaError_t copy(void* d, const void* s, size_t n, cudaMemcpyKind k) {
 // the tests' side
 extern "C" {
 void fake_device(int d) { g_dev = d; }
+void fake_sms(int d, int n) { g_sms[d] = n; }
 void fake_pending(int e) { g_last = (cudaError_t)e; }
 void fake_fail(const char* part) { g_fail = part; }       // launches of kernels so named are refused
 void fake_status(int bits) { g_status = bits; }           // or-ed into every int read back
 void fake_clear() { g_log.clear(); }
-const char* fake_log() { return g_log.c_str(); }          // launched kernels, one per line
+const char* fake_log() { return g_log.c_str(); }          // launches, one per line: kernel@grid x,grid y
 }
 
 extern "C" {
@@ -73,8 +74,9 @@ cudaError_t __cudaLaunchKernel(cudaKernel_t k, dim3 g, dim3 b, void**, size_t sm
   if (smem > 48 * 1024 && (int)smem > g_optin[{g_dev, (const void*)k}]) return fail(cudaErrorInvalidValue);
   if (!g.x || !g.y || !g.z || g.y > 65535 || g.z > 65535 || !b.x || b.x * b.y * b.z > 1024)
     return fail(cudaErrorInvalidConfiguration);
-  if (g_capture) g_capture->push_back(name);
-  else g_log += name + "\n";
+  const std::string note = name + "@" + std::to_string(g.x) + "," + std::to_string(g.y);
+  if (g_capture) g_capture->push_back(note);
+  else g_log += note + "\n";
   return cudaSuccess;
 }
 cudaError_t cudaFuncSetAttribute(const void* f, cudaFuncAttribute a, int v) {
@@ -85,7 +87,7 @@ cudaError_t cudaFuncSetAttribute(const void* f, cudaFuncAttribute a, int v) {
 
 cudaError_t cudaGetDeviceCount(int* n) { return *n = DEVICES, cudaSuccess; }
 cudaError_t cudaGetDevice(int* d) { return *d = g_dev, cudaSuccess; }
-cudaError_t cudaDeviceGetAttribute(int* v, cudaDeviceAttr, int) { return *v = 152, cudaSuccess; }
+cudaError_t cudaDeviceGetAttribute(int* v, cudaDeviceAttr, int d) { return *v = g_sms[d], cudaSuccess; }
 cudaError_t cudaDeviceSynchronize() { return cudaSuccess; }
 const char* cudaGetErrorString(cudaError_t) { return "an error of the test's making"; }
 cudaError_t cudaPeekAtLastError() { return g_last; }

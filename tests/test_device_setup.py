@@ -49,3 +49,18 @@ def test_ensemble_on_second_device(library, monkeypatch):
         seen.append(rt.kernels())
         ens.close()
     assert seen[0] and seen[1] == seen[0]
+
+
+def test_grids_follow_the_device(tmp_path, monkeypatch):
+    """Two blocks a matrix where the device has two SMs for each, four where it has more."""
+    rt = fake.use(monkeypatch, fake.fake_runtime(tmp_path))   # its own copy: SM counts are kept
+    model = _model(4)                                         # 2 states x 3 modes
+    rt.lib.fake_sms(1, 13)
+    A, psi = random_state(model)
+    for device, blocks in ((0, 4), (1, 2)):
+        rt.lib.fake_device(device)
+        core = capi.GpuCore(model)
+        rt.launches()
+        core.calc_derivs(A, psi)
+        assert [x[1:] for x in rt.launches() if "reginv" in x[0]] == [(6, blocks)]
+        core.close()
