@@ -107,11 +107,13 @@ struct ProdBatch {
   long long nblocks = 0;
   int maxn = 0;
   int prec = 0;                  // 1 FP32, else FP64 accuracy (digit products)
+  bool plain = true;             // no factor but one, nothing accumulated
   double flops = 0, bytes = 0;   // algorithmic work of one launch
   void add(const cplx* X, cplx* Y, const cplx* M, int ldm, int conjT, const std::vector<int>& shape, int mode,
            int nout, cplx alpha, int accumulate, int xfmt = TF_C64, int yfmt = TF_C64) {
     if (yfmt != TF_C64 && (accumulate || alpha.x != 1.0 || alpha.y != 0.0))
       throw StatusError(MCTDH_EARG, "FP32 output needs alpha = 1 without accumulation");
+    plain = plain && !accumulate && alpha.x == 1.0 && alpha.y == 0.0;
     ProdDesc pd;
     memset(&pd, 0, sizeof(pd));
     pd.xfmt = xfmt;
@@ -243,6 +245,7 @@ struct HoleBatch {
 void merge_prod(ProdBatch& d, const ProdBatch& s) {
   d.h.insert(d.h.end(), s.h.begin(), s.h.end());
   d.prec = s.prec;
+  d.plain = d.plain && s.plain;
 }
 void merge_hole(HoleBatch& d, const HoleBatch& s) {
   d.h.insert(d.h.end(), s.h.begin(), s.h.end());
@@ -2200,7 +2203,7 @@ struct StreamSwap {
 void run_prod(Ctx& c, const ProdBatch& b) {
   if (b.h.empty()) return;
   ProfScope ps(c, KP_PROD, b.flops, b.bytes);
-  launch_prod(b.d, (int)b.h.size(), b.nblocks, b.maxn, c.d_status, c.st, b.prec);
+  launch_prod(b.d, (int)b.h.size(), b.nblocks, b.maxn, b.plain, c.d_status, c.st, b.prec);
   c.count();
 }
 void run_hole(Ctx& c, const HoleBatch& b) {
@@ -4563,7 +4566,7 @@ void ens_destroy(Ens* E) {
 
 void ens_run_prod(Ens& E, const ProdBatch& b) {
   if (b.h.empty()) return;
-  launch_prod(b.d, (int)b.h.size(), b.nblocks, b.maxn, E.status_d, E.st, b.prec, E.tune_tc ? 2 : 0, E.persist_prod);
+  launch_prod(b.d, (int)b.h.size(), b.nblocks, b.maxn, b.plain, E.status_d, E.st, b.prec, E.tune_tc ? 2 : 0, E.persist_prod);
   ++E.launches;
 }
 void ens_run_hole(Ens& E, const HoleBatch& b) {

@@ -488,9 +488,10 @@ __global__ void __launch_bounds__(LU_MAXROWS) lu_panel_kernel(const GwpCYDesc* _
 // for its columns (the blocks of the first row of blocks store the result as U), then
 // subtracts the rank-8 product as exact digit products (fixed.cuh; a warp's 16 rows are
 // the MMA's rows, the (re, im) of four columns its columns, as in the mode products),
-// where FP64 would take 18 us of an SM's FP64 pipe per block.
+// where FP64 would take 18 us of an SM's FP64 pipe per block; elements small against the
+// factors (a panel whose rows and columns are graded) are done in FP64.
 __global__ void __launch_bounds__(256) lu_update_kernel(const GwpCYDesc* __restrict__ descs, int j0) {
-  constexpr int NS = 8;
+  constexpr int NS = FX_NS, SH = fx_headroom(LU_PW);
   const GwpCYDesc& d = descs[blockIdx.z];
   const int nG = d.nG;
   if (j0 >= nG) return;
@@ -532,13 +533,14 @@ __global__ void __launch_bounds__(256) lu_update_kernel(const GwpCYDesc* __restr
   }
   __syncthreads();
   unsigned er[2];
-  bool bad = false;
+  bool bad = false, live[2];
 #pragma unroll
   for (int f = 0; f < 2; ++f) {
     unsigned mag = max(fx_mag(x[f][0]), fx_mag(x[f][1]));
     mag = max(mag, __shfl_xor_sync(0xffffffffu, mag, 1));
     mag = max(mag, __shfl_xor_sync(0xffffffffu, mag, 2));
     bad = bad || !fx_ok(mag);
+    live[f] = mag != 0u;
     er[f] = fx_ebits(mag);
   }
   cplx y[2][2];   // in flight during the products
@@ -555,7 +557,7 @@ __global__ void __launch_bounds__(256) lu_update_kernel(const GwpCYDesc* __restr
 #pragma unroll
     for (int k = 0; k < 2; ++k) {
       unsigned s[NS];
-      fx_digits<NS>(x[f][k].x, x[f][k].y, er[f], er[f], s);
+      fx_digits(x[f][k].x, x[f][k].y, er[f], er[f], s);
 #pragma unroll
       for (int i = 0; i < NS; ++i) A[i][2 * k + f] = s[i];
     }
@@ -568,13 +570,14 @@ __global__ void __launch_bounds__(256) lu_update_kernel(const GwpCYDesc* __restr
     mag = max(mag, __shfl_xor_sync(0xffffffffu, mag, 2));
     const bool slow = __any_sync(0xffffffffu, bad || !fx_ok(mag));
     const unsigned ec = fx_ebits(mag);
-    const unsigned es = fx_exp(__shfl_sync(0xffffffffu, ec, 8 * q), 0u, 44);
+    const unsigned ecol = __shfl_sync(0xffffffffu, ec, 8 * q), es = fx_exp(ecol, 0u, 44 + SH);
+    const bool lcol = __shfl_sync(0xffffffffu, mag, 8 * q) != 0u;
     const int col = c0 + 32 * blockIdx.x + 4 * t + q;
     float c[NS][4];
     if (!slow) {
       unsigned s0[NS], s1[NS];
-      fx_digits<NS>(m0.x, m0.y, ec, ec, s0);
-      fx_digits<NS>(m1.x, m1.y, ec, ec, s1);
+      fx_digits(m0.x, m0.y, ec, ec, s0);
+      fx_digits(m1.x, m1.y, ec, ec, s1);
 #pragma unroll
       for (int i = 0; i < NS; ++i) {   // column re: (Mr, -Mi); column im: (Mi, Mr)
         const unsigned w0 = (g & 1) ? __byte_perm(s0[i], s0[i], 0x1032) : s0[i] ^ 0x80000000u;
@@ -586,10 +589,15 @@ __global__ void __launch_bounds__(256) lu_update_kernel(const GwpCYDesc* __restr
 #pragma unroll
     for (int f = 0; f < 2; ++f) {
       if (row[f] < 0 || col > nG) continue;
-      cplx v;
+      cplx v = mkc(0.0, 0.0);
+      bool fp64 = slow;
       if (!slow) {
-        v = mkc(fx_double(fx_join<NS>(c, 2 * f), es + er[f]), fx_double(fx_join<NS>(c, 2 * f + 1), es + er[f]));
-      } else {
+        const long long re = fx_join(c, 2 * f, fx_pow2(SH)), im = fx_join(c, 2 * f + 1, fx_pow2(SH));
+        v = mkc(fx_double(re, es + er[f]), fx_double(im, es + er[f]));
+        // both the product and the element below 2^-8 of the largest factors' product
+        fp64 = fx_small(re, im, fx_small_limit(SH)) && live[f] && lcol && fx_mag(y[tt][f]) < er[f] + ecol - (1029u << 20);
+      }
+      if (fp64) {
         v = mkc(0.0, 0.0);
         for (int k = 0; k < pw; ++k) cfma(v, d.M[row[f] + ld * (j0 + k)], T[4 * t + q][k]);
       }

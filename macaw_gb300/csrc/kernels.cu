@@ -136,11 +136,11 @@ int sm_count() {
 // tc: 0 CUDA-core kernel, 1 tensor cores from the configured SPF count on,
 // 2 tensor cores for every size they take (the ensemble autotuner's candidate).
 // persist > 0: at most that many persistent CTAs walk the blocks.
-void launch_prod(const ProdDesc* d_descs, int ndesc, long long nblocks, int maxn, int* status, cudaStream_t st,
+void launch_prod(const ProdDesc* d_descs, int ndesc, long long nblocks, int maxn, bool plain, int* status, cudaStream_t st,
                  int prec, int tc, int persist) {
   if (ndesc <= 0 || nblocks <= 0) return;
   if (prec != 1) {
-    launch_prod_fx(d_descs, ndesc, nblocks, maxn, status, st, persist);
+    launch_prod_fx(d_descs, ndesc, nblocks, maxn, plain, status, st, persist);
     return;
   }
   if (tc && tc_enabled() && launch_prod_tc(d_descs, ndesc, nblocks, maxn, status, st, tc == 2)) return;

@@ -254,9 +254,9 @@ bool launch_prod_tc(const ProdDesc* d_descs, int ndesc, long long nblocks, int m
 int tc_timeout_flag(bool clear);
 // the settings that choose the captured kernels, as one number
 int tc_config();
-// persist > 0: at most `persist` persistent CTAs walk the batch's blocks; status: the
-// word that takes DEVST_TC_WAIT
-void launch_prod(const ProdDesc* d_descs, int ndesc, long long nblocks, int maxn, int* status, cudaStream_t st,
+// persist > 0: at most `persist` persistent CTAs walk the batch's blocks; plain: alpha = 1
+// and no accumulation in the whole batch; status: the word that takes DEVST_TC_WAIT
+void launch_prod(const ProdDesc* d_descs, int ndesc, long long nblocks, int maxn, bool plain, int* status, cudaStream_t st,
                  int prec = 0, int tc = 1, int persist = 0);
 // a batch of contractions: descriptors with n1, n2 <= 8 first
 struct HoleLaunch {
@@ -289,9 +289,9 @@ void launch_rk_end(cplx* y5, cplx* diff, const cplx* base, const StageArgs& a, c
                    const unsigned char* elem_mode, long long off, long long n, cudaStream_t st);
 // FP64 accuracy as exact digit products on the tensor cores (fixed.cu); launched by
 // launch_prod / launch_hole
-void launch_prod_fx(const ProdDesc* d_descs, int ndesc, long long nblocks, int maxn, int* status, cudaStream_t st,
-                    int persist);
-// ... with tcgen05 MMAs, nin and nout <= 16 (tc.cu)
+void launch_prod_fx(const ProdDesc* d_descs, int ndesc, long long nblocks, int maxn, bool plain, int* status,
+                    cudaStream_t st, int persist);
+// ... with tcgen05 MMAs, nin and nout <= 16, plain (tc.cu)
 void launch_prod_digits_tc(const ProdDesc* d_descs, int ndesc, long long nblocks, int maxn, int* status, cudaStream_t st);
 void launch_hole_fx(const HoleLaunch& b, cudaStream_t st, int persist, const cplx* ybase = nullptr);
 void launch_reduce(const RedTarget* d_tg, int ntg, const RedTerm* d_terms, cudaStream_t st);

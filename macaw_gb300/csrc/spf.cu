@@ -12,8 +12,7 @@
 #include "fixed.cuh"
 
 #define SPF_THREADS 256
-#define SPF_NS 8
-#define SPF_CHUNK 9      // steps of eight columns between flushes: 9 x 16 x 7 x 2^14 < 2^24
+#define SPF_CHUNK 9      // steps of eight columns between flushes: 5 x 16 x 8 x 2^14 < 2^24 per half
 #define SPF_COLS (8 * SPF_CHUNK)
 
 #define SPF_PITCH (SPF_ROWS + 2)   // staged rows of a column: the lanes' 16-byte reads meet no bank twice
@@ -22,14 +21,20 @@
 struct RowShared {
   cplx x[SPF_CHUNK][8][SPF_PITCH];         // the CTA's rows of a chunk of steps
   union {
-    uint2 W[SPF_CHUNK][2][SPF_NS][32];     // digits of eight columns of the matrix (j2 = q and q + 4)
+    uint2 W[SPF_CHUNK][2][FX_NS][32];     // digits of eight columns of the matrix (j2 = q and q + 4)
     struct {
-      unsigned char small[sizeof(uint2) * SPF_CHUNK * 2 * SPF_NS * 32 - 8192];
-      cplx other[4][2][2][32];             // the second warps' sums, once W is read
+      unsigned char small[sizeof(uint2) * SPF_CHUNK * 2 * FX_NS * 32 - 8192 - 2048];
+      float tother[4][2][2][32];           // the second warps' sums of |x||rm| and their
+      cplx other[4][2][2][32];             // sums, once W is read
     };
   };
-  unsigned colmag[MAXN_SPF];
+  unsigned colmag[8], top;                 // largest elements of the columns j1 (scaled), of the matrix
+  unsigned scale[SPF_COLS];                // the columns' scaling
 };
+// the scaling of a column whose rm are zero: its x, brought out of range by it, count for
+// nothing, and the digits of either are zero
+#define SPF_EMPTY 0x7ff00000u
+#define SPF_SCALE_MAX 400
 
 __device__ __forceinline__ void copy_async16(void* dst, const void* src) {
   asm volatile("cp.async.ca.shared.global [%0], [%1], 16;" ::"r"((unsigned)__cvta_generic_to_shared(dst)), "l"(src)
@@ -50,24 +55,32 @@ __device__ __forceinline__ void stage_rows(RowShared& S, int s0, int ns, Col&& c
   }
 }
 
+// 2^e as FP32 for e <= 0, zero where that is no normal number
+__device__ __forceinline__ float spf_pow2(int e) { return e > -127 ? __int_as_float((e + 127) << 23) : 0.f; }
+
 // The CTA's rows row0 .. row0 + 63 of sum_j x(row, j) rm(j1, j) over ncols columns for all
 // j1 < n: warps w and w + 4 own 16 rows (the MMA's rows) and every second step, the
-// columns are the (re, im) of four j1; a row
-// has one exponent per chunk of steps, a column j1 of the matrices another.  col(j)
-// returns the j-th column of x and of rm, a step is eight of them (whatever operators
-// they belong to); the first chunk is staged already.
+// columns are the (re, im) of four j1.  Column j of x is multiplied and rm(., j) divided
+// by a power of two that makes the rm(., j) alike in size, whatever the operators' units;
+// then a row has one exponent per chunk of steps, a column j1 of the matrices another.
+// col(j) returns the j-th column of x and of rm, a step is eight of them (whatever
+// operators they belong to); the first chunk is staged already.
 // put(row, j1, value) takes the results (warps 0 - 3); rows from G on are skipped.  The
-// matrices are cut while the rows are on their way.  Operands outside
-// the exponent range are multiplied in FP64.
+// matrices are cut while the rows are on their way.  Operands outside the exponent range
+// are multiplied in FP64, and so are elements whose sum of |x||rm| (one more MMA, on the
+// leading digits) is below 2^-6 .. 2^-8 of the product of the largest elements.
 template <typename Col, typename Put>
 __device__ __forceinline__ void row_products(RowShared& S, int ncols, Col&& col, int n, int G, int row0, Put&& put) {
-  constexpr int NS = SPF_NS;
+  constexpr int NS = FX_NS;
   const int nsteps = (ncols + 7) / 8;
   const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5, g = lane >> 2, q = lane & 3;
   const int half = warp >> 2, lr = 16 * (warp & 3) + g;   // the lane's rows: lr, lr + 8
   auto& other = S.other;
   for (int j0 = 0; j0 < n; j0 += 8) {   // eight outputs per pass
     cplx sum[2][2];                     // [group of four j1][row]
+    // sums of |x||rm|, and of the products of largest elements, both times 2^-eref
+    float tsum[2][2] = {{0.f, 0.f}, {0.f, 0.f}}, bsum[2][2] = {{0.f, 0.f}, {0.f, 0.f}};
+    int eref[2][2] = {{0, 0}, {0, 0}};
     for (int s0 = 0; s0 < nsteps; s0 += SPF_CHUNK) {
       const int ns = min(SPF_CHUNK, nsteps - s0);
       if (s0 || (j0 && nsteps > SPF_CHUNK)) {
@@ -75,30 +88,46 @@ __device__ __forceinline__ void row_products(RowShared& S, int ncols, Col&& col,
         stage_rows(S, s0, ns, col, ncols, G, row0);
       }
       if (tid < 8) S.colmag[tid] = 0u;
+      if (tid == 8) S.top = 0u;
       __syncthreads();
       const int nc = min(8, n - j0);
-      for (int e0 = tid; e0 < 64 * ns; e0 += 3 * SPF_THREADS) {   // (j, j1), three loads in flight
-        unsigned m[3];
+      // (j, j1): at most three per thread, the eight of a column in neighbouring lanes
+      constexpr int PER = (64 * SPF_CHUNK + SPF_THREADS - 1) / SPF_THREADS;
+      unsigned m[PER], rmag[PER];
 #pragma unroll
-        for (int i = 0; i < 3; ++i) {
-          const int e = e0 + i * SPF_THREADS, j = 8 * s0 + (e >> 3);
-          m[i] = e < 64 * ns && j < ncols && (e & 7) < nc ? fx_mag(col(j).rm[j0 + (e & 7)]) : 0u;
-        }
-        const unsigned all = max(m[0], max(m[1], m[2]));
-        if (all) atomicMax(&S.colmag[e0 & 7], all);
+      for (int i = 0; i < PER; ++i) {
+        const int e = tid + i * SPF_THREADS, j = 8 * s0 + (e >> 3);
+        m[i] = e < 64 * ns && j < ncols && (e & 7) < nc ? fx_mag(col(j).rm[j0 + (e & 7)]) : 0u;
+      }
+#pragma unroll
+      for (int i = 0; i < PER; ++i) {
+        rmag[i] = m[i];
+#pragma unroll
+        for (int o = 1; o < 8; o <<= 1) rmag[i] = max(rmag[i], __shfl_xor_sync(0xffffffffu, rmag[i], o));
+        if ((tid & 7) == 0 && rmag[i]) atomicMax(&S.top, rmag[i]);
+      }
+      __syncthreads();
+      const unsigned top = S.top & FX_EBITS;
+#pragma unroll
+      for (int i = 0; i < PER; ++i) {
+        const int e = tid + i * SPF_THREADS;
+        if (e >= 64 * ns) break;
+        const unsigned b = min(top - (rmag[i] & FX_EBITS), (unsigned)SPF_SCALE_MAX << 20);
+        if ((e & 7) == 0) S.scale[e >> 3] = rmag[i] ? b : SPF_EMPTY;
+        if (m[i]) atomicMax(&S.colmag[e & 7], m[i] + b);
       }
       __syncthreads();
       bool bad = tid < nc && !fx_ok(S.colmag[tid]);
       for (int w = warp; w < 2 * ns; w += SPF_THREADS / 32) {
         const int t = w & 1, s = w >> 1, j1 = 4 * t + (g >> 1);
         if (4 * t >= nc) continue;
-        const int jc = 8 * (s0 + s) + q;
+        const int jl = 8 * s + q, jc = 8 * s0 + jl;
         unsigned d0[NS], d1[NS];
         const cplx m0 = (j1 < nc && jc < ncols) ? col(jc).rm[j0 + j1] : mkc(0, 0);
         const cplx m1 = (j1 < nc && jc + 4 < ncols) ? col(jc + 4).rm[j0 + j1] : mkc(0, 0);
-        const unsigned em = fx_ebits(S.colmag[j1]);
-        fx_digits<NS>(m0.x, m0.y, em, em, d0);
-        fx_digits<NS>(m1.x, m1.y, em, em, d1);
+        const unsigned em = fx_ebits(S.colmag[j1]), b0 = S.scale[jl], b1 = S.scale[jl + 4];
+        fx_digits(m0.x, m0.y, em - b0, em - b0, d0);
+        fx_digits(m1.x, m1.y, em - b1, em - b1, d1);
 #pragma unroll
         for (int i = 0; i < NS; ++i) {   // column re: (Mr, -Mi); column im: (Mi, Mr)
           const unsigned w0 = (g & 1) ? __byte_perm(d0[i], d0[i], 0x1032) : d0[i] ^ 0x80000000u;
@@ -108,17 +137,29 @@ __device__ __forceinline__ void row_products(RowShared& S, int ncols, Col&& col,
       }
       copy_async_wait();
       __syncthreads();
-      unsigned mag[2] = {0u, 0u};
+      unsigned mag[2];
+      {
+        int most[2] = {0, 0};        // scaled
+        unsigned raw[2] = {0u, 0u};
 #pragma unroll 3
-      for (int s = 0; s < ns; ++s)
+        for (int s = 0; s < ns; ++s)
 #pragma unroll
-        for (int f = 0; f < 2; ++f)
-          mag[f] = max(mag[f], max(fx_mag(S.x[s][q][lr + 8 * f]), fx_mag(S.x[s][q + 4][lr + 8 * f])));
+          for (int h = 0; h < 2; ++h) {
+            const unsigned b = S.scale[8 * s + q + 4 * h];
 #pragma unroll
-      for (int f = 0; f < 2; ++f) {
-        mag[f] = max(mag[f], __shfl_xor_sync(0xffffffffu, mag[f], 1));
-        mag[f] = max(mag[f], __shfl_xor_sync(0xffffffffu, mag[f], 2));
-        bad = bad || !fx_ok(mag[f]);
+            for (int f = 0; f < 2; ++f) {
+              const unsigned x = fx_mag(S.x[s][q + 4 * h][lr + 8 * f]);
+              raw[f] = max(raw[f], b == SPF_EMPTY && x < FX_EBITS ? 0u : x);
+              most[f] = max(most[f], (int)(x - b));
+            }
+          }
+#pragma unroll
+        for (int f = 0; f < 2; ++f) {
+          most[f] = max(most[f], __shfl_xor_sync(0xffffffffu, most[f], 1));
+          most[f] = max(most[f], __shfl_xor_sync(0xffffffffu, most[f], 2));
+          mag[f] = (unsigned)most[f];
+          bad = bad || !fx_ok(mag[f]) || raw[f] >= FX_EBITS || (raw[f] && !mag[f]);
+        }
       }
       const unsigned eb[2] = {fx_ebits(mag[0]), fx_ebits(mag[1])};
       if (__syncthreads_or(bad)) {   // the pass in FP64
@@ -132,31 +173,39 @@ __device__ __forceinline__ void row_products(RowShared& S, int ncols, Col&& col,
         goto next_pass;
       }
       {
-        float c[2][NS][4];
+        float c[2][NS][4], ct[2][4];
 #pragma unroll
         for (int t = 0; t < 2; ++t)
 #pragma unroll
-          for (int i = 0; i < NS; ++i)
+          for (int k = 0; k < 4; ++k) {
+            ct[t][k] = 0.f;
 #pragma unroll
-            for (int k = 0; k < 4; ++k) c[t][i][k] = 0.f;
+            for (int i = 0; i < NS; ++i) c[t][i][k] = 0.f;
+          }
         for (int s = half; s < ns; s += 2) {
-          unsigned A[NS][4];
+          unsigned A[NS][4], ta[4];
 #pragma unroll
-          for (int f = 0; f < 2; ++f)
+          for (int h = 0; h < 2; ++h) {
+            const unsigned b = S.scale[8 * s + q + 4 * h];
 #pragma unroll
-            for (int h = 0; h < 2; ++h) {
+            for (int f = 0; f < 2; ++f) {
               unsigned d[NS];
               const cplx x = S.x[s][q + 4 * h][lr + 8 * f];
-              fx_digits<NS>(x.x, x.y, eb[f], eb[f], d);
+              fx_digits(x.x, x.y, eb[f] + b, eb[f] + b, d);
 #pragma unroll
               for (int i = 0; i < NS; ++i) A[i][2 * h + f] = d[i];
+              ta[2 * h + f] = fx_lead(d[0], d[1]);
             }
+          }
 #pragma unroll
           for (int t = 0; t < 2; ++t) {
             if (4 * t < nc) {
+              uint2 w0;
 #pragma unroll
               for (int i = 0; i < NS; ++i) {
                 const uint2 w = S.W[s][t][i][lane];
+                if (i == 0) w0 = w;
+                if (i == 1) fx_mma16(ct[t], ta, fx_lead(w0.x, w.x), fx_lead(w0.y, w.y), false);
 #pragma unroll
                 for (int j = 0; j + i < NS; ++j) fx_mma16(c[t][i + j], A[j], w.x, w.y, false);
               }
@@ -166,32 +215,48 @@ __device__ __forceinline__ void row_products(RowShared& S, int ncols, Col&& col,
 #pragma unroll
         for (int t = 0; t < 2; ++t) {
           if (4 * t < nc) {
-            const unsigned em = fx_ebits(S.colmag[4 * t + q]);
+            const unsigned cm = S.colmag[4 * t + q], em = fx_ebits(cm);
 #pragma unroll
             for (int f = 0; f < 2; ++f) {
-              const unsigned es = fx_exp(em, eb[f], 43);
-              const cplx v =
-                  mkc(fx_double(fx_join_wide<NS, 1>(c[t], 2 * f), es), fx_double(fx_join_wide<NS, 1>(c[t], 2 * f + 1), es));
+              const unsigned es = fx_exp(em, eb[f], 44);
+              const cplx v = mkc(fx_double(fx_join_wide(c[t], 2 * f, 1.f), es), fx_double(fx_join_wide(c[t], 2 * f + 1, 1.f), es));
               sum[t][f] = s0 ? cadd(sum[t][f], v) : v;
+              if (cm && mag[f]) {
+                const int e = (int)(em >> 20) + (int)(eb[f] >> 20), up = max(e, eref[t][f]);
+                const float keep = spf_pow2(eref[t][f] - up), add = spf_pow2(e - up);
+                tsum[t][f] = fmaf(tsum[t][f], keep, (ct[t][2 * f] + ct[t][2 * f + 1]) * add);
+                bsum[t][f] = fmaf(bsum[t][f], keep, add);
+                eref[t][f] = up;
+              }
             }
           }
         }
       }
-      __syncthreads();   // colmag and W are read
+      __syncthreads();   // colmag, scale and W are read
     }
     if (half)
 #pragma unroll
       for (int t = 0; t < 2; ++t)
 #pragma unroll
-        for (int f = 0; f < 2; ++f) other[warp & 3][t][f][lane] = nsteps ? sum[t][f] : mkc(0, 0);
+        for (int f = 0; f < 2; ++f) {
+          other[warp & 3][t][f][lane] = nsteps ? sum[t][f] : mkc(0, 0);
+          S.tother[warp & 3][t][f][lane] = tsum[t][f];
+        }
     __syncthreads();
     if (!half)
 #pragma unroll
       for (int t = 0; t < 2; ++t)
 #pragma unroll
         for (int f = 0; f < 2; ++f)
-          if (j0 + 4 * t + q < n && row0 + lr + 8 * f < G)
-            put(row0 + lr + 8 * f, j0 + 4 * t + q, nsteps ? cadd(sum[t][f], other[warp & 3][t][f][lane]) : mkc(0, 0));
+          if (j0 + 4 * t + q < n && row0 + lr + 8 * f < G) {
+            const int row = row0 + lr + 8 * f, j1 = j0 + 4 * t + q;
+            cplx v = nsteps ? cadd(sum[t][f], other[warp & 3][t][f][lane]) : mkc(0, 0);
+            if (tsum[t][f] + S.tother[warp & 3][t][f][lane] < FX_LOW * bsum[t][f]) {   // the element in FP64
+              v = mkc(0, 0);
+              for (int j = 0; j < ncols; ++j) cfma(v, col(j).x[row], col(j).rm[j1]);
+            }
+            put(row, j1, v);
+          }
   next_pass:;
   }
 }
@@ -284,19 +349,20 @@ static_assert(sizeof(SpfSmall) <= sizeof(RowShared::W) && offsetof(SpfSmall, red
               "takes the place of the digits, red alone that of the second warps' sums");
 
 // so = (phi^H phi, phi^H dphi) of the CTA's 64 rows: warp w takes 16 rows of the first
-// as in the contraction kernel for n <= 8 (seven digits, weights above 2^-64), warp w + 4
-// of the second; the four warps' sums are added in order.
+// as in the contraction kernel for n <= 8, warp w + 4 of the second, sums that are small
+// against the columns' largest elements again in FP64; the four warps' sums are added in
+// order.
 __device__ __forceinline__ void contract_rows(SpfSmall& T) {
-  constexpr int NS = 7, ND = 8;
+  constexpr int NS = FX_NS;
   const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5, g = lane >> 2, q = lane & 3;
-  const int which = warp >> 2, r0 = 16 * (warp & 3) + 2 * q;
+  const int which = warp >> 2, r0 = 16 * (warp & 3);
   const cplx (*Y)[SPF_PITCH] = which ? T.dph : T.phs;
   unsigned mx = 0u, my = 0u;
   cplx x[4], y[4];
 #pragma unroll
   for (int f = 0; f < 4; ++f) {
-    x[f] = T.phs[g][r0 + (f & 1) + 8 * (f >> 1)];
-    y[f] = Y[g][r0 + (f & 1) + 8 * (f >> 1)];
+    x[f] = T.phs[g][r0 + 2 * q + (f & 1) + 8 * (f >> 1)];
+    y[f] = Y[g][r0 + 2 * q + (f & 1) + 8 * (f >> 1)];
     mx = max(mx, fx_mag(x[f]));
     my = max(my, fx_mag(y[f]));
   }
@@ -307,40 +373,49 @@ __device__ __forceinline__ void contract_rows(SpfSmall& T) {
   }
   const unsigned ex = fx_ebits(mx), ey = fx_ebits(my);
   unsigned A[NS][4], B[NS][4];   // (re, im) of fibres 2 q, 2 q + 1, then of 2 q + 8, 2 q + 9
+  unsigned ta[4], tb[2];
 #pragma unroll
   for (int h = 0; h < 2; ++h) {
     unsigned s[NS];
-    fx_digits<NS>(x[2 * h].x, x[2 * h + 1].x, ex, ex, s);
+    fx_digits(x[2 * h].x, x[2 * h + 1].x, ex, ex, s);
 #pragma unroll
     for (int k = 0; k < NS; ++k) A[k][2 * h] = s[k];
-    fx_digits<NS>(x[2 * h].y, x[2 * h + 1].y, ex, ex, s);
+    ta[2 * h] = fx_lead(s[0], s[1]);
+    fx_digits(x[2 * h].y, x[2 * h + 1].y, ex, ex, s);
 #pragma unroll
     for (int k = 0; k < NS; ++k) A[k][2 * h + 1] = s[k];
-    fx_digits<NS>(y[2 * h].x, y[2 * h + 1].x, ey, ey, s);
+    ta[2 * h + 1] = fx_lead(s[0], s[1]);
+    fx_digits(y[2 * h].x, y[2 * h + 1].x, ey, ey, s);
 #pragma unroll
     for (int k = 0; k < NS; ++k) B[k][2 * h] = s[k];
-    fx_digits<NS>(y[2 * h].y, y[2 * h + 1].y, ey, ey, s);
+    tb[h] = fx_lead(s[0], s[1]);
+    fx_digits(y[2 * h].y, y[2 * h + 1].y, ey, ey, s);
 #pragma unroll
     for (int k = 0; k < NS; ++k) B[k][2 * h + 1] = s[k];
+    tb[h] = fx_add_half2(tb[h], fx_lead(s[0], s[1]));
   }
-  float cr[ND][4], ci[ND][4];
+  float cr[NS][4], ci[NS][4], ct[4];
 #pragma unroll
   for (int i = 0; i < NS; ++i)
 #pragma unroll
-    for (int j = 0; j < NS && j + i < ND; ++j) {
-      const bool first = i == 0 || (i == 1 && j == NS - 1);   // the first product of weight i + j
-      fx_mma16(cr[i + j], A[i], B[j][0], B[j][2], first);
-      fx_mma16(ci[i + j], A[i], B[j][1], B[j][3], first);
+    for (int j = 0; j + i < NS; ++j) {
+      fx_mma16(cr[i + j], A[i], B[j][0], B[j][2], i == 0);   // the first product of weight i + j
+      fx_mma16(ci[i + j], A[i], B[j][1], B[j][3], i == 0);
     }
-  const unsigned e2[2] = {__shfl_sync(0xffffffffu, ey, 8 * q), __shfl_sync(0xffffffffu, ey, 8 * q + 4)};
+  fx_mma16(ct, ta, tb[0], tb[1], true);
 #pragma unroll
   for (int i = 0; i < 2; ++i) {
-    const long long re = fx_join_wide<ND, 1>(cr, i) + fx_join_wide<ND, 1>(ci, 2 + i);
-    const long long im = fx_join_wide<ND, 1>(ci, i) - fx_join_wide<ND, 1>(cr, 2 + i);
-    const unsigned es = fx_exp(ex, e2[i], 43);
-    T.red[warp & 3][64 * which + g + 8 * (2 * q + i)] = mkc(fx_double(re, es), fx_double(im, es));
+    const unsigned es = fx_exp(ex, __shfl_sync(0xffffffffu, ey, 8 * q + 4 * i), 44);
+    const unsigned wy = __shfl_sync(0xffffffffu, my, 8 * q + 4 * i);
+    cplx v = mkc(fx_double(fx_join_wide(cr, i, 1.f) + fx_join_wide(ci, 2 + i, 1.f), es),
+                 fx_double(fx_join_wide(ci, i, 1.f) - fx_join_wide(cr, 2 + i, 1.f), es));
+    if (mx && wy && ct[i] + ct[2 + i] < FX_LOW) {
+      v = mkc(0.0, 0.0);
+      for (int r = 0; r < 16; ++r) cfma_conj(v, T.phs[g][r0 + r], Y[2 * q + i][r0 + r]);
+    }
+    T.red[warp & 3][64 * which + g + 8 * (2 * q + i)] = v;
   }
-  const bool slow = __syncthreads_or(!fx_ok(mx) || !fx_ok(my));
+  const bool slow = __syncthreads_or(mx >= (FX_EMAX + 1u) << 20 || my >= (FX_EMAX + 1u) << 20);
   if (tid >= 128) return;
   cplx v = mkc(0.0, 0.0);
   if (slow) {
@@ -368,92 +443,44 @@ __device__ __forceinline__ cplx stage_sum(const SpfStage& g, long long e) {
 
 // Solve from T.so and subtract the CTA's rows of phi X; with g.on also the next stage's
 // input (the CTA's rows of phi are in shared memory by now, so it may replace them).  A
-// warp has 16 rows and four columns of phi X, one set of digit products (in FP64 the 8 n
-// instructions a row and column pair took 4.7 us at n = 8).
+// thread has row threadIdx.x % 64 of columns threadIdx.x / 64 and + 4.  In FP64: eight
+// instructions a row and column pair of warps.  Digit products were 2.4 us faster at n = 8
+// and 400 points, but cut the rows of phi and X by their largest elements.
 __device__ __forceinline__ bool solve_project(SpfSmall& T, const SpfDesc& d, int row0, cplx* o, const SpfStage& g) {
-  constexpr int NS = SPF_NS;
-  const int n = d.n, G = d.G, lane = threadIdx.x & 31, warp = threadIdx.x >> 5, gl = lane >> 2, q = lane & 3;
-  const int lr = 16 * (warp & 3) + gl, j0 = 4 * (warp >> 2), j = j0 + q;   // elements (lr, j), (lr + 8, j)
+  const int n = d.n, G = d.G, row = threadIdx.x & (SPF_ROWS - 1), jr = threadIdx.x / SPF_ROWS;
+  const bool in = row0 + row < G;
   cplx ss[2], bs[2];
   double dt = 0.0;
   if (g.on) {
     dt = g.dt_mode[g.elem_mode[d.out_offset - g.off]];
 #pragma unroll
-    for (int f = 0; f < 2; ++f) {
-      ss[f] = bs[f] = mkc(0.0, 0.0);
-      if (row0 + lr + 8 * f < G && j < n) {
-        const long long e = d.out_offset + row0 + lr + 8 * f + (long long)G * j;
-        ss[f] = stage_sum(g, e);
-        bs[f] = g.base[e];
+    for (int i = 0; i < 2; ++i) {
+      ss[i] = bs[i] = mkc(0.0, 0.0);
+      if (in && jr + 4 * i < n) {
+        const long long e = d.out_offset + row0 + row + (long long)G * (jr + 4 * i);
+        ss[i] = stage_sum(g, e);
+        bs[i] = g.base[e];
       }
     }
-  }
-  // the rows of phi, cut ahead of the solve
-  unsigned A[NS][4], er[2];
-  bool bad = false;
-#pragma unroll
-  for (int f = 0; f < 2; ++f) {
-    const cplx x0 = T.phs[q][lr + 8 * f], x1 = T.phs[q + 4][lr + 8 * f];
-    const cplx y0 = q < n ? x0 : mkc(0.0, 0.0), y1 = q + 4 < n ? x1 : mkc(0.0, 0.0);
-    unsigned mag = row0 + lr + 8 * f < G ? max(fx_mag(y0), fx_mag(y1)) : 0u;
-    mag = max(mag, __shfl_xor_sync(0xffffffffu, mag, 1));
-    mag = max(mag, __shfl_xor_sync(0xffffffffu, mag, 2));
-    bad = bad || !fx_ok(mag);
-    er[f] = fx_ebits(mag);
-    unsigned s[NS];
-    fx_digits<NS>(y0.x, y0.y, er[f], er[f], s);
-#pragma unroll
-    for (int i = 0; i < NS; ++i) A[i][f] = s[i];
-    fx_digits<NS>(y1.x, y1.y, er[f], er[f], s);
-#pragma unroll
-    for (int i = 0; i < NS; ++i) A[i][2 + f] = s[i];
   }
   const bool ok = solve_elimination<1>(
       n, [&](int i, int c) { return c < n ? T.so[i + 8 * c] : T.so[64 + i + 8 * (c - n)]; }, T.colb, T.rowb, T.Xt);
   __syncthreads();
-  if (j0 >= n) return ok;   // whole warps
-  cplx v[2];
-  const int jo = j0 + (gl >> 1);
-  const cplx m0 = jo < n && q < n ? T.Xt[jo + n * q] : mkc(0.0, 0.0);
-  const cplx m1 = jo < n && q + 4 < n ? T.Xt[jo + n * (q + 4)] : mkc(0.0, 0.0);
-  unsigned mag = max(fx_mag(m0), fx_mag(m1));
-  mag = max(mag, __shfl_xor_sync(0xffffffffu, mag, 1));
-  mag = max(mag, __shfl_xor_sync(0xffffffffu, mag, 2));
-  if (__any_sync(0xffffffffu, bad || !fx_ok(mag))) {
 #pragma unroll
-    for (int f = 0; f < 2; ++f) {
-      v[f] = mkc(0.0, 0.0);
-      if (j < n)
-        for (int k = 0; k < n; ++k) cfma(v[f], T.phs[k][lr + 8 * f], T.Xt[j + n * k]);
+  for (int i = 0; i < 2; ++i) {
+    const int j = jr + 4 * i;
+    if (!in || j >= n) break;
+    cplx v = T.dph[j][row];
+    for (int k = 0; k < n; ++k) {
+      const cplx x = T.phs[k][row], c = T.Xt[j + n * k];
+      v.x = fma(-x.x, c.x, fma(x.y, c.y, v.x));
+      v.y = fma(-x.x, c.y, fma(-x.y, c.x, v.y));
     }
-  } else {
-    const unsigned ec = fx_ebits(mag);
-    const unsigned es = fx_exp(__shfl_sync(0xffffffffu, ec, 8 * q), 0u, 44);
-    unsigned s0[NS], s1[NS];
-    fx_digits<NS>(m0.x, m0.y, ec, ec, s0);
-    fx_digits<NS>(m1.x, m1.y, ec, ec, s1);
-    float c[NS][4];
-#pragma unroll
-    for (int i = 0; i < NS; ++i) {   // column re: (Mr, -Mi); column im: (Mi, Mr)
-      const unsigned w0 = (gl & 1) ? __byte_perm(s0[i], s0[i], 0x1032) : s0[i] ^ 0x80000000u;
-      const unsigned w1 = (gl & 1) ? __byte_perm(s1[i], s1[i], 0x1032) : s1[i] ^ 0x80000000u;
-#pragma unroll
-      for (int k = 0; k + i < NS; ++k) fx_mma16(c[i + k], A[k], w0, w1, i == 0);
-    }
-#pragma unroll
-    for (int f = 0; f < 2; ++f)
-      v[f] = mkc(fx_double(fx_join<NS>(c, 2 * f), es + er[f]), fx_double(fx_join<NS>(c, 2 * f + 1), es + er[f]));
-  }
-#pragma unroll
-  for (int f = 0; f < 2; ++f) {
-    const int row = lr + 8 * f;
-    if (row0 + row >= G || j >= n) continue;
-    const cplx w = csub(T.dph[j][row], v[f]);
     const long long e = row0 + row + (long long)G * j;
-    o[e] = w;
+    o[e] = v;
     if (g.on) {
-      const cplx s = mkc(fma(g.last, w.x, ss[f].x), fma(g.last, w.y, ss[f].y));
-      g.out[d.out_offset + e] = mkc(fma(dt, s.x, bs[f].x), fma(dt, s.y, bs[f].y));
+      const cplx s = mkc(fma(g.last, v.x, ss[i].x), fma(g.last, v.y, ss[i].y));
+      g.out[d.out_offset + e] = mkc(fma(dt, s.x, bs[i].x), fma(dt, s.y, bs[i].y));
     }
   }
   return ok;

@@ -226,7 +226,8 @@ __global__ void __launch_bounds__(TC_ROWS) prod_tc_kernel(const ProdDesc* __rest
 }
 
 // ---------------------------------------------------------------------------
-// Mode products of FP64 accuracy as exact digit products (fixed.cuh) with tcgen05.  A
+// Mode products of FP64 accuracy as digit products (fixed.cuh) with tcgen05 (factors of
+// one, nothing accumulated: ProdBatch::plain).  A
 // tile is 128 fibres, one per thread and MMA row; the thread cuts its fibre into eight
 // FP16 digits of one exponent, digit i of all fibres being operand A_i (128 x 2 nin).
 // The matrix's digits lie side by side as columns, B = [B_0 B_1 .. B_7] (WC columns
@@ -246,6 +247,42 @@ struct DigitTile {
   static constexpr uint32_t COLS = 8 * WC;       // TMEM columns
   static constexpr uint32_t SMEM = 8 * A + B;
 };
+// The outputs of a fibre whose T = sum |x||m| does not show the digits to be accurate, from
+// the leading ones in shared memory: a row of A_0, A_1 and the re columns of B_0, B_1.
+template <int NG>
+static __device__ __noinline__ unsigned digits_low(const unsigned char* a, const unsigned char* b, int nout) {
+  using T = DigitTile<NG>;
+  float x[4 * NG], any = 0.f;
+#pragma unroll
+  for (int k = 0; k < NG; ++k) {
+    const uint4 u = *reinterpret_cast<const uint4*>(a + k * 128), v = *reinterpret_cast<const uint4*>(a + T::A + k * 128);
+    x[4 * k] = fx_lead_sum(u.x, v.x);
+    x[4 * k + 1] = fx_lead_sum(u.y, v.y);
+    x[4 * k + 2] = fx_lead_sum(u.z, v.z);
+    x[4 * k + 3] = fx_lead_sum(u.w, v.w);
+    any += x[4 * k] + x[4 * k + 1] + x[4 * k + 2] + x[4 * k + 3];
+  }
+  if (any == 0.f) return 0u;   // a fibre of zeros
+  unsigned low = 0u;
+#pragma unroll 1
+  for (int o = 0; o < nout; ++o) {
+    const int n0 = 2 * o, n1 = T::WC + 2 * o;
+    const unsigned char* b0 = b + (n0 >> 3) * T::SBO + (n0 & 7) * 16;
+    const unsigned char* b1 = b + (n1 >> 3) * T::SBO + (n1 & 7) * 16;
+    float t = 0.f;
+#pragma unroll
+    for (int k = 0; k < NG; ++k) {
+      const uint4 u = *reinterpret_cast<const uint4*>(b0 + k * 128), v = *reinterpret_cast<const uint4*>(b1 + k * 128);
+      t = fmaf(x[4 * k], fx_lead_sum(u.x, v.x), t);
+      t = fmaf(x[4 * k + 1], fx_lead_sum(u.y, v.y), t);
+      t = fmaf(x[4 * k + 2], fx_lead_sum(u.z, v.z), t);
+      t = fmaf(x[4 * k + 3], fx_lead_sum(u.w, v.w), t);
+    }
+    if (t < FX_LOW) low |= 1u << o;
+  }
+  return low;
+}
+
 template <int NG>
 __global__ void __launch_bounds__(128, NG <= 2 ? 4 : 2)
     prod_digits_kernel(const ProdDesc* __restrict__ descs, int ndesc, long long ntiles, int* status) {
@@ -253,7 +290,8 @@ __global__ void __launch_bounds__(128, NG <= 2 ? 4 : 2)
   extern __shared__ __align__(128) unsigned char tc_smem[];   // A_0 .. A_7, B
   __shared__ __align__(8) uint64_t bar;
   __shared__ uint32_t s_tmem;
-  __shared__ unsigned rowexp[4 * NG];
+  __shared__ unsigned rowexp[4 * NG], colmag[4 * NG];
+  __shared__ __align__(16) unsigned scale[4 * NG];
   __shared__ int s_bad;
   const int tid = threadIdx.x, warp = tid >> 5;
   long long t0 = ntiles * blockIdx.x / gridDim.x;
@@ -272,7 +310,8 @@ __global__ void __launch_bounds__(128, NG <= 2 ? 4 : 2)
   int di = t0 < tend ? warp_find_desc(descs, ndesc, t0) : 0;
   for (; ok && t0 < tend; ++di) {
     const ProdDesc& d = descs[di];
-    const int nin = d.nin, nout = d.nout;
+    const int nin = d.nin, nout = d.nout, sh = fx_headroom(nin);
+    const float pw = fx_pow2(sh);
     const unsigned L = (unsigned)d.L, nfib = (unsigned)(d.L * d.R);
     const long long dend = min(tend, d.block_start + (long long)((nfib + 127) / 128));
     const long long Lx = d.L * (nin - 1), Ly = d.L * (nout - 1);
@@ -289,25 +328,43 @@ __global__ void __launch_bounds__(128, NG <= 2 ? 4 : 2)
       }
     };
     fetch();
-    // the matrix: a row's exponent, then its digits
+    // the matrix and the sample of the scaling are on their way together; then a row's
+    // exponent, its digits
+    constexpr int PM = (T::WC / 2 * (T::K / 2) + 127) / 128;
+    cplx mv[PM];
+#pragma unroll
+    for (int i = 0; i < PM; ++i) {
+      const int e = tid + 128 * i, jo = e / (T::K / 2), ji = e % (T::K / 2);
+      mv[i] = mkc(0.0, 0.0);
+      if (jo < nout && ji < nin) mv[i] = d.conjT ? cconj(d.M[ji + (long long)d.ldm * jo]) : d.M[jo + (long long)d.ldm * ji];
+    }
     __syncthreads();   // B of the descriptor before is read (its MMAs are complete)
     if (tid < 4 * NG) rowexp[tid] = 0u;
     if (tid == 0) s_bad = 0;
+    fx_column_sizes(d, colmag);
     __syncthreads();
-    for (int e = tid; e < T::WC / 2 * 4 * NG; e += 128) {
-      const int jo = e / (4 * NG), ji = e % (4 * NG);
-      if (jo < nout && ji < nin)
-        atomicMax(&rowexp[jo], fx_mag(d.conjT ? d.M[ji + (long long)d.ldm * jo] : d.M[jo + (long long)d.ldm * ji]));
+    bool scaled;
+    {   // every warp for itself: the same values
+      const unsigned b = fx_column_scale(colmag, nin);
+      if ((tid & 31) < 4 * NG) scale[tid & 31] = b;
+      scaled = __any_sync(0xffffffffu, b);
+    }
+    __syncwarp();
+#pragma unroll
+    for (int i = 0; i < PM; ++i) {
+      const int e = tid + 128 * i, jo = e / (T::K / 2), ji = e % (T::K / 2);
+      if (jo < nout && ji < nin) atomicMax(&rowexp[jo], fx_scaled_down(fx_mag(mv[i]), scale[ji]));
     }
     __syncthreads();
     if (tid < nout && !fx_ok(rowexp[tid])) s_bad = 1;
-    for (int e = tid; e < T::WC / 2 * (T::K / 2); e += 128) {
-      const int jo = e / (T::K / 2), ji = e % (T::K / 2);
-      cplx m = mkc(0.0, 0.0);
-      if (jo < nout && ji < nin) m = d.conjT ? cconj(d.M[ji + (long long)d.ldm * jo]) : d.M[jo + (long long)d.ldm * ji];
-      const unsigned eb = jo < nout ? fx_ebits(rowexp[jo]) : fx_ebits(0u);
+#pragma unroll
+    for (int q = 0; q < PM; ++q) {
+      const int e = tid + 128 * q, jo = e / (T::K / 2), ji = e % (T::K / 2);
+      if (e >= T::WC / 2 * (T::K / 2)) break;
+      const cplx m = mv[q];
+      const unsigned eb = (jo < nout ? fx_ebits(rowexp[jo]) : fx_ebits(0u)) + (ji < nin ? scale[ji] : 0u);
       unsigned s[8];
-      fx_digits<8>(m.x, m.y, eb, eb, s);
+      fx_digits(m.x, m.y, eb, eb, s);
       unsigned char* b = tc_smem + 8 * T::A + (ji >> 2) * 128 + (ji & 3) * 4;
 #pragma unroll
       for (int i = 0; i < 8; ++i) {   // columns re: (Mr, -Mi), im: (Mi, Mr)
@@ -316,19 +373,28 @@ __global__ void __launch_bounds__(128, NG <= 2 ? 4 : 2)
         *reinterpret_cast<unsigned*>(b + (n >> 3) * T::SBO + ((n & 7) + 1) * 16) = __byte_perm(s[i], s[i], 0x1032);
       }
     }
-    const bool plain = !d.accumulate && d.alpha.x == 1.0 && d.alpha.y == 0.0;
     for (; t0 < dend; ++t0) {
+      if (scaled) {
+#pragma unroll
+        for (int k = 0; k < NG; ++k) {
+          const uint4 b = reinterpret_cast<const uint4*>(scale)[k];
+          x[4 * k] = fx_scale_up(x[4 * k], b.x);
+          x[4 * k + 1] = fx_scale_up(x[4 * k + 1], b.y);
+          x[4 * k + 2] = fx_scale_up(x[4 * k + 2], b.z);
+          x[4 * k + 3] = fx_scale_up(x[4 * k + 3], b.w);
+        }
+      }
       unsigned mag = 0u;
 #pragma unroll
       for (int j = 0; j < 4 * NG; ++j) mag = max(mag, fx_mag(x[j]));
       const unsigned eb = fx_ebits(mag);
-      const unsigned ef = fx_exp(eb, 0u, 44);
+      const unsigned ef = fx_exp(eb, 0u, 44 + sh);
       bool bad = !fx_ok(mag);
 #pragma unroll
       for (int k = 0; k < NG; ++k) {
         unsigned s[4][8];
 #pragma unroll
-        for (int j = 0; j < 4; ++j) fx_digits<8>(x[4 * k + j].x, x[4 * k + j].y, eb, eb, s[j]);
+        for (int j = 0; j < 4; ++j) fx_digits(x[4 * k + j].x, x[4 * k + j].y, eb, eb, s[j]);
         unsigned char* a = tc_smem + (tid >> 3) * T::SBO + k * 128 + (tid & 7) * 16;
 #pragma unroll
         for (int i = 0; i < 8; ++i)
@@ -361,6 +427,7 @@ __global__ void __launch_bounds__(128, NG <= 2 ? 4 : 2)
       parity ^= 1;
       tc_fence_after();
       const bool act = pc < nfib;
+      unsigned least = 0xffffffffu;   // below 2 fx_small_limit: an output may be too small for its digits
       cplx* y = d.Y + ((long long)pc + Ly * rc);
 #pragma unroll
       for (int h = 0; h < NG; ++h) {
@@ -371,16 +438,18 @@ __global__ void __launch_bounds__(128, NG <= 2 ? 4 : 2)
         for (int o = 0; o < 4; ++o) {
           if (4 * h + o < nout) {
             const unsigned es = fx_ebits(rowexp[4 * h + o]) + ef;
-            cplx v = mkc(fx_double(fx_join<8>(c, 2 * o), es), fx_double(fx_join<8>(c, 2 * o + 1), es));
-            if (!plain) {
-              v = cmul(d.alpha, v);
-              if (d.accumulate && act) v = cadd(v, y[(long long)L * (4 * h + o)]);
-            }
-            if (act && !bad) y[(long long)L * (4 * h + o)] = v;
+            const long long re = fx_join(c, 2 * o, pw), im = fx_join(c, 2 * o + 1, pw);
+            least = min(least, fx_small_word(re, im, fx_small_limit(sh)));
+            if (act && !bad) y[(long long)L * (4 * h + o)] = mkc(fx_double(re, es), fx_double(im, es));
           }
         }
       }
-      if (act && bad) prod_fibre_fp64(d, pc - L * rc, rc);
+      if (act && bad) {
+        prod_fibre_fp64(d, pc - L * rc, rc);
+      } else if (act && least < 2 * fx_small_limit(sh)) {
+        const unsigned low = digits_low<NG>(tc_smem + (tid >> 3) * T::SBO + (tid & 7) * 16, tc_smem + 8 * T::A, nout);
+        if (low) prod_outputs_fp64(d, pc, low, 0, 1);
+      }
     }
     t0 = dend;
   }
