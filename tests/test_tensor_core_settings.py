@@ -1,12 +1,13 @@
 """The tensor-core settings choose the kernels of the calls made after them, also where
 an EOM evaluation is replayed from a graph; MACAW_GB300_TC=0 keeps every tcgen05 kernel
-out.  On the stand-in runtime, by the names of the launched kernels."""
+out; FP64-accurate mode products of two tiles per CTA and more take its digit kernel.  On the stand-in runtime, by the names of the launched kernels."""
 import pytest
 
 from macaw_gb300 import capi
-from macaw_gb300.generate import qvc
+from macaw_gb300.generate import gmctdh16, qvc
 from tests import fake
 from tests.helpers import random_state
+from tests.test_gpu_large_batches import SIZES, _model as large
 
 
 def _model(modes):
@@ -38,3 +39,25 @@ def test_switch_covers_the_digit_products(tmp_path, monkeypatch, value, modes, d
     core.calc_derivs(A, psi)
     assert any("prod_digits_kernel" in k for k in rt.kernels()) == digits
     assert capi.tensor_core_status()["enabled"] == int(value)
+
+
+# the sizes of test_gpu_large_batches, whose first products fill two tiles per CTA
+@pytest.mark.parametrize("sizes, form", list(zip(SIZES, "2234")))
+def test_large_batches_take_the_digit_kernel(tmp_path, monkeypatch, sizes, form):
+    rt = fake.use(monkeypatch, fake.fake_runtime(tmp_path))
+    model = large(sizes)
+    core = capi.GpuCore(model)
+    core.calc_derivs(*random_state(model))
+    products = [k for k in rt.kernels() if "prod_" in k]
+    assert f"prod_digits_kernelILi{form}E" in products[0]
+
+
+# 65,536 fibres of a Gaussian mode for each of two states: S^-1 A, then dA -= tau A
+def test_accumulating_batches_do_not(tmp_path, monkeypatch):
+    rt = fake.use(monkeypatch, fake.fake_runtime(tmp_path))
+    model = gmctdh16(ngwp=16, gwp_dofs=2, dvr_grid=18, dvr_nspf=16)
+    core = capi.GpuCore(model)
+    core.calc_derivs(*random_state(model))
+    products = [k for k in rt.kernels() if "prod_" in k]
+    assert all("prod_digits_kernelILi4E" in k for k in products[:-1])
+    assert "prod_fx_kernelILi4E" in products[-1]
