@@ -46,12 +46,11 @@ MFX_EPOCHS = 12
 MFX_GATE = 0.5
 # ncu DRAM bytes per algorithmic byte of a kernel class in the benchmark regime
 # (one capture of the profile case), and what bounds each class there
-# DRAM bytes per algorithmic byte of the mode products: 177.5 MB of DRAM traffic
-# over 461 MB of operand bytes in the eight mode-product launches of one ncu
-# capture of the profile case at precision 5 (`--profile-case --precision 5
-# --profile-from-fs 1`: five compensated mean-field chain launches, three FP32
-# H_B*B launches)
-TRAFFIC_PER_ALG_BYTE = {"mode_product": 0.385}
+# DRAM bytes per algorithmic byte of the mode products: 3.40 GB of DRAM traffic over
+# 8.20 GB of operand bytes in the 192 mode-product launches (48 of digit products, 144
+# FP32 ones of H_B*B) of one ncu capture of the profile case at precision 5
+# (`--profile-case --precision 5 --profile-from-fs 1`, three CMF2 steps)
+TRAFFIC_PER_ALG_BYTE = {"mode_product": 0.414}
 ROOF_BOUND = {"mode_product": "hbm", "hole_contract": "hbm", "spf_derivative": "hbm"}
 ROOF_NOTE = {"mode_product": "not HBM: the mean-field products of FP64 accuracy are bound by instruction issue "
                              "(cutting and joining digits), the FP32 H_B products by load latency; operands "

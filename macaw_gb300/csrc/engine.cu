@@ -159,7 +159,8 @@ struct ProdBatch {
 inline int hole_nblk(const HoleDesc& d, int tpb, int cap) {
   const long long ntiles = (d.L * d.R + HOLE_TILE - 1) / HOLE_TILE;
   // the wide form's blocks (two per SM) cost more to start: 283 blocks took 20.5 us
-  // where 478 took 25.8 (mixed counts of 5 to 9, 56,007 coefficients)
+  // where 478 took 25.8 (mixed counts of 5 to 9, 56,007 coefficients; measured before
+  // it kept windows)
   const long long work = std::max(d.n1, d.n2) <= 8 ? ntiles : ntiles * ((d.n1 + 15) / 16) * ((d.n2 + 15) / 16);
   return (int)std::min({std::max(work / tpb, 1LL), ntiles, (long long)std::min(cap, HOLE_NBLK_MAX)});
 }
@@ -1346,7 +1347,7 @@ void plan_eom(Ctx& c) {
   // Modes on which the pair's terms carry the same matrix (SPF overlaps, mostly) go to
   // the two ends, so that the terms share the chains' beginnings; products with the same
   // input and matrix are computed once (8-SPF QVC model, eight general
-  // terms: 68 -> 57 products, 260 -> 226 us).
+  // terms: 68 -> 57 products, which took 260 and 226 us).
   // The order changes only the rounding; FP32 products, whose rounding shows, pairs
   // with one term, and pairs whose tensors would grow by it (states of different SPF
   // counts) keep the reference order.
@@ -2970,7 +2971,9 @@ void lan_check(Ctx& c, LanRun& R) {
 }
 
 // Eigenpairs of the real symmetric tridiagonal matrix (d, e): implicit QL with
-// Wilkinson's shift, rotations accumulated into z (n x n, column r the vector of d[r]).
+// Wilkinson's shift, rotations accumulated into z (n x n, column r the vector of d[r]): the
+// implicit QL algorithm of Martin and Wilkinson (Numerische Mathematik 12, 1968; EISPACK's
+// imtql2, also its way on where a rotation underflows).
 // On the host: at n <= 20 it takes a few microseconds where one warp of the GPU, whose
 // FP64 chains are serial, took 143 (n = 7).
 void tridiag_eig(int n, double* d, double* e, double* z) {
@@ -4244,7 +4247,7 @@ void download(Ctx& c, const cplx* src, double* A, double* psi) {
 // Calc_Derivs on host arrays with the coefficients copied in while the operators act on
 // the SPFs, which do not need them.  The results leave once the status is known: a call
 // that fails leaves the caller's arrays alone.  From OVERLAP_MIN coefficients (0.5 MB,
-// about 10 us); not for packets, whose host arrays are gathered by state.
+// whose copy takes about 10 us); not for packets, whose host arrays are gathered by state.
 #define OVERLAP_MIN 32768
 bool overlapped_copies(const Ctx& c) {
   return c.naconftot >= OVERLAP_MIN && c.npk == 1 && !c.pk_on && !c.pk_mult && c.modes_gwp.empty() && !c.profiling &&

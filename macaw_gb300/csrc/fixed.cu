@@ -1,6 +1,6 @@
-// Mode products and single-hole contractions of FP64 accuracy as exact digit
-// products on the tensor cores (fixed.cuh) for sm_103a: precision 0, and the
-// FP64-accurate products and contractions of the mixed modes.
+// Mode products and single-hole contractions of FP64 accuracy as digit products on the
+// tensor cores (fixed.cuh) for sm_103a: precision 0, and the FP64-accurate products and
+// contractions of the mixed modes.
 #include <algorithm>
 
 #include "kernels.cuh"
@@ -257,8 +257,9 @@ static void prod_fx_go(const ProdDesc* d, int nd, long long nblocks, int persist
 // The tcgen05 form (tc.cu) takes batches of 5 to 16 SPFs that give every one of its CTAs
 // (four per SM up to 8 SPFs, two above) at least two tiles of 128 fibres, so that the
 // matrix digits and the pipeline's start are paid for: 57 products of 32,768 fibres of 8
-// took 191 us against 226, of 248,832 fibres of 12 2,206 against 2,900; a batch of 700
-// tiles of 5 to 9 took 19 against 17.
+// take 229 us against 271, of 248,832 fibres of 12 2,560 against 3,230; just above the
+// line, with 6 to 8 SPFs, 22 against 27.  Below it a batch of 700 tiles of 5 to 9 took
+// 19 against 17 (measured before either kernel formed T).
 void launch_prod_fx(const ProdDesc* d, int nd, long long nblocks, int maxn, bool plain, int* status, cudaStream_t st,
                     int persist) {
   if (plain && persist <= 0 && tc_enabled() && maxn > 4 && maxn <= 16 && nblocks >= (maxn <= 8 ? 8 : 4) * (long long)sm_count()) {
@@ -281,12 +282,14 @@ void launch_prod_fx(const ProdDesc* d, int nd, long long nblocks, int maxn, bool
 // X columns, its columns the re, then the im of eight Y columns, its inner dimension the
 // fibres; lanes load what they hold, nothing is staged.  A column has one exponent per
 // window of at most HOLE_FLUSH groups, from the window's first group; elements above it
-// end the window.  A window's sums go to FP64, exactly but for the dropped digits.  One more MMA sums |x||y| of the leading
-// digits: pairs where that is below 2^-6 .. 2^-8 of the product of the columns' largest
-// elements (columns graded in opposite directions) are summed again in FP64.  On states of the models here
-// that is none to one window in a hundred, and the windows of 128 neighbouring fibres are
-// what keeps it so (interleaved over the warps, one in ten).  The last block of a
-// descriptor to finish adds the blocks' partials in block order into the first.
+// end the window.  A window's sums go to FP64, exactly but for the dropped digits.  One more
+// MMA sums |x||y| of the leading digits: pairs where that is below 2^-6 .. 2^-8 of the
+// product of the columns' largest elements (columns graded in opposite directions) are
+// summed again in FP64.  On states of the models here that is none to one window in a
+// hundred, and the windows of 128 neighbouring fibres are what keeps it so (interleaved
+// over the warps, one in ten).  The last block of a descriptor to finish adds the blocks'
+// partials in block order into the first.  42 contractions of 32,768 fibres of 8: 148 us,
+// of which 14 are for windows and |x||y|; bound by cutting operands (ALU).
 // ---------------------------------------------------------------------------
 #define HOLE_FLUSH 8     // groups of 16 fibres between flushes: 128 x 8 x 2^14 = 2^24
 #define HOLE_WARPS 4     // per block; twice as many where n1 or n2 is above eight
@@ -616,6 +619,8 @@ __device__ __forceinline__ void hole_fx_block(const HoleDesc& d, int b, const cp
 // read it (an uint4 per lane, digit and group of 16 fibres: re, im of fibres 2 q, 2 q + 1,
 // then of 2 q + 8, 2 q + 9), and every warp takes a pair block of the tile.  Where every
 // pair block cut its own operands, cutting bound the kernel (ALU 52 %, tensor pipe 36 %).
+// 42 contractions of 12 SPFs (8,957,952 coefficients): 3,040 us, of which 760 are for the
+// exponents of windows and the sums |x||y|.
 // A column block of at most four columns puts re and im side by side into one MMA.
 // Warps 0-3 cut the next stage while warps 4-7 multiply this one: with every warp doing
 // both in turn the phases of a block did not overlap.

@@ -1,4 +1,4 @@
-// Exact digit arithmetic for the FP64 contractions on the tensor cores (sm_103a).
+// Digit arithmetic for the FP64 contractions on the tensor cores (sm_103a).
 //
 // GB300 issues one warp-wide FP64 instruction per SM sub-partition every 62-64
 // cycles (measured 1.83 DFMA per SM and cycle, 0.53 TFMA/s on 152 SMs); its FP16
@@ -250,8 +250,8 @@ static __device__ __noinline__ void prod_outputs_fp64(const ProdDesc& d, unsigne
 // over FX_SAMPLE fibres spread over the tensor, the same for every CTA and kernel: any
 // powers of two are right, and fibres that these do not suit show in the sums (from the
 // largest elements, which one fibre decides, ten times as many).  Empty columns count
-// as the weakest; columns within 2^FX_SCALE_MIN of each other are left alone, which
-// saves a tenth of the products' instructions.  In exponent words; lane j returns b(j).
+// as the weakest; columns within 2^FX_SCALE_MIN of each other are left alone,
+// as a sample's mean is no better than that.  In exponent words; lane j returns b(j).
 #define FX_SCALE_MAX 60
 #define FX_SCALE_MIN 1
 #define FX_SAMPLE 32

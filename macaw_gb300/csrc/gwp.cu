@@ -404,7 +404,7 @@ __device__ cplx warp_sum(cplx v) {
 }
 
 // LU factorisation of the bordered system in panels of LU_PW columns, two launches per
-// panel (384 unknowns, two systems: 48 panels of 17.5 and updates of 8.9 us,
+// panel (384 unknowns, two systems: 48 panels of 17.5 and updates of 9.0 us,
 // where a Householder QR of [C; eps I] took 48 launches of 127).
 //
 // Panel: one block per system, a row of the panel per thread in registers.  Rows stay
@@ -486,7 +486,7 @@ __global__ void __launch_bounds__(LU_MAXROWS) lu_panel_kernel(const GwpCYDesc* _
 // Trailing update: a block takes 32 of the remaining rows and 32 of the remaining
 // columns (the right-hand side is the last).  It solves the panel's unit lower triangle
 // for its columns (the blocks of the first row of blocks store the result as U), then
-// subtracts the rank-8 product as exact digit products (fixed.cuh; a warp's 16 rows are
+// subtracts the rank-8 product as digit products (fixed.cuh; a warp's 16 rows are
 // the MMA's rows, the (re, im) of four columns its columns, as in the mode products),
 // where FP64 would take 18 us of an SM's FP64 pipe per block; elements small against the
 // factors (a panel whose rows and columns are graded) are done in FP64.

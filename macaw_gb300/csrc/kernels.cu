@@ -1,10 +1,11 @@
 // FP64 kernels of the G-MCTDH equation-of-motion path for sm_103a.
 //
-// On GB300 FP64 runs on the CUDA cores at a small fraction of the FP32 rate, so
-// these kernels are written to spend FP64 FMAs only on the algebra the EOM needs:
-// each fibre of a tensor is read once into registers (mode products), fibre tiles
-// are staged in shared memory for the single-hole contractions, and reductions
-// are two-stage with a fixed summation order so reruns are bitwise identical.
+// The FP32 forms of the mode products and single-hole contractions (precision 1) and
+// what the FP64-accurate ones (fixed.cu, tc.cu) are launched by; one-mode operators, sums
+// of terms, regularised inverses, integrator stages.  FP64 is the scarce unit of this
+// chip, so these kernels spend it only on the algebra the EOM needs, each fibre of a
+// tensor is read once, and reductions are two-stage with a fixed summation order, so
+// that reruns are bitwise identical.
 #include <algorithm>
 #include <atomic>
 

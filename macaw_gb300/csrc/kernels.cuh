@@ -287,7 +287,7 @@ int launch_spf(const SpfDesc* d_descs, int ndesc, long long ntiles, int maxn, co
 // diff = y5 - y4
 void launch_rk_end(cplx* y5, cplx* diff, const cplx* base, const StageArgs& a, const double* c4, const double* dt_mode,
                    const unsigned char* elem_mode, long long off, long long n, cudaStream_t st);
-// FP64 accuracy as exact digit products on the tensor cores (fixed.cu); launched by
+// FP64 accuracy as digit products on the tensor cores (fixed.cu); launched by
 // launch_prod / launch_hole
 void launch_prod_fx(const ProdDesc* d_descs, int ndesc, long long nblocks, int maxn, bool plain, int* status,
                     cudaStream_t st, int persist);

@@ -1,4 +1,4 @@
-// SPF derivatives of the grid modes (derivatives.f90:94-153) for sm_103a: exact digit
+// SPF derivatives of the grid modes (derivatives.f90:94-153) for sm_103a: digit
 // products on the tensor cores (fixed.cuh) for the operator sum and the contractions,
 // FP64 for the small solve:
 //  (1) dphi = f sum_k ophi_k rhom1MF_k^T, 64 grid rows per CTA;

@@ -227,17 +227,18 @@ __global__ void __launch_bounds__(TC_ROWS) prod_tc_kernel(const ProdDesc* __rest
 
 // ---------------------------------------------------------------------------
 // Mode products of FP64 accuracy as digit products (fixed.cuh) with tcgen05 (factors of
-// one, nothing accumulated: ProdBatch::plain).  A
-// tile is 128 fibres, one per thread and MMA row; the thread cuts its fibre into eight
-// FP16 digits of one exponent, digit i of all fibres being operand A_i (128 x 2 nin).
-// The matrix's digits lie side by side as columns, B = [B_0 B_1 .. B_7] (WC columns
-// each: the (re, im) of the outputs), and D = [D_0 .. D_7] holds the sums of equal weight
-// in TMEM: A_i times the first 8 - i blocks adds into D_i .. D_7, so a K step of a tile
-// takes eight MMAs of N = WC (8 - i).  A thread reads its fibre's sums back, joins and
-// rounds them: no shuffles, no fragments in registers.  Bound by the instructions that
-// cut and join (about 50 per complex number on either side; issue 48 %, FP64 pipe 42 % for
-// the conversions) at the occupancy that registers and TMEM leave: the products of the
-// 8-SPF QVC model's EOM 226 -> 191 us, with 12 SPFs 2,900 -> 2,206.
+// one, nothing accumulated: ProdBatch::plain).  A tile is 128 fibres, one per thread and
+// MMA row; the thread cuts its fibre into eight FP16 digits of one exponent, digit i of
+// all fibres being operand A_i (128 x 2 nin).  The matrix's digits lie side by side as
+// columns, B = [B_0 B_1 .. B_7] (WC columns each: the (re, im) of the outputs), and
+// D = [D_0 .. D_7] holds the sums of equal weight in TMEM: A_i times the first 8 - i
+// blocks adds into D_i .. D_7, so a K step of a tile takes eight MMAs of N = WC (8 - i).
+// A thread reads its fibre's sums back, joins and rounds them: no shuffles, no fragments
+// in registers; the outputs too small for the digits' bound it sums again in FP64.  Bound
+// by the instructions that scale, cut and join (about 50 per complex number on either
+// side) at the occupancy that registers and TMEM leave.  The products of the 8-SPF QVC
+// model's EOM take 229 us (271 with mma.sync), of which 38 are for the scaling and the
+// test of the outputs; with 12 SPFs 2,560 (3,230) and 350.
 // ---------------------------------------------------------------------------
 template <int NG>   // groups of four j
 struct DigitTile {
