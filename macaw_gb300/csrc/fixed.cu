@@ -325,7 +325,8 @@ static __device__ void dot_block(const HoleDesc& d, int b, cplx* red) {
 }
 
 // The block's contraction in FP64 from global memory, for operands outside the
-// exponent range (fibres p0 .. p1): a pair per warp, its lanes over the fibres.
+// exponent range (fibres p0 .. p1): a pair per warp, its lanes over the fibres.  With every
+// block of the 42 contractions of 32,768 fibres of 8 here: 1,454 us against 148.
 static __device__ __noinline__ void hole_block_fp64(const HoleDesc& d, const cplx* Y, int b, unsigned p0, unsigned p1) {
   const long long L = d.L;
   const int lane = threadIdx.x & 31, nwarp = blockDim.x >> 5;
